@@ -20,6 +20,7 @@
 #include "afr_implicit.cuh"
 #include "afr_mixed.cuh"
 #include "afr_p0.cuh"
+#include "afr_prism.cuh"
 #include "afr_sst.cuh"
 
 using namespace afr;
@@ -67,6 +68,13 @@ struct afr_handle {
   MxOps mo{};
   MxFace mf{};
   MxBuf mb{};
+  // prisms whose operators have tensor-product structure (afr_prism.cuh)
+  bool px = false;
+  PxOps<2, 3> px1{};
+  PxOps<3, 4> px2{};
+  PxGeom pg{};
+  unsigned px_faces = 0;  // bit (axis*2 + side): faces whose point fields some slot reads
+  bool px_points = false;  // some face point interpolates from the point fields
   int mx_pre_blocks = 0, mx_cell_blocks = 0;  // resident CTAs of the persistent kernels
   int mx_pre_per_sm = 0, mx_pre_max_per_sm = 0, n_sms = 0;
   int mx_pre_occ = 0, mx_vol_occ = 0;          // occupancy-API CTAs per SM, before the tensor-memory cap
@@ -395,6 +403,16 @@ struct Launch {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_mx_update<S, NP, MXU2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)MxUpdSmem<S, NP, MXU2>::total);
+    if constexpr (PXD) {
+      auto* fv = k_px_cell<PXN1, PXNF, PXC, true>;
+      auto* fi = k_px_cell<PXN1, PXNF, PXC, false>;
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(fv, cudaFuncAttributeMaxDynamicSharedMemorySize, PxS::total);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(fi, cudaFuncAttributeMaxDynamicSharedMemorySize, PxS::total);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fv, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fi, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    }
     // the largest shared-memory carveout for the two persistent kernels, whose
     // shared memory sets how many CTAs fit on an SM
     if (e == cudaSuccess)
@@ -433,11 +451,35 @@ struct Launch {
         h->g, h->ops, h->fc, a, h->mb.RV, h->mb.Jm, h->mo.rdet);
   }
   static int n_ranges(const afr_handle* h) { return (h->n_prism > 0 ? 1 : 0) + (h->N > h->n_prism ? 1 : 0); }
+  // structured prisms: one kernel forms the face-point fields and the volume terms
+  static constexpr bool PXD = S == 8 || S == 27;
+  static constexpr int PXN1 = S == 8 ? 2 : 3, PXNF = S == 8 ? 3 : 4, PXC = S == 8 ? 6 : 2;
+  using PxS = PxSmem<PXN1, PXNF, PXC>;
+  static bool px_range(const afr_handle* h, int r) { return PXD && h->px && r == 0; }
+  static cudaError_t px_cell(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
+    if constexpr (PXD) {
+      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
+      const auto* op = [&] {
+        if constexpr (S == 8) return &h->px1;
+        else return &h->px2;
+      }();
+      auto* fn = visc ? k_px_cell<PXN1, PXNF, PXC, true> : k_px_cell<PXN1, PXNF, PXC, false>;
+      fn<<<nb, 32 * PX_WARPS, PxS::total, st>>>(*op, h->pg, h->mb.XF, h->px_points ? h->mb.PFm : nullptr, h->mb.RV,
+                                                h->mb.FW, h->px_faces, U, h->nv, nut, (float)h->prm.mu, 0, n);
+      return cudaGetLastError();
+    }
+    return cudaErrorNotSupported;
+  }
   static cudaError_t mx_pre(afr_handle* h, const double* U, const double* nut, bool grads, cudaStream_t st) {
     const int ranges[3] = {0, h->n_prism, h->N};
     for (int r = 0; r < 2; ++r) {
       const int n = ranges[r + 1] - ranges[r];
       if (n <= 0) continue;
+      if (px_range(h, r)) {
+        const cudaError_t e = px_cell(h, U, nut, grads, n, st);
+        if (e != cudaSuccess) return e;
+        continue;
+      }
       const int tiles = (n + MX_PRE_CELLS - 1) / MX_PRE_CELLS;
       k_mx_pre<S, NP><<<std::min(tiles, h->mx_pre_blocks), MX_THREADS, mx_pre_smem(), st>>>(
           h->g, h->mo, h->mb, U, h->nv, nut, grads ? 1 : 0, ranges[r], ranges[r + 1], h->status);
@@ -464,7 +506,7 @@ struct Launch {
     const int ranges[3] = {0, h->n_prism, h->N};
     for (int r = 0; r < 2; ++r) {
       const int n = ranges[r + 1] - ranges[r];
-      if (n <= 0) continue;
+      if (n <= 0 || px_range(h, r)) continue;
       const int tiles = (n + MXC - 1) / MXC;
       k_mx_vol<S, FN, MXC><<<std::min(tiles, h->mx_cell_blocks), MX_VOL_THREADS, mx_vol_smem(), st>>>(
           h->g, h->mo, a.Ucur, h->nv, a.inviscid_only, (float)h->prm.mu, h->mb.PFm, h->mb.RV, ranges[r],
@@ -492,7 +534,10 @@ struct Launch {
     cudaError_t r = mx ? mx_pre(h, U, nut, grads, st) : pre(h, U, nut, grads, st);
     if (r != cudaSuccess) return r;
     if (tm) tm->mark(st);
-    if (nl) *nl += (mx ? n_ranges(h) : 1) + (h->slots.n > 0 ? 1 : 0) + (mx ? 2 : 1) * n_ranges(h);
+    if (nl) {
+      const int face = !mx || !h->mx_paired ? (h->slots.n > 0 ? 1 : 0) : (h->mx_npairs > 0 ? 1 : 0) + (h->mx_nrest > 0 ? 1 : 0);
+      *nl += (mx ? 3 : 2) * n_ranges(h) - (mx && h->px ? 1 : 0) + face;
+    }
     if (mx) return mx_stage(h, a, st, tm);
     r = stage(h, a, st, tm);
     if (tm) tm->mark(st);  // the plain form has no separate update kernel: an empty interval
@@ -860,8 +905,17 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
                   std::string("the mixed form needs operators with row l1 norms <= 1e6 (FP32 accumulation); the ") +
                       (t == 0 ? "prism" : "tet") + " operators of this order reach " + std::to_string(l1));
   }
+  // prisms with tensor-product operators take k_px_cell; everything else the
+  // tensor-core kernels
+  if (h->n_prism > 0) {
+    if (h->order == 1)
+      h->px = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], Wkeep[0].data(), h->px1);
+    else if (h->order == 2)
+      h->px = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], Wkeep[0].data(), h->px2);
+  }
+  const bool tcr = !h->px || h->N > h->n_prism;  // some cells run on the tensor-core kernels
   for (int t = 0; t < 2; ++t) {
-    if (Wkeep[t].empty()) continue;
+    if (Wkeep[t].empty() || (t == 0 && h->px)) continue;
     const double* c2f = m->c2f[t];
     const double* D3 = m->D_3d[t];
     const double* Wt = Wkeep[t].data();
@@ -902,20 +956,24 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   if ((rc = dalloc(h, &md, N * S * 3)) || (rc = dalloc(h, &hc, N))) return rc;
   h->mo.MD = md;
   h->mo.hcell = hc;
-  float4 *adjf32, *adjs32, *invs32;
-  if ((rc = dalloc(h, &adjf32, N * (size_t)h->Fn * 3)) || (rc = dalloc(h, &adjs32, N * (size_t)S * 3)) ||
-      (rc = dalloc(h, &invs32, N * (size_t)S * 3)))
+  float4 *adjf32 = nullptr, *adjs32 = nullptr, *invs32 = nullptr;
+  if (tcr && ((rc = dalloc(h, &adjf32, N * (size_t)h->Fn * 3)) || (rc = dalloc(h, &adjs32, N * (size_t)S * 3)) ||
+              (rc = dalloc(h, &invs32, N * (size_t)S * 3))))
     return rc;
+  float *padjs = nullptr, *padjf = nullptr;
+  const size_t NP = h->n_prism;
+  if (h->px && ((rc = dalloc(h, &padjs, NP * S * 9)) || (rc = dalloc(h, &padjf, NP * h->Fn * 9)))) return rc;
   h->mo.adjf = adjf32;
   h->mo.adjs = adjs32;
   h->mo.invs = invs32;
   double* rdet;
   if ((rc = dalloc(h, &rdet, N * (size_t)S))) return rc;
   h->mo.rdet = rdet;
-  const int FW = h->order <= 2 ? 18 : 5;
-  float *xf, *pfm, *jm;
+  h->pg = PxGeom{padjs, padjf, md, rdet};
+  const int FW = h->order <= 2 ? MX_XF : 5;
+  float *xf, *pfm = nullptr, *jm;
   const size_t ns = h->slots.n;
-  if ((rc = dalloc(h, &xf, N * FW * 6 * P)) || (rc = dalloc(h, &pfm, N * S * 20)) || (rc = dalloc(h, &jm, ns * P * 10 + 4)))  // 16 bytes of slack: the update kernel copies 16-byte-rounded slot ranges
+  if ((rc = dalloc(h, &xf, N * FW * 6 * P)) || (rc = dalloc(h, &jm, ns * P * 10 + 4)))  // 16 bytes of slack: the update kernel copies 16-byte-rounded slot ranges
     return rc;
   float* rv;
   if ((rc = dalloc(h, &rv, N * S * 10))) return rc;
@@ -943,9 +1001,15 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
               break;
     }
     const size_t nrows = N * (size_t)h->Fn * 3, nsrows = N * (size_t)S * 3;
-    k_mx_rows_f32<<<(unsigned)((nrows + 255) / 256), 256, 0, st>>>(h->g.adj_fine, nrows, adjf32);
-    k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.adj, nsrows, adjs32);
-    k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv, nsrows, invs32);
+    if (tcr) {
+      k_mx_rows_f32<<<(unsigned)((nrows + 255) / 256), 256, 0, st>>>(h->g.adj_fine, nrows, adjf32);
+      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.adj, nsrows, adjs32);
+      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv, nsrows, invs32);
+    }
+    if (h->px) {
+      k_px_planes<<<(unsigned)((NP * h->Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, h->Fn, padjf);
+      k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, S, padjs);
+    }
     k_mx_rdet<<<(unsigned)((N * (size_t)S + 255) / 256), 256, 0, st>>>(h->g.det, N * (size_t)S, rdet);
     cudaError_t r = cudaGetLastError();
     return r != cudaSuccess ? r : LL::mx_grids(h);
@@ -968,8 +1032,17 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
     if (e == cudaSuccess) e = cudaMemcpy(hflag.data(), h->slots.flags, ns * 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
     std::vector<int32_t> nb_slot(h->F, -1);
-    for (size_t sl = 0; sl < ns; ++sl)
-      if (hflag[sl] & 1) nb_slot[hface[sl]] = (int32_t)sl;
+    for (size_t sl = 0; sl < ns; ++sl) {
+      const int fl = hflag[sl];
+      if (fl & 1) nb_slot[hface[sl]] = (int32_t)sl;
+      h->px_faces |= 1u << (((fl >> 2) & 3) * 2 + ((fl & 16) ? 1 : 0));
+      if (fl & 2) continue;  // boundary: no other side
+      for (int i = 0; i < P; ++i) {
+        const int o = hofp[sl * P + i];
+        if (o == MX_OFP_GENERAL) h->px_points = true;
+        else h->px_faces |= 1u << (o / P);
+      }
+    }
     std::vector<int2> pairs;
     std::vector<uint8_t> taken(nt, 0);
     for (size_t sl = 0; sl < ns; ++sl) {
@@ -1006,6 +1079,10 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
     h->mx_nrest = (int)rest.size();
     h->mx_paired = true;
   }
+  // point fields: the tensor-core volume kernel's input and the source of the
+  // interpolated face points
+  if ((tcr || h->px_points) && (rc = dalloc(h, &pfm, N * S * MX_PF))) return rc;
+  h->mb.PFm = pfm;
   h->prec = AFR_PREC_MIXED;
   // The FP64 fine-point adjugates were needed only for MD and the FP32 copy;
   // the FP64 solution-point adjugates only for the set-up and the SST kernels.
@@ -1881,7 +1958,7 @@ int afr_autotune(afr_handle* h, const double* U, const double* nu_t, int32_t* ch
   }
   const double* nut = h->prm.turb == AFR_TURB_SST ? nu_t : nullptr;
   // coordinate search: pre-pass CTAs per SM, face-kernel block, update-kernel cells per CTA
-  {
+  if (!h->px || h->N > h->n_prism) {  // the tensor-core pre-pass runs
     int best = h->mx_pre_per_sm;
     float tb = 1e30f;
     for (int c = 1; c <= h->mx_pre_max_per_sm; ++c) {

@@ -215,6 +215,29 @@ __device__ __forceinline__ void viscous_flux(const T q[5], const T gv[9], const 
   G[2][4] = (u * t02 + v * t12 + w * t22) + (-k * gT[2]);
 }
 
+// viscous_flux from the symmetric gradient sg = (S00, S11, S22, S01, S02, S12),
+// S_ij = (d_j u_i + d_i u_j) / 2, the only combinations of the velocity
+// gradient it contains; components 1..4 (the mass flux is zero)
+template <class T>
+__device__ __forceinline__ void viscous_flux_sym(const T vel[3], const T sg[6], const T gT[3], T mu, T mu_t,
+                                                 T G[3][4]) {
+  const T mt = mu + mu_t;
+  const T ld = T(-2.0 / 3.0) * mt * (sg[0] + sg[1] + sg[2]);
+  const T t00 = T(2.0) * mt * sg[0] + ld;
+  const T t11 = T(2.0) * mt * sg[1] + ld;
+  const T t22 = T(2.0) * mt * sg[2] + ld;
+  const T t01 = T(2.0) * mt * sg[3], t02 = T(2.0) * mt * sg[4], t12 = T(2.0) * mt * sg[5];
+  const T cp = T(GAMMA * R_AIR / (GAMMA - 1.0));
+  const T k = mu * cp / T(PR) + mu_t * cp / T(PR_T);
+  const T u = vel[0], v = vel[1], w = vel[2];
+  G[0][0] = t00; G[0][1] = t01; G[0][2] = t02;
+  G[1][0] = t01; G[1][1] = t11; G[1][2] = t12;
+  G[2][0] = t02; G[2][1] = t12; G[2][2] = t22;
+  G[0][3] = (u * t00 + v * t01 + w * t02) + (-k * gT[0]);
+  G[1][3] = (u * t01 + v * t11 + w * t12) + (-k * gT[1]);
+  G[2][3] = (u * t02 + v * t12 + w * t22) + (-k * gT[2]);
+}
+
 // conserved -> primitive without pressure floor (core/fr_residual/inviscid.py:38-47)
 __device__ __forceinline__ void cons_to_prim(const double* U, double q[5]) {
   const double rho = fmax(U[0], 1e-10);

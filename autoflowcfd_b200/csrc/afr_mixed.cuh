@@ -77,12 +77,17 @@ struct MxFace {
   const uint8_t* ofp;   // (n_slots*NP) face point of the other side, (ax*2+side)*NP + j, or MX_OFP_GENERAL
 };
 
+// Point fields: q (5), symmetric velocity gradient (S00, S11, S22, S01, S02,
+// S12: the viscous flux holds no other combination), grad T (3), mu_t.
+constexpr int MX_XF = 15;  // fields per face point, in that order
+constexpr int MX_PF = 16;  // floats per solution point: gradients (9), mu_t, q (5), 1 unused
+
 struct MxBuf {
-  float* XF;   // (N, FW, 6*NP) point fields at every face point of the cell
-  float* PFm;  // (N, S, 20) gradients of u, v, w, T (12), mu_t, q (5), 2 unused
+  float* XF;   // (N, 6, FW, NP) point fields at the face points, one contiguous block per face of the cell
+  float* PFm;  // (N, S, MX_PF)
   float* Jm;   // (n_slots, NP, 10) inviscid and viscous jumps
   float* RV;   // (N, S, 10) inviscid and viscous volume terms
-  int FW;      // 18 (q 5, grads 12, mu_t) or 5 (inviscid handles)
+  int FW;      // MX_XF (orders 1, 2) or 5 (order 3: inviscid only)
 };
 
 namespace mxd {
@@ -240,7 +245,7 @@ __device__ __forceinline__ bool wait_commit(uint64_t* bar, uint32_t& phase, unsi
 // ---------------------------------------------------------------------------
 template <int S, int NP>
 struct MxPreSmem {
-  static constexpr int Sq = pad16(S), NFP = 6 * NP, NB1 = 3 * Sq, NB2MAX = 144;
+  static constexpr int Sq = pad16(S), NFP = 6 * NP, NB1 = 3 * Sq, NB2MAX = 128;
   static constexpr int oB1 = 0;                        // D3g image (hi|lo)
   static constexpr int oA2 = oB1 + NB1 * Sq * 4;       // E image
   static constexpr int oA1 = oA2 + 128 * Sq * 4;       // gradient inputs, rows phi*8 + c
@@ -277,8 +282,8 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
   double* sM = reinterpret_cast<double*>(smem + L::oM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int FW = mb.FW;
-  visc = visc && FW >= 18;
-  const int nfw = visc ? 18 : 5;  // fields extrapolated by this call
+  visc = visc && FW >= MX_XF;
+  const int nfw = visc ? MX_XF : 5;  // fields extrapolated by this call
   const int NB2 = pad16(nfw * C);
   const int ct = cell_type(g, cell_base);
 
@@ -377,9 +382,10 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
       const double* q = sQ + (c * S + s) * 6;
       if (c < nc) {
         const float mutf = (visc && nut) ? float(q[0] * nut_at(c, s)) : 0.f;
-        float4* o = reinterpret_cast<float4*>(mb.PFm + ((size_t)(e0 + c) * S + s) * 20);
-        o[3] = make_float4(mutf, float(q[0]), float(q[1]), float(q[2]));
-        o[4] = make_float4(float(q[3]), float(q[4]), 0.f, 0.f);
+        float* o = mb.PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+        *reinterpret_cast<float2*>(o + 10) = make_float2(float(q[0]), float(q[1]));
+        *reinterpret_cast<float4*>(o + 12) = make_float4(float(q[2]), float(q[3]), float(q[4]), 0.f);
+        o[9] = mutf;
       }
       if (visc) {
         const double phi[4] = {q[1], q[2], q[3], q[5]};
@@ -387,7 +393,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
         for (int f = 0; f < 4; ++f)
           mxd::st_split(sA1, 128 * Sq, tc::kmajor_index(f * C + c, s, 128), float(phi[f] - sM[c * 9 + 5 + f]));
         const double mut = (c < nc && nut) ? q[0] * nut_at(c, s) : 0.0;
-        mxd::st_split(sB2, NB2 * Sq, tc::kmajor_index(17 * C + c, s, NB2), float(mut));
+        mxd::st_split(sB2, NB2 * Sq, tc::kmajor_index(14 * C + c, s, NB2), float(mut));
       }
 #pragma unroll
       for (int v = 0; v < 5; ++v)
@@ -423,7 +429,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
       // physical gradients (core/fr_operators/gradients.py:23-64) and mu_t
       for (int t = tid; t < C * S; t += MX_THREADS) {
         const int c = t % C, s = t / C;
-        float gr[12];
+        float gr[12], pf[9];
         if (c < nc) {
           const float4* inv = L::STG ? sInvs + (c * S + s) * 3 : mo.invs + ((size_t)(e0 + c) * S + s) * 3;
           float iv[9];
@@ -440,16 +446,24 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
 #pragma unroll
             for (int n = 0; n < 3; ++n)
               gr[f * 3 + n] = gs[0 * 4 + f] * iv[0 * 3 + n] + gs[1 * 4 + f] * iv[1 * 3 + n] + gs[2 * 4 + f] * iv[2 * 3 + n];
-          float4* o = reinterpret_cast<float4*>(mb.PFm + ((size_t)(e0 + c) * S + s) * 20);
-          o[0] = make_float4(gr[0], gr[1], gr[2], gr[3]);
-          o[1] = make_float4(gr[4], gr[5], gr[6], gr[7]);
-          o[2] = make_float4(gr[8], gr[9], gr[10], gr[11]);
+          pf[0] = gr[0];
+          pf[1] = gr[4];
+          pf[2] = gr[8];
+          pf[3] = 0.5f * (gr[1] + gr[3]);
+          pf[4] = 0.5f * (gr[2] + gr[6]);
+          pf[5] = 0.5f * (gr[5] + gr[7]);
+#pragma unroll
+          for (int n = 0; n < 3; ++n) pf[6 + n] = gr[9 + n];
+          float* o = mb.PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+          *reinterpret_cast<float4*>(o) = make_float4(pf[0], pf[1], pf[2], pf[3]);
+          *reinterpret_cast<float4*>(o + 4) = make_float4(pf[4], pf[5], pf[6], pf[7]);
+          o[8] = pf[8];
         } else {
 #pragma unroll
-          for (int k = 0; k < 12; ++k) gr[k] = 0.f;
+          for (int k = 0; k < 9; ++k) pf[k] = 0.f;
         }
 #pragma unroll
-        for (int k = 0; k < 12; ++k) mxd::st_split(sB2, NB2 * Sq, tc::kmajor_index((5 + k) * C + c, s, NB2), gr[k]);
+        for (int k = 0; k < 9; ++k) mxd::st_split(sB2, NB2 * Sq, tc::kmajor_index((5 + k) * C + c, s, NB2), pf[k]);
       }
       tc::fence_async_smem();
       __syncthreads();
@@ -480,7 +494,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
               const int c = j * CPC + cc;
               if (c < nc) {
                 const float val = f < 5 ? float(sM[c * 9 + f] + (double)vc[cc]) : vc[cc];
-                mb.XF[((size_t)(e0 + c) * FW + f) * NFP + fp] = val;
+                mb.XF[(((size_t)(e0 + c) * 6 + fp / NP) * FW + f) * NP + fp % NP] = val;
               }
             }
           }
@@ -509,7 +523,7 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
 template <int NP>
 __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& st, const MxFace& mf, const MxBuf& mb,
                                              const double* __restrict__ hcell, float mu, int visc, int t,
-                                             const float (&ow)[18], const float (&ot)[18]) {
+                                             const float (&ow)[MX_XF], const float (&ot)[MX_XF]) {
   const int sl = t / NP, i = t % NP;
   const int f = st.face[sl];
   const int e = st.cell[sl];
@@ -533,21 +547,20 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
 #pragma unroll
   for (int v = 0; v < 5; ++v) Jo[v] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
   if (visc) {
-    float qa[5], ga[13];
+    float av[MX_XF];  // the common flux: both sides' averages
 #pragma unroll
-    for (int v = 0; v < 5; ++v) qa[v] = 0.5f * (ow[v] + ot[v]);
-#pragma unroll
-    for (int k = 0; k < 13; ++k) ga[k] = 0.5f * (ow[5 + k] + ot[5 + k]);
-    float Gc[3][5], Go[3][5];
-    viscous_flux<float>(qa, ga, ga + 9, mu, ga[12], Gc);
-    viscous_flux<float>(ow, ow + 5, ow + 14, mu, ow[17], Go);
+    for (int k = 1; k < MX_XF; ++k) av[k] = 0.5f * (ow[k] + ot[k]);
+    float Gc[3][4], Go[3][4];
+    viscous_flux_sym<float>(av + 1, av + 5, av + 11, mu, av[14], Gc);
+    viscous_flux_sym<float>(ow + 1, ow + 5, ow + 11, mu, ow[14], Go);
     float jv[5];
+    jv[0] = 0.f;
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
-      jv[v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
+    for (int v = 0; v < 4; ++v)
+      jv[1 + v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
     if (bnd) {
       // interior penalty (core/fr_operators/flux_kernels.py:140-200)
-      const float eta = float(C_IP) * (mu + ow[17]) / float(hcell[e]);
+      const float eta = float(C_IP) * (mu + ow[14]) / float(hcell[e]);
       const float scale = eta * ar.w * side;
 #pragma unroll
       for (int v = 1; v < 4; ++v) jv[v] += -scale * (ow[v] - ot[v]);
@@ -555,6 +568,12 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
 #pragma unroll
     for (int v = 0; v < 5; ++v) Jo[5 + v] = jv[v];
   }
+}
+
+// face point fp = (axis*2+side)*NP + i of cell e: field k at [k * NP]
+template <int NP>
+__device__ __forceinline__ const float* mx_face_row(const MxBuf& mb, int e, int fp) {
+  return mb.XF + ((size_t)e * 6 + fp / NP) * mb.FW * NP + fp % NP;
 }
 
 template <int S, int NP>
@@ -566,7 +585,6 @@ __global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, 
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (rest ? n_rest : st.n * NP)) return;
   const int t = rest ? rest[idx] : idx;
-  constexpr int NFP = 6 * NP;
   const int sl = t / NP, i = t % NP;
   const int f = st.face[sl];
   const int e = st.cell[sl];
@@ -574,13 +592,12 @@ __global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, 
   const bool is_owner = (fl & 1) == 0;
   const bool bnd = (fl & 2) != 0;
   const int ax = (fl >> 2) & 3;
-  const int FW = mb.FW;
-  const int nf = visc ? 18 : 5;
-  float ow[18], ot[18];
+  const int nf = visc ? MX_XF : 5;
+  float ow[MX_XF], ot[MX_XF];
   {
-    const float* xo = mb.XF + (size_t)e * FW * NFP + (ax * 2 + ((fl & 16) ? 1 : 0)) * NP + i;
+    const float* xo = mx_face_row<NP>(mb, e, (ax * 2 + ((fl & 16) ? 1 : 0)) * NP + i);
 #pragma unroll
-    for (int k = 0; k < 18; ++k) ow[k] = k < nf ? __ldg(xo + k * NFP) : 0.f;
+    for (int k = 0; k < MX_XF; ++k) ow[k] = k < nf ? __ldg(xo + k * NP) : 0.f;
   }
   const double* tnp = fc.tnormal + ((size_t)f * NP + i) * 3;
   const float tn[3] = {float(tnp[0]), float(tnp[1]), float(tnp[2])};
@@ -590,18 +607,18 @@ __global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, 
 #pragma unroll
     for (int v = 0; v < 5; ++v) ot[v] = gq[v];
 #pragma unroll
-    for (int k = 5; k < 18; ++k) ot[k] = ow[k];
+    for (int k = 5; k < MX_XF; ++k) ot[k] = ow[k];
   } else if (mf.ofp[t] != MX_OFP_GENERAL) {
     // matched rows come from the record's other cell (either source slot may hold them)
     const int oc = is_owner ? fc.neighbor[f] : fc.owner[f];
-    const float* xn = mb.XF + (size_t)oc * FW * NFP + mf.ofp[t];
+    const float* xn = mx_face_row<NP>(mb, oc, mf.ofp[t]);
 #pragma unroll
-    for (int k = 0; k < 18; ++k) ot[k] = k < nf ? __ldg(xn + k * NFP) : 0.f;
+    for (int k = 0; k < MX_XF; ++k) ot[k] = k < nf ? __ldg(xn + k * NP) : 0.f;
   } else {
     // interpolation from the source cells' point fields (sum src0 then src1,
     // zero weights skipped as in core/fr_residual/inviscid_kernel_colored.py:117-121)
 #pragma unroll
-    for (int k = 0; k < 18; ++k) ot[k] = 0.f;
+    for (int k = 0; k < MX_XF; ++k) ot[k] = 0.f;
     for (int src = 0; src < 2; ++src) {
       const int c = src == 0 ? st.c0[sl] : st.c1[sl];
       if (c < 0) continue;
@@ -609,19 +626,18 @@ __global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, 
                                              : fmat(fc.ow_m0, fc.ow_m0i, f, i, NP, S))
                                  : (is_owner ? fmat(fc.nb_m1, fc.nb_m1i, st.i1[sl], i, NP, S)
                                              : fmat(fc.ow_m1, fc.ow_m1i, st.i1[sl], i, NP, S));
-      const float* pf = mb.PFm + (size_t)c * S * 20;
+      const float* pf = mb.PFm + (size_t)c * S * MX_PF;
       for (int s = 0; s < S; ++s) {
         const float w = float(__ldg(M + s * NP));
         if (w == 0.f) continue;
-        const float4* p4 = reinterpret_cast<const float4*>(pf + s * 20);
-        const float4 x3 = __ldg(p4 + 3), x4 = __ldg(p4 + 4);
-        ot[0] += w * x3.y; ot[1] += w * x3.z; ot[2] += w * x3.w; ot[3] += w * x4.x; ot[4] += w * x4.y;
+        const float4* p4 = reinterpret_cast<const float4*>(pf + s * MX_PF);
+        const float4 x2 = __ldg(p4 + 2), x3 = __ldg(p4 + 3);
+        ot[0] += w * x2.z; ot[1] += w * x2.w; ot[2] += w * x3.x; ot[3] += w * x3.y; ot[4] += w * x3.z;
         if (visc) {
-          const float4 x0 = __ldg(p4), x1 = __ldg(p4 + 1), x2 = __ldg(p4 + 2);
+          const float4 x0 = __ldg(p4), x1 = __ldg(p4 + 1);
           ot[5] += w * x0.x;  ot[6] += w * x0.y;  ot[7] += w * x0.z;  ot[8] += w * x0.w;
           ot[9] += w * x1.x;  ot[10] += w * x1.y; ot[11] += w * x1.z; ot[12] += w * x1.w;
-          ot[13] += w * x2.x; ot[14] += w * x2.y; ot[15] += w * x2.z; ot[16] += w * x2.w;
-          ot[17] += w * x3.x;
+          ot[13] += w * x2.x; ot[14] += w * x2.y;
         }
       }
     }
@@ -639,7 +655,6 @@ __global__ void __launch_bounds__(256, 3) k_mx_face_pair(Faces fc, Bc bc, SlotTa
                                                       const int2* __restrict__ pairs, int n_pairs) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_pairs) return;
-  constexpr int NFP = 6 * NP;
   const int2 pr = pairs[idx];
   const int t = pr.x, t2 = pr.y;
   const int sl = t / NP, i = t % NP;
@@ -647,17 +662,16 @@ __global__ void __launch_bounds__(256, 3) k_mx_face_pair(Faces fc, Bc bc, SlotTa
   const int e = st.cell[sl];
   const int fl = st.flags[sl];
   const int ax = (fl >> 2) & 3;
-  const int FW = mb.FW;
-  const int nf = visc ? 18 : 5;
+  const int nf = visc ? MX_XF : 5;
   const int oc = fc.neighbor[f];
-  float ra[18], rb[18];
+  float ra[MX_XF], rb[MX_XF];
   {
-    const float* xa = mb.XF + (size_t)e * FW * NFP + (ax * 2 + ((fl & 16) ? 1 : 0)) * NP + i;
-    const float* xb = mb.XF + (size_t)oc * FW * NFP + mf.ofp[t];
+    const float* xa = mx_face_row<NP>(mb, e, (ax * 2 + ((fl & 16) ? 1 : 0)) * NP + i);
+    const float* xb = mx_face_row<NP>(mb, oc, mf.ofp[t]);
 #pragma unroll
-    for (int k = 0; k < 18; ++k) {
-      ra[k] = k < nf ? __ldg(xa + k * NFP) : 0.f;
-      rb[k] = k < nf ? __ldg(xb + k * NFP) : 0.f;
+    for (int k = 0; k < MX_XF; ++k) {
+      ra[k] = k < nf ? __ldg(xa + k * NP) : 0.f;
+      rb[k] = k < nf ? __ldg(xb + k * NP) : 0.f;
     }
   }
   mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, t, ra, rb);
@@ -775,7 +789,7 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
       mxd::prefetch_l2(mo.adjf, (size_t)g.N * FN * 48, en * FN * 48, nn * FN * 48);
       if (!L::STG) mxd::prefetch_l2(Ucur, NS * nv * 8, en * S * nv * 8, nn * S * nv * 8);
       if (visc) {
-        mxd::prefetch_l2(PFm, NS * 80, en * S * 80, nn * S * 80);
+        mxd::prefetch_l2(PFm, NS * MX_PF * 4, en * S * MX_PF * 4, nn * S * MX_PF * 4);
         mxd::prefetch_l2(mo.adjs, NS * 48, en * S * 48, nn * S * 48);
       }
     }
@@ -833,21 +847,21 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
           for (int v = 0; v < 5; ++v) Gt[m][v] = 0.f;
         if (live) {
           const size_t p = (size_t)(e0 + c) * S + s;
-          const float4* pf = reinterpret_cast<const float4*>(PFm + p * 20);
-          const float4 g0 = __ldg(pf), g1 = __ldg(pf + 1), g2 = __ldg(pf + 2), g3 = __ldg(pf + 3);
+          const float4* pf = reinterpret_cast<const float4*>(PFm + p * MX_PF);
+          const float4 g0 = __ldg(pf), g1 = __ldg(pf + 1), g2 = __ldg(pf + 2);
           const float4* am = mo.adjs + p * 3;
-          float q[5];
+          float vel[3];
 #pragma unroll
-          for (int v = 0; v < 5; ++v) q[v] = float(sQ[(c * S + s) * 5 + v]);
-          const float gv[9] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x};
-          const float gT[3] = {g2.y, g2.z, g2.w};
-          float G[3][5];
-          viscous_flux<float>(q, gv, gT, mu, g3.x, G);
+          for (int d = 0; d < 3; ++d) vel[d] = float(sQ[(c * S + s) * 5 + 1 + d]);
+          const float sg[6] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y};
+          const float gT[3] = {g1.z, g1.w, g2.x};
+          float G[3][4];
+          viscous_flux_sym<float>(vel, sg, gT, mu, g2.y, G);
 #pragma unroll
           for (int m = 0; m < 3; ++m) {
             const float4 x = __ldg(am + m);
 #pragma unroll
-            for (int v = 0; v < 5; ++v) Gt[m][v] = x.x * G[0][v] + x.y * G[1][v] + x.z * G[2][v];
+            for (int v = 0; v < 4; ++v) Gt[m][1 + v] = x.x * G[0][v] + x.y * G[1][v] + x.z * G[2][v];
           }
         }
 #pragma unroll

@@ -1,0 +1,573 @@
+// Mixed-precision cell kernel of prisms whose operators have tensor-product
+// structure in the collapsed coordinates (a, b, c): point s = (a*N1 + b)*N1 + c.
+//
+//   D_3d[.,.,0]  couples points of one a-line (same b, c), the same weights on
+//   every line; D_3d[.,.,2] likewise along c; D_3d[.,.,1] couples the points of
+//   one triangle plane (same c).
+//   boundary_extrap reads one a-line (axis 0), one triangle plane (axis 1) or
+//   one c-line (axis 2) per face point.
+//   c2f and the folded W = f2c*D_fine (per reference axis m) are Kronecker
+//   products triangle (x) c-line.
+//
+// The reference's prism operators have this structure to rounding (entries
+// outside it are 1e-16 to 6e-15 of the largest); afr_create tests for it
+// (px_operators) and takes this kernel instead of k_mx_pre + k_mx_vol, which
+// stay for every other operator set (tets, P3).
+//
+// Why: with the structure a P2 cell needs 9 k multiply-adds instead of the
+// 45 k of the dense products, so plain FP32 (whose products carry 24 bits
+// instead of the 16 of a BF16 hi+lo pair) is no longer bound by arithmetic,
+// and everything a cell needs for the face-point fields, the viscous and the
+// inviscid volume terms is formed in one pass over the state: 9.7 KB per P2
+// cell instead of 19 KB for the two tensor-core kernels.
+//
+// A warp owns CW whole cells from load to store, so the phases are separated
+// by __syncwarp only and the warps of an SM drift apart and overlap one
+// another's loads and arithmetic.  CW is chosen so that the items of the
+// phases fill the 32 lanes: P2, CW = 2: 27 + 27 points, 30 (cell, variable,
+// c-level), 32 (cell, fine triangle point), 30 (cell, field); P1, CW = 6: 48,
+// 60, 54 and 90 in two or three rounds.  The operators arrive as a kernel
+// parameter: every index into them is a compile-time constant, so they are
+// operands from the constant bank and cost no loads.
+#pragma once
+#include "afr_mixed.cuh"
+
+namespace afr {
+
+constexpr int PX_WARPS = 4;
+
+template <int N1, int NF>
+struct PxOps {
+  static constexpr int NT = N1 * N1, MT = NF * NF;
+  float E02[2][2][N1];   // extrapolation along a (0) and c (1): [which][side][point of the line]
+  float E1[2][N1][NT];   // extrapolation to the b faces: [side][a of the face point][triangle point]
+  float D0[N1][N1], D2[N1][N1], D1[NT][NT];
+  float Ct[MT][NT], Cc[NF][N1];      // c2f = Ct (x) Cc
+  float Wt[3][NT][MT], Wc[3][N1][NF];  // W per axis = Wt (x) Wc
+};
+
+// per-cell metrics in the order the lanes read them
+struct PxGeom {
+  const float* adjs;   // (N, 9, S) solution-point adjugates, entry m*3 + n
+  const float* adjf;   // (N, 9, MT, NF) fine-point adjugates, fine point = triangle point * NF + c-level
+  const double* MD;    // (N, S, 3)
+  const double* rdet;  // (N, S)
+};
+
+template <int N1, int NF, int CW>
+struct PxSmem {
+  static constexpr int S = N1 * N1 * N1, NT = N1 * N1, MT = NF * NF;
+  static constexpr int TP = MT == 16 ? 20 : 12;  // triangle row stride: 16-byte rows on distinct banks
+  static constexpr int FS = S | 1;               // field row stride (odd)
+  static constexpr int nH = 15 * N1 * TP;        // c-contracted fluxes; before: state, gradient inputs, fluxes; face fields
+  static constexpr int nX = MX_XF * FS, nY = 5 * N1 * TP;
+  static constexpr int oX = nH, oY = (oX + nX + 3) / 4 * 4, oRef = oY + nY, oF = oRef + 8;
+  static constexpr int cell = (oF + 30 + 3) / 4 * 4;  // floats per cell
+  static constexpr int oDev = 16 * S, oG = oDev + 4 * S;  // inside H, after the staged state (8 doubles per point)
+  static_assert(oG + 12 * S <= nH && 6 * MX_XF * NT <= nH && 10 * S <= nH, "phases share the H block");
+  static constexpr int total = PX_WARPS * CW * cell * 4;
+};
+
+template <int N1, int NF, int CW, bool VISC>
+__global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
+    k_px_cell(const __grid_constant__ PxOps<N1, NF> op, PxGeom pg, float* __restrict__ XF, float* __restrict__ PFm,
+              float* __restrict__ RV, int FW, unsigned face_mask, const double* __restrict__ U, int nv,
+              const double* __restrict__ nut, float mu, int cell_base, int cell_end) {
+  using L = PxSmem<N1, NF, CW>;
+  constexpr int S = L::S, NT = L::NT, MT = L::MT, TP = L::TP, FS = L::FS, NP = NT;
+  constexpr int CPR = 32 / S;                 // cells per round of the point phases
+  constexpr int PR = (CW + CPR - 1) / CPR;    // rounds
+  extern __shared__ __align__(16) float smf[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e0 = cell_base + (blockIdx.x * PX_WARPS + warp) * CW;
+  const int nc = min(CW, cell_end - e0);
+  if (nc <= 0) return;  // whole warps; no block barrier below
+  float* sw = smf + warp * CW * L::cell;
+  // point lanes: the same solution point every round
+  const int s = lane % S, pc = lane / S;
+  const int tri = s / N1, cc = s % N1;
+
+  // ---- state and nu_t of the warp's cells ----
+  for (int c = 0; c < nc; ++c) {
+    double* d = reinterpret_cast<double*>(sw + c * L::cell);
+    const double* ub = U + (size_t)(e0 + c) * S * nv;
+    for (int t = lane; t < S * nv; t += 32) cp_async8(d + t, ub + t);
+    if (VISC && nut)
+      for (int t = lane; t < S; t += 32) cp_async8(d + 7 * S + t, nut + (size_t)(e0 + c) * S + t);
+  }
+  cp_async_wait_all();
+  __syncwarp();
+
+  // ---- primitives; deviations from the cell's reference point ----
+  float uf[PR][3], mut[PR];
+#pragma unroll
+  for (int r = 0; r < PR; ++r) {
+    const int c = r * CPR + pc;
+    const bool in = pc < CPR && c < CW;
+    float* sc = sw + (in ? c : 0) * L::cell;
+    double q[6] = {1.0, 0.0, 0.0, 0.0, 1.0, 1.0};
+    mut[r] = 0.f;
+    if (in && c < nc) {
+      const double* d = reinterpret_cast<const double*>(sc);
+      mxd::prim_T(d + s * nv, q);
+      if (VISC && nut) mut[r] = float(q[0] * d[7 * S + s]);
+    }
+    float dev[6];
+    constexpr int MID = S / 2;  // the point whose value is the cell's reference state
+#pragma unroll
+    for (int v = 0; v < 6; ++v) {
+      const float ref = __shfl_sync(0xffffffffu, float(q[v]), (pc < CPR ? pc : 0) * S + MID);
+      dev[v] = float(q[v] - double(ref));
+      if (in && s == MID) sc[L::oRef + v] = ref;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) uf[r][d] = float(q[1 + d]);
+    if (in) {
+#pragma unroll
+      for (int v = 0; v < 5; ++v) sc[L::oX + v * FS + s] = dev[v];
+      if (VISC) *reinterpret_cast<float4*>(sc + L::oDev + 4 * s) = make_float4(dev[1], dev[2], dev[3], dev[5]);
+    }
+    if (PFm && in && c < nc) {
+      float* o = PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+#pragma unroll
+      for (int v = 0; v < 5; ++v) o[10 + v] = float(q[v]);
+    }
+  }
+  __syncwarp();
+
+  float vis[PR][4];
+  if constexpr (VISC) {
+    // this lane's rows of the derivative operators
+    float d0[N1], d1[NT], d2[N1];
+#pragma unroll
+    for (int l = 0; l < N1; ++l) {
+      d0[l] = op.D0[tri / N1][l];
+      d2[l] = op.D2[cc][l];
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) d1[t] = op.D1[tri][t];
+    float rd[PR];
+#pragma unroll
+    for (int r = 0; r < PR; ++r) {
+      const int c = r * CPR + pc;
+      const bool in = pc < CPR && c < CW;
+      float* sc = sw + (in ? c : 0) * L::cell;
+      float aj[9];
+      rd[r] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) aj[k] = 0.f;
+      if (in && c < nc) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) aj[k] = __ldg(pg.adjs + ((size_t)(e0 + c) * 9 + k) * S + s);
+        rd[r] = float(__ldg(pg.rdet + (size_t)(e0 + c) * S + s));
+      }
+      // reference-space gradients of u, v, w, T
+      const float4* dv = reinterpret_cast<const float4*>(sc + L::oDev);
+      float g[3][4];
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) g[m][f] = 0.f;
+      auto acc = [](float (&o)[4], float w, const float4& x) {
+        o[0] += w * x.x;
+        o[1] += w * x.y;
+        o[2] += w * x.z;
+        o[3] += w * x.w;
+      };
+#pragma unroll
+      for (int l = 0; l < N1; ++l) {
+        acc(g[0], d0[l], dv[l * NT + s % NT]);
+        acc(g[2], d2[l], dv[s - cc + l]);
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) acc(g[1], d1[t], dv[t * N1 + cc]);
+      // physical gradients: inverse Jacobian = adjugate / det
+      float gr[4][3];
+#pragma unroll
+      for (int f = 0; f < 4; ++f)
+#pragma unroll
+        for (int n = 0; n < 3; ++n)
+          gr[f][n] = rd[r] * (g[0][f] * aj[n] + g[1][f] * aj[3 + n] + g[2][f] * aj[6 + n]);
+      const float sym[6] = {gr[0][0], gr[1][1], gr[2][2], 0.5f * (gr[0][1] + gr[1][0]), 0.5f * (gr[0][2] + gr[2][0]),
+                            0.5f * (gr[1][2] + gr[2][1])};
+      float G[3][4];
+      viscous_flux_sym(uf[r], sym, gr[3], mu, mut[r], G);
+      if (in) {
+        float* x = sc + L::oX + 5 * FS + s;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) x[k * FS] = sym[k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) x[(6 + k) * FS] = gr[3][k];
+        x[9 * FS] = mut[r];
+        float4* gt = reinterpret_cast<float4*>(sc + L::oG);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          float h[4];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) h[v] = aj[m * 3] * G[0][v] + aj[m * 3 + 1] * G[1][v] + aj[m * 3 + 2] * G[2][v];
+          gt[m * S + s] = make_float4(h[0], h[1], h[2], h[3]);
+        }
+      }
+      if (PFm && in && c < nc) {
+        float* o = PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) o[k] = sym[k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) o[6 + k] = gr[3][k];
+        o[9] = mut[r];
+      }
+    }
+    __syncwarp();
+    // viscous divergence / det (the mass component is zero)
+#pragma unroll
+    for (int r = 0; r < PR; ++r) {
+      const int c = r * CPR + pc;
+      const float* sc = sw + (pc < CPR && c < CW ? c : 0) * L::cell;
+      const float4* gt = reinterpret_cast<const float4*>(sc + L::oG);
+      float o[4] = {0.f, 0.f, 0.f, 0.f};
+      auto acc = [&](float w, const float4& x) {
+        o[0] += w * x.x;
+        o[1] += w * x.y;
+        o[2] += w * x.z;
+        o[3] += w * x.w;
+      };
+#pragma unroll
+      for (int l = 0; l < N1; ++l) {
+        acc(d0[l], gt[l * NT + s % NT]);
+        acc(d2[l], gt[2 * S + s - cc + l]);
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) acc(d1[t], gt[S + t * N1 + cc]);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) vis[r][v] = o[v] * rd[r];
+    }
+    __syncwarp();  // H is reused for the face-point fields
+  }
+
+  // ---- extrapolation: one lane per (cell, field), the field in registers ----
+  constexpr int NFL = VISC ? MX_XF : 5;
+  for (int it = lane; it < CW * NFL; it += 32) {
+    const int c = it / NFL, f = it - c * NFL;
+    float* sc = sw + c * L::cell;
+    float x[S];
+    const float* xs = sc + L::oX + f * FS;
+#pragma unroll
+    for (int j = 0; j < S; ++j) x[j] = xs[j];
+    const float base = f < 5 ? sc[L::oRef + f] : 0.f;  // the extrapolation reproduces constants
+    float* o = sc + f * NP;                            // face k's point i at o[k * MX_XF * NP + i]
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        float a0 = 0.f, a2 = 0.f;
+#pragma unroll
+        for (int l = 0; l < N1; ++l) {
+          a0 += op.E02[0][sd][l] * x[l * NT + i];
+          a2 += op.E02[1][sd][l] * x[i * N1 + l];
+        }
+        o[sd * MX_XF * NP + i] = base + a0;
+        o[(4 + sd) * MX_XF * NP + i] = base + a2;
+      }
+      if (face_mask >> (2 + sd) & 1) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          float a1 = 0.f;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) a1 += op.E1[sd][i / N1][t] * x[t * N1 + i % N1];
+          o[(2 + sd) * MX_XF * NP + i] = base + a1;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  // face-point fields of the faces that some slot reads, one contiguous block per face
+  for (int c = 0; c < nc; ++c) {
+    const float* sc = sw + c * L::cell;
+    float* dst = XF + (size_t)(e0 + c) * 6 * FW * NP;
+    if (VISC && FW == MX_XF) {
+      constexpr int HB = MX_XF * NP;  // floats per face block
+      for (int t = lane; t < 6 * HB / 2; t += 32) {
+        const bool use = (face_mask >> (2 * t / HB) & 1) | (face_mask >> ((2 * t + 1) / HB) & 1);
+        if (use) reinterpret_cast<float2*>(dst)[t] = reinterpret_cast<const float2*>(sc)[t];
+      }
+    } else {
+      for (int t = lane; t < 6 * 5 * NP; t += 32) {
+        const int k = t / (5 * NP), j = t - k * (5 * NP);
+        if (face_mask >> k & 1) dst[k * FW * NP + j] = sc[k * MX_XF * NP + j];
+      }
+    }
+  }
+  if constexpr (VISC) {
+    // the gradient fields are consumed: their rows park the viscous terms
+#pragma unroll
+    for (int r = 0; r < PR; ++r) {
+      const int c = r * CPR + pc;
+      if (pc < CPR && c < CW) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) sw[c * L::cell + L::oX + (5 + v) * FS + s] = vis[r][v];
+      }
+    }
+  }
+
+  // ---- c2f, triangle part: one lane per (cell, variable, c-level) ----
+  for (int it = lane; it < CW * 5 * N1; it += 32) {
+    const int c = it / (5 * N1), vk = it - c * (5 * N1), v = vk / N1, k = vk - v * N1;
+    float* sc = sw + c * L::cell;
+    float x[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) x[t] = sc[L::oX + v * FS + t * N1 + k];
+    float* y = sc + L::oY + vk * TP;
+#pragma unroll
+    for (int t4 = 0; t4 < (MT + 3) / 4; ++t4) {
+      float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (t4 * 4 + j < MT) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) z[j] += op.Ct[t4 * 4 + j][t] * x[t];
+        }
+      *reinterpret_cast<float4*>(y + t4 * 4) = make_float4(z[0], z[1], z[2], z[3]);
+    }
+  }
+  // Euler flux at the reference state, FP64: lane = (cell, direction)
+  if (lane < 3 * CW) {
+    const int c = lane / 3, n = lane % 3;
+    float* sc = sw + c * L::cell;
+    const float* rf = sc + L::oRef;
+    const double q[5] = {rf[0], rf[1], rf[2], rf[3], rf[4]};
+    const double un = n == 0 ? q[1] : (n == 1 ? q[2] : q[3]);
+    const double m = q[0] * un;
+    double* F = reinterpret_cast<double*>(sc + L::oF) + n * 5;
+    F[0] = m;
+    F[1] = m * q[1] + (n == 0 ? q[4] : 0.0);
+    F[2] = m * q[2] + (n == 1 ? q[4] : 0.0);
+    F[3] = m * q[3] + (n == 2 ? q[4] : 0.0);
+    F[4] = un * (GAMMA / (GAMMA - 1.0) * q[4] + 0.5 * q[0] * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]));
+  }
+  __syncwarp();
+
+  // ---- fine points: one lane per (cell, fine triangle point) walks the
+  // c-line: c2f along c, flux deviation, contravariant components, and the
+  // c part of W accumulated in registers ----
+  for (int it = lane; it < CW * MT; it += 32) {
+    const int c = it / MT, t = it - c * MT;
+    float* sc = sw + c * L::cell;
+    float af[9][NF];
+    {
+      const float* ap = pg.adjf + ((size_t)(e0 + (c < nc ? c : 0)) * 9 * MT + t) * NF;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        if constexpr (NF == 4) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(ap + (size_t)k * MT * NF));
+          af[k][0] = x.x;
+          af[k][1] = x.y;
+          af[k][2] = x.z;
+          af[k][NF - 1] = x.w;
+        } else {
+#pragma unroll
+          for (int l = 0; l < NF; ++l) af[k][l] = __ldg(ap + (size_t)k * MT * NF + l);
+        }
+      }
+    }
+    float y[5][N1], qb[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      qb[v] = sc[L::oRef + v];
+#pragma unroll
+      for (int k = 0; k < N1; ++k) y[v][k] = sc[L::oY + (v * N1 + k) * TP + t];
+    }
+    float h[3][5][N1];
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+      for (int v = 0; v < 5; ++v)
+#pragma unroll
+        for (int k = 0; k < N1; ++k) h[m][v][k] = 0.f;
+#pragma unroll
+    for (int l = 0; l < NF; ++l) {
+      float dq[5], dF[3][5];
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        dq[v] = 0.f;
+#pragma unroll
+        for (int k = 0; k < N1; ++k) dq[v] += op.Cc[l][k] * y[v][k];
+      }
+      mxd::euler_flux_delta(qb, dq, dF);
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          const float ft = af[m * 3][l] * dF[0][v] + af[m * 3 + 1][l] * dF[1][v] + af[m * 3 + 2][l] * dF[2][v];
+#pragma unroll
+          for (int k = 0; k < N1; ++k) h[m][v][k] += op.Wc[m][k][l] * ft;
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+      for (int v = 0; v < 5; ++v)
+#pragma unroll
+        for (int k = 0; k < N1; ++k) sc[((m * 5 + v) * N1 + k) * TP + t] = h[m][v][k];
+  }
+  __syncwarp();
+
+  // ---- W, triangle part: one lane per (cell, variable, c-level) ----
+  for (int it = lane; it < CW * 5 * N1; it += 32) {
+    const int c = it / (5 * N1), vk = it - c * (5 * N1), v = vk / N1, k = vk - v * N1;
+    float* sc = sw + c * L::cell;
+    float o[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) o[j] = 0.f;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const float4* hp = reinterpret_cast<const float4*>(sc + (m * 5 * N1 + vk) * TP);
+#pragma unroll
+      for (int t4 = 0; t4 < (MT + 3) / 4; ++t4) {
+        const float4 x = hp[t4];
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (t4 * 4 + i < MT) {
+#pragma unroll
+            for (int j = 0; j < NT; ++j) o[j] += op.Wt[m][j][t4 * 4 + i] * xv[i];
+          }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j) sc[L::oX + v * FS + j * N1 + k] = o[j];  // the deviations are consumed
+  }
+  __syncwarp();
+
+  // ---- volume terms: -(W*dFt + MD*F(ref)) / det and the viscous part ----
+#pragma unroll
+  for (int r = 0; r < PR; ++r) {
+    const int c = r * CPR + pc;
+    if (pc < CPR && c < nc) {
+      float* sc = sw + c * L::cell;
+      const size_t p = (size_t)(e0 + c) * S + s;
+      const double md0 = __ldg(pg.MD + p * 3), md1 = __ldg(pg.MD + p * 3 + 1), md2 = __ldg(pg.MD + p * 3 + 2);
+      const double rdet = __ldg(pg.rdet + p);
+      const double* F = reinterpret_cast<const double*>(sc + L::oF);
+      const float* x = sc + L::oX + s;
+      float o[10];
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const double mdf = md0 * F[v] + md1 * F[5 + v] + md2 * F[10 + v];
+        o[v] = float(-(double(x[v * FS]) + mdf) * rdet);
+        o[5 + v] = (VISC && v > 0) ? x[(4 + v) * FS] : 0.f;
+      }
+      float2* tile = reinterpret_cast<float2*>(sc + 10 * s);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) tile[k] = make_float2(o[2 * k], o[2 * k + 1]);
+    }
+  }
+  __syncwarp();
+  for (int c = 0; c < nc; ++c) {
+    const float2* src = reinterpret_cast<const float2*>(sw + c * L::cell);
+    float2* dst = reinterpret_cast<float2*>(RV + (size_t)(e0 + c) * S * 10);
+    for (int t = lane; t < 5 * S; t += 32) dst[t] = src[t];
+  }
+}
+
+// FP64 3 x 3 metric entries (npts per cell, 9 each) -> FP32 planes (N, 9, npts)
+__global__ void k_px_planes(const double* __restrict__ adj, size_t ncells, int npts, float* __restrict__ out) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ncells * npts * 9) return;
+  const int p = (int)(t % npts), k = (int)(t / npts % 9);
+  const size_t c = t / ((size_t)npts * 9);
+  out[t] = float(adj[(c * npts + p) * 9 + k]);
+}
+
+// ---- host: operator structure ----
+// Kronecker factors of an (R*r) x (K*k) operator at a(row, col): A = T (R x K)
+// (x) c (r x k); false when the operator is not such a product to tol of its
+// largest entry
+template <class Get>
+inline bool px_kron(int R, int r, int K, int k, Get a, double tol, std::vector<double>& T, std::vector<double>& c) {
+  double big = 0.0;
+  int pi = 0, pj = 0;
+  for (int i = 0; i < R * r; ++i)
+    for (int j = 0; j < K * k; ++j) {
+      const double x = std::fabs(a(i, j));
+      if (!(x <= 1e300)) return false;
+      if (x > big) {
+        big = x;
+        pi = i;
+        pj = j;
+      }
+    }
+  if (big == 0.0) return false;
+  T.assign((size_t)R * K, 0.0);
+  c.assign((size_t)r * k, 0.0);
+  for (int i = 0; i < R; ++i)
+    for (int j = 0; j < K; ++j) T[i * K + j] = a(i * r + pi % r, j * k + pj % k);
+  for (int i = 0; i < r; ++i)
+    for (int j = 0; j < k; ++j) c[i * k + j] = a(pi / r * r + i, pj / k * k + j) / a(pi, pj);
+  for (int i = 0; i < R * r; ++i)
+    for (int j = 0; j < K * k; ++j)
+      if (std::fabs(a(i, j) - T[(i / r) * K + j / k] * c[(i % r) * k + j % k]) > tol * big) return false;
+  return true;
+}
+
+// The structured operators of a prism set, or false when an operator lacks the
+// structure: D (S, S, 3), E (3, 2, P, S), c2f (Fn, S), W (S, Fn, 3).
+// tol: 1e-12 of an operator's largest entry, a hundred times what the
+// reference's own operators show and far below the 6e-8 of the FP32 copies.
+template <int N1, int NF>
+inline bool px_operators(const double* D, const double* E, const double* c2f, const double* W, PxOps<N1, NF>& o) {
+  constexpr int NT = N1 * N1, S = NT * N1, MT = NF * NF, FN = MT * NF, P = NT;
+  constexpr double TOL = 1e-12;
+  double big = 0.0;
+  for (int i = 0; i < S * S * 3; ++i) big = std::max(big, std::fabs(D[i]));
+  auto d = [&](int s, int j, int m) { return D[((size_t)s * S + j) * 3 + m]; };
+  for (int s = 0; s < S; ++s)
+    for (int j = 0; j < S; ++j) {
+      const int a = s / NT, c = s % N1, a2 = j / NT, c2 = j % N1, t = s / N1, t2 = j / N1;
+      const double w0 = s % NT == j % NT ? d(a * NT, a2 * NT, 0) : 0.0;
+      const double w1 = c == c2 ? d(t * N1, t2 * N1, 1) : 0.0;
+      const double w2 = t == t2 ? d(c, c2, 2) : 0.0;
+      if (!(std::fabs(d(s, j, 0) - w0) <= TOL * big && std::fabs(d(s, j, 1) - w1) <= TOL * big &&
+            std::fabs(d(s, j, 2) - w2) <= TOL * big))
+        return false;
+    }
+  for (int i = 0; i < N1; ++i)
+    for (int j = 0; j < N1; ++j) {
+      o.D0[i][j] = (float)d(i * NT, j * NT, 0);
+      o.D2[i][j] = (float)d(i, j, 2);
+    }
+  for (int i = 0; i < NT; ++i)
+    for (int j = 0; j < NT; ++j) o.D1[i][j] = (float)d(i * N1, j * N1, 1);
+  auto e = [&](int ax, int sd, int i, int s) { return E[(((size_t)ax * 2 + sd) * P + i) * S + s]; };
+  big = 0.0;
+  for (int i = 0; i < 6 * P * S; ++i) big = std::max(big, std::fabs(E[i]));
+  for (int sd = 0; sd < 2; ++sd) {
+    for (int i = 0; i < P; ++i)
+      for (int s = 0; s < S; ++s) {
+        const double w0 = s % NT == i ? e(0, sd, 0, s / NT * NT) : 0.0;
+        const double w1 = s % N1 == i % N1 ? e(1, sd, i / N1 * N1, s / N1 * N1) : 0.0;
+        const double w2 = s / N1 == i ? e(2, sd, 0, s % N1) : 0.0;
+        if (!(std::fabs(e(0, sd, i, s) - w0) <= TOL * big && std::fabs(e(1, sd, i, s) - w1) <= TOL * big &&
+              std::fabs(e(2, sd, i, s) - w2) <= TOL * big))
+          return false;
+      }
+    for (int l = 0; l < N1; ++l) {
+      o.E02[0][sd][l] = (float)e(0, sd, 0, l * NT);
+      o.E02[1][sd][l] = (float)e(2, sd, 0, l);
+    }
+    for (int a = 0; a < N1; ++a)
+      for (int t = 0; t < NT; ++t) o.E1[sd][a][t] = (float)e(1, sd, a * N1, t * N1);
+  }
+  std::vector<double> T, c;
+  if (!px_kron(MT, NF, NT, N1, [&](int i, int j) { return c2f[(size_t)i * S + j]; }, TOL, T, c)) return false;
+  for (int i = 0; i < MT * NT; ++i) o.Ct[i / NT][i % NT] = (float)T[i];
+  for (int i = 0; i < NF * N1; ++i) o.Cc[i / N1][i % N1] = (float)c[i];
+  for (int m = 0; m < 3; ++m) {
+    if (!px_kron(NT, N1, MT, NF, [&](int i, int j) { return W[((size_t)i * FN + j) * 3 + m]; }, TOL, T, c))
+      return false;
+    for (int i = 0; i < NT * MT; ++i) o.Wt[m][i / MT][i % MT] = (float)T[i];
+    for (int i = 0; i < N1 * NF; ++i) o.Wc[m][i / NF][i % NF] = (float)c[i];
+  }
+  return true;
+}
+
+}  // namespace afr
