@@ -86,7 +86,7 @@ struct afr_handle {
   int32_t* mx_rest = nullptr;
   int mx_npairs = 0, mx_nrest = 0;
   bool mx_paired = false;
-  int mx_upd_var = 1;       // update-kernel cells per CTA: 0 = half, 1 = base, 2 = double
+  int mx_upd_var = 1;       // update-kernel warps per CTA: 2, 4 or 8 (variant 0, 1, 2)
   // dual-time / IMEX buffers, allocated by the first call of either scheme
   double* iRinv = nullptr;   // (N,S,nv) inviscid residual (dU/dt)
   double* iRvisc = nullptr;  // (N,S,nv) viscous residual (dU/dt)
@@ -380,11 +380,8 @@ struct Launch {
   }
   // ---- mixed-precision form ----
   static constexpr int MXC = 16;                            // cells per volume-kernel tile
-  static constexpr int MXU = S <= 8 ? 16 : (S <= 27 ? 4 : 2);  // cells per update-kernel CTA
   static size_t mx_pre_smem() { return MxPreSmem<S, NP>::total; }
   static size_t mx_vol_smem() { return MxVolSmem<S, FN, MXC>::total; }
-  static constexpr int MXU0 = MXU / 2 > 0 ? MXU / 2 : 1, MXU2 = MXU * 2;  // autotuner candidates
-  static size_t mx_upd_smem() { return MxUpdSmem<S, NP, MXU>::total; }
   // resident CTAs per SM of the persistent kernels, capped by tensor memory (512 columns per SM)
   static cudaError_t mx_grids(afr_handle* h) {
     int dev = 0, sms = 0, bp = 0, bc = 0;
@@ -395,14 +392,7 @@ struct Launch {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_mx_vol<S, FN, MXC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_vol_smem());
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mx_update<S, NP, MXU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)mx_upd_smem());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mx_update<S, NP, MXU0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)MxUpdSmem<S, NP, MXU0>::total);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mx_update<S, NP, MXU2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)MxUpdSmem<S, NP, MXU2>::total);
+      e = cudaFuncSetAttribute(k_mx_update<S, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 8));
     if constexpr (PXD) {
       auto* fv = k_px_cell<PXN1, PXNF, PXC, true>;
       auto* fi = k_px_cell<PXN1, PXNF, PXC, false>;
@@ -445,10 +435,10 @@ struct Launch {
     h->n_sms = sms;
     return cudaSuccess;
   }
-  template <int CPB>
-  static void mx_update_launch(afr_handle* h, const StageArgs& a, int n, cudaStream_t st) {
-    k_mx_update<S, NP, CPB><<<(n + CPB - 1) / CPB, MxUpdSmem<S, NP, CPB>::THREADS, MxUpdSmem<S, NP, CPB>::total, st>>>(
-        h->g, h->ops, h->fc, a, h->mb.RV, h->mb.Jm, h->mo.rdet);
+  static void mx_update_launch(afr_handle* h, const StageArgs& a, int ct, int n, cudaStream_t st) {
+    const int warps = 2 << h->mx_upd_var, per = warps * MxUpd<S>::CW;
+    k_mx_update<S, NP><<<(n + per - 1) / per, 32 * warps, MxUpd<S>::bytes(h->nv, warps), st>>>(
+        h->ops, h->fc, a, ct, h->mb.RV, h->mb.Jm, h->mo.rdet);
   }
   static int n_ranges(const afr_handle* h) { return (h->n_prism > 0 ? 1 : 0) + (h->N > h->n_prism ? 1 : 0); }
   // structured prisms: one kernel forms the face-point fields and the volume terms
@@ -520,9 +510,7 @@ struct Launch {
       a.cell_end = ranges[r + 1];
       const int n = a.cell_end - a.cell_base;
       if (n <= 0) continue;
-      if (h->mx_upd_var == 0) mx_update_launch<MXU0>(h, a, n, st);
-      else if (h->mx_upd_var == 2) mx_update_launch<MXU2>(h, a, n, st);
-      else mx_update_launch<MXU>(h, a, n, st);
+      mx_update_launch(h, a, r, n, st);
     }
     return cudaGetLastError();
   }
@@ -973,10 +961,10 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   const int FW = h->order <= 2 ? MX_XF : 5;
   float *xf, *pfm = nullptr, *jm;
   const size_t ns = h->slots.n;
-  if ((rc = dalloc(h, &xf, N * FW * 6 * P)) || (rc = dalloc(h, &jm, ns * P * 10 + 4)))  // 16 bytes of slack: the update kernel copies 16-byte-rounded slot ranges
+  if ((rc = dalloc(h, &xf, N * FW * 6 * P)) || (rc = dalloc(h, &jm, ns * P * 9)))
     return rc;
   float* rv;
-  if ((rc = dalloc(h, &rv, N * S * 10))) return rc;
+  if ((rc = dalloc(h, &rv, N * S * 9))) return rc;
   h->mb = MxBuf{xf, pfm, jm, rv, FW};
   float4* arow;
   uint8_t* ofp;
@@ -1957,7 +1945,7 @@ int afr_autotune(afr_handle* h, const double* U, const double* nu_t, int32_t* ch
     return fail(h, AFR_ENOMEM, "autotune scratch");
   }
   const double* nut = h->prm.turb == AFR_TURB_SST ? nu_t : nullptr;
-  // coordinate search: pre-pass CTAs per SM, face-kernel block, update-kernel cells per CTA
+  // coordinate search: pre-pass CTAs per SM, face-kernel block, update-kernel warps per CTA
   if (!h->px || h->N > h->n_prism) {  // the tensor-core pre-pass runs
     int best = h->mx_pre_per_sm;
     float tb = 1e30f;

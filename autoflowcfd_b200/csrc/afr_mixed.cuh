@@ -20,7 +20,7 @@
 //              cells' FP32 point fields with the reference's matrices;
 //   k_mx_vol   per C-cell tile (persistent): c2f, viscous D_3d and the folded
 //              W = f2c*D_fine divergence as GEMMs -> volume terms (FP32);
-//   k_mx_update per few cells: lifting in ascending color order, outlier
+//   k_mx_update a warp per few cells: lifting in ascending color order, outlier
 //              zeroing, SSP-RK3 combination, positivity (FP64), filter (an
 //              FP64 product on the tensor path).
 //
@@ -85,8 +85,8 @@ constexpr int MX_PF = 16;  // floats per solution point: gradients (9), mu_t, q 
 struct MxBuf {
   float* XF;   // (N, 6, FW, NP) point fields at the face points, one contiguous block per face of the cell
   float* PFm;  // (N, S, MX_PF)
-  float* Jm;   // (n_slots, NP, 10) inviscid and viscous jumps
-  float* RV;   // (N, S, 10) inviscid and viscous volume terms
+  float* Jm;   // (n_slots, 9, NP) jumps: inviscid (5), viscous momentum and energy (4)
+  float* RV;   // (N, 9, S) volume terms, in the same order
   int FW;      // MX_XF (orders 1, 2) or 5 (order 3: inviscid only)
 };
 
@@ -543,9 +543,9 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
   float Fc[5], Fp[3][5];
   ausm_up<float>(ow, ot, dir, Fc);
   euler_flux<float>(ow, Fp);
-  float* Jo = mb.Jm + (size_t)t * 10;
+  float* Jo = mb.Jm + (size_t)sl * 9 * NP + i;
 #pragma unroll
-  for (int v = 0; v < 5; ++v) Jo[v] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
+  for (int v = 0; v < 5; ++v) Jo[v * NP] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
   if (visc) {
     float av[MX_XF];  // the common flux: both sides' averages
 #pragma unroll
@@ -553,20 +553,19 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
     float Gc[3][4], Go[3][4];
     viscous_flux_sym<float>(av + 1, av + 5, av + 11, mu, av[14], Gc);
     viscous_flux_sym<float>(ow + 1, ow + 5, ow + 11, mu, ow[14], Go);
-    float jv[5];
-    jv[0] = 0.f;
+    float jv[4];  // momentum and energy (no viscous mass flux)
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      jv[1 + v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
+      jv[v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
     if (bnd) {
       // interior penalty (core/fr_operators/flux_kernels.py:140-200)
       const float eta = float(C_IP) * (mu + ow[14]) / float(hcell[e]);
       const float scale = eta * ar.w * side;
 #pragma unroll
-      for (int v = 1; v < 4; ++v) jv[v] += -scale * (ow[v] - ot[v]);
+      for (int v = 0; v < 3; ++v) jv[v] += -scale * (ow[1 + v] - ot[1 + v]);
     }
 #pragma unroll
-    for (int v = 0; v < 5; ++v) Jo[5 + v] = jv[v];
+    for (int v = 0; v < 4; ++v) Jo[(5 + v) * NP] = jv[v];
   }
 }
 
@@ -680,8 +679,8 @@ __global__ void __launch_bounds__(256, 3) k_mx_face_pair(Faces fc, Bc bc, SlotTa
 
 // ---------------------------------------------------------------------------
 // volume kernel: persistent over C-cell tiles, tensor-core contractions.
-// Writes the volume terms RV (N, S, 10) FP32: inviscid -(W*Ft + MD*F(qbar))/det
-// (5) and viscous D_3d*Gt/det (5).
+// Writes the volume terms RV (N, 9, S) FP32: inviscid -(W*Ft + MD*F(qbar))/det
+// (5) and the momentum and energy rows of the viscous D_3d*Gt/det (4).
 // ---------------------------------------------------------------------------
 constexpr int MX_VOL_THREADS = 512;
 
@@ -697,7 +696,7 @@ struct MxVolSmem {
   static constexpr int szAc = 128 * Sq * 4, szAD = VP ? 128 * 3 * Sq * 4 : 0, szAW = 128 * 3 * Fq * 4;
   static constexpr int szR1 = cmax(szAc + szAD, szAW);
   static constexpr int oR2 = oR1 + szR1;  // q (FP64) before the first product, then dq, then the RV tile
-  static constexpr int szR2 = cmax(cmax(C * QS * 4, C * S * 5 * 8), C * S * 10 * 4);
+  static constexpr int szR2 = cmax(cmax(C * QS * 4, C * S * 5 * 8), C * S * 9 * 4);
   static constexpr int oX = oR2 + szR2;
   // doubles: qbar, F(qbar); with VP also det and the metric divergence of the tile
   static constexpr int nX = C * 5 + C * 15 + (VP ? C * S * 4 : 0);
@@ -965,8 +964,8 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int s = ch * 8 + j;
-            if (s < S && c < nc)
-              sR[(c * S + s) * 10 + 5 + v] = visc ? float(double(v8[j] + w8[j]) * sDet[c * S + s]) : 0.f;
+            if (s < S && c < nc && v > 0)
+              sR[(c * 9 + 4 + v) * S + s] = visc ? float(double(v8[j] + w8[j]) * sDet[c * S + s]) : 0.f;
           }
         }
       }
@@ -991,7 +990,7 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
               const double* md = L::VP ? sMD + (c * S + s) * 3 : mo.MD + p * 3;
               const double rdj = L::VP ? sDet[c * S + s] : __ldg(mo.rdet + p);
               const double mdf = md[0] * sFb[c * 15 + v] + md[1] * sFb[c * 15 + 5 + v] + md[2] * sFb[c * 15 + 10 + v];
-              sR[(c * S + s) * 10 + v] = float(-(double(v8[j] + w8[j]) + mdf) * rdj);
+              sR[(c * 9 + v) * S + s] = float(-(double(v8[j] + w8[j]) + mdf) * rdj);
             }
           }
         }
@@ -999,7 +998,7 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
     }
     __syncthreads();
     // coalesced store of the tile's volume terms (cells e0 .. e0+nc are contiguous)
-    mxd::copy_f32(RV + (size_t)e0 * S * 10, sR, nc * S * 10);
+    mxd::copy_f32(RV + (size_t)e0 * S * 9, sR, nc * S * 9);
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -1014,342 +1013,335 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-// update kernel: CPB cells per CTA.  Lifting of the face jumps in ascending
-// color order (staged in shared memory), outlier zeroing, then the SSP-RK3
+// update kernel: a warp owns CW whole cells from load to store.  Lifting of the
+// face jumps in ascending color order, outlier zeroing, then the SSP-RK3
 // combination, positivity and filter in FP64 (or the residual-only outputs).
 //
-// The tile's inputs are contiguous blocks (the cells e0 .. e0+nc of the state,
-// step-start state, volume terms, reciprocal det and dt, and the slots of
-// those cells' jumps); each arrives in shared memory by one bulk asynchronous
-// copy (cp.async.bulk, completion counted in bytes on an mbarrier).  A block
-// whose address or size is not a multiple of 16 bytes (odd first cell of a
-// range, odd last tile) is copied by 8-byte asynchronous copies instead.
-// Shared-memory rows keep the global layout: state rows of n_vars doubles (an
-// odd stride, so threads reading consecutive points use distinct banks).
+// A lane owns a solution point (S <= 27; two at S = 64; four cells side by
+// side at S = 8), so the residual, the outlier test and the RK combination
+// stay in registers and the phases need no block barrier: the block-wide form
+// of this kernel spent 2,600 instructions per P2 cell, most of them index
+// arithmetic around shared-memory tiles.  The volume terms and the jumps are
+// stored field-major (planes of points), so every load of a lane's values is
+// one coalesced access.  CW = 3 at P2 and P3 makes the filter's 5*CW = 15
+// columns two nearly full column tiles of the FP64 tensor product.
 // ---------------------------------------------------------------------------
-constexpr int MX_UPD_MAXSLOT = 6;  // slots per cell staged in shared memory (more: read from global)
+constexpr int MX_UPD_SLOTS = 5;  // slots per cell whose jumps are loaded together (more: one by one)
 
-__host__ __device__ constexpr int align16(int b) { return (b + 15) / 16 * 16; }
-
-template <int S, int NP, int CPB>
-struct MxUpdSmem {
-  static constexpr int THREADS = 256;
-  static constexpr int NVMAX = 7;
-  // byte offsets; bulk-copy destinations 16-byte aligned
-  static constexpr int bU = 0;                                        // CPB*S*nv doubles
-  static constexpr int bU0 = align16(bU + CPB * S * NVMAX * 8);       // step-start state
-  static constexpr int bRV = align16(bU0 + CPB * S * NVMAX * 8);      // CPB*S*10 floats
-  static constexpr int bRd = align16(bRV + CPB * S * 10 * 4);         // CPB*S doubles
-  static constexpr int bDt = align16(bRd + CPB * S * 8);              // CPB*S doubles
-  static constexpr int bJ = align16(bDt + CPB * S * 8);               // jumps, 16-byte lead
-  static constexpr int bRi = align16(bJ + CPB * MX_UPD_MAXSLOT * NP * 10 * 4 + 16);  // CPB*S*5 doubles
-  static constexpr int bRv = bRi + CPB * S * 5 * 8;                   // CPB*S*5 doubles
-  static constexpr int bW = bRv + CPB * S * 5 * 8;                    // outliers: CPB*2*OUT_WORK doubles
-  static constexpr int bP = bW + CPB * 2 * OUT_WORK * 8;              // 2*CPB*S doubles
-  static constexpr int bG = bP + 2 * CPB * S * 8;                     // g_left, g_right (8 doubles)
-  static constexpr int bI = bG + 8 * 8;                               // ints
-  static constexpr int nI = CPB * MX_UPD_MAXSLOT + CPB + 1 + 6 * S;
-  static constexpr int total = bI + nI * 4;
+template <int S>
+struct MxUpd {
+  static constexpr int PL = (S + 31) / 32;            // points per lane
+  static constexpr int CPR = S < 32 ? 32 / S : 1;     // cells side by side in a warp
+  static constexpr int CW = S == 8 ? 8 : 3;           // cells per warp
+  static constexpr int PR = CW / CPR;                 // rounds
+  static_assert(CW % CPR == 0, "whole rounds");
+  // shared memory: g' per (side, axis, point), face point per (axis, point);
+  // per warp two state tiles (current state, then the filtered one; step-start state, then the output)
+  static constexpr int tab = 6 * S * 8 + (3 * S * 4 + 15) / 16 * 16;
+  __host__ __device__ static constexpr int warp_bytes(int nv) { return 2 * CW * S * nv * 8; }
+  static constexpr int bytes(int nv, int warps) { return tab + warps * warp_bytes(nv); }
 };
 
 namespace mxd {
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(bytes)
-               : "memory");
+
+// maximum over the lanes of a cell
+template <int S>
+__device__ __forceinline__ unsigned cell_max(unsigned x) {
+  if constexpr (S == 8) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
+    return x;
+  } else {
+    return __reduce_max_sync(0xffffffffu, x);
+  }
 }
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   tc::smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
-               : "memory");
+
+// lanes of this cell where p holds
+template <int S>
+__device__ __forceinline__ unsigned cell_ballot(bool p, int grp) {
+  const unsigned b = __ballot_sync(0xffffffffu, p);
+  return S == 8 ? (b >> (8 * grp)) & 0xffu : b;
 }
-__device__ __forceinline__ bool bulk_ok(const void* src, size_t bytes) {
-  return ((reinterpret_cast<uintptr_t>(src) | bytes) & 15u) == 0 && bytes > 0;
+
+template <int S>
+__device__ __forceinline__ double cell_sum(double x) {
+#pragma unroll
+  for (int o = 1; o < (S == 8 ? 8 : 32); o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
 }
-// 8-byte asynchronous copies of a block whose bulk copy is not possible
-__device__ __forceinline__ void copy8(void* dst, const void* src, size_t bytes) {
-  for (size_t t = threadIdx.x; t < bytes / 8; t += blockDim.x)
-    cp_async8(static_cast<char*>(dst) + 8 * t, static_cast<const char*>(src) + 8 * t);
+
+// True when the outlier rule (|R| > 1e4 * max(median |R|, 1e-9 mean |U|,
+// 1e-300) is zeroed, core/fr_operators/troubled_cell.py:346-408) provably
+// zeroes nothing of a column: at least as many values as lie at or above the
+// median's rank reach 1e-4 of an upper bound of the largest one.  The bound is
+// the largest high word plus one, so one integer maximum and one ballot
+// decide; columns that fail (or hold a NaN or infinity) take outlier_exact.
+template <int S, int PL>
+__device__ __forceinline__ bool outlier_clear(const double (&x)[PL], const bool (&on)[PL], int grp) {
+  constexpr int NEED = S - ((S & 1) ? S / 2 : S / 2 - 1);
+  unsigned hw = 0u;
+#pragma unroll
+  for (int l = 0; l < PL; ++l) hw = max(hw, on[l] ? (unsigned)__double2hiint(x[l]) & 0x7fffffffu : 0u);
+  hw = cell_max<S>(hw);
+  if (hw >= 0x7fe00000u) return false;
+  const double hi = __hiloint2double((int)hw + 1, 0);
+  const double p = hi * 1.0000000001e-4;  // 1e4 * p >= hi after rounding
+  int cnt = 0;
+#pragma unroll
+  for (int l = 0; l < PL; ++l) cnt += __popc(cell_ballot<S>(on[l] && fabs(x[l]) >= p, grp));
+  return cnt >= NEED || hi <= 1e-297;
+}
+
+// the rule itself: stable ranks over the cell's points, median, zeroing
+template <int S, int PL>
+__device__ __noinline__ void outlier_exact(double (&x)[PL], const double (&u)[PL], const bool (&on)[PL], int grp,
+                                           int s0) {
+  double acc = 0.0;
+#pragma unroll
+  for (int l = 0; l < PL; ++l) acc += on[l] ? fabs(u[l]) : 0.0;
+  const double mean = cell_sum<S>(acc) / S;
+  int rank[PL];
+#pragma unroll
+  for (int l = 0; l < PL; ++l) rank[l] = 0;
+  for (int j = 0; j < S; ++j) {
+    double src = x[0];
+    if constexpr (PL > 1) src = j >= 32 ? x[PL - 1] : x[0];
+    const double y = fabs(__shfl_sync(0xffffffffu, src, (S == 8 ? 8 * grp : 0) + (j & 31)));
+#pragma unroll
+    for (int l = 0; l < PL; ++l) {
+      const double a = fabs(x[l]);
+      rank[l] += (y < a) || (y == a && j < s0 + 32 * l);
+    }
+  }
+  auto at_rank = [&](int r) {  // |x| of the point with rank r (0 where a NaN leaves none)
+    double v = 0.0;
+#pragma unroll
+    for (int l = 0; l < PL; ++l) {
+      const unsigned b = cell_ballot<S>(on[l] && rank[l] == r, grp);
+      const double y = fabs(__shfl_sync(0xffffffffu, x[l], (S == 8 ? 8 * grp : 0) + (b ? __ffs(b) - 1 : 0)));
+      if (b) v = y;
+    }
+    return v;
+  };
+  const double med = (S & 1) ? at_rank(S / 2) : 0.5 * (at_rank(S / 2 - 1) + at_rank(S / 2));
+  const double thr = 1e4 * fmax(fmax(med, 1e-9 * mean), 1e-300);
+#pragma unroll
+  for (int l = 0; l < PL; ++l)
+    if (fabs(x[l]) > thr) x[l] = 0.0;
 }
 }  // namespace mxd
 
-// Outlier zeroing of the mixed update kernel (same rule as
-// suppress_outliers_cells, core/fr_operators/troubled_cell.py:346-408): the
-// column statistics -- mean |U|, min and max |R|, NaN, and the count against
-// the lower bound of the median -- by four threads per column (aligned lane
-// groups, combined with shuffles) instead of one.  Reference rows have stride
-// ldU.  work >= OUT_WORK doubles per block (block b < nc: sRi of cell b,
-// nc + b: sRv of cell b).
-template <int S>
-__device__ void mx_suppress_outliers(double* sRi, double* sRv, const double* sU, int ldU, int nc, bool visc,
-                                     double* work) {
-  constexpr int NEED = S - ((S & 1) ? S / 2 : S / 2 - 1);  // elements at or above the (lower) middle rank
-  const int nb = nc * (visc ? 2 : 1);
-  const int ncol = nb * 5;
-  const int n4 = (ncol * 4 + (int)blockDim.x - 1) / (int)blockDim.x * (int)blockDim.x;
-  int flagged = 0;
-  for (int base = 0; base < n4; base += blockDim.x) {
-    const int t = base + threadIdx.x;
-    const bool on = t < ncol * 4;
-    const int col = on ? (t >> 2) : 0, sub = t & 3;
-    const int bb = col / 5, v = col % 5;
-    const double* R = bb < nc ? sRi + bb * S * 5 : sRv + (bb - nc) * S * 5;
-    const double* Ur = sU + (bb % nc) * S * ldU;
-    double acc = 0.0, lo = INFINITY, hi = 0.0;
-    int nan = 0;
-    if (on)
-      for (int s = sub; s < S; s += 4) {
-        acc += fabs(Ur[s * ldU + v]);
-        const double x = fabs(R[s * 5 + v]);
-        lo = fmin(lo, x);
-        hi = fmax(hi, x);
-        nan |= isnan(x) ? 1 : 0;
-      }
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-      acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-      nan |= __shfl_xor_sync(0xffffffffu, nan, o);
-    }
-    const double mean = acc / S;
-    bool skip = !nan && hi <= 1e4 * fmax(fmax(lo, 1e-9 * mean), 1e-300);
-    double bound = lo;
-    bool count = !nan && !skip;
-    double p = hi * 1e-4;
-    if (count) {
-      // next double up (p is finite and >= 0 here: its bit pattern plus one)
-      for (int it = 0; it < 4 && 1e4 * p < hi; ++it) p = __longlong_as_double(__double_as_longlong(p) + 1);
-      count = 1e4 * p >= hi;
-    }
-    int cnt = 0;
-    if (on && count)
-      for (int s = sub; s < S; s += 4) cnt += fabs(R[s * 5 + v]) >= p;
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if (count && cnt >= NEED) {
-      skip = true;
-      bound = p;
-    }
-    if (on && sub == 0) {
-      double* w = work + bb * OUT_WORK;
-      w[5 + v] = mean;
-      w[v] = bound;
-      w[20 + v] = skip ? 0.0 : 1.0;
-      flagged |= !skip;
-    }
-  }
-  if (!__syncthreads_or(flagged)) return;  // no column takes the rank pass: nothing is zeroed
-  for (int t = threadIdx.x; t < nb * S * 5; t += blockDim.x) {
-    const int bb = t / (S * 5), r = t % (S * 5), s = r / 5, v = r % 5;
-    double* w = work + bb * OUT_WORK;
-    if (w[20 + v] != 0.0) outlier_rank<S>(bb < nc ? sRi + bb * S * 5 : sRv + (bb - nc) * S * 5, s, v, w);
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nb * S * 5; t += blockDim.x) {
-    const int bb = t / (S * 5), r = t % (S * 5), v = r % 5;
-    const double* w = work + bb * OUT_WORK;
-    if (w[20 + v] != 0.0) outlier_zero(bb < nc ? sRi + bb * S * 5 : sRv + (bb - nc) * S * 5, r, v, w, S & 1);
-  }
-  __syncthreads();
-}
-
-template <int S, int NP, int CPB>
-__global__ void __launch_bounds__(MxUpdSmem<S, NP, CPB>::THREADS, 5)
-    k_mx_update(Geom g, Ops ops, Faces fc, StageArgs a, const float* __restrict__ RV, const float* __restrict__ Jm,
+template <int S, int NP>
+__global__ void __launch_bounds__(256, S == 64 ? 2 : 3)
+    k_mx_update(Ops ops, Faces fc, StageArgs a, int ct, const float* __restrict__ RV, const float* __restrict__ Jm,
                 const double* __restrict__ rdet) {
-  using L = MxUpdSmem<S, NP, CPB>;
-  extern __shared__ __align__(128) uint8_t smb[];
-  __shared__ uint64_t bar;
-  double* sU = reinterpret_cast<double*>(smb + L::bU);
-  double* sU0 = reinterpret_cast<double*>(smb + L::bU0);
-  float* sRVf = reinterpret_cast<float*>(smb + L::bRV);
-  double* sRd = reinterpret_cast<double*>(smb + L::bRd);
-  double* sDt = reinterpret_cast<double*>(smb + L::bDt);
-  double* sRi = reinterpret_cast<double*>(smb + L::bRi);
-  double* sRv = reinterpret_cast<double*>(smb + L::bRv);
-  double* work = reinterpret_cast<double*>(smb + L::bW);
-  double* part = reinterpret_cast<double*>(smb + L::bP);
-  double* sGw = reinterpret_cast<double*>(smb + L::bG);  // [0..3] g_left, [4..7] g_right
-  int* sFl = reinterpret_cast<int*>(smb + L::bI);
-  int* sPtr = sFl + CPB * MX_UPD_MAXSLOT;
-  int* sDfp = sPtr + CPB + 1;
-  int* sDco = sDfp + 3 * S;
-  const int e0 = a.cell_base + blockIdx.x * CPB;
-  const int nc = min(CPB, a.cell_end - e0);
-  const int ct = cell_type(g, e0);
+  using L = MxUpd<S>;
+  constexpr int PL = L::PL, CPR = L::CPR, CW = L::CW, PR = L::PR;
+  extern __shared__ __align__(16) uint8_t smb[];
+  double* sG = reinterpret_cast<double*>(smb);
+  int* sFp = reinterpret_cast<int*>(smb + 6 * S * 8);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nv = a.nv;
-  const bool visc = !a.inviscid_only;
-  const int tid = threadIdx.x;
-  constexpr int N1D = S == 8 ? 2 : (S == 27 ? 3 : 4);
-  const int k_beg = fc.slot_ptr[e0], k_end = fc.slot_ptr[e0 + nc];
-  const bool staged = (k_end - k_beg) <= CPB * MX_UPD_MAXSLOT;
-  // jump block: bytes [jb0, jb1) of Jm rounded out to 16-byte boundaries (the
-  // allocation carries 16 bytes of slack); the tile's first jump sits jlead
-  // bytes into the staged copy
-  const size_t jb0 = (size_t)k_beg * NP * 40, jb1 = (size_t)k_end * NP * 40;
-  const size_t ja0 = jb0 & ~size_t(15), ja1 = (jb1 + 15) & ~size_t(15);
-  const float* sJ = reinterpret_cast<const float*>(smb + L::bJ + (jb0 - ja0));
-  {
-    const size_t ub = (size_t)nc * S * nv * 8, pb = (size_t)nc * S * 8, rb = (size_t)nc * S * 40;
-    const double* uc = a.Ucur + (size_t)e0 * S * nv;
-    const double* u0 = a.U0 + (size_t)e0 * S * nv;
-    const float* rv = RV + (size_t)e0 * S * 10;
-    const double* rd = rdet + (size_t)e0 * S;
-    const double* dt = a.stage >= 0 ? a.dt + (size_t)e0 * S : nullptr;
-    const char* jsrc = reinterpret_cast<const char*>(Jm) + ja0;
-    const bool bu = mxd::bulk_ok(uc, ub), bu0 = a.stage >= 0 && mxd::bulk_ok(u0, ub), brv = mxd::bulk_ok(rv, rb),
-               brd = mxd::bulk_ok(rd, pb), bdt = a.stage >= 0 && mxd::bulk_ok(dt, pb),
-               bj = staged && k_end > k_beg;  // rounded out: always aligned
-    if (tid == 0) {
-      tc::mbar_init(&bar, 1);
-      tc::fence_mbar_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const uint32_t tx = (bu ? ub : 0) + (bu0 ? ub : 0) + (brv ? rb : 0) + (brd ? pb : 0) + (bdt ? pb : 0) +
-                          (bj ? ja1 - ja0 : 0);
-      mxd::mbar_expect_tx(&bar, tx);
-      if (bu) mxd::bulk_g2s(sU, uc, (uint32_t)ub, &bar);
-      if (bu0) mxd::bulk_g2s(sU0, u0, (uint32_t)ub, &bar);
-      if (brv) mxd::bulk_g2s(sRVf, rv, (uint32_t)rb, &bar);
-      if (brd) mxd::bulk_g2s(sRd, rd, (uint32_t)pb, &bar);
-      if (bdt) mxd::bulk_g2s(sDt, dt, (uint32_t)pb, &bar);
-      if (bj) mxd::bulk_g2s(smb + L::bJ, jsrc, (uint32_t)(ja1 - ja0), &bar);
-    }
-    if (!bu) mxd::copy8(sU, uc, ub);
-    if (a.stage >= 0 && !bu0) mxd::copy8(sU0, u0, ub);
-    if (!brv) mxd::copy8(sRVf, rv, rb);
-    if (!brd) mxd::copy8(sRd, rd, pb);
-    if (a.stage >= 0 && !bdt) mxd::copy8(sDt, dt, pb);
-    for (int t = tid; t < 3 * S; t += blockDim.x) {
-      sDfp[t] = ops.dist_fp[t];
-      sDco[t] = ops.dist_co[t];
-    }
-    if (tid < N1D) {
-      sGw[tid] = ops.g_left[tid];
-      sGw[4 + tid] = ops.g_right[tid];
-    }
-    if (tid <= nc) sPtr[tid] = fc.slot_ptr[e0 + tid];
-    if (staged)
-      for (int t = tid; t < k_end - k_beg; t += blockDim.x) sFl[t] = a.slot_flags[k_beg + t];
-    mxd::cp_async_wait_all();
-    uint32_t ph = 0;
-    if (!mxd::wait_commit(&bar, ph, a.status)) {
-      // the status reports the time-out; wait once more (bounded) so that no
-      // copy is still writing this CTA's shared memory when it moves on
-      uint32_t ph0 = 0;
-      tc::mbar_wait(&bar, ph0);
-    }
+  for (int t = threadIdx.x; t < 3 * S; t += blockDim.x) {
+    const int co = ops.dist_co[t];
+    sG[t] = ops.g_left[co];
+    sG[3 * S + t] = ops.g_right[co];
+    sFp[t] = ops.dist_fp[t];
   }
   __syncthreads();
-  // lift the jumps of each cell's slots, ascending color order; two threads
-  // per point, one for the inviscid and one for the viscous jumps
-  for (int t = tid; t < 2 * nc * S; t += blockDim.x) {
-    const int p = t >> 1, half = t & 1;
-    if (half && !visc) {
-      sRv[p * 5 + 0] = sRv[p * 5 + 1] = sRv[p * 5 + 2] = sRv[p * 5 + 3] = sRv[p * 5 + 4] = 0.0;
+  const int e0 = a.cell_base + (blockIdx.x * (blockDim.x >> 5) + warp) * CW;
+  const int nc = min(CW, a.cell_end - e0);
+  if (nc <= 0) return;  // whole warps; no block barrier below
+  double* sU = reinterpret_cast<double*>(smb + L::tab + warp * L::warp_bytes(nv));
+  double* s0 = sU + CW * S * nv;
+  const bool visc = !a.inviscid_only;
+  const bool step = a.stage >= 0;
+  if (step) {
+    const double* uc = a.Ucur + (size_t)e0 * S * nv;
+    for (int t = lane; t < nc * S * nv; t += 32) cp_async8(sU + t, uc + t);
+    if (a.stage > 0) {  // stage 0 starts from the current state
+      const double* u0 = a.U0 + (size_t)e0 * S * nv;
+      for (int t = lane; t < nc * S * nv; t += 32) cp_async8(s0 + t, u0 + t);
+    }
+    cp_async_commit();
+  }
+  const int grp = S < 32 ? lane / S : 0;  // cell side of the warp
+  const int sp = S < 32 ? lane % S : lane;
+#pragma unroll 1
+  for (int r = 0; r < PR; ++r) {
+    const int c = r * CPR + grp;
+    const int e = e0 + c;
+    const bool live = grp < CPR && c < nc;
+    double x[9][PL];  // dU/dt: inviscid 0..4, viscous momentum and energy 5..8
+    double rd[PL];
+    bool on[PL];
+#pragma unroll
+    for (int l = 0; l < PL; ++l) on[l] = live && sp + 32 * l < S;
+    // jumps of the cell's slots, ascending color order
+    double cx[9][PL];
+#pragma unroll
+    for (int v = 0; v < 9; ++v)
+#pragma unroll
+      for (int l = 0; l < PL; ++l) cx[v][l] = 0.0;
+    const int k0 = live ? fc.slot_ptr[e] : 0, n = live ? fc.slot_ptr[e + 1] - k0 : 0;
+    float rv[9][PL];
+#pragma unroll
+    for (int l = 0; l < PL; ++l) {
+      const size_t p = (size_t)e * S + sp + 32 * l;
+      rd[l] = on[l] ? __ldg(rdet + p) : 0.0;
+#pragma unroll
+      for (int v = 0; v < 9; ++v)
+        rv[v][l] = on[l] && (v < 5 || visc) ? __ldg(RV + ((size_t)e * 9 + v) * S + sp + 32 * l) : 0.f;
+    }
+    for (int kb = 0; kb < n; kb += MX_UPD_SLOTS) {
+      int fl[MX_UPD_SLOTS];
+#pragma unroll
+      for (int j = 0; j < MX_UPD_SLOTS; ++j) fl[j] = kb + j < n ? __ldg(a.slot_flags + k0 + kb + j) : -1;
+#pragma unroll
+      for (int l = 0; l < PL; ++l) {
+#pragma unroll
+        for (int j = 0; j < MX_UPD_SLOTS; ++j) {
+          float jv[9];
+          double gw = 0.0;
+#pragma unroll
+          for (int v = 0; v < 9; ++v) jv[v] = 0.f;
+          if (on[l] && fl[j] >= 0) {
+            const int ax = (fl[j] >> 2) & 3;
+            gw = sG[((fl[j] & 16) ? 3 * S : 0) + ax * S + sp + 32 * l];
+            const float* Jk = Jm + (size_t)(k0 + kb + j) * 9 * NP + sFp[ax * S + sp + 32 * l];
+#pragma unroll
+            for (int v = 0; v < 9; ++v)
+              if (v < 5 || visc) jv[v] = __ldg(Jk + v * NP);
+          }
+#pragma unroll
+          for (int v = 0; v < 9; ++v) cx[v][l] += gw * double(jv[v]);
+        }
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < PL; ++l)
+#pragma unroll
+      for (int v = 0; v < 9; ++v)  // inviscid corrections enter with -g', viscous with +g'
+        x[v][l] = double(rv[v][l]) + (v < 5 ? -cx[v][l] : cx[v][l]) * rd[l];
+    // outliers: a column that is not provably free of them takes the exact rule
+    unsigned bad = 0u;
+#pragma unroll
+    for (int v = 0; v < 9; ++v)
+      if (v < 5 || visc) bad |= mxd::outlier_clear<S, PL>(x[v], on, grp) ? 0u : 1u << v;
+    bad = S == 8 ? __reduce_or_sync(0xffffffffu, bad) : bad;
+    if (bad) {
+#pragma unroll
+      for (int v = 0; v < 9; ++v)
+        if (bad >> v & 1u) {
+          double u[PL];
+#pragma unroll
+          for (int l = 0; l < PL; ++l)
+            u[l] = on[l] ? a.Ucur[((size_t)e * S + sp + 32 * l) * nv + (v < 5 ? v : v - 4)] : 0.0;
+          mxd::outlier_exact<S, PL>(x[v], u, on, grp, sp);
+        }
+    }
+    if (!step) {
+      // residual-only outputs: assembled as rows, stored as blocks below
+#pragma unroll
+      for (int l = 0; l < PL; ++l)
+        if (on[l]) {
+          double* ri = sU + (c * S + sp + 32 * l) * nv;
+          double* rw = s0 + (c * S + sp + 32 * l) * nv;
+#pragma unroll
+          for (int v = 0; v < 7; ++v)
+            if (v < nv) {
+              ri[v] = v < 5 ? x[v < 5 ? v : 0][l] : 0.0;
+              rw[v] = (v > 0 && v < 5 && visc) ? x[v > 0 && v < 5 ? 4 + v : 0][l] : 0.0;
+            }
+        }
       continue;
     }
-    const int b = p / S, s = p - b * S;
-    double cx[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int k = sPtr[b]; k < sPtr[b + 1]; ++k) {
-      const int fl = staged ? sFl[k - k_beg] : a.slot_flags[k];
-      const int ax = (fl >> 2) & 3;
-      const int fp = sDfp[ax * S + s];
-      const double gw = sGw[((fl & 16) ? 4 : 0) + sDco[ax * S + s]];
-      const float* Jk = (staged ? sJ + ((k - k_beg) * NP + fp) * 10 : Jm + ((size_t)k * NP + fp) * 10) + 5 * half;
-#pragma unroll
-      for (int v = 0; v < 5; ++v) cx[v] += gw * double(Jk[v]);
+    if (r == 0) {
+      cp_async_wait0();
+      __syncwarp();
     }
-    const double rdj = sRd[p];
-    const float* rp = sRVf + p * 10 + 5 * half;
-    double* out = half ? sRv : sRi;
-    const double sg = half ? 1.0 : -1.0;  // inviscid corrections enter with -g', viscous with +g'
+    // RK stage combination + positivity, in place over the state tile
+    double sq = 0.0, sr = 0.0;
 #pragma unroll
-    for (int v = 0; v < 5; ++v) out[p * 5 + v] = double(rp[v]) + sg * cx[v] * rdj;
-  }
-  __syncthreads();
-  mx_suppress_outliers<S>(sRi, sRv, sU, nv, nc, visc, work);
-
-  if (a.stage < 0) {
-    for (int p = tid; p < nc * S; p += blockDim.x)
-      for (int v = 0; v < nv; ++v) {
-        const size_t o = ((size_t)e0 * S + p) * nv + v;
-        if (a.Rinv) a.Rinv[o] = v < 5 ? sRi[p * 5 + v] : 0.0;
-        if (a.Rvisc) a.Rvisc[o] = (v < 5 && visc) ? sRv[p * 5 + v] : 0.0;
+    for (int l = 0; l < PL; ++l)
+      if (on[l]) {
+        double Lr[5], un[7];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          Lr[v] = x[v][l] + (v > 0 ? x[v > 0 ? 4 + v : 0][l] : 0.0);
+          sq += Lr[v] * Lr[v];
+        }
+        sr += Lr[0] * Lr[0];
+        const double dts = __ldg(a.dt + (size_t)e * S + sp + 32 * l);
+        double* uc = sU + (c * S + sp + 32 * l) * nv;
+        const double* u0 = a.stage > 0 ? s0 + (c * S + sp + 32 * l) * nv : uc;
+        const double w0 = a.stage == 0 ? 0.0 : (a.stage == 1 ? 0.75 : 1.0 / 3.0);
+        const double w1 = a.stage == 0 ? 1.0 : (a.stage == 1 ? 0.25 : 2.0 / 3.0);
+#pragma unroll
+        for (int v = 0; v < 7; ++v) {
+          const double b = v < nv ? (a.stage == 0 ? uc[v] : w0 * u0[v] + w1 * uc[v]) : 0.0;
+          un[v] = v < 5 ? b + (w1 * dts) * Lr[v < 5 ? v : 0] : b;
+        }
+        // positivity (core/time_integration/positivity.py:13-45), one reciprocal of rho
+        const double rho = fmax(un[0], 1e-6);
+        un[0] = rho;
+        const double rr = 1.0 / rho;
+        double vel[3] = {un[1] * rr, un[2] * rr, un[3] * rr};
+        const double v2 = vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2];
+        double ke = 0.5 * rho * v2;
+        if (v2 > 9.9e7) {  // near or above the speed limit of 1e4
+          const double vm = sqrt(v2);
+          if (vm > 1e4) {
+            const double cf = 1e4 / vm;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              vel[d] *= cf;
+              un[1 + d] = rho * vel[d];
+            }
+          }
+          ke = 0.5 * rho * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
+        }
+        const double pr = (GAMMA - 1.0) * (un[4] - ke);
+        if (pr < 1.0) un[4] = 1.0 / (GAMMA - 1.0) + ke;
+        un[5] = fmax(un[5], 0.0);
+        un[6] = fmax(un[6], 1e-8);
+#pragma unroll
+        for (int v = 0; v < 7; ++v)
+          if (v < nv) uc[v] = un[v];
       }
+    if (a.stage == 0) {
+      const double acc = mxd::cell_sum<S>(sq), acc_rho = mxd::cell_sum<S>(sr);
+      if (live && sp == 0) {
+        a.norm_part[e] = acc;
+        a.norm_rho_part[e] = acc_rho;
+        // a non-finite dU/dt anywhere in the cell makes its partial non-finite
+        if (!isfinite(acc) && a.status) atomicOr(a.status, (unsigned)DS_NONFINITE);
+      }
+    }
+  }
+  __syncwarp();
+  const int nst = nc * S * nv;
+  if (!step) {
+    if (a.Rinv)
+      for (int t = lane; t < nst; t += 32) a.Rinv[(size_t)e0 * S * nv + t] = sU[t];
+    if (a.Rvisc)
+      for (int t = lane; t < nst; t += 32) a.Rvisc[(size_t)e0 * S * nv + t] = s0[t];
     return;
   }
-  // RK stage combination + positivity, in place over the state tile (loops
-  // over the 8 possible variables, unrolled, so the arrays stay in registers)
-  for (int p = tid; p < nc * S; p += blockDim.x) {
-    double Lr[8], un[8];
-    double sq_sum = 0.0;
-#pragma unroll
-    for (int v = 0; v < 8; ++v) Lr[v] = v < 5 ? sRi[p * 5 + v] + (visc ? sRv[p * 5 + v] : 0.0) : 0.0;
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-      if (v < nv) sq_sum += Lr[v] * Lr[v];
-    const double dts = sDt[p];
-    const double* u0 = sU0 + p * nv;
-    double* uc = sU + p * nv;
-    if (a.stage == 0) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) un[v] = v < nv ? u0[v] + dts * Lr[v] : 0.0;
-    } else if (a.stage == 1) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) un[v] = v < nv ? (0.75 * u0[v] + 0.25 * uc[v]) + (0.25 * dts) * Lr[v] : 0.0;
-    } else {
-#pragma unroll
-      for (int v = 0; v < 8; ++v)
-        un[v] = v < nv ? (1.0 / 3.0 * u0[v] + 2.0 / 3.0 * uc[v]) + (2.0 / 3.0 * dts) * Lr[v] : 0.0;
+  // modal filter of the first five variables: one FP64 tensor-core product per
+  // warp (rows s, columns (cell, variable), K = the cell's points) into the
+  // step-start tile, which the stage no longer needs
+  if (nv > 5)
+    for (int p = lane; p < nc * S; p += 32) {
+      s0[p * nv + 5] = sU[p * nv + 5];
+      if (nv > 6) s0[p * nv + 6] = sU[p * nv + 6];
     }
-    // positivity (core/time_integration/positivity.py:13-45), one reciprocal of rho
-    const double rho = fmax(un[0], 1e-6);
-    un[0] = rho;
-    const double rr = 1.0 / rho;
-    double vel[3] = {un[1] * rr, un[2] * rr, un[3] * rr};
-    const double vm = sqrt(vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
-    if (vm > 1e4) {
-      const double cf = 1e4 / vm;
-      for (int d = 0; d < 3; ++d) { vel[d] *= cf; un[1 + d] = rho * vel[d]; }
-    }
-    const double ke = 0.5 * rho * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
-    const double pr = (GAMMA - 1.0) * (un[4] - ke);
-    if (pr < 1.0) un[4] = 1.0 / (GAMMA - 1.0) + ke;
-    if (nv > 5) un[5] = fmax(un[5], 0.0);
-    if (nv > 6) un[6] = fmax(un[6], 1e-8);
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-      if (v < nv) uc[v] = un[v];
-    part[p] = sq_sum;
-    part[CPB * S + p] = Lr[0] * Lr[0];
-  }
-  __syncthreads();
-  // modal filter as one FP64 tensor-core product per tile: rows s, columns
-  // (cell, variable) of the first five variables, K = the cell's points; the
-  // outputs are assembled in the residual buffers (no longer needed) and
-  // stored as one contiguous block
-  double* sOut = sRi;  // (nc*S, nv) row-major, fits in sRi + sRv
-  dmma_product_f(
-      S, 5 * nc, S, ops.ffilt[ct],
-      [&](int j, int col) { return sU[((col / 5) * S + j) * nv + col % 5]; },
-      [&](int s, int col, double x) { sOut[((col / 5) * S + s) * nv + col % 5] = x; });
-  for (int p = tid; p < nc * S; p += blockDim.x)
-    for (int v = 5; v < nv; ++v) sOut[p * nv + v] = sU[p * nv + v];
-  __syncthreads();
-  for (int t = tid; t < nc * S * nv; t += blockDim.x) a.Unext[(size_t)e0 * S * nv + t] = sOut[t];
-  if (a.stage == 0 && tid < nc) {
-    double acc = 0.0;
-    for (int s = 0; s < S; ++s) acc += part[tid * S + s];
-    a.norm_part[e0 + tid] = acc;
-    double acc_rho = 0.0;
-    for (int s = 0; s < S; ++s) acc_rho += part[CPB * S + tid * S + s];
-    a.norm_rho_part[e0 + tid] = acc_rho;
-    // a non-finite dU/dt anywhere in the cell makes its partial non-finite
-    if (!isfinite(acc) && a.status) atomicOr(a.status, (unsigned)DS_NONFINITE);
-  }
+  dmma_warp_rb_f<(S + 7) / 8, (5 * CW + 7) / 8, S>(
+      S, 5 * nc, ops.ffilt[ct], [&](int j, int col) { return sU[((col / 5) * S + j) * nv + col % 5]; },
+      [&](int m, int col, double v) { s0[((col / 5) * S + m) * nv + col % 5] = v; });
+  __syncwarp();
+  double* out = a.Unext + (size_t)e0 * S * nv;
+  for (int t = lane; t < nst; t += 32) out[t] = s0[t];
 }
 
 // ---------------------------------------------------------------------------

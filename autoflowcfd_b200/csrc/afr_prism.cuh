@@ -64,7 +64,7 @@ struct PxSmem {
   static constexpr int oX = nH, oY = (oX + nX + 3) / 4 * 4, oRef = oY + nY, oF = oRef + 8;
   static constexpr int cell = (oF + 30 + 3) / 4 * 4;  // floats per cell
   static constexpr int oDev = 16 * S, oG = oDev + 4 * S;  // inside H, after the staged state (8 doubles per point)
-  static_assert(oG + 12 * S <= nH && 6 * MX_XF * NT <= nH && 10 * S <= nH, "phases share the H block");
+  static_assert(oG + 12 * S <= nH && 6 * MX_XF * NT <= nH, "phases share the H block");
   static constexpr int total = PX_WARPS * CW * cell * 4;
 };
 
@@ -449,23 +449,14 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
       const double rdet = __ldg(pg.rdet + p);
       const double* F = reinterpret_cast<const double*>(sc + L::oF);
       const float* x = sc + L::oX + s;
-      float o[10];
+      float* o = RV + (size_t)(e0 + c) * 9 * S + s;
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
         const double mdf = md0 * F[v] + md1 * F[5 + v] + md2 * F[10 + v];
-        o[v] = float(-(double(x[v * FS]) + mdf) * rdet);
-        o[5 + v] = (VISC && v > 0) ? x[(4 + v) * FS] : 0.f;
+        o[v * S] = float(-(double(x[v * FS]) + mdf) * rdet);
+        if (VISC && v > 0) o[(4 + v) * S] = x[(4 + v) * FS];
       }
-      float2* tile = reinterpret_cast<float2*>(sc + 10 * s);
-#pragma unroll
-      for (int k = 0; k < 5; ++k) tile[k] = make_float2(o[2 * k], o[2 * k + 1]);
     }
-  }
-  __syncwarp();
-  for (int c = 0; c < nc; ++c) {
-    const float2* src = reinterpret_cast<const float2*>(sw + c * L::cell);
-    float2* dst = reinterpret_cast<float2*>(RV + (size_t)(e0 + c) * S * 10);
-    for (int t = lane; t < 5 * S; t += 32) dst[t] = src[t];
   }
 }
 
