@@ -82,10 +82,9 @@ struct afr_handle {
   int mx_face_block = 128;  // threads per face-kernel CTA: 64, 128 or 256
   // matched interior face points paired across the face's two slots, and the
   // remaining slot points (boundary, interpolated, unpaired)
-  int2* mx_pairs = nullptr;
+  MxPair* mx_pairs = nullptr;
   int32_t* mx_rest = nullptr;
   int mx_npairs = 0, mx_nrest = 0;
-  bool mx_paired = false;
   int mx_upd_var = 1;       // update-kernel warps per CTA: 2, 4 or 8 (variant 0, 1, 2)
   // dual-time / IMEX buffers, allocated by the first call of either scheme
   double* iRinv = nullptr;   // (N,S,nv) inviscid residual (dU/dt)
@@ -477,21 +476,11 @@ struct Launch {
     return cudaGetLastError();
   }
   static cudaError_t mx_stage(afr_handle* h, StageArgs a, cudaStream_t st, StepTimer* tm) {
-    const int nt = h->slots.n * NP;
-    const int fb = h->mx_face_block;
-    if (h->mx_paired) {
-      if (h->mx_npairs > 0)
-        k_mx_face_pair<S, NP><<<(h->mx_npairs + fb - 1) / fb, fb, 0, st>>>(
-            h->fc, h->bc, h->slots, h->mf, h->mb, h->mo.hcell, (float)h->prm.mu, a.inviscid_only ? 0 : 1,
-            h->mx_pairs, h->mx_npairs);
-      if (h->mx_nrest > 0)
-        k_mx_face<S, NP><<<(h->mx_nrest + fb - 1) / fb, fb, 0, st>>>(
-            h->fc, h->bc, h->slots, h->mf, h->mb, h->mo.hcell, (float)h->prm.mu, a.inviscid_only ? 0 : 1,
-            h->mx_rest, h->mx_nrest);
-    } else if (nt > 0) {
-      k_mx_face<S, NP><<<(nt + fb - 1) / fb, fb, 0, st>>>(h->fc, h->bc, h->slots, h->mf, h->mb, h->mo.hcell,
-                                                           (float)h->prm.mu, a.inviscid_only ? 0 : 1, nullptr, 0);
-    }
+    const int fb = h->mx_face_block, rb = (h->mx_nrest + fb - 1) / fb, pb = (h->mx_npairs + fb - 1) / fb;
+    if (rb + pb > 0)
+      k_mx_face<S, NP><<<rb + pb, fb, 0, st>>>(h->fc, h->bc, h->slots, h->mf, h->mb, h->mo.hcell, (float)h->prm.mu,
+                                               a.inviscid_only ? 0 : 1, h->mx_rest, h->mx_nrest, rb, h->mx_pairs,
+                                               h->mx_npairs);
     if (tm) tm->mark(st);
     const int ranges[3] = {0, h->n_prism, h->N};
     for (int r = 0; r < 2; ++r) {
@@ -522,10 +511,7 @@ struct Launch {
     cudaError_t r = mx ? mx_pre(h, U, nut, grads, st) : pre(h, U, nut, grads, st);
     if (r != cudaSuccess) return r;
     if (tm) tm->mark(st);
-    if (nl) {
-      const int face = !mx || !h->mx_paired ? (h->slots.n > 0 ? 1 : 0) : (h->mx_npairs > 0 ? 1 : 0) + (h->mx_nrest > 0 ? 1 : 0);
-      *nl += (mx ? 3 : 2) * n_ranges(h) - (mx && h->px ? 1 : 0) + face;
-    }
+    if (nl) *nl += (mx ? 3 : 2) * n_ranges(h) - (mx && h->px ? 1 : 0) + (h->slots.n > 0 ? 1 : 0);
     if (mx) return mx_stage(h, a, st, tm);
     r = stage(h, a, st, tm);
     if (tm) tm->mark(st);  // the plain form has no separate update kernel: an empty interval
@@ -1014,10 +1000,11 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   if (ns > 0) {
     const size_t nt = ns * P;
     std::vector<uint8_t> hofp(nt);
-    std::vector<int32_t> hface(ns), hflag(ns);
+    std::vector<int32_t> hface(ns), hflag(ns), hcell(ns);
     e = cudaMemcpy(hofp.data(), ofp, nt, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(hface.data(), h->slots.face, ns * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(hflag.data(), h->slots.flags, ns * 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(hcell.data(), h->slots.cell, ns * 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
     std::vector<int32_t> nb_slot(h->F, -1);
     for (size_t sl = 0; sl < ns; ++sl) {
@@ -1031,8 +1018,15 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
         else h->px_faces |= 1u << (o / P);
       }
     }
-    std::vector<int2> pairs;
+    std::vector<MxPair> pairs;
     std::vector<uint8_t> taken(nt, 0);
+    if (N * 6 * P >= ((size_t)1 << 31)) return fail(h, AFR_EUNSUPPORTED, "more than 2^31 face points");
+    auto row = [&](size_t sl, int i) -> uint32_t {
+      const int fl = hflag[sl];
+      const uint32_t face = ((fl >> 2) & 3) * 2 + ((fl & 16) ? 1 : 0);
+      return (((uint32_t)hcell[sl] * 6 + face) * P + i) | ((fl & 16) ? 0x80000000u : 0u);
+    };
+    pairs.reserve(nt / 2);
     for (size_t sl = 0; sl < ns; ++sl) {
       const int fl = hflag[sl];
       if ((fl & 1) || (fl & 2)) continue;  // owner sides of interior faces
@@ -1047,7 +1041,7 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
         if (o == MX_OFP_GENERAL || o / P != code2) continue;
         const size_t t2 = (size_t)s2 * P + o % P;
         if (hofp[t2] != code * P + i || taken[t2]) continue;
-        pairs.push_back(make_int2((int)t, (int)t2));
+        pairs.push_back(MxPair{(int32_t)t, (int32_t)t2, row(sl, i), row(s2, o % P)});
         taken[t] = taken[t2] = 1;
       }
     }
@@ -1056,16 +1050,15 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
       if (!taken[t]) rest.push_back((int32_t)t);
     int32_t* dpairs = nullptr;
     int32_t* drest = nullptr;
-    if (!pairs.empty() && (rc = upload(h, &dpairs, reinterpret_cast<const int32_t*>(pairs.data()), pairs.size() * 2, st)))
+    if (!pairs.empty() && (rc = upload(h, &dpairs, reinterpret_cast<const int32_t*>(pairs.data()), pairs.size() * 4, st)))
       return rc;
     if (!rest.empty() && (rc = upload(h, &drest, rest.data(), rest.size(), st))) return rc;
     e = cudaStreamSynchronize(st);  // host vectors leave scope
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
-    h->mx_pairs = reinterpret_cast<int2*>(dpairs);
+    h->mx_pairs = reinterpret_cast<MxPair*>(dpairs);
     h->mx_rest = drest;
     h->mx_npairs = (int)pairs.size();
     h->mx_nrest = (int)rest.size();
-    h->mx_paired = true;
   }
   // point fields: the tensor-core volume kernel's input and the source of the
   // interpolated face points

@@ -12,7 +12,7 @@
 //   k_mx_pre   per 8-cell tile: gradients of (u,v,w,T) (D_3d as a GEMM) and the
 //              extrapolation of all point fields to every face point of the
 //              cell (boundary_extrap of all six faces stacked as one GEMM);
-//   k_mx_face  per (slot, flux point): AUSM+up and BR1 jumps.  Where the
+//   k_mx_face  per pair of slot flux points: AUSM+up and BR1 jumps.  Where the
 //              other side's interpolation row equals one of that cell's own
 //              extrapolation rows (matched once at create: every prism face
 //              point, most tet face points) the other side is read from its
@@ -73,8 +73,20 @@ struct MxOps {
 constexpr uint8_t MX_OFP_GENERAL = 255;  // other side by interpolation from point fields
 
 struct MxFace {
-  const float4* arow;   // (n_slots*NP) own adjugate row at the flux point, and its norm
+  // (n_slots*NP) own adjugate row at the flux point, and its norm; the norm is
+  // negative where the alignment fallback replaces the row's direction by the
+  // face normal (both are geometry: decided once)
+  const float4* arow;
   const uint8_t* ofp;   // (n_slots*NP) face point of the other side, (ax*2+side)*NP + j, or MX_OFP_GENERAL
+};
+
+// A matched pair of slot points: everything the paired face kernel needs to
+// find its data, in one 16-byte load (the chain pair -> slot -> face -> cells
+// was three dependent loads).  Rows are (cell*6 + face)*NP + point with the
+// slot's side in the sign bit.
+struct MxPair {
+  int32_t t, t2;        // owner- and neighbour-side slot points
+  uint32_t row, row2;   // their own face-point rows
 };
 
 // Point fields: q (5), symmetric velocity gradient (S00, S11, S22, S01, S02,
@@ -515,31 +527,27 @@ __global__ void __launch_bounds__(MX_THREADS, 2)  // 64 registers: two CTAs per 
 }
 
 // ---------------------------------------------------------------------------
-// face kernel: one thread per (slot, flux point), fields read at face points
+// face kernel: one thread per pair of slot points (or single slot point), fields read at face points
 // ---------------------------------------------------------------------------
 // The jumps of slot point t from its own face-point fields ow and the other
 // side's ot (core/fr_residual/inviscid_kernel_colored.py:86-236,
 // core/fr_residual/viscous_flux_kernel.py:335-520)
 template <int NP>
 __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& st, const MxFace& mf, const MxBuf& mb,
-                                             const double* __restrict__ hcell, float mu, int visc, int t,
-                                             const float (&ow)[MX_XF], const float (&ot)[MX_XF]) {
+                                             const double* __restrict__ hcell, float mu, int visc, int t, float side,
+                                             bool bnd, const float (&ow)[MX_XF], const float (&ot)[MX_XF]) {
   const int sl = t / NP, i = t % NP;
-  const int f = st.face[sl];
-  const int e = st.cell[sl];
-  const int fl = st.flags[sl];
-  const bool is_owner = (fl & 1) == 0;
-  const bool bnd = (fl & 2) != 0;
-  const float side = (fl & 16) ? 1.f : -1.f;
-  const double* tnp = fc.tnormal + ((size_t)f * NP + i) * 3;
-  const float tn[3] = {float(tnp[0]), float(tnp[1]), float(tnp[2])};
   const float4 ar = mf.arow[t];
   const float a0 = ar.x, a1 = ar.y, a2 = ar.z;
-  const float mag = fmaxf(ar.w, 1e-30f);
-  float dir[3] = {a0 / mag * side, a1 / mag * side, a2 / mag * side};
-  const float sg = is_owner ? 1.f : -1.f;
-  const float t0 = sg * tn[0], t1 = sg * tn[1], t2 = sg * tn[2];
-  if (dir[0] * t0 + dir[1] * t1 + dir[2] * t2 < 0.5f) { dir[0] = t0; dir[1] = t1; dir[2] = t2; }
+  const float mag = fmaxf(fabsf(ar.w), 1e-30f), rm = side / mag;
+  float dir[3] = {a0 * rm, a1 * rm, a2 * rm};
+  if (ar.w < 0.f) {  // alignment fallback: the face normal, outward from this side
+    const int f = st.face[sl];
+    const double* tnp = fc.tnormal + ((size_t)f * NP + i) * 3;
+    const float sg = (st.flags[sl] & 1) == 0 ? 1.f : -1.f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) dir[d] = sg * float(tnp[d]);
+  }
   float Fc[5], Fp[3][5];
   ausm_up<float>(ow, ot, dir, Fc);
   euler_flux<float>(ow, Fp);
@@ -559,8 +567,8 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
       jv[v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
     if (bnd) {
       // interior penalty (core/fr_operators/flux_kernels.py:140-200)
-      const float eta = float(C_IP) * (mu + ow[14]) / float(hcell[e]);
-      const float scale = eta * ar.w * side;
+      const float eta = float(C_IP) * (mu + ow[14]) / float(hcell[st.cell[sl]]);
+      const float scale = eta * fabsf(ar.w) * side;
 #pragma unroll
       for (int v = 0; v < 3; ++v) jv[v] += -scale * (ow[1 + v] - ot[1 + v]);
     }
@@ -575,15 +583,12 @@ __device__ __forceinline__ const float* mx_face_row(const MxBuf& mb, int e, int 
   return mb.XF + ((size_t)e * 6 + fp / NP) * mb.FW * NP + fp % NP;
 }
 
+// a slot point outside the pairs (boundary, interpolated or without a matched
+// partner)
 template <int S, int NP>
-__global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, MxFace mf, MxBuf mb,
-                                                 const double* __restrict__ hcell, float mu, int visc,
-                                                 const int32_t* __restrict__ rest, int n_rest) {
-  // slot points not taken by the paired kernel (boundary, interpolated or
-  // without a matched partner); all of them when rest is null
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (rest ? n_rest : st.n * NP)) return;
-  const int t = rest ? rest[idx] : idx;
+__device__ __forceinline__ void mx_face_single(const Faces& fc, const Bc& bc, const SlotTable& st, const MxFace& mf,
+                                               const MxBuf& mb, const double* __restrict__ hcell, float mu, int visc,
+                                               int t) {
   const int sl = t / NP, i = t % NP;
   const int f = st.face[sl];
   const int e = st.cell[sl];
@@ -641,40 +646,42 @@ __global__ void __launch_bounds__(256) k_mx_face(Faces fc, Bc bc, SlotTable st, 
       }
     }
   }
-  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, t, ow, ot);
+  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, t, (fl & 16) ? 1.f : -1.f, bnd, ow, ot);
 }
 
 // Matched interior face points in pairs: slot point t (owner side) and its
 // partner t2 (the neighbour side's slot point at the matched face point) read
 // the same two face-point rows, own and other swapped; one thread loads them
-// once and forms both jumps
+// once and forms both jumps.  The first rest_blocks CTAs take the points
+// outside the pairs: one launch, so that their longer load chains run under
+// the pairs instead of after them.  80 registers (three 256-thread CTAs).
 template <int S, int NP>
-__global__ void __launch_bounds__(256, 3) k_mx_face_pair(Faces fc, Bc bc, SlotTable st, MxFace mf, MxBuf mb,
-                                                      const double* __restrict__ hcell, float mu, int visc,
-                                                      const int2* __restrict__ pairs, int n_pairs) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256, 3) k_mx_face(Faces fc, Bc bc, SlotTable st, MxFace mf, MxBuf mb,
+                                                    const double* __restrict__ hcell, float mu, int visc,
+                                                    const int32_t* __restrict__ rest, int n_rest, int rest_blocks,
+                                                    const MxPair* __restrict__ pairs, int n_pairs) {
+  if ((int)blockIdx.x < rest_blocks) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n_rest) mx_face_single<S, NP>(fc, bc, st, mf, mb, hcell, mu, visc, rest[j]);
+    return;
+  }
+  const int idx = ((int)blockIdx.x - rest_blocks) * blockDim.x + threadIdx.x;
   if (idx >= n_pairs) return;
-  const int2 pr = pairs[idx];
-  const int t = pr.x, t2 = pr.y;
-  const int sl = t / NP, i = t % NP;
-  const int f = st.face[sl];
-  const int e = st.cell[sl];
-  const int fl = st.flags[sl];
-  const int ax = (fl >> 2) & 3;
+  const int4 pr = __ldg(reinterpret_cast<const int4*>(pairs) + idx);
   const int nf = visc ? MX_XF : 5;
-  const int oc = fc.neighbor[f];
   float ra[MX_XF], rb[MX_XF];
   {
-    const float* xa = mx_face_row<NP>(mb, e, (ax * 2 + ((fl & 16) ? 1 : 0)) * NP + i);
-    const float* xb = mx_face_row<NP>(mb, oc, mf.ofp[t]);
+    const uint32_t r0 = (uint32_t)pr.z & 0x7fffffffu, r1 = (uint32_t)pr.w & 0x7fffffffu;
+    const float* xa = mb.XF + (size_t)(r0 / NP) * mb.FW * NP + r0 % NP;
+    const float* xb = mb.XF + (size_t)(r1 / NP) * mb.FW * NP + r1 % NP;
 #pragma unroll
     for (int k = 0; k < MX_XF; ++k) {
       ra[k] = k < nf ? __ldg(xa + k * NP) : 0.f;
       rb[k] = k < nf ? __ldg(xb + k * NP) : 0.f;
     }
   }
-  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, t, ra, rb);
-  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, t2, rb, ra);
+  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, pr.x, pr.z < 0 ? 1.f : -1.f, false, ra, rb);
+  mx_face_jump<NP>(fc, st, mf, mb, hcell, mu, visc, pr.y, pr.w < 0 ? 1.f : -1.f, false, rb, ra);
 }
 
 // ---------------------------------------------------------------------------
@@ -1093,12 +1100,20 @@ __device__ __forceinline__ bool outlier_clear(const double (&x)[PL], const bool 
 }
 
 // the rule itself: stable ranks over the cell's points, median, zeroing
+// (a call: kept out of the registers of the common path)
+template <int PL>
+struct Vals {
+  double v[PL];
+};
 template <int S, int PL>
-__device__ __noinline__ void outlier_exact(double (&x)[PL], const double (&u)[PL], const bool (&on)[PL], int grp,
-                                           int s0) {
+__device__ __noinline__ Vals<PL> outlier_exact(Vals<PL> X, Vals<PL> u, int grp, int s0, bool live) {
+  double(&x)[PL] = X.v;
+  bool on[PL];
+#pragma unroll
+  for (int l = 0; l < PL; ++l) on[l] = live && s0 + 32 * l < S;
   double acc = 0.0;
 #pragma unroll
-  for (int l = 0; l < PL; ++l) acc += on[l] ? fabs(u[l]) : 0.0;
+  for (int l = 0; l < PL; ++l) acc += on[l] ? fabs(u.v[l]) : 0.0;
   const double mean = cell_sum<S>(acc) / S;
   int rank[PL];
 #pragma unroll
@@ -1128,6 +1143,7 @@ __device__ __noinline__ void outlier_exact(double (&x)[PL], const double (&u)[PL
 #pragma unroll
   for (int l = 0; l < PL; ++l)
     if (fabs(x[l]) > thr) x[l] = 0.0;
+  return X;
 }
 }  // namespace mxd
 
@@ -1233,11 +1249,15 @@ __global__ void __launch_bounds__(256, S == 64 ? 2 : 3)
 #pragma unroll
       for (int v = 0; v < 9; ++v)
         if (bad >> v & 1u) {
-          double u[PL];
+          mxd::Vals<PL> u, X;
 #pragma unroll
-          for (int l = 0; l < PL; ++l)
-            u[l] = on[l] ? a.Ucur[((size_t)e * S + sp + 32 * l) * nv + (v < 5 ? v : v - 4)] : 0.0;
-          mxd::outlier_exact<S, PL>(x[v], u, on, grp, sp);
+          for (int l = 0; l < PL; ++l) {
+            X.v[l] = x[v][l];
+            u.v[l] = on[l] ? a.Ucur[((size_t)e * S + sp + 32 * l) * nv + (v < 5 ? v : v - 4)] : 0.0;
+          }
+          X = mxd::outlier_exact<S, PL>(X, u, grp, sp, live);
+#pragma unroll
+          for (int l = 0; l < PL; ++l) x[v][l] = X.v[l];
         }
     }
     if (!step) {
@@ -1368,7 +1388,14 @@ __global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow
     a1 += w * ad[1];
     a2 += w * ad[2];
   }
-  arow[t] = make_float4(float(a0), float(a1), float(a2), float(sqrt(a0 * a0 + a1 * a1 + a2 * a2)));
+  {
+    // the direction is compared with the face normal in the face kernel's own FP32 arithmetic
+    const float4 ar = make_float4(float(a0), float(a1), float(a2), float(sqrt(a0 * a0 + a1 * a1 + a2 * a2)));
+    const float mag = fmaxf(ar.w, 1e-30f), rm = (sb ? 1.f : -1.f) / mag, sg = is_owner ? 1.f : -1.f;
+    const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
+    const float al = ar.x * rm * (sg * float(tn[0])) + ar.y * rm * (sg * float(tn[1])) + ar.z * rm * (sg * float(tn[2]));
+    arow[t] = make_float4(ar.x, ar.y, ar.z, al < 0.5f ? -mag : ar.w);
+  }
   if (bnd) {
     ofp[t] = 0;
     return;
