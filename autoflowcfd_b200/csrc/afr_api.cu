@@ -85,7 +85,7 @@ struct afr_handle {
   MxPair* mx_pairs = nullptr;
   int32_t* mx_rest = nullptr;
   int mx_npairs = 0, mx_nrest = 0;
-  int mx_upd_var = 1;       // update-kernel warps per CTA: 2, 4 or 8 (variant 0, 1, 2)
+  int mx_upd_var = 2;       // update-kernel warps per CTA: 1, 2 or 4 (variant 0, 1, 2)
   // dual-time / IMEX buffers, allocated by the first call of either scheme
   double* iRinv = nullptr;   // (N,S,nv) inviscid residual (dU/dt)
   double* iRvisc = nullptr;  // (N,S,nv) viscous residual (dU/dt)
@@ -391,7 +391,7 @@ struct Launch {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_mx_vol<S, FN, MXC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_vol_smem());
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mx_update<S, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 8));
+      e = cudaFuncSetAttribute(k_mx_update<S, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
     if constexpr (PXD) {
       auto* fv = k_px_cell<PXN1, PXNF, PXC, true>;
       auto* fi = k_px_cell<PXN1, PXNF, PXC, false>;
@@ -435,7 +435,7 @@ struct Launch {
     return cudaSuccess;
   }
   static void mx_update_launch(afr_handle* h, const StageArgs& a, int ct, int n, cudaStream_t st) {
-    const int warps = 2 << h->mx_upd_var, per = warps * MxUpd<S>::CW;
+    const int warps = 1 << h->mx_upd_var, per = warps * MxUpd<S>::CW;
     k_mx_update<S, NP><<<(n + per - 1) / per, 32 * warps, MxUpd<S>::bytes(h->nv, warps), st>>>(
         h->ops, h->fc, a, ct, h->mb.RV, h->mb.Jm, h->mo.rdet);
   }

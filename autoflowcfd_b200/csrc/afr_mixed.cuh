@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(MX_VOL_THREADS, 1)
 // one coalesced access.  CW = 3 at P2 and P3 makes the filter's 5*CW = 15
 // columns two nearly full column tiles of the FP64 tensor product.
 // ---------------------------------------------------------------------------
-constexpr int MX_UPD_SLOTS = 5;  // slots per cell whose jumps are loaded together (more: one by one)
+constexpr int MX_UPD_SLOTS = 5;  // slots of a prism, whose jumps are loaded together (other counts: one by one)
 
 template <int S>
 struct MxUpd {
@@ -1148,7 +1148,7 @@ __device__ __noinline__ Vals<PL> outlier_exact(Vals<PL> X, Vals<PL> u, int grp, 
 }  // namespace mxd
 
 template <int S, int NP>
-__global__ void __launch_bounds__(256, S == 64 ? 2 : 3)
+__global__ void __launch_bounds__(128, S == 64 ? 3 : 5)
     k_mx_update(Ops ops, Faces fc, StageArgs a, int ct, const float* __restrict__ RV, const float* __restrict__ Jm,
                 const double* __restrict__ rdet) {
   using L = MxUpd<S>;
@@ -1183,54 +1183,76 @@ __global__ void __launch_bounds__(256, S == 64 ? 2 : 3)
   }
   const int grp = S < 32 ? lane / S : 0;  // cell side of the warp
   const int sp = S < 32 ? lane % S : lane;
+  // slot ranges (lane c: cell c's first slot) and flags (lane j: slots kb + j and kb + 32 + j)
+  const int ptr = __ldg(fc.slot_ptr + e0 + min(lane, nc));
+  const int kb = __shfl_sync(0xffffffffu, ptr, 0), ke = __shfl_sync(0xffffffffu, ptr, nc);
+  const bool flags_held = ke - kb <= (CW * MX_UPD_SLOTS > 32 ? 64 : 32);
+  const int fl = kb + lane < ke ? __ldg(a.slot_flags + kb + lane) : 0;
+  const int fl2 = kb + 32 + lane < ke ? __ldg(a.slot_flags + kb + 32 + lane) : 0;
 #pragma unroll 1
   for (int r = 0; r < PR; ++r) {
-    const int c = r * CPR + grp;
-    const int e = e0 + c;
+    const int c = r * CPR + (grp < CPR ? grp : 0);
     const bool live = grp < CPR && c < nc;
+    const int e = e0 + (c < nc ? c : 0);  // lanes without a cell read one that exists
     double x[9][PL];  // dU/dt: inviscid 0..4, viscous momentum and energy 5..8
     double rd[PL];
     bool on[PL];
 #pragma unroll
     for (int l = 0; l < PL; ++l) on[l] = live && sp + 32 * l < S;
-    // jumps of the cell's slots, ascending color order
     double cx[9][PL];
 #pragma unroll
     for (int v = 0; v < 9; ++v)
 #pragma unroll
       for (int l = 0; l < PL; ++l) cx[v][l] = 0.0;
-    const int k0 = live ? fc.slot_ptr[e] : 0, n = live ? fc.slot_ptr[e + 1] - k0 : 0;
+    const int k0 = __shfl_sync(0xffffffffu, ptr, c < nc ? c : 0);
+    const int n = __shfl_sync(0xffffffffu, ptr, (c < nc ? c : 0) + 1) - k0;
     float rv[9][PL];
 #pragma unroll
     for (int l = 0; l < PL; ++l) {
-      const size_t p = (size_t)e * S + sp + 32 * l;
-      rd[l] = on[l] ? __ldg(rdet + p) : 0.0;
+      rd[l] = __ldg(rdet + (size_t)e * S + sp + 32 * l);
 #pragma unroll
       for (int v = 0; v < 9; ++v)
-        rv[v][l] = on[l] && (v < 5 || visc) ? __ldg(RV + ((size_t)e * 9 + v) * S + sp + 32 * l) : 0.f;
+        rv[v][l] = v < 5 || visc ? __ldg(RV + ((size_t)e * 9 + v) * S + sp + 32 * l) : 0.f;
     }
-    for (int kb = 0; kb < n; kb += MX_UPD_SLOTS) {
-      int fl[MX_UPD_SLOTS];
-#pragma unroll
-      for (int j = 0; j < MX_UPD_SLOTS; ++j) fl[j] = kb + j < n ? __ldg(a.slot_flags + k0 + kb + j) : -1;
+    // jumps of the cell's slots, ascending color order
+    if (flags_held && __all_sync(0xffffffffu, n == MX_UPD_SLOTS)) {
+      // five slots, as every prism has: all loads of a point in flight at once
 #pragma unroll
       for (int l = 0; l < PL; ++l) {
+        float jv[MX_UPD_SLOTS][9];
+        int gi[MX_UPD_SLOTS];
 #pragma unroll
         for (int j = 0; j < MX_UPD_SLOTS; ++j) {
-          float jv[9];
-          double gw = 0.0;
-#pragma unroll
-          for (int v = 0; v < 9; ++v) jv[v] = 0.f;
-          if (on[l] && fl[j] >= 0) {
-            const int ax = (fl[j] >> 2) & 3;
-            gw = sG[((fl[j] & 16) ? 3 * S : 0) + ax * S + sp + 32 * l];
-            const float* Jk = Jm + (size_t)(k0 + kb + j) * 9 * NP + sFp[ax * S + sp + 32 * l];
-#pragma unroll
-            for (int v = 0; v < 9; ++v)
-              if (v < 5 || visc) jv[v] = __ldg(Jk + v * NP);
+          const int q = k0 - kb + j;
+          int f = __shfl_sync(0xffffffffu, fl, q & 31);
+          if constexpr (CW * MX_UPD_SLOTS > 32) {
+            const int f2 = __shfl_sync(0xffffffffu, fl2, q & 31);
+            f = q < 32 ? f : f2;
           }
+          const int as = ((f >> 2) & 3) * S + sp + 32 * l;
+          gi[j] = ((f & 16) ? 3 * S : 0) + as;
+          const float* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
 #pragma unroll
-          for (int v = 0; v < 9; ++v) cx[v][l] += gw * double(jv[v]);
+          for (int v = 0; v < 9; ++v) jv[j][v] = v < 5 || visc ? __ldg(Jk + v * NP) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < MX_UPD_SLOTS; ++j) {
+          const double gw = sG[gi[j]];
+#pragma unroll
+          for (int v = 0; v < 9; ++v) cx[v][l] += gw * double(jv[j][v]);
+        }
+      }
+    } else {
+      for (int j = 0; j < n; ++j) {
+        const int f = __ldg(a.slot_flags + k0 + j);
+#pragma unroll
+        for (int l = 0; l < PL; ++l) {
+          const int as = ((f >> 2) & 3) * S + sp + 32 * l;
+          const double gw = sG[((f & 16) ? 3 * S : 0) + as];
+          const float* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
+#pragma unroll
+          for (int v = 0; v < 9; ++v)
+            if (v < 5 || visc) cx[v][l] += gw * double(__ldg(Jk + v * NP));
         }
       }
     }
