@@ -21,6 +21,7 @@
 #include "afr_mixed.cuh"
 #include "afr_p0.cuh"
 #include "afr_prism.cuh"
+#include "afr_prism_sst.cuh"
 #include "afr_sst.cuh"
 
 using namespace afr;
@@ -48,7 +49,7 @@ struct afr_handle {
   double* pt = nullptr;
   double* cfp = nullptr;
   double* sp8 = nullptr;
-  uint8_t* wall_face = nullptr;
+  SstFace* sst_faces = nullptr;
   uint8_t* cd_wall = nullptr;
   double* area_w = nullptr;
   int32_t* cd_faces = nullptr;
@@ -69,9 +70,14 @@ struct afr_handle {
   MxFace mf{};
   MxBuf mb{};
   // prisms whose operators have tensor-product structure (afr_prism.cuh)
-  bool px = false;
-  PxOps<2, 3> px1{};
-  PxOps<3, 4> px2{};
+  bool px = false;    // the mixed form's cell kernel
+  bool px64 = false;  // the FP64 kernels
+  double* px_rows = nullptr;  // derivative rows of the prism points (see px_rows in afr_prism.cuh)
+  double px_dev = INFINITY;  // worst deviation of the prism operators from the structure
+  PxOps<float, 2, 3> px1{};
+  PxOps<float, 3, 4> px2{};
+  PxOps<double, 2, 3> pxd1{};
+  PxOps<double, 3, 4> pxd2{};
   PxGeom pg{};
   unsigned px_faces = 0;  // bit (axis*2 + side): faces whose point fields some slot reads
   bool px_points = false;  // some face point interpolates from the point fields
@@ -314,24 +320,43 @@ static cudaError_t resident_ctas(const void* fn, int threads, size_t dyn_smem, i
 }
 
 // SST source, transport and point-implicit update of one step (the three
-// per-step kernels); cells of each type in their own launches
+// per-step kernels); cells of each type in their own launches.  Structured
+// prisms of the mixed form take the line and plane derivatives of
+// afr_prism_sst.cuh; the plain form keeps every entry of the operators: those
+// outside the structure are 1e-15 of the largest, yet leaving them out moves
+// omega by 2e-8 after twelve steps of the SST growth (8e-11 with them).
 template <int S, int NP>
 cudaError_t sst_launch(afr_handle* h, const SstArgs& a, cudaStream_t st, StepTimer* tm) {
   constexpr int CPB = SstTile<S>::CPB, TH = SstTile<S>::THREADS;
+  constexpr bool PXD = S == 8 || S == 27;
   const int ranges[3] = {0, h->n_prism, h->N};
   for (int r = 0; r < 2; ++r) {
     const int n = ranges[r + 1] - ranges[r];
-    if (n > 0) k_sst_point<S><<<(n + CPB - 1) / CPB, TH, 0, st>>>(h->g, h->ops, a, ranges[r], ranges[r + 1]);
+    if (n <= 0) continue;
+    if constexpr (PXD) {
+      if (r == 0 && h->px64 && h->prec == AFR_PREC_MIXED) {
+        constexpr int N1 = S == 8 ? 2 : 3, per = PXS_WARPS * PxsSmem<N1>::CPR;
+        k_pxs_point<N1><<<(n + per - 1) / per, 32 * PXS_WARPS, PxsSmem<N1>::total, st>>>(h->px_rows, h->g, a, 0, n);
+        continue;
+      }
+    }
+    k_sst_point<S><<<(n + CPB - 1) / CPB, TH, 0, st>>>(h->g, h->ops, a, ranges[r], ranges[r + 1]);
   }
   if (tm) tm->mark(st);
   if (h->F > 0)
-    k_sst_face<S, NP><<<(h->F + SST_FACE_WARPS - 1) / SST_FACE_WARPS, 32 * SST_FACE_WARPS, 0, st>>>(h->g, h->ops,
-                                                                                                    h->fc, a);
+    k_sst_face<S, NP><<<(h->F + SST_FACE_WARPS - 1) / SST_FACE_WARPS, 32 * SST_FACE_WARPS, 0, st>>>(h->ops, h->fc, a);
   if (tm) tm->mark(st);
   for (int r = 0; r < 2; ++r) {
     const int n = ranges[r + 1] - ranges[r];
-    if (n > 0)
-      k_sst_update<S, NP><<<(n + CPB - 1) / CPB, TH, 0, st>>>(h->g, h->ops, h->fc, a, ranges[r], ranges[r + 1]);
+    if (n <= 0) continue;
+    if constexpr (PXD) {
+      if (r == 0 && h->px64 && h->prec == AFR_PREC_MIXED) {
+        constexpr int per = PXS_WARPS * (32 / S);
+        k_pxs_update<S, NP><<<(n + per - 1) / per, 32 * PXS_WARPS, 0, st>>>(h->ops, h->fc, a, 0, n);
+        continue;
+      }
+    }
+    k_sst_update<S, NP><<<(n + CPB - 1) / CPB, TH, 0, st>>>(h->g, h->ops, h->fc, a, ranges[r], ranges[r + 1]);
   }
   if (tm) tm->mark(st);
   return cudaGetLastError();
@@ -881,12 +906,9 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   }
   // prisms with tensor-product operators take k_px_cell; everything else the
   // tensor-core kernels
-  if (h->n_prism > 0) {
-    if (h->order == 1)
-      h->px = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], Wkeep[0].data(), h->px1);
-    else if (h->order == 2)
-      h->px = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], Wkeep[0].data(), h->px2);
-  }
+  h->px = h->px_dev <= 1e-12;
+  if (h->px && h->order == 1) h->px1 = px_float(h->pxd1);
+  if (h->px && h->order == 2) h->px2 = px_float(h->pxd2);
   const bool tcr = !h->px || h->N > h->n_prism;  // some cells run on the tensor-core kernels
   for (int t = 0; t < 2; ++t) {
     if (Wkeep[t].empty() || (t == 0 && h->px)) continue;
@@ -1332,6 +1354,20 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     h->ops.f2c[t] = f2c;
     h->ops.filt[t] = flt;
   }
+  // tensor-product structure of the prism operators (afr_prism.cuh).  The
+  // mixed form takes it up to 1e-12 of an operator's largest entry (its FP32
+  // copies round at 6e-8), the FP64 kernels up to 2e-13; the reference's
+  // operators deviate by 1e-15 to 3e-14.
+  if (h->n_prism > 0 && h->order == 1)
+    h->px_dev = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], m->f2c[0], m->D_fine[0], h->pxd1);
+  if (h->n_prism > 0 && h->order == 2)
+    h->px_dev = px_operators(m->D_3d[0], m->boundary_extrap, m->c2f[0], m->f2c[0], m->D_fine[0], h->pxd2);
+  h->px64 = h->px_dev <= 2e-13;
+  if (h->px64) {
+    const std::vector<double> r = h->order == 1 ? px_rows<2>(m->D_3d[0]) : px_rows<3>(m->D_3d[0]);
+    if ((rc = upload(h, &h->px_rows, r.data(), r.size(), st))) return bail(rc);
+    cudaStreamSynchronize(st);  // r leaves scope
+  }
   {
     double *ex, *gl, *gr;
     int32_t *dfp, *dco;
@@ -1512,9 +1548,6 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     if ((rc = upload(h, &bq, m->bc_Q, nb * 5, st))) return bail(rc);
     if ((rc = upload(h, &bp, m->bc_p_out, nb, st))) return bail(rc);
     h->bc = Bc{m->n_bc, bt, bn, bw, bq, bp};
-    std::vector<uint8_t> wall(F);
-    for (size_t f = 0; f < F; ++f) wall[f] = (m->is_boundary[f] && m->bc_type[m->bc_group[f]] == AFR_BC_WALL) ? 1 : 0;
-    if ((rc = upload(h, &h->wall_face, wall.data(), F, st))) return bail(rc);
     cudaStreamSynchronize(st);
   }
   if (m->cd_wall_face && m->true_area_weight) {
@@ -1540,7 +1573,30 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
   if ((rc = dalloc(h, &h->red_part, (N * S + RED_CHUNK - 1) / RED_CHUNK + 1))) return bail(rc);
   if (prm->turb == AFR_TURB_SST) {
     if ((rc = dalloc(h, &h->pt, N * S * 5))) return bail(rc);
-    if ((rc = dalloc(h, &h->cfp, F * P * 4))) return bail(rc);
+    if ((rc = dalloc(h, &h->cfp, F * P * 2))) return bail(rc);
+    // face records of the transport
+    const int32_t *i0 = nullptr, *i1 = nullptr;  // matrix rows (dense meshes: the record's own)
+    if (m->src_mat_table) {
+      i0 = m->nb_src0_mat_index;
+      i1 = m->nb_src1_mat_index;
+    }
+    std::vector<SstFace> rec(F);
+    for (size_t f = 0; f < F; ++f) {
+      const int32_t o = (int32_t)m->owner_cell[f];
+      const int64_t s1 = m->nb_src1_idx[f];
+      SstFace& q = rec[f];
+      q.owner = o;
+      q.group = ((o < h->n_prism ? 0 : 1) * 3 + (int)m->owner_axis[f]) * 2 + (m->owner_side[f] <= 0.0 ? 0 : 1);
+      q.c0 = (int32_t)m->nb_src0_cell[f];
+      q.m0 = i0 ? i0[f] : (int32_t)f;
+      q.c1 = s1 >= 0 ? (int32_t)m->nb_src1_cell[s1] : -1;
+      q.m1 = s1 >= 0 ? (i1 ? i1[s1] : (int32_t)s1) : 0;
+      q.flags = (q.c0 < 0 && s1 < 0 ? 1 : 0) |
+                (m->is_boundary[f] && m->bc_type[m->bc_group[f]] == AFR_BC_WALL ? 2 : 0);
+      q.pad = 0;
+    }
+    if ((rc = upload(h, &h->sst_faces, rec.data(), F, st))) return bail(rc);
+    cudaStreamSynchronize(st);  // rec leaves scope
     if ((rc = dalloc(h, &h->sp8, N * S * 8))) return bail(rc);
   }
   if (prm->precision == AFR_PREC_MIXED && (rc = mixed_setup(h, m, Wkeep, st))) return bail(rc);
@@ -1590,7 +1646,7 @@ int afr_sst_update(afr_handle* h, const double* U, const double* dt_local, doubl
   if (!h || !U || !dt_local || !k || !omega || !nu_t) return AFR_EINVAL;
   if (h->prm.turb != AFR_TURB_SST) return fail(h, AFR_EINVAL, "handle was created without SST");
   cudaStream_t st = (cudaStream_t)stream;
-  SstArgs s{U, dt_local, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->wall_face, diag, h->nv, h->prm.mu};
+  SstArgs s{U, dt_local, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->sst_faces, diag, h->nv, h->prm.mu};
   cudaError_t e = dispatch(h, [&](auto L) { return L.sst(h, s, st); });
   if (e != cudaSuccess) return cuda_fail(h, e, "sst update");
   return check_status(h, st);
@@ -1613,7 +1669,7 @@ static int step_impl(afr_handle* h, double* U, double* k, double* omega, double*
   cudaError_t e = dispatch(h, [&](auto L) {
     cudaError_t r = cudaSuccess;
     if (sst) {
-      SstArgs s{U, h->dt, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->wall_face, nullptr, h->nv, h->prm.mu};
+      SstArgs s{U, h->dt, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->sst_faces, nullptr, h->nv, h->prm.mu};
       r = L.sst(h, s, st, tm);
       nl += 3;
       if (r != cudaSuccess) return r;
@@ -1728,7 +1784,7 @@ int imp_preamble(afr_handle* h, double* U, double* k, double* omega, double* nu_
   if (rc) return rc;
   if (sst) {
     cudaError_t e = dispatch(h, [&](auto L) {
-      SstArgs s{U, turb_dt ? turb_dt : h->dt, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->wall_face, nullptr, h->nv,
+      SstArgs s{U, turb_dt ? turb_dt : h->dt, k, omega, nu_t, h->pt, h->sp8, h->cfp, h->sst_faces, nullptr, h->nv,
                 h->prm.mu};
       return L.sst(h, s, st, nullptr);
     });

@@ -36,14 +36,14 @@ namespace afr {
 
 constexpr int PX_WARPS = 4;
 
-template <int N1, int NF>
+template <class T, int N1, int NF>
 struct PxOps {
   static constexpr int NT = N1 * N1, MT = NF * NF;
-  float E02[2][2][N1];   // extrapolation along a (0) and c (1): [which][side][point of the line]
-  float E1[2][N1][NT];   // extrapolation to the b faces: [side][a of the face point][triangle point]
-  float D0[N1][N1], D2[N1][N1], D1[NT][NT];
-  float Ct[MT][NT], Cc[NF][N1];      // c2f = Ct (x) Cc
-  float Wt[3][NT][MT], Wc[3][N1][NF];  // W per axis = Wt (x) Wc
+  T E02[2][2][N1];   // extrapolation along a (0) and c (1): [which][side][point of the line]
+  T E1[2][N1][NT];   // extrapolation to the b faces: [side][a of the face point][triangle point]
+  T D0[N1][N1], D2[N1][N1], D1[NT][NT];
+  T Ct[MT][NT], Cc[NF][N1];        // c2f = Ct (x) Cc
+  T Wt[3][NT][MT], Wc[3][N1][NF];  // W per axis = Wt (x) Wc
 };
 
 // per-cell metrics in the order the lanes read them
@@ -70,7 +70,7 @@ struct PxSmem {
 
 template <int N1, int NF, int CW, bool VISC>
 __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
-    k_px_cell(const __grid_constant__ PxOps<N1, NF> op, PxGeom pg, float* __restrict__ XF, float* __restrict__ PFm,
+    k_px_cell(const __grid_constant__ PxOps<float, N1, NF> op, PxGeom pg, float* __restrict__ XF, float* __restrict__ PFm,
               float* __restrict__ RV, int FW, unsigned face_mask, const double* __restrict__ U, int nv,
               const double* __restrict__ nut, float mu, int cell_base, int cell_end) {
   using L = PxSmem<N1, NF, CW>;
@@ -470,24 +470,25 @@ __global__ void k_px_planes(const double* __restrict__ adj, size_t ncells, int n
 }
 
 // ---- host: operator structure ----
-// Kronecker factors of an (R*r) x (K*k) operator at a(row, col): A = T (R x K)
-// (x) c (r x k); false when the operator is not such a product to tol of its
-// largest entry
+// Each test returns its worst deviation relative to the operator's largest
+// entry (infinity where the structure is absent altogether).
+
+// Kronecker factors of an (R*r) x (K*k) operator at a(row, col): A = T (R x K) (x) c (r x k)
 template <class Get>
-inline bool px_kron(int R, int r, int K, int k, Get a, double tol, std::vector<double>& T, std::vector<double>& c) {
-  double big = 0.0;
+inline double px_kron(int R, int r, int K, int k, Get a, std::vector<double>& T, std::vector<double>& c) {
+  double big = 0.0, dev = 0.0;
   int pi = 0, pj = 0;
   for (int i = 0; i < R * r; ++i)
     for (int j = 0; j < K * k; ++j) {
       const double x = std::fabs(a(i, j));
-      if (!(x <= 1e300)) return false;
+      if (!(x <= 1e300)) return INFINITY;
       if (x > big) {
         big = x;
         pi = i;
         pj = j;
       }
     }
-  if (big == 0.0) return false;
+  if (big == 0.0) return INFINITY;
   T.assign((size_t)R * K, 0.0);
   c.assign((size_t)r * k, 0.0);
   for (int i = 0; i < R; ++i)
@@ -496,69 +497,131 @@ inline bool px_kron(int R, int r, int K, int k, Get a, double tol, std::vector<d
     for (int j = 0; j < k; ++j) c[i * k + j] = a(pi / r * r + i, pj / k * k + j) / a(pi, pj);
   for (int i = 0; i < R * r; ++i)
     for (int j = 0; j < K * k; ++j)
-      if (std::fabs(a(i, j) - T[(i / r) * K + j / k] * c[(i % r) * k + j % k]) > tol * big) return false;
-  return true;
+      dev = std::max(dev, std::fabs(a(i, j) - T[(i / r) * K + j / k] * c[(i % r) * k + j % k]));
+  return dev / big;
 }
 
-// The structured operators of a prism set, or false when an operator lacks the
-// structure: D (S, S, 3), E (3, 2, P, S), c2f (Fn, S), W (S, Fn, 3).
-// tol: 1e-12 of an operator's largest entry, a hundred times what the
-// reference's own operators show and far below the 6e-8 of the FP32 copies.
-template <int N1, int NF>
-inline bool px_operators(const double* D, const double* E, const double* c2f, const double* W, PxOps<N1, NF>& o) {
-  constexpr int NT = N1 * N1, S = NT * N1, MT = NF * NF, FN = MT * NF, P = NT;
-  constexpr double TOL = 1e-12;
-  double big = 0.0;
-  for (int i = 0; i < S * S * 3; ++i) big = std::max(big, std::fabs(D[i]));
+// Line and plane factors of a derivative operator D (S, S, 3), S = n^3
+template <int n>
+inline double px_lines(const double* D, double (&D0)[n][n], double (&D1)[n * n][n * n], double (&D2)[n][n]) {
+  constexpr int NT = n * n, S = NT * n;
   auto d = [&](int s, int j, int m) { return D[((size_t)s * S + j) * 3 + m]; };
+  double big = 0.0, dev = 0.0;
   for (int s = 0; s < S; ++s)
     for (int j = 0; j < S; ++j) {
-      const int a = s / NT, c = s % N1, a2 = j / NT, c2 = j % N1, t = s / N1, t2 = j / N1;
-      const double w0 = s % NT == j % NT ? d(a * NT, a2 * NT, 0) : 0.0;
-      const double w1 = c == c2 ? d(t * N1, t2 * N1, 1) : 0.0;
-      const double w2 = t == t2 ? d(c, c2, 2) : 0.0;
-      if (!(std::fabs(d(s, j, 0) - w0) <= TOL * big && std::fabs(d(s, j, 1) - w1) <= TOL * big &&
-            std::fabs(d(s, j, 2) - w2) <= TOL * big))
-        return false;
+      const double w[3] = {s % NT == j % NT ? d(s / NT * NT, j / NT * NT, 0) : 0.0,
+                           s % n == j % n ? d(s / n * n, j / n * n, 1) : 0.0,
+                           s / n == j / n ? d(s % n, j % n, 2) : 0.0};
+      for (int m = 0; m < 3; ++m) {
+        if (!(std::fabs(d(s, j, m)) <= 1e300)) return INFINITY;
+        big = std::max(big, std::fabs(d(s, j, m)));
+        dev = std::max(dev, std::fabs(d(s, j, m) - w[m]));
+      }
     }
-  for (int i = 0; i < N1; ++i)
-    for (int j = 0; j < N1; ++j) {
-      o.D0[i][j] = (float)d(i * NT, j * NT, 0);
-      o.D2[i][j] = (float)d(i, j, 2);
+  if (big == 0.0) return INFINITY;
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) {
+      D0[i][j] = d(i * NT, j * NT, 0);
+      D2[i][j] = d(i, j, 2);
     }
   for (int i = 0; i < NT; ++i)
-    for (int j = 0; j < NT; ++j) o.D1[i][j] = (float)d(i * N1, j * N1, 1);
+    for (int j = 0; j < NT; ++j) D1[i][j] = d(i * n, j * n, 1);
+  return dev / big;
+}
+
+// Derivative rows of every point for the FP64 kernels: (2*n + n*n, S), the
+// point's weights along its a-line, triangle plane and c-line; each line also
+// takes an equal share of the row's entries outside the structure.
+template <int n>
+inline std::vector<double> px_rows(const double* D) {
+  constexpr int NT = n * n, S = NT * n;
+  std::vector<double> out((size_t)(2 * n + NT) * S);
+  for (int s = 0; s < S; ++s)
+    for (int m = 0; m < 3; ++m) {
+      const int cnt = m == 1 ? NT : n;
+      std::vector<double> w(cnt, 0.0);
+      double rest = 0.0;
+      for (int j = 0; j < S; ++j) {
+        const double x = D[((size_t)s * S + j) * 3 + m];
+        if (m == 0 && j % NT == s % NT) w[j / NT] = x;
+        else if (m == 1 && j % n == s % n) w[j / n] = x;
+        else if (m == 2 && j / n == s / n) w[j % n] = x;
+        else rest += x;
+      }
+      const int base = m == 0 ? 0 : (m == 1 ? n : n + NT);
+      for (int l = 0; l < cnt; ++l) out[(size_t)(base + l) * S + s] = w[l] + rest / cnt;
+    }
+  return out;
+}
+
+// The structured operators of a prism set and their worst deviation from the
+// given ones: D (S, S, 3), E (3, 2, P, S), c2f (Fn, S), f2c (S, Fn), Df (Fn, Fn, 3).
+template <int N1, int NF>
+inline double px_operators(const double* D, const double* E, const double* c2f, const double* f2c, const double* Df,
+                           PxOps<double, N1, NF>& o) {
+  constexpr int NT = N1 * N1, S = NT * N1, MT = NF * NF, FN = MT * NF, P = NT;
+  double dev = px_lines<N1>(D, o.D0, o.D1, o.D2);
   auto e = [&](int ax, int sd, int i, int s) { return E[(((size_t)ax * 2 + sd) * P + i) * S + s]; };
-  big = 0.0;
-  for (int i = 0; i < 6 * P * S; ++i) big = std::max(big, std::fabs(E[i]));
+  double big = 0.0, de = 0.0;
+  for (int i = 0; i < 6 * P * S; ++i) {
+    if (!(std::fabs(E[i]) <= 1e300)) return INFINITY;
+    big = std::max(big, std::fabs(E[i]));
+  }
+  if (big == 0.0) return INFINITY;
   for (int sd = 0; sd < 2; ++sd) {
     for (int i = 0; i < P; ++i)
       for (int s = 0; s < S; ++s) {
         const double w0 = s % NT == i ? e(0, sd, 0, s / NT * NT) : 0.0;
         const double w1 = s % N1 == i % N1 ? e(1, sd, i / N1 * N1, s / N1 * N1) : 0.0;
         const double w2 = s / N1 == i ? e(2, sd, 0, s % N1) : 0.0;
-        if (!(std::fabs(e(0, sd, i, s) - w0) <= TOL * big && std::fabs(e(1, sd, i, s) - w1) <= TOL * big &&
-              std::fabs(e(2, sd, i, s) - w2) <= TOL * big))
-          return false;
+        de = std::max(de, std::max(std::fabs(e(0, sd, i, s) - w0),
+                                   std::max(std::fabs(e(1, sd, i, s) - w1), std::fabs(e(2, sd, i, s) - w2))));
       }
     for (int l = 0; l < N1; ++l) {
-      o.E02[0][sd][l] = (float)e(0, sd, 0, l * NT);
-      o.E02[1][sd][l] = (float)e(2, sd, 0, l);
+      o.E02[0][sd][l] = e(0, sd, 0, l * NT);
+      o.E02[1][sd][l] = e(2, sd, 0, l);
     }
     for (int a = 0; a < N1; ++a)
-      for (int t = 0; t < NT; ++t) o.E1[sd][a][t] = (float)e(1, sd, a * N1, t * N1);
+      for (int t = 0; t < NT; ++t) o.E1[sd][a][t] = e(1, sd, a * N1, t * N1);
   }
+  dev = std::max(dev, de / big);
   std::vector<double> T, c;
-  if (!px_kron(MT, NF, NT, N1, [&](int i, int j) { return c2f[(size_t)i * S + j]; }, TOL, T, c)) return false;
-  for (int i = 0; i < MT * NT; ++i) o.Ct[i / NT][i % NT] = (float)T[i];
-  for (int i = 0; i < NF * N1; ++i) o.Cc[i / N1][i % N1] = (float)c[i];
-  for (int m = 0; m < 3; ++m) {
-    if (!px_kron(NT, N1, MT, NF, [&](int i, int j) { return W[((size_t)i * FN + j) * 3 + m]; }, TOL, T, c))
-      return false;
-    for (int i = 0; i < NT * MT; ++i) o.Wt[m][i / MT][i % MT] = (float)T[i];
-    for (int i = 0; i < N1 * NF; ++i) o.Wc[m][i / NF][i % NF] = (float)c[i];
-  }
-  return true;
+  dev = std::max(dev, px_kron(MT, NF, NT, N1, [&](int i, int j) { return c2f[(size_t)i * S + j]; }, T, c));
+  if (!(dev < 1.0)) return INFINITY;
+  for (int i = 0; i < MT * NT; ++i) o.Ct[i / NT][i % NT] = T[i];
+  for (int i = 0; i < NF * N1; ++i) o.Cc[i / N1][i % N1] = c[i];
+  // W = f2c * D_fine from the factors of both: (T (x) c) * (a-line, plane, c-line)
+  dev = std::max(dev, px_kron(NT, N1, MT, NF, [&](int i, int j) { return f2c[(size_t)i * FN + j]; }, T, c));
+  double f0[NF][NF], f1[MT][MT], f2[NF][NF];
+  dev = std::max(dev, px_lines<NF>(Df, f0, f1, f2));
+  if (!(dev < 1.0)) return INFINITY;
+  for (int r = 0; r < NT; ++r)
+    for (int t = 0; t < MT; ++t) {
+      double w0 = 0.0, w1 = 0.0;
+      for (int l = 0; l < NF; ++l) w0 += T[r * MT + l * NF + t % NF] * f0[l][t / NF];
+      for (int l = 0; l < MT; ++l) w1 += T[r * MT + l] * f1[l][t];
+      o.Wt[0][r][t] = w0;
+      o.Wt[1][r][t] = w1;
+      o.Wt[2][r][t] = T[r * MT + t];
+    }
+  for (int k = 0; k < N1; ++k)
+    for (int l = 0; l < NF; ++l) {
+      double w2 = 0.0;
+      for (int j = 0; j < NF; ++j) w2 += c[k * NF + j] * f2[j][l];
+      o.Wc[0][k][l] = o.Wc[1][k][l] = c[k * NF + l];
+      o.Wc[2][k][l] = w2;
+    }
+  return dev;
+}
+
+template <int N1, int NF>
+inline PxOps<float, N1, NF> px_float(const PxOps<double, N1, NF>& d) {
+  PxOps<float, N1, NF> f;
+  static_assert(sizeof(f) * 2 == sizeof(d), "the same fields");
+  const double* x = reinterpret_cast<const double*>(&d);
+  float* y = reinterpret_cast<float*>(&f);
+  for (size_t i = 0; i < sizeof(f) / sizeof(float); ++i) y[i] = (float)x[i];
+  return f;
 }
 
 }  // namespace afr

@@ -11,16 +11,26 @@
 
 namespace afr {
 
+// One face record of the transport in two 16-byte loads: the owner's cell and
+// extrapolation row group, the neighbour-side sources and their matrices.
+struct SstFace {
+  int32_t owner, group;  // group: (cell type * 3 + axis) * 2 + (side > 0)
+  int32_t c0, m0;        // first source cell (-1: none) and matrix row
+  int32_t c1, m1;        // second source
+  int32_t flags;         // bit 0: no source (boundary), bit 1: wall
+  int32_t pad;
+};
+
 struct SstArgs {
   const double* U;      // (N,S,nv) step-start state
   const double* dt;     // (N,S)
   double* k;            // (N,S) in/out
   double* w;            // (N,S) in/out
   double* nut;          // (N,S) in/out (kinematic eddy viscosity)
-  double* pt;           // (N,S,5) scratch: Sk, Sw, beta_blend, gamma_k, gamma_w
+  double* pt;           // (N,S,5) scratch: Sk, Sw, beta_blend, gamma_k, gamma_w; structured prisms: see k_pxs_point
   double* sp8;          // (N,S,8) scratch: rho, u, v, w, k, omega, gamma_k, gamma_w (face gathers)
-  double* cfp;          // (F,P,4) scratch: conv_k, diff_k, conv_w, diff_w face corrections
-  const uint8_t* wall_face;  // (F) WALL boundary faces (k Dirichlet-zero ghost)
+  double* cfp;          // (F,P,2) scratch: face corrections of k and omega, convection minus diffusion
+  const SstFace* faces; // (F) what the face kernel needs of a record
   double* dbg;          // optional (N,S,4): Sk, Sw, transport_k, transport_w
   int nv;
   double mu;            // molecular viscosity of the mean flow
@@ -48,15 +58,95 @@ __device__ __forceinline__ double sst_F1(double k, double w, double d, double nu
   return tanh(a2 * a2);  // arg1**4 (sst.py:92-141); within an ulp of pow(a, 4)
 }
 
-__device__ __forceinline__ double sst_F2(double k, double w, double d, double nu) {
-  w = fmax(w, 1e-10);
-  k = fmax(k, 1e-10);
-  d = fmax(d, 1e-10);
-  const double sk = sqrt(k);
-  double a = fmax(2.0 * sk / (SST_BSTAR * w * d), 500.0 * nu / (d * d * w));
-  if (!isfinite(a)) a = 1e150;
-  a = fmin(a, 1e150);
-  return tanh(a * a);
+// tanh of a non-negative argument; 1 - 2 exp(-2x) rounds to 1 from x = 19.07 on
+__device__ __forceinline__ double sst_tanh(double x) { return x >= 20.0 ? 1.0 : tanh(x); }
+
+// F1 from its argument: tanh(arg^4), arg as sst_F1 caps it
+__device__ __forceinline__ double sst_blend(double a, double cap) {
+  if (!isfinite(a)) a = cap;
+  a = fmin(a, cap);
+  const double a2 = a * a;
+  return sst_tanh(a2 * a2);
+}
+
+struct SstPoint {
+  double nut, Sk, Sw, beta, gk, gw;
+};
+
+// the closure at one point: gradients gp of rho u, rho v, rho w, k, omega
+// (rows), clamped density, k, omega, wall distance, molecular viscosity
+__device__ __forceinline__ SstPoint sst_closure(double (&gp)[5][3], double rho, double kf, double wf, double d,
+                                                double mu) {
+  // |grad| <= 1e6 clip of grad k, grad omega
+#pragma unroll
+  for (int q = 3; q < 5; ++q) {
+    const double m2 = gp[q][0] * gp[q][0] + gp[q][1] * gp[q][1] + gp[q][2] * gp[q][2];
+    if (m2 > 0.999999e12) {  // near or above the limit
+      const double mag = sqrt(m2);
+      if (mag > 1e6) {
+        double sc = 1e6 / fmax(mag, 1e-10);
+        sc = fmin(fmax(sc, 0.0), 1.0);
+        for (int n = 0; n < 3; ++n) gp[q][n] *= sc;
+      }
+    }
+  }
+  // strain magnitude of the conserved-momentum gradient
+  double ss = 0.0;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) {
+      const double sij = 0.5 * (gp[i][j] + gp[j][i]);
+      ss += sij * sij;
+    }
+  const double Sm = sqrt(2.0 * ss);
+  const double gd = gp[3][0] * gp[4][0] + gp[3][1] * gp[4][1] + gp[3][2] * gp[4][2];
+  // --- compute_source_terms ---
+  const double rrho = 1.0 / fmax(rho, 1e-10);  // one reciprocal: each use within an ulp of a division
+  const double nu = MU_SOURCE * rrho;
+  const double k_s = fmin(kf, 1e40);
+  const double w_s = fmax(fmin(wf, 1e40), 1e-10);
+  // The blending arguments (sst.py:92-179) of the source terms and of the
+  // transport share everything but the viscosity, and each quotient is a
+  // product with one of four reciprocals (a few ulp from the division): the
+  // closure's cost is its divisions, square roots and tanh.
+  const double wc = fmax(w_s, 1e-10), kc = fmax(k_s, 1e-10), dc = fmax(d, 1e-10);
+  const double rw = 1.0 / wc, rd = 1.0 / dc;
+  const double CD = fmax(2.0 * rho * SST_SW2 * rw * gd, 1e-10);
+  const double t1 = sqrt(kc) * (rw * rd) * (1.0 / SST_BSTAR);
+  const double t2 = 500.0 * nu * (rd * rd * rw);
+  const double t3 = 4.0 * rho * SST_SW2 * kc * (rd * rd) / CD;
+  const double F1 = sst_blend(fmin(fmax(t1, t2), t3), 1e75);
+  double a2 = fmax(2.0 * t1, t2);
+  if (!isfinite(a2)) a2 = 1e150;
+  a2 = fmin(a2, 1e150);
+  const double F2 = sst_tanh(a2 * a2);
+  const double beta = F1 * SST_B1 + (1.0 - F1) * SST_B2;
+  double nut = SST_A1 * kc / fmax(SST_A1 * wc, F2 * fmax(Sm, 1e-10));
+  nut = fmin(nut, SST_TVR * MU_SOURCE * rrho);
+  if (!isfinite(nut)) nut = 0.0;
+  double Pk = nut * rho * (Sm * Sm);
+  Pk = fmin(Pk, 10.0 * SST_BSTAR * rho * k_s * w_s);
+  const double Dk = rho * SST_BSTAR * k_s * w_s;
+  const double g1 = SST_B1 / SST_BSTAR - SST_SW1 * SST_KAPPA * SST_KAPPA / sqrt(SST_BSTAR);
+  const double g2 = SST_B2 / SST_BSTAR - SST_SW2 * SST_KAPPA * SST_KAPPA / sqrt(SST_BSTAR);
+  const double gam = F1 * g1 + (1.0 - F1) * g2;
+  const double Pw = rho * gam * (Sm * Sm);
+  const double Dw = rho * beta * (w_s * w_s);
+  const double CDw = 2.0 * rho * (1.0 - F1) * SST_SW2 * rw * gd;
+  const double Sk = dfinite(Pk - Dk);
+  const double Sw = dfinite(Pw - Dw + CDw);
+  // --- transport diffusion coefficients (mu = molecular viscosity of the mean flow) ---
+  // (the transport does not cap k and omega at 1e40)
+  double F1t;
+  if (kf <= 1e40 && wf <= 1e40) {
+    F1t = sst_blend(fmin(fmax(t1, 500.0 * (mu * rrho) * (rd * rd * rw)), t3), 1e75);
+  } else {
+    const double CD2 = fmax(2.0 * rho * SST_SW2 / fmax(wf, 1e-10) * gd, 1e-10);
+    F1t = sst_F1(kf, wf, d, mu * rrho, rho, CD2);
+  }
+  const double sk = F1t * SST_SK1 + (1.0 - F1t) * SST_SK2;
+  const double sw = F1t * SST_SW1 + (1.0 - F1t) * SST_SW2;
+  const double rnut = rho * nut;
+  return SstPoint{nut, Sk, Sw, beta, mu + sk * rnut, mu + sw * rnut};
 }
 
 // SST cells per CTA (the three per-cell SST kernels)
@@ -120,69 +210,21 @@ __global__ void __launch_bounds__(128) k_sst_point(Geom g, Ops ops, SstArgs a, i
         for (int m = 0; m < 3; ++m) acc += gcs[(s * 3 + m) * 5 + q] * inv[m * 3 + n];
         gp[q][n] = acc;
       }
-    // |grad| <= 1e6 clip of grad k, grad omega
-    for (int q = 3; q < 5; ++q) {
-      const double mag = sqrt(gp[q][0] * gp[q][0] + gp[q][1] * gp[q][1] + gp[q][2] * gp[q][2]);
-      if (mag > 1e6) {
-        double sc = 1e6 / fmax(mag, 1e-10);
-        sc = fmin(fmax(sc, 0.0), 1.0);
-        for (int n = 0; n < 3; ++n) gp[q][n] *= sc;
-      }
-    }
     const double* u = sU + t * nv;
     const double rho = fmax(u[0], 1e-10);
     const double kf = f[t * 5 + 3], wf = f[t * 5 + 4];
-    const double d = g.wall_dist[p];
-    // strain magnitude of the conserved-momentum gradient
-    double ss = 0.0;
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) {
-        const double sij = 0.5 * (gp[i][j] + gp[j][i]);
-        ss += sij * sij;
-      }
-    const double Sm = sqrt(2.0 * ss);
-    const double gd = gp[3][0] * gp[4][0] + gp[3][1] * gp[4][1] + gp[3][2] * gp[4][2];
-    // --- compute_source_terms ---
-    const double rrho = 1.0 / fmax(rho, 1e-10);  // one reciprocal: each use within an ulp of a division
-    const double nu = MU_SOURCE * rrho;
-    const double k_s = fmin(kf, 1e40);
-    const double w_s = fmax(fmin(wf, 1e40), 1e-10);
-    const double CD = fmax(2.0 * rho * SST_SW2 / w_s * gd, 1e-10);
-    const double F1 = sst_F1(k_s, w_s, d, nu, rho, CD);
-    const double F2 = sst_F2(k_s, w_s, d, nu);
-    const double beta = F1 * SST_B1 + (1.0 - F1) * SST_B2;
-    double nut = SST_A1 * fmax(k_s, 1e-10) / fmax(SST_A1 * fmax(w_s, 1e-10), F2 * fmax(Sm, 1e-10));
-    nut = fmin(nut, SST_TVR * MU_SOURCE * rrho);
-    if (!isfinite(nut)) nut = 0.0;
-    double Pk = nut * rho * (Sm * Sm);
-    Pk = fmin(Pk, 10.0 * SST_BSTAR * rho * k_s * w_s);
-    const double Dk = rho * SST_BSTAR * k_s * w_s;
-    const double g1 = SST_B1 / SST_BSTAR - SST_SW1 * SST_KAPPA * SST_KAPPA / sqrt(SST_BSTAR);
-    const double g2 = SST_B2 / SST_BSTAR - SST_SW2 * SST_KAPPA * SST_KAPPA / sqrt(SST_BSTAR);
-    const double gam = F1 * g1 + (1.0 - F1) * g2;
-    const double Pw = rho * gam * (Sm * Sm);
-    const double Dw = rho * beta * (w_s * w_s);
-    const double CDw = 2.0 * rho * (1.0 - F1) * SST_SW2 / w_s * gd;
-    const double Sk = dfinite(Pk - Dk);
-    const double Sw = dfinite(Pw - Dw + CDw);
-    // --- transport diffusion coefficients (mu = molecular viscosity of the mean flow) ---
-    const double nu_m = a.mu * rrho;
-    const double CD2 = fmax(2.0 * rho * SST_SW2 / fmax(wf, 1e-10) * gd, 1e-10);
-    const double F1t = sst_F1(kf, wf, d, nu_m, rho, CD2);
-    const double sk = F1t * SST_SK1 + (1.0 - F1t) * SST_SK2;
-    const double sw = F1t * SST_SW1 + (1.0 - F1t) * SST_SW2;
-    const double rnut = rho * nut;
-    a.nut[p] = nut;
+    const SstPoint o = sst_closure(gp, rho, kf, wf, g.wall_dist[p], a.mu);
+    const double rrho = 1.0 / rho;
+    a.nut[p] = o.nut;
     // outputs staged in this point's own rows (read above by this thread only),
     // then stored as contiguous blocks
-    const double gk = a.mu + sk * rnut, gw = a.mu + sw * rnut;
     const double r1 = u[1] * rrho, r2 = u[2] * rrho, r3 = u[3] * rrho;
-    double* o = f + t * 5;
-    o[0] = Sk;
-    o[1] = Sw;
-    o[2] = beta;
-    o[3] = gk;
-    o[4] = gw;
+    double* o5 = f + t * 5;
+    o5[0] = o.Sk;
+    o5[1] = o.Sw;
+    o5[2] = o.beta;
+    o5[3] = o.gk;
+    o5[4] = o.gw;
     double* o8 = sInv + t * 9;
     o8[0] = rho;
     o8[1] = r1;
@@ -190,8 +232,8 @@ __global__ void __launch_bounds__(128) k_sst_point(Geom g, Ops ops, SstArgs a, i
     o8[3] = r3;
     o8[4] = kf;
     o8[5] = wf;
-    o8[6] = gk;
-    o8[7] = gw;
+    o8[6] = o.gk;
+    o8[7] = o.gw;
   }
   __syncthreads();
   double* pt = a.pt + (size_t)e0 * S * 5;
@@ -205,27 +247,27 @@ __global__ void __launch_bounds__(128) k_sst_point(Geom g, Ops ops, SstArgs a, i
 // tensor path (mma.sync m8n8k4 .f64): owner side (face points x S) x (S x 8
 // packed point values), neighbour side per source cell (face points x S) x
 // (S x k, omega, gamma_k, gamma_w); the second source is added to the first as
-// in the reference.  Lanes 0..P-1 then form the corrections.
+// in the reference.  Lanes 0..P-1 then form the corrections.  (One thread per
+// face point with plain multiply-adds over the rows' nonzeros, and a warp per
+// face with its rows staged in shared memory, are slower: 75 and 91 us against
+// 58 us on 16,150 P2 prisms; their row loads wait on one another.)
 constexpr int SST_FACE_WARPS = 4;
 
 template <int S, int NP>
-__global__ void __launch_bounds__(32 * SST_FACE_WARPS, 16) k_sst_face(Geom g, Ops ops, Faces fc, SstArgs a) {
+__global__ void __launch_bounds__(32 * SST_FACE_WARPS, 16) k_sst_face(Ops ops, Faces fc, SstArgs a) {
   constexpr int W = SST_FACE_WARPS, RW = 17;  // RW: po (8), pn of the first (4) and second (4) source, pad
   constexpr int MT = (NP + 7) / 8;            // row tiles of the face points
   __shared__ double sR[W][NP * RW];
   const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f = blockIdx.x * W + wi;
   if (f >= fc.F) return;  // whole warps: only warp-level synchronisation below
-  const int oc = fc.owner[f];
-  const int c0 = fc.nb_c0[f], i1 = fc.nb_i1[f];
-  const int c1 = i1 >= 0 ? fc.nb_c1[i1] : -1;
-  const bool bnd = c0 < 0 && i1 < 0;
+  const int4* rp = reinterpret_cast<const int4*>(a.faces + f);
+  const int4 r0 = __ldg(rp), r1 = __ldg(rp + 1);  // owner, group, c0, m0 | c1, m1, flags
+  const int oc = r0.x, c0 = r0.z, c1 = r1.x;
+  const bool bnd = (r1.z & 1) != 0;
   double* R = sR[wi];
   {
-    const int ct = cell_type(g, oc);
-    const int ax = fc.o_axis[f];
-    const double* Ef =
-        ops.fextrap + (((size_t)ct * 3 + ax) * 2 + (fc.o_side[f] <= 0.0 ? 0 : 1)) * (MT * ((S + 3) / 4) * 32);
+    const double* Ef = ops.fextrap + (size_t)r0.y * (MT * ((S + 3) / 4) * 32);
     const double* X = a.sp8 + (size_t)oc * S * 8;
     dmma_warp_rb_f<MT, 1, S>(
         NP, 8, Ef, [&](int s, int n) { return __ldg(X + s * 8 + n); },
@@ -236,7 +278,7 @@ __global__ void __launch_bounds__(32 * SST_FACE_WARPS, 16) k_sst_face(Geom g, Op
       const int c = src == 0 ? c0 : c1;
       if (c < 0) continue;
       const double* X = a.sp8 + (size_t)c * S * 8 + 4;
-      const double* M = src == 0 ? fmat(fc.nb_m0, fc.nb_m0i, f, 0, NP, S) : fmat(fc.nb_m1, fc.nb_m1i, i1, 0, NP, S);
+      const double* M = src == 0 ? fc.nb_m0 + (size_t)r0.w * S * NP : fc.nb_m1 + (size_t)r1.y * S * NP;
       dmma_warp_rb<MT, 1, S>(
           NP, 4, [&](int i, int s) { return __ldg(M + s * NP + i); }, [&](int s, int n) { return __ldg(X + s * 8 + n); },
           [&](int i, int n, double x) { R[i * RW + 8 + src * 4 + n] = x; });
@@ -249,7 +291,7 @@ __global__ void __launch_bounds__(32 * SST_FACE_WARPS, 16) k_sst_face(Geom g, Op
 #pragma unroll
     for (int c = 0; c < 8; ++c) po[c] = r[c];
     if (bnd) {
-      const bool wz = a.wall_face[f] != 0;
+      const bool wz = (r1.z & 2) != 0;
       pn[0] = wz ? -po[4] : po[4];
       pn[1] = po[5];
       pn[2] = po[6];
@@ -263,13 +305,12 @@ __global__ void __launch_bounds__(32 * SST_FACE_WARPS, 16) k_sst_face(Geom g, Op
     }
     const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
     const double mflux = ((po[0] * po[1]) * tn[0] + (po[0] * po[2]) * tn[1]) + (po[0] * po[3]) * tn[2];
-    double* o = a.cfp + ((size_t)f * NP + i) * 4;
     const double upk = mflux >= 0.0 ? po[4] : pn[0];
     const double upw = mflux >= 0.0 ? po[5] : pn[1];
-    o[0] = mflux * (upk - po[4]);
-    o[1] = (0.5 * (po[6] + pn[2])) * (0.5 * (po[4] + pn[0]) - po[4]);
-    o[2] = mflux * (upw - po[5]);
-    o[3] = (0.5 * (po[7] + pn[3])) * (0.5 * (po[5] + pn[1]) - po[5]);
+    // the convective correction enters the residual with +, the diffusive one with -
+    reinterpret_cast<double2*>(a.cfp)[(size_t)f * NP + i] =
+        make_double2(mflux * (upk - po[4]) - (0.5 * (po[6] + pn[2])) * (0.5 * (po[4] + pn[0]) - po[4]),
+                     mflux * (upw - po[5]) - (0.5 * (po[7] + pn[3])) * (0.5 * (po[5] + pn[1]) - po[5]));
   }
 }
 
@@ -289,7 +330,7 @@ __global__ void __launch_bounds__(128) k_sst_update(Geom g, Ops ops, Faces fc, S
   __shared__ double sP[CPB * S * 9];
   __shared__ double gc[CPB * S * 3 * 2];  // reference-space grads of k, w
   // contravariant fluxes (conv k, diff k, conv w, diff w); then the face
-  // corrections of the tile's transport slots (slot j's face rows at Ft + j*NP*4)
+  // corrections of the tile's transport slots (slot j's face rows at Ft + j*NP*2)
   __shared__ __align__(16) double Ft[CPB * S * 3 * 4];
   // inverse Jacobians (rows of 9) until the fluxes are formed; then R (volume
   // residuals, then with the interface corrections), T (transport k, w +
@@ -309,7 +350,7 @@ __global__ void __launch_bounds__(128) k_sst_update(Geom g, Ops ops, Faces fc, S
   const int ct = cell_type(g, e0);
   // the tile's transport slots are contiguous (cell-major)
   const int k_beg = fc.tslot_ptr[e0], k_end = fc.tslot_ptr[e0 + nc];
-  const bool staged = (k_end - k_beg) * NP * 4 <= CPB * S * 12 && k_end - k_beg <= CPB * SST_STAGE_SLOTS;
+  const bool staged = (k_end - k_beg) * NP * 2 <= CPB * S * 12 && k_end - k_beg <= CPB * SST_STAGE_SLOTS;
   double* sC = Ft;
   // the tile's blocks are contiguous: asynchronous copies, all in flight at once
   {
@@ -392,10 +433,10 @@ __global__ void __launch_bounds__(128) k_sst_update(Geom g, Ops ops, Faces fc, S
   // the fluxes are consumed: the slots' face corrections arrive in their space
   __syncthreads();
   if (staged) {
-    for (int t = threadIdx.x; t < (k_end - k_beg) * NP * 2; t += blockDim.x) {
-      const int j = t / (NP * 2), q = t - j * (NP * 2);
+    for (int t = threadIdx.x; t < (k_end - k_beg) * NP; t += blockDim.x) {
+      const int j = t / NP, q = t - j * NP;
       const int face = sCode[j] >> 4;
-      cp_async16(sC + j * NP * 4 + 2 * q, a.cfp + (size_t)face * NP * 4 + 2 * q);
+      cp_async16(sC + (j * NP + q) * 2, a.cfp + ((size_t)face * NP + q) * 2);
     }
     cp_async_wait_all();
   }
@@ -405,33 +446,25 @@ __global__ void __launch_bounds__(128) k_sst_update(Geom g, Ops ops, Faces fc, S
     const int s = p % S;
     const int e = e0 + p / S;
     const double rdj = sRd[p];
-    double C[4] = {0.0, 0.0, 0.0, 0.0};
+    double C[2] = {0.0, 0.0};
     const int sb = fc.tslot_ptr[e], se = fc.tslot_ptr[e + 1];
     for (int k = sb; k < se; ++k) {
       const int code = staged ? sCode[k - k_beg] : __ldg(fc.tslot + k);
       const int ax = (code >> 2) & 3;
       const double gw = sG[((code & 1) ? 4 : 0) + sDco[ax * S + s]];
       const int fp = sDfp[ax * S + s];
-      double2 c01, c23;
-      if (staged) {
-        const double2* cr = reinterpret_cast<const double2*>(sC + ((k - k_beg) * NP + fp) * 4);
-        c01 = cr[0];
-        c23 = cr[1];
+      const double2 cv = staged ? *reinterpret_cast<const double2*>(sC + ((k - k_beg) * NP + fp) * 2)
+                                : __ldg(reinterpret_cast<const double2*>(a.cfp) + (size_t)(code >> 4) * NP + fp);
+      if (code & 2) {
+        C[0] += (gw * cv.x) * rdj;
+        C[1] += (gw * cv.y) * rdj;
       } else {
-        const double2* cr = reinterpret_cast<const double2*>(a.cfp + ((size_t)(code >> 4) * NP + fp) * 4);
-        c01 = __ldg(cr);
-        c23 = __ldg(cr + 1);
-      }
-      const double cv[4] = {c01.x, c01.y, c23.x, c23.y};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double contrib = gw * cv[q];
-        if (code & 2) C[q] += contrib * rdj;
-        else C[q] -= contrib * rdj;
+        C[0] -= (gw * cv.x) * rdj;
+        C[1] -= (gw * cv.y) * rdj;
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) Ref[p * 4 + q] = C[q];  // staged: R is complete only after the barrier below
+    for (int q = 0; q < 2; ++q) Ref[p * 2 + q] = C[q];  // staged: R is complete only after the barrier below
   }
   __syncthreads();
   // the fluxes are consumed: their space receives the tile's point sources
@@ -446,13 +479,8 @@ __global__ void __launch_bounds__(128) k_sst_update(Geom g, Ops ops, Faces fc, S
   }
   for (int p = threadIdx.x; p < nc * S; p += blockDim.x) {
     const double rho = sP[p * 9];
-    const double* Cp = Ref + p * 4;
-    const double conv_k = R[p * 4 + 0] + Cp[0];
-    const double diff_k = R[p * 4 + 1] - Cp[1];
-    const double conv_w = R[p * 4 + 2] + Cp[2];
-    const double diff_w = R[p * 4 + 3] - Cp[3];
-    T[p * 5 + 0] = (conv_k + diff_k) / fmax(rho, 1e-10);
-    T[p * 5 + 1] = (conv_w + diff_w) / fmax(rho, 1e-10);
+    T[p * 5 + 0] = (R[p * 4 + 0] + R[p * 4 + 1] + Ref[p * 2 + 0]) / fmax(rho, 1e-10);
+    T[p * 5 + 1] = (R[p * 4 + 2] + R[p * 4 + 3] + Ref[p * 2 + 1]) / fmax(rho, 1e-10);
     T[p * 5 + 2] = 0.0; T[p * 5 + 3] = 0.0; T[p * 5 + 4] = 0.0;
   }
   __syncthreads();
