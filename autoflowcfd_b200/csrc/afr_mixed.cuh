@@ -1090,13 +1090,13 @@ __device__ __forceinline__ bool outlier_clear(const double (&x)[PL], const bool 
 #pragma unroll
   for (int l = 0; l < PL; ++l) hw = max(hw, on[l] ? (unsigned)__double2hiint(x[l]) & 0x7fffffffu : 0u);
   hw = cell_max<S>(hw);
-  if (hw >= 0x7fe00000u) return false;
+  const bool finite = hw < 0x7fe00000u;  // no early return: every lane of the warp takes part in the ballots
   const double hi = __hiloint2double((int)hw + 1, 0);
   const double p = hi * 1.0000000001e-4;  // 1e4 * p >= hi after rounding
   int cnt = 0;
 #pragma unroll
   for (int l = 0; l < PL; ++l) cnt += __popc(cell_ballot<S>(on[l] && fabs(x[l]) >= p, grp));
-  return cnt >= NEED || hi <= 1e-297;
+  return finite && (cnt >= NEED || hi <= 1e-297);
 }
 
 // the rule itself: stable ranks over the cell's points, median, zeroing
