@@ -36,8 +36,8 @@ struct afr_handle {
   Faces fc{};
   Bc bc{};
   // scratch
-  double* PF = nullptr;       // (N,S,18) point fields of the state being evaluated
-  double* J = nullptr;        // (n_slots,P,10) face jumps of the residual slots
+  double* PF = nullptr;       // (N,S,16) point fields of the state being evaluated
+  double* J = nullptr;        // (n_slots,9,P) face jumps of the residual slots
   SlotTable slots{};
   double* Ua = nullptr;
   double* Ub = nullptr;
@@ -78,7 +78,10 @@ struct afr_handle {
   PxOps<float, 3, 4> px2{};
   PxOps<double, 2, 3> pxd1{};
   PxOps<double, 3, 4> pxd2{};
-  PxGeom pg{};
+  PxGeom<float> pg{};
+  PxGeom<double> pgd{};
+  double* RVd = nullptr;       // (N, 9, S) volume terms (plain form of structured prisms)
+  double4* slot_rows = nullptr;  // (n_slots, P) own adjugate rows (plain form)
   unsigned px_faces = 0;  // bit (axis*2 + side): faces whose point fields some slot reads
   bool px_points = false;  // some face point interpolates from the point fields
   int mx_pre_blocks = 0, mx_cell_blocks = 0;  // resident CTAs of the persistent kernels
@@ -244,7 +247,7 @@ __global__ void k_force(Geom g, Ops ops, Faces fc, const int32_t* faces, int nf,
   const double* E = ops.extrap + (((size_t)ct * 3 + ax) * 2 + (fc.o_side[f] < 0.0 ? 0 : 1)) * NP * S;
   double fp[3] = {0, 0, 0}, fv[3] = {0, 0, 0};
   for (int i = 0; i < NP; ++i) {
-    double pf = 0.0, mt = 0.0, gv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double pf = 0.0, mt = 0.0, sg[6] = {0, 0, 0, 0, 0, 0};  // S00, S11, S22, S01, S02, S12
     for (int s = 0; s < S; ++s) {
       const size_t p = (size_t)oc * S + s;
       const double* u = U + p * nv;
@@ -254,17 +257,17 @@ __global__ void k_force(Geom g, Ops ops, Faces fc, const int32_t* faces, int nf,
       const double w = E[i * S + s];
       pf += w * pr;
       if (nut) mt += w * (rho * nut[p]);
-      for (int k = 0; k < 9; ++k) gv[k] += w * PF[p * PFW + 5 + k];
+      for (int k = 0; k < 6; ++k) sg[k] += w * PF[p * PFW + 5 + k];
     }
     const double* n = fc.tnormal + ((size_t)f * NP + i) * 3;
     const double aw = area_w[(size_t)f * NP + i];
     for (int d = 0; d < 3; ++d) fp[d] += pf * n[d] * aw;
     const double mtot = mu + mt;
-    const double div = gv[0] + gv[4] + gv[8];
+    const double div = sg[0] + sg[1] + sg[2];
     for (int r = 0; r < 3; ++r) {
       double tr = 0.0;
       for (int c = 0; c < 3; ++c) {
-        const double sij = 0.5 * (gv[r * 3 + c] + gv[c * 3 + r]);
+        const double sij = r == c ? sg[r] : sg[2 + r + c];
         const double tau = 2.0 * mtot * sij + ((r == c) ? (-2.0 / 3.0 * mtot) * div : 0.0);
         tr += tau * n[c];
       }
@@ -366,11 +369,74 @@ template <int S, int FN, int NP, int N1D>
 struct Launch {
   static constexpr int CPB = S <= 8 ? 8 : (S <= 27 ? 2 : 1);
   static size_t cell_smem() { return sizeof(double) * CellSmem<S, FN, CPB, NP>::total; }
-  static cudaError_t pre(afr_handle* h, const double* U, const double* nut, bool grads, cudaStream_t st) {
+  // structured prisms: one kernel forms the face-point fields and the volume terms
+  static constexpr bool PXD = S == 8 || S == 27;
+  static constexpr int PXN1 = S == 8 ? 2 : 3, PXNF = S == 8 ? 3 : 4, PXC = S == 8 ? 6 : 2;
+  using PxS = PxSmem<float, PXN1, PXNF, PXC>;
+  using PxSD = PxSmem<double, PXN1, PXNF, PXC>;
+  static bool px_range(const afr_handle* h, int r) { return PXD && h->px && r == 0; }
+  static cudaError_t px_cell(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
+    if constexpr (PXD) {
+      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
+      const auto* op = [&] {
+        if constexpr (S == 8) return &h->px1;
+        else return &h->px2;
+      }();
+      auto* fn = visc ? k_px_cell<float, PXN1, PXNF, PXC, true> : k_px_cell<float, PXN1, PXNF, PXC, false>;
+      fn<<<nb, 32 * PX_WARPS, PxS::total, st>>>(*op, h->pg, h->mb.XF, h->px_points ? h->mb.PFm : nullptr, h->mb.RV,
+                                                h->mb.FW, h->px_faces, U, h->nv, nut, (float)h->prm.mu, 0, n);
+      return cudaGetLastError();
+    }
+    return cudaErrorNotSupported;
+  }
+  // shared-memory limits of the plain form's kernels, once per process
+  static void set_attrs() {
+    static const bool done = [] {
+      const size_t smem = cell_smem();
+      cudaFuncSetAttribute(k_cell<S, FN, NP, CPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_update<S, NP, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
+      if constexpr (PXD) {
+        cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             PxSD::total);
+        cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             PxSD::total);
+      }
+      return true;
+    }();
+    (void)done;
+  }
+  // the plain form's structured prisms
+  static bool px64_range(const afr_handle* h, int r) {
+    return PXD && r == 0 && h->px64 && h->prec == AFR_PREC_FP64 && h->RVd;
+  }
+  static cudaError_t px_cell64(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
+    if constexpr (PXD) {
+      set_attrs();
+      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
+      const auto* op = [&] {
+        if constexpr (S == 8) return &h->pxd1;
+        else return &h->pxd2;
+      }();
+      auto* fn = visc ? k_px_cell<double, PXN1, PXNF, PXC, true> : k_px_cell<double, PXN1, PXNF, PXC, false>;
+      fn<<<nb, 32 * PX_WARPS, PxSD::total, st>>>(*op, h->pgd, nullptr, h->PF, h->RVd, 0, 0u, U, h->nv, nut,
+                                                 h->prm.mu, 0, n);
+      return cudaGetLastError();
+    }
+    return cudaErrorNotSupported;
+  }
+  // point fields of every cell by the generic kernel; with vol, structured
+  // prisms take k_px_cell, which also forms their volume terms
+  static cudaError_t pre(afr_handle* h, const double* U, const double* nut, bool grads, cudaStream_t st,
+                         bool vol = false) {
     constexpr int CPB = PreTile<S>::CPB;
     const int ranges[3] = {0, h->n_prism, h->N};
     for (int r = 0; r < 2; ++r) {
       const int n = ranges[r + 1] - ranges[r];
+      if (vol && px64_range(h, r) && n > 0) {
+        const cudaError_t e = px_cell64(h, U, nut, grads, n, st);
+        if (e != cudaSuccess) return e;
+        continue;
+      }
       if (n > 0)
         k_pre<S><<<(n + CPB - 1) / CPB, 128, 0, st>>>(h->g, h->ops, U, h->nv, nut, grads ? 1 : 0, h->PF, ranges[r],
                                                       ranges[r + 1]);
@@ -382,14 +448,10 @@ struct Launch {
     const int nwarps = (h->slots.n + SPW - 1) / SPW;
     if (nwarps > 0)
       k_face<S, NP><<<(nwarps + FACE_WARPS - 1) / FACE_WARPS, 32 * FACE_WARPS, 0, st>>>(
-          h->g, h->ops, h->fc, h->bc, h->slots, h->PF, h->prm.mu, a.inviscid_only ? 0 : 1, h->J);
+          h->g, h->ops, h->fc, h->bc, h->slots, h->PF, h->slot_rows, h->prm.mu, a.inviscid_only ? 0 : 1, h->J);
     if (tm) tm->mark(st);
     const size_t smem = cell_smem();
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_cell<S, FN, NP, CPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      attr = true;
-    }
+    set_attrs();
     a.N = h->N;
     a.slot_flags = h->slots.flags;
     const int ranges[3] = {0, h->n_prism, h->N};
@@ -398,6 +460,12 @@ struct Launch {
       a.cell_end = ranges[r + 1];
       const int n = a.cell_end - a.cell_base;
       if (n <= 0) continue;
+      if (px64_range(h, r)) {
+        constexpr int warps = 4, per = warps * MxUpd<S>::CW;
+        k_update<S, NP, double><<<(n + per - 1) / per, 32 * warps, MxUpd<S>::bytes(h->nv, warps), st>>>(
+            h->ops, h->fc, a, r, h->RVd, h->J, h->pgd.rdet);
+        continue;
+      }
       k_cell<S, FN, NP, CPB><<<(n + CPB - 1) / CPB, CELL_THREADS, smem, st>>>(h->g, h->ops, h->fc, a, h->J);
     }
     return cudaGetLastError();
@@ -416,10 +484,10 @@ struct Launch {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_mx_vol<S, FN, MXC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_vol_smem());
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mx_update<S, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
+      e = cudaFuncSetAttribute(k_update<S, NP, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
     if constexpr (PXD) {
-      auto* fv = k_px_cell<PXN1, PXNF, PXC, true>;
-      auto* fi = k_px_cell<PXN1, PXNF, PXC, false>;
+      auto* fv = k_px_cell<float, PXN1, PXNF, PXC, true>;
+      auto* fi = k_px_cell<float, PXN1, PXNF, PXC, false>;
       if (e == cudaSuccess) e = cudaFuncSetAttribute(fv, cudaFuncAttributeMaxDynamicSharedMemorySize, PxS::total);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(fi, cudaFuncAttributeMaxDynamicSharedMemorySize, PxS::total);
       if (e == cudaSuccess)
@@ -461,29 +529,10 @@ struct Launch {
   }
   static void mx_update_launch(afr_handle* h, const StageArgs& a, int ct, int n, cudaStream_t st) {
     const int warps = 1 << h->mx_upd_var, per = warps * MxUpd<S>::CW;
-    k_mx_update<S, NP><<<(n + per - 1) / per, 32 * warps, MxUpd<S>::bytes(h->nv, warps), st>>>(
+    k_update<S, NP, float><<<(n + per - 1) / per, 32 * warps, MxUpd<S>::bytes(h->nv, warps), st>>>(
         h->ops, h->fc, a, ct, h->mb.RV, h->mb.Jm, h->mo.rdet);
   }
   static int n_ranges(const afr_handle* h) { return (h->n_prism > 0 ? 1 : 0) + (h->N > h->n_prism ? 1 : 0); }
-  // structured prisms: one kernel forms the face-point fields and the volume terms
-  static constexpr bool PXD = S == 8 || S == 27;
-  static constexpr int PXN1 = S == 8 ? 2 : 3, PXNF = S == 8 ? 3 : 4, PXC = S == 8 ? 6 : 2;
-  using PxS = PxSmem<PXN1, PXNF, PXC>;
-  static bool px_range(const afr_handle* h, int r) { return PXD && h->px && r == 0; }
-  static cudaError_t px_cell(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
-    if constexpr (PXD) {
-      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
-      const auto* op = [&] {
-        if constexpr (S == 8) return &h->px1;
-        else return &h->px2;
-      }();
-      auto* fn = visc ? k_px_cell<PXN1, PXNF, PXC, true> : k_px_cell<PXN1, PXNF, PXC, false>;
-      fn<<<nb, 32 * PX_WARPS, PxS::total, st>>>(*op, h->pg, h->mb.XF, h->px_points ? h->mb.PFm : nullptr, h->mb.RV,
-                                                h->mb.FW, h->px_faces, U, h->nv, nut, (float)h->prm.mu, 0, n);
-      return cudaGetLastError();
-    }
-    return cudaErrorNotSupported;
-  }
   static cudaError_t mx_pre(afr_handle* h, const double* U, const double* nut, bool grads, cudaStream_t st) {
     const int ranges[3] = {0, h->n_prism, h->N};
     for (int r = 0; r < 2; ++r) {
@@ -533,7 +582,7 @@ struct Launch {
   static cudaError_t eval(afr_handle* h, StageArgs a, const double* U, const double* nut, bool grads,
                           cudaStream_t st, StepTimer* tm = nullptr, int* nl = nullptr) {
     const bool mx = h->prec == AFR_PREC_MIXED;
-    cudaError_t r = mx ? mx_pre(h, U, nut, grads, st) : pre(h, U, nut, grads, st);
+    cudaError_t r = mx ? mx_pre(h, U, nut, grads, st) : pre(h, U, nut, grads, st, true);
     if (r != cudaSuccess) return r;
     if (tm) tm->mark(st);
     if (nl) *nl += (mx ? 3 : 2) * n_ranges(h) - (mx && h->px ? 1 : 0) + (h->slots.n > 0 ? 1 : 0);
@@ -868,6 +917,57 @@ int afr_destroy(afr_handle* h) {
   return AFR_OK;
 }
 
+static void release_alloc(afr_handle* h, const double*& p, size_t n) {
+  auto it = std::find(h->allocs.begin(), h->allocs.end(), (void*)p);
+  if (it == h->allocs.end()) return;
+  h->allocs.erase(it);
+  cudaFree((void*)p);
+  h->bytes -= n * sizeof(double);
+  p = nullptr;
+}
+
+// Tables of the plain form at orders 1-3: the slots' own adjugate rows, and for
+// structured prisms the metrics in lane order, the metric divergence MD and
+// 1/det.  The fine-point adjugates stay only for cells on the generic kernels.
+static int plain_setup(afr_handle* h, cudaStream_t st) {
+  const size_t N = h->N, S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism;
+  int rc;
+  if ((rc = dalloc(h, &h->slot_rows, ns * P))) return rc;
+  double *adjs = nullptr, *adjf = nullptr, *md = nullptr, *rdet = nullptr;
+  if (h->px64 && ((rc = dalloc(h, &adjs, NP * S * 9)) || (rc = dalloc(h, &adjf, NP * Fn * 9)) ||
+                  (rc = dalloc(h, &md, N * S * 3)) || (rc = dalloc(h, &rdet, N * S)) ||
+                  (rc = dalloc(h, &h->RVd, NP * S * 9))))
+    return rc;
+  const unsigned nb = (unsigned)((ns * P + 127) / 128), nmd = (unsigned)((N * S * 3 + 255) / 256);
+  switch (h->order) {
+    case 1:
+      if (ns) k_slot_rows<8, 4><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+      if (h->px64) k_mx_md<8, 27><<<nmd, 256, 0, st>>>(h->g, h->ops, md);
+      break;
+    case 2:
+      if (ns) k_slot_rows<27, 9><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+      if (h->px64) k_mx_md<27, 64><<<nmd, 256, 0, st>>>(h->g, h->ops, md);
+      break;
+    default:
+      if (ns) k_slot_rows<64, 16><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+  }
+  if (h->px64) {
+    const int nf = h->order == 1 ? 3 : 4;
+    k_px_planes<<<(unsigned)((NP * Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, (int)Fn, nf, adjf);
+    k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, (int)S, 1, adjs);
+    k_mx_rdet<<<(unsigned)((N * S + 255) / 256), 256, 0, st>>>(h->g.det, N * S, rdet);
+    h->pgd = PxGeom<double>{adjs, adjf, md, rdet, h->px_rows};
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_fail(h, e, "plain-form set-up");
+  if (h->px64 && h->n_prism == h->N) {
+    release_alloc(h, h->g.adj_fine, N * Fn * 9);
+    release_alloc(h, h->g.adj, N * S * 9);
+  }
+  return AFR_OK;
+}
+
 // Tables of the mixed-precision form: operator images, metric divergence,
 // interior-penalty lengths, per-slot adjugate rows and the conforming-face
 // match of the other side's face point.
@@ -965,7 +1065,14 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   double* rdet;
   if ((rc = dalloc(h, &rdet, N * (size_t)S))) return rc;
   h->mo.rdet = rdet;
-  h->pg = PxGeom{padjs, padjf, md, rdet};
+  float* prows = nullptr;
+  if (h->px) {
+    const std::vector<double> r = h->order == 1 ? px_rows<2>(m->D_3d[0]) : px_rows<3>(m->D_3d[0]);
+    const std::vector<float> rf(r.begin(), r.end());
+    if ((rc = upload(h, &prows, rf.data(), rf.size(), st))) return rc;
+    cudaStreamSynchronize(st);  // rf leaves scope
+  }
+  h->pg = PxGeom<float>{padjs, padjf, md, rdet, prows};
   const int FW = h->order <= 2 ? MX_XF : 5;
   float *xf, *pfm = nullptr, *jm;
   const size_t ns = h->slots.n;
@@ -1003,8 +1110,8 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
       k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv, nsrows, invs32);
     }
     if (h->px) {
-      k_px_planes<<<(unsigned)((NP * h->Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, h->Fn, padjf);
-      k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, S, padjs);
+      k_px_planes<<<(unsigned)((NP * h->Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, h->Fn, 1, padjf);
+      k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, S, 1, padjs);
     }
     k_mx_rdet<<<(unsigned)((N * (size_t)S + 255) / 256), 256, 0, st>>>(h->g.det, N * (size_t)S, rdet);
     cudaError_t r = cudaGetLastError();
@@ -1087,18 +1194,11 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   if ((tcr || h->px_points) && (rc = dalloc(h, &pfm, N * S * MX_PF))) return rc;
   h->mb.PFm = pfm;
   h->prec = AFR_PREC_MIXED;
-  // The FP64 fine-point adjugates were needed only for MD and the FP32 copy;
-  // the FP64 solution-point adjugates only for the set-up and the SST kernels.
-  auto release = [&](const double*& p, size_t n) {
-    auto it = std::find(h->allocs.begin(), h->allocs.end(), (void*)p);
-    if (it == h->allocs.end()) return;
-    h->allocs.erase(it);
-    cudaFree((void*)p);
-    h->bytes -= n * sizeof(double);
-    p = nullptr;
-  };
+  // The FP64 adjugates were needed only for MD, the slot rows and the FP32
+  // copies.
+  auto release = [&](const double*& p, size_t n) { release_alloc(h, p, n); };
   release(h->g.adj_fine, N * (size_t)h->Fn * 9);
-  if (h->prm.turb != AFR_TURB_SST) release(h->g.adj, N * (size_t)S * 9);
+  release(h->g.adj, N * (size_t)S * 9);
   // The dense per-record interpolation matrices are read afterwards only by
   // the general (unmatched) face points and by the SST face kernel: release
   // them when neither exists.
@@ -1535,7 +1635,7 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     cudaStreamSynchronize(st);
     h->slots = SlotTable{(int32_t)ns, d_f, d_c, d_fl, d_0, d_1, d_i1};
     // FP64 jumps: the plain stage of orders 1-3 only
-    if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = dalloc(h, &h->J, ns * P * 10))) return bail(rc);
+    if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = dalloc(h, &h->J, ns * P * 9))) return bail(rc);
   }
   // ---- boundary condition table ----
   {
@@ -1600,6 +1700,7 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     if ((rc = dalloc(h, &h->sp8, N * S * 8))) return bail(rc);
   }
   if (prm->precision == AFR_PREC_MIXED && (rc = mixed_setup(h, m, Wkeep, st))) return bail(rc);
+  if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = plain_setup(h, st))) return bail(rc);
   if (h->order == 0 && (rc = p0_setup(h, m, st))) return bail(rc);
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return bail(cuda_fail(h, e, "afr_create"));

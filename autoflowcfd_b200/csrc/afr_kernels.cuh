@@ -19,7 +19,7 @@ struct StageArgs {
   const double* U0;     // step-start state (RK combination)
   const double* U1;     // stage-1 state (RK stage 2 combination)
   double* Unext;        // output state (N,S,nv)
-  const double* PF;     // (N,S,18) point fields of Ucur (k_pre)
+  const double* PF;     // (N,S,16) point fields of Ucur (k_pre)
   const double* nut;    // (N,S) kinematic eddy viscosity or null
   const double* dt;     // (N,S)
   double* Rinv;         // residual-only mode outputs (N,S,nv), may be null
@@ -258,12 +258,14 @@ __device__ void suppress_outliers_cells(double* sRi, double* sRv, const double* 
 }
 
 // ---------------------------------------------------------------------------
-// per-point pre-pass: PF (N,S,18) = primitive q(5) (no pressure floor,
-// core/fr_residual/inviscid.py:38-47), grads of u,v,w (9) and T (3)
+// per-point pre-pass: PF (N,S,16) = primitive q(5) (no pressure floor,
+// core/fr_residual/inviscid.py:38-47), symmetric velocity gradient (6: the
+// viscous flux holds no other combination) and grad T (3)
 // (core/fr_operators/gradients.py:23-64 as used by
-// core/fr_residual/viscous_flux.py:161-166), mu_t = max(rho,1e-10) * nu_t (1)
+// core/fr_residual/viscous_flux.py:161-166), mu_t = max(rho,1e-10) * nu_t (1),
+// one unused (128-byte rows)
 // ---------------------------------------------------------------------------
-constexpr int PFW = 18;
+constexpr int PFW = 16;
 
 template <int S>
 struct PreTile {
@@ -292,7 +294,8 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
     cons_to_prim(u, q);
     double* o = sPF + t * PFW;
     for (int v = 0; v < 5; ++v) o[v] = q[v];
-    o[17] = nut ? fmax(u[0], 1e-10) * nut[p] : 0.0;
+    o[15] = 0.0;
+    o[14] = nut ? fmax(u[0], 1e-10) * nut[p] : 0.0;
     f[t * 4 + 0] = q[1];
     f[t * 4 + 1] = q[2];
     f[t * 4 + 2] = q[3];
@@ -308,15 +311,27 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
       double inv[9];
       const double* ip = g.inv + ((size_t)e0 * S + t) * 9;
       for (int k = 0; k < 9; ++k) inv[k] = __ldg(ip + k);
-      for (int c = 0; c < 12; ++c) {
-        const int q = c / 3, n = c % 3;  // c = q*3+n: q in (u,v,w,T)
-        double acc = 0.0;
-        for (int m = 0; m < 3; ++m) acc += gc[(t * 3 + m) * 4 + q] * inv[m * 3 + n];
-        sPF[t * PFW + 5 + c] = acc;
+      double gr[4][3];  // rows u, v, w, T
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          double acc = 0.0;
+          for (int m = 0; m < 3; ++m) acc += gc[(t * 3 + m) * 4 + q] * inv[m * 3 + n];
+          gr[q][n] = acc;
+        }
+      double* o = sPF + t * PFW + 5;
+#pragma unroll
+      for (int n = 0; n < 3; ++n) {
+        o[n] = gr[n][n];
+        o[6 + n] = gr[3][n];
       }
+      o[3] = 0.5 * (gr[0][1] + gr[1][0]);
+      o[4] = 0.5 * (gr[0][2] + gr[2][0]);
+      o[5] = 0.5 * (gr[1][2] + gr[2][1]);
     }
   } else {
-    for (int t = threadIdx.x; t < nc * S * 12; t += blockDim.x) sPF[(t / 12) * PFW + 5 + t % 12] = 0.0;
+    for (int t = threadIdx.x; t < nc * S * 9; t += blockDim.x) sPF[(t / 9) * PFW + 5 + t % 9] = 0.0;
   }
   __syncthreads();
   double* out = PF + (size_t)e0 * S * PFW;
@@ -328,7 +343,7 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
 // face record whose own extrapolation + correction lifting lands on a cell
 // (core/fr_residual/inviscid_kernel_colored.py:86-157 owner side, :159-236
 // neighbour side; core/fr_residual/viscous_flux_kernel.py:335-520).  Writes
-// the inviscid and viscous flux jumps J (n_slots, NP, 10).
+// the inviscid and viscous flux jumps J (n_slots, 9, NP).
 // Slot flags: bit0 neighbour side, bit1 boundary face, bits2-3 axis, bit4 side>0.
 // ---------------------------------------------------------------------------
 struct SlotTable {
@@ -430,29 +445,30 @@ __device__ __forceinline__ void dmma_warp_rb_f(int M, int N, const double* __res
 // Face kernel: one warp per group of SPW = 32 / NP slots (a slot is one side
 // of one face record whose correction lifts into a cell; lane = slot-in-group
 // * NP + flux point in the flux phase).  Per slot, the own side's
-// extrapolation E * [q, adjugate row of the face's axis, grads, mu_t] and the
+// extrapolation E * [q, grads, mu_t] and the
 // other side's interpolation M_src0 * [q, grads, mu_t] (+ M_src1 * ...) are
 // FP64 tensor-core products into the warp's shared rows; the lanes then form
 // the ghost state, AUSM+up with the alignment fallback and the BR1 common
 // flux with the boundary penalty
 // (core/fr_residual/inviscid_kernel_colored.py:86-236,
 // core/fr_residual/viscous_flux_kernel.py:335-520) and write the jumps
-// J (n_slots, NP, 10).  A weight of zero contributes nothing to the products
+// J (n_slots, 9, NP: inviscid 5, viscous momentum and energy 4).  A weight of zero contributes nothing to the products
 // while the state is finite (the reference skips zero weights,
 // inviscid_kernel_colored.py:117-121; a non-finite state makes the step
 // non-finite either way).
 // Slot flags: bit0 neighbour side, bit1 boundary face, bits2-3 axis, bit4 side>0.
 constexpr int FACE_WARPS = 4;
-constexpr int FW_OWN = 21, FW_OTH = 18;  // doubles per face point: own side, other side
+constexpr int FW_F = 15;  // doubles per face point and side
 
 template <int S, int NP>
 __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Faces fc, Bc bc, SlotTable st,
-                                                          const double* __restrict__ PF, double mu, int visc,
+                                                          const double* __restrict__ PF,
+                                                          const double4* __restrict__ arow, double mu, int visc,
                                                           double* __restrict__ J) {
   constexpr int SPW = 32 / NP;  // slots per warp
   constexpr int MT = (NP + 7) / 8;  // row tiles of the face points
-  __shared__ double sOw[FACE_WARPS][SPW * NP * FW_OWN];
-  __shared__ double sOt[FACE_WARPS][SPW * NP * FW_OTH];
+  __shared__ double sOw[FACE_WARPS][SPW * NP * FW_F];
+  __shared__ double sOt[FACE_WARPS][SPW * NP * FW_F];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sl0 = (blockIdx.x * FACE_WARPS + warp) * SPW;
   if (sl0 >= st.n) return;  // whole warps leave together
@@ -469,27 +485,24 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
     const int ax = (fl >> 2) & 3;
     const int sb = (fl & 16) ? 1 : 0;
     const int ct = cell_type(g, e);
-    // own side: rows face points, columns [q(5), adj row(3), grads + mu_t(13)]
+    // own side: rows face points, columns [q(5), grads + mu_t(10)]
     const double* Ef = ops.fextrap + (((size_t)ct * 3 + ax) * 2 + sb) * (MT * ((S + 3) / 4) * 32);
     const double* pf = PF + (size_t)e * S * PFW;
-    const double* ad = g.adj + (size_t)e * S * 9 + ax * 3;
-    double* ow = ow_s + j * NP * FW_OWN;
+    double* ow = ow_s + j * NP * FW_F;
     {
-      auto fb = [&](int s, int n) {
-        return n < 5 ? __ldg(pf + s * PFW + n) : (n < 8 ? __ldg(ad + s * 9 + (n - 5)) : __ldg(pf + s * PFW + n - 3));
-      };
-      auto fc_ = [&](int i, int n, double x) { ow[i * FW_OWN + n] = x; };
-      if (visc) dmma_warp_rb_f<MT, 3, S>(NP, FW_OWN, Ef, fb, fc_);
-      else dmma_warp_rb_f<MT, 1, S>(NP, 8, Ef, fb, fc_);  // columns 8.. are not read without viscosity
+      auto fb = [&](int s, int n) { return __ldg(pf + s * PFW + n); };
+      auto fc_ = [&](int i, int n, double x) { ow[i * FW_F + n] = x; };
+      if (visc) dmma_warp_rb_f<MT, 2, S>(NP, FW_F, Ef, fb, fc_);
+      else dmma_warp_rb_f<MT, 1, S>(NP, 5, Ef, fb, fc_);  // columns 5.. are not read without viscosity
     }
     // other side: the interpolation sources (the first, then the second added)
-    double* ot = ot_s + j * NP * FW_OTH;
+    double* ot = ot_s + j * NP * FW_F;
     if (!bnd) {
       for (int src = 0; src < 2; ++src) {
         const int c = src == 0 ? st.c0[sl] : st.c1[sl];
         if (c < 0) {
           if (src == 0)
-            for (int t = lane; t < NP * FW_OTH; t += 32) ot[t] = 0.0;
+            for (int t = lane; t < NP * FW_F; t += 32) ot[t] = 0.0;
           continue;
         }
         const double* M = src == 0 ? (is_owner ? fmat(fc.nb_m0, fc.nb_m0i, f, 0, NP, S)
@@ -501,10 +514,10 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
         auto fa = [&](int i, int s) { return __ldg(M + s * NP + i); };
         auto fb = [&](int s, int n) { return __ldg(pc + s * PFW + n); };
         auto fc_ = [&](int i, int n, double x) {
-          if (src == 0) ot[i * FW_OTH + n] = x;
-          else ot[i * FW_OTH + n] += x;
+          if (src == 0) ot[i * FW_F + n] = x;
+          else ot[i * FW_F + n] += x;
         };
-        if (visc) dmma_warp_rb<MT, 3, S>(NP, FW_OTH, fa, fb, fc_);
+        if (visc) dmma_warp_rb<MT, 2, S>(NP, FW_F, fa, fb, fc_);
         else dmma_warp_rb<MT, 1, S>(NP, 5, fa, fb, fc_);  // columns 5.. are not read without viscosity
       }
     }
@@ -520,43 +533,46 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
   const bool is_owner = (fl & 1) == 0;
   const bool bnd = (fl & 2) != 0;
   const double side = (fl & 16) ? 1.0 : -1.0;
-  double ow[21], ot[18];
+  double ow[FW_F], ot[FW_F];
 #pragma unroll
-  for (int k = 0; k < 21; ++k) ow[k] = (k < 8 || visc) ? ow_s[(j * NP + i) * FW_OWN + k] : 0.0;
+  for (int k = 0; k < FW_F; ++k) ow[k] = (k < 5 || visc) ? ow_s[(j * NP + i) * FW_F + k] : 0.0;
   const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
   if (bnd) {
-    double qo[5], n[3], gq[5];
-    for (int v = 0; v < 5; ++v) qo[v] = ow[v];
+    double n[3], gq[5];
     for (int d = 0; d < 3; ++d) n[d] = tn[d];
-    ghost_state(bc, fc.bc_group[f], qo, n, gq);
+    ghost_state(bc, fc.bc_group[f], ow, n, gq);
     for (int v = 0; v < 5; ++v) ot[v] = gq[v];
-    for (int k = 0; k < 13; ++k) ot[5 + k] = ow[8 + k];
+    for (int k = 5; k < FW_F; ++k) ot[k] = ow[k];
   } else {
 #pragma unroll
-    for (int k = 0; k < 18; ++k) ot[k] = (k < 5 || visc) ? ot_s[(j * NP + i) * FW_OTH + k] : 0.0;
+    for (int k = 0; k < FW_F; ++k) ot[k] = (k < 5 || visc) ? ot_s[(j * NP + i) * FW_F + k] : 0.0;
   }
-  // pointwise fluxes
-  const double a0 = ow[5], a1 = ow[6], a2 = ow[7];
-  double mag = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
-  if (mag < 1e-300) mag = 1e-300;
+  // pointwise fluxes; the own adjugate row and its norm are geometry, formed at
+  // create (a negative norm marks the alignment fallback)
+  const double4 ar = arow[(size_t)sl * NP + i];
+  const double a0 = ar.x, a1 = ar.y, a2 = ar.z;
+  const double mag = fabs(ar.w);
   double dir[3] = {a0 / mag * side, a1 / mag * side, a2 / mag * side};
-  const double sg = is_owner ? 1.0 : -1.0;
-  const double t0 = sg * tn[0], t1 = sg * tn[1], t2 = sg * tn[2];
-  if (dir[0] * t0 + dir[1] * t1 + dir[2] * t2 < 0.5) { dir[0] = t0; dir[1] = t1; dir[2] = t2; }
+  if (ar.w < 0.0) {
+    const double sg = is_owner ? 1.0 : -1.0;
+    dir[0] = sg * tn[0];
+    dir[1] = sg * tn[1];
+    dir[2] = sg * tn[2];
+  }
   double Fc[5], Fp[3][5];
   ausm_up(ow, ot, dir, Fc);
   euler_flux(ow, Fp);
-  double* Jo = J + ((size_t)sl * NP + i) * 10;
-  for (int v = 0; v < 5; ++v) Jo[v] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
+  double* Jo = J + (size_t)sl * 9 * NP + i;
+  for (int v = 0; v < 5; ++v) Jo[v * NP] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
   if (visc) {
-    double qa[5], ga[13];
-    for (int v = 0; v < 5; ++v) qa[v] = 0.5 * (ow[v] + ot[v]);
-    for (int k = 0; k < 13; ++k) ga[k] = 0.5 * (ow[8 + k] + ot[5 + k]);
-    double Gc[3][5], Go[3][5];
-    viscous_flux(qa, ga, ga + 9, mu, ga[12], Gc);
-    viscous_flux(ow, ow + 8, ow + 17, mu, ow[20], Go);
-    double jv[5];
-    for (int v = 0; v < 5; ++v)
+    double av[FW_F];  // the common flux: both sides' averages
+#pragma unroll
+    for (int k = 1; k < FW_F; ++k) av[k] = 0.5 * (ow[k] + ot[k]);
+    double Gc[3][4], Go[3][4];
+    viscous_flux_sym(av + 1, av + 5, av + 11, mu, av[14], Gc);
+    viscous_flux_sym(ow + 1, ow + 5, ow + 11, mu, ow[14], Go);
+    double jv[4];
+    for (int v = 0; v < 4; ++v)
       jv[v] = (a0 * Gc[0][v] + a1 * Gc[1][v] + a2 * Gc[2][v]) - (a0 * Go[0][v] + a1 * Go[1][v] + a2 * Go[2][v]);
     if (bnd) {
       // interior-penalty term on boundary faces (core/fr_operators/flux_kernels.py:140-200);
@@ -566,12 +582,39 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
       vol_o /= S;
       double h = pow(vol_o, 1.0 / 3.0);
       if (h < 1e-300) h = 1e-300;
-      const double eta = C_IP * (mu + ow[20]) / h;
+      const double eta = C_IP * (mu + ow[14]) / h;
       const double scale = eta * sqrt(a0 * a0 + a1 * a1 + a2 * a2) * side;
-      for (int v = 1; v < 4; ++v) jv[v] += -scale * (ow[v] - ot[v]);
+      for (int v = 0; v < 3; ++v) jv[v] += -scale * (ow[1 + v] - ot[1 + v]);
     }
-    for (int v = 0; v < 5; ++v) Jo[5 + v] = jv[v];
+    for (int v = 0; v < 4; ++v) Jo[(5 + v) * NP] = jv[v];
   }
+}
+
+// own adjugate row of the face's axis at every slot flux point (E * adj) and
+// its norm, negative where the row's direction falls back to the face normal
+// (alignment below 0.5, core/fr_residual/inviscid_kernel_colored.py:104-108)
+template <int S, int NP>
+__global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __restrict__ arow) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)st.n * NP) return;
+  const int sl = (int)(t / NP), i = (int)(t % NP);
+  const int f = st.face[sl], e = st.cell[sl], fl = st.flags[sl];
+  const int ax = (fl >> 2) & 3, sb = (fl & 16) ? 1 : 0;
+  const double* Er = ops.extrap + ((((size_t)cell_type(g, e) * 3 + ax) * 2 + sb) * NP + i) * S;
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+  for (int s = 0; s < S; ++s) {
+    const double w = Er[s];
+    const double* ad = g.adj + ((size_t)e * S + s) * 9 + ax * 3;
+    a0 += w * ad[0];
+    a1 += w * ad[1];
+    a2 += w * ad[2];
+  }
+  double mag = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
+  if (mag < 1e-300) mag = 1e-300;
+  const double side = sb ? 1.0 : -1.0, sg = (fl & 1) == 0 ? 1.0 : -1.0;
+  const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
+  const double al = a0 / mag * side * (sg * tn[0]) + a1 / mag * side * (sg * tn[1]) + a2 / mag * side * (sg * tn[2]);
+  arow[t] = make_double4(a0, a1, a2, al < 0.5 ? -mag : mag);
 }
 
 // ---------------------------------------------------------------------------
@@ -587,7 +630,7 @@ constexpr int CELL_MAXSLOT = 6;  // slots per cell staged in shared memory (more
 
 template <int S, int FN, int CPB, int NPMAX>
 struct CellSmem {
-  static constexpr int oPF = 0;                    // CPB*S*18
+  static constexpr int oPF = 0;                    // CPB*S*16
   static constexpr int oAdj = oPF + CPB * S * PFW; // CPB*S*9
   static constexpr int oU = oAdj + CPB * S * 9;    // CPB*S*US
   static constexpr int oDet = oU + CPB * S * US;    // CPB*S
@@ -597,7 +640,7 @@ struct CellSmem {
   static constexpr int oFt = oQf + CPB * FN * 5;   // CPB*FN*15
   static constexpr int oGt = oFt + CPB * FN * 15;  // CPB*S*15
   static constexpr int oJ = oGt + CPB * S * 15;    // staged jumps of the CTA's slots
-  static constexpr int oWp = oJ + CPB * CELL_MAXSLOT * NPMAX * 10;  // 2 halves of the W divergence
+  static constexpr int oWp = oJ + CPB * CELL_MAXSLOT * NPMAX * 9;  // 2 halves of the W divergence
   static constexpr int oAf = oWp + 2 * CPB * S * 5;  // CPB*FN*9 adjugates at the fine points
   static constexpr int work = oAf + CPB * FN * 9;     // CPB*2*OUT_WORK (outliers) + 32
   static constexpr int total = work + CPB * 2 * OUT_WORK + 32;
@@ -638,8 +681,8 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   const bool staged = (k_end - k_beg) <= CPB * CELL_MAXSLOT;
   double* sJ = sm + L::oJ;
   if (staged)
-    for (int t = tid; t < (k_end - k_beg) * NP * 10; t += blockDim.x)
-      cp_async8(sJ + t, J + (size_t)k_beg * NP * 10 + t);
+    for (int t = tid; t < (k_end - k_beg) * NP * 9; t += blockDim.x)
+      cp_async8(sJ + t, J + (size_t)k_beg * NP * 9 + t);
   cp_async_wait_all();
   __syncthreads();
 
@@ -653,14 +696,15 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   }
   if (visc) {
     for (int t = tid; t < nc * S; t += blockDim.x) {
-      double q[5], G[3][5];
+      double G[3][4];
       const double* p = sPF + t * PFW;
-      for (int v = 0; v < 5; ++v) q[v] = p[v];
-      viscous_flux(q, p + 5, p + 14, a.mu, p[17], G);
+      viscous_flux_sym(p + 1, p + 5, p + 11, a.mu, p[14], G);
       const double* am = sAdj + t * 9;
-      for (int m = 0; m < 3; ++m)
-        for (int v = 0; v < 5; ++v)
-          sGt[(t * 3 + m) * 5 + v] = am[m * 3 + 0] * G[0][v] + am[m * 3 + 1] * G[1][v] + am[m * 3 + 2] * G[2][v];
+      for (int m = 0; m < 3; ++m) {
+        sGt[(t * 3 + m) * 5] = 0.0;
+        for (int v = 0; v < 4; ++v)
+          sGt[(t * 3 + m) * 5 + 1 + v] = am[m * 3 + 0] * G[0][v] + am[m * 3 + 1] * G[1][v] + am[m * 3 + 2] * G[2][v];
+      }
     }
   }
   __syncthreads();
@@ -711,9 +755,9 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
       const int ax = (fl >> 2) & 3;
       const int fp = ops.dist_fp[ax * S + s];
       const double gw = ((fl & 16) ? ops.g_right : ops.g_left)[ops.dist_co[ax * S + s]];
-      const double* Jk = staged ? sJ + ((k - k_beg) * NP + fp) * 10 : J + ((size_t)k * NP + fp) * 10;
-      ci += -(gw * Jk[v]) * rdj;
-      if (visc) cv += (gw * Jk[5 + v]) * rdj;
+      const double* Jk = staged ? sJ + (k - k_beg) * 9 * NP + fp : J + (size_t)k * 9 * NP + fp;
+      ci += -(gw * Jk[v * NP]) * rdj;
+      if (visc && v > 0) cv += (gw * Jk[(4 + v) * NP]) * rdj;
     }
     sRi[t] = sRi[t] + ci;
     if (visc) sRv[t] = sRv[t] + cv;

@@ -20,7 +20,7 @@
 //              cells' FP32 point fields with the reference's matrices;
 //   k_mx_vol   per C-cell tile (persistent): c2f, viscous D_3d and the folded
 //              W = f2c*D_fine divergence as GEMMs -> volume terms (FP32);
-//   k_mx_update a warp per few cells: lifting in ascending color order, outlier
+//   k_update a warp per few cells: lifting in ascending color order, outlier
 //              zeroing, SSP-RK3 combination, positivity (FP64), filter (an
 //              FP64 product on the tensor path).
 //
@@ -210,24 +210,25 @@ __device__ __forceinline__ void cell_point(int idx, int npts, int& c, int& p) {
 
 // F(qbar + dq) - F(qbar) for the Euler flux, written as telescoped products so
 // that no large terms cancel (qbar, dq primitive: rho, u, v, w, p).
-__device__ __forceinline__ void euler_flux_delta(const float qb[5], const float dq[5], float dF[3][5]) {
-  const float rb = qb[0], dr = dq[0], dp = dq[4];
-  const float ub[3] = {qb[1], qb[2], qb[3]}, du[3] = {dq[1], dq[2], dq[3]};
-  const float u[3] = {ub[0] + du[0], ub[1] + du[1], ub[2] + du[2]};
-  const float g1 = float(GAMMA / (GAMMA - 1.0));
-  const float uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-  const float d_uu = (u[0] + ub[0]) * du[0] + (u[1] + ub[1]) * du[1] + (u[2] + ub[2]) * du[2];
-  const float p = qb[4] + dp;
-  const float r = rb + dr;
-  const float e = g1 * p + 0.5f * r * uu;                 // rho H
-  const float de = g1 * dp + 0.5f * (dr * uu + rb * d_uu);
+template <class T>
+__device__ __forceinline__ void euler_flux_delta(const T qb[5], const T dq[5], T dF[3][5]) {
+  const T rb = qb[0], dr = dq[0], dp = dq[4];
+  const T ub[3] = {qb[1], qb[2], qb[3]}, du[3] = {dq[1], dq[2], dq[3]};
+  const T u[3] = {ub[0] + du[0], ub[1] + du[1], ub[2] + du[2]};
+  const T g1 = T(GAMMA / (GAMMA - 1.0));
+  const T uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+  const T d_uu = (u[0] + ub[0]) * du[0] + (u[1] + ub[1]) * du[1] + (u[2] + ub[2]) * du[2];
+  const T p = qb[4] + dp;
+  const T r = rb + dr;
+  const T e = g1 * p + T(0.5) * r * uu;                 // rho H
+  const T de = g1 * dp + T(0.5) * (dr * uu + rb * d_uu);
 #pragma unroll
   for (int n = 0; n < 3; ++n) {
-    const float dm = dr * u[n] + rb * du[n];              // delta(rho u_n)
-    const float mb = rb * ub[n];
+    const T dm = dr * u[n] + rb * du[n];              // delta(rho u_n)
+    const T mb = rb * ub[n];
     dF[n][0] = dm;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) dF[n][1 + j] = dm * u[j] + mb * du[j] + (n == j ? dp : 0.f);
+    for (int j = 0; j < 3; ++j) dF[n][1 + j] = dm * u[j] + mb * du[j] + (n == j ? dp : T(0));
     dF[n][4] = du[n] * e + ub[n] * de;
   }
 }
@@ -1147,10 +1148,11 @@ __device__ __noinline__ Vals<PL> outlier_exact(Vals<PL> X, Vals<PL> u, int grp, 
 }
 }  // namespace mxd
 
-template <int S, int NP>
-__global__ void __launch_bounds__(128, S == 64 ? 3 : 5)
-    k_mx_update(Ops ops, Faces fc, StageArgs a, int ct, const float* __restrict__ RV, const float* __restrict__ Jm,
-                const double* __restrict__ rdet) {
+// T: float (mixed form) or double (plain form of structured prisms).
+template <int S, int NP, class T>
+__global__ void __launch_bounds__(128, S == 64 || sizeof(T) == 8 ? 3 : 5)
+    k_update(Ops ops, Faces fc, StageArgs a, int ct, const T* __restrict__ RV, const T* __restrict__ Jm,
+             const double* __restrict__ rdet) {
   using L = MxUpd<S>;
   constexpr int PL = L::PL, CPR = L::CPR, CW = L::CW, PR = L::PR;
   extern __shared__ __align__(16) uint8_t smb[];
@@ -1206,20 +1208,20 @@ __global__ void __launch_bounds__(128, S == 64 ? 3 : 5)
       for (int l = 0; l < PL; ++l) cx[v][l] = 0.0;
     const int k0 = __shfl_sync(0xffffffffu, ptr, c < nc ? c : 0);
     const int n = __shfl_sync(0xffffffffu, ptr, (c < nc ? c : 0) + 1) - k0;
-    float rv[9][PL];
+    T rv[9][PL];
 #pragma unroll
     for (int l = 0; l < PL; ++l) {
       rd[l] = __ldg(rdet + (size_t)e * S + sp + 32 * l);
 #pragma unroll
       for (int v = 0; v < 9; ++v)
-        rv[v][l] = v < 5 || visc ? __ldg(RV + ((size_t)e * 9 + v) * S + sp + 32 * l) : 0.f;
+        rv[v][l] = v < 5 || visc ? __ldg(RV + ((size_t)e * 9 + v) * S + sp + 32 * l) : T(0);
     }
     // jumps of the cell's slots, ascending color order
     if (flags_held && __all_sync(0xffffffffu, n == MX_UPD_SLOTS)) {
       // five slots, as every prism has: all loads of a point in flight at once
 #pragma unroll
       for (int l = 0; l < PL; ++l) {
-        float jv[MX_UPD_SLOTS][9];
+        T jv[MX_UPD_SLOTS][9];
         int gi[MX_UPD_SLOTS];
 #pragma unroll
         for (int j = 0; j < MX_UPD_SLOTS; ++j) {
@@ -1231,9 +1233,9 @@ __global__ void __launch_bounds__(128, S == 64 ? 3 : 5)
           }
           const int as = ((f >> 2) & 3) * S + sp + 32 * l;
           gi[j] = ((f & 16) ? 3 * S : 0) + as;
-          const float* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
+          const T* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
 #pragma unroll
-          for (int v = 0; v < 9; ++v) jv[j][v] = v < 5 || visc ? __ldg(Jk + v * NP) : 0.f;
+          for (int v = 0; v < 9; ++v) jv[j][v] = v < 5 || visc ? __ldg(Jk + v * NP) : T(0);
         }
 #pragma unroll
         for (int j = 0; j < MX_UPD_SLOTS; ++j) {
@@ -1249,7 +1251,7 @@ __global__ void __launch_bounds__(128, S == 64 ? 3 : 5)
         for (int l = 0; l < PL; ++l) {
           const int as = ((f >> 2) & 3) * S + sp + 32 * l;
           const double gw = sG[((f & 16) ? 3 * S : 0) + as];
-          const float* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
+          const T* Jk = Jm + (size_t)(k0 + j) * 9 * NP + sFp[as];
 #pragma unroll
           for (int v = 0; v < 9; ++v)
             if (v < 5 || visc) cx[v][l] += gw * double(__ldg(Jk + v * NP));

@@ -47,42 +47,75 @@ struct PxOps {
 };
 
 // per-cell metrics in the order the lanes read them
+template <class T>
 struct PxGeom {
-  const float* adjs;   // (N, 9, S) solution-point adjugates, entry m*3 + n
-  const float* adjf;   // (N, 9, MT, NF) fine-point adjugates, fine point = triangle point * NF + c-level
+  const T* adjs;       // (N, 9, S) solution-point adjugates, entry m*3 + n
+  // fine-point adjugates (fine point = triangle point * NF + c-level): FP32
+  // (N, 9, MT, NF), a lane's c-line in one vector; FP64 (N, NF, 9, MT), level by level
+  const T* adjf;
   const double* MD;    // (N, S, 3)
   const double* rdet;  // (N, S)
+  const T* rows;       // derivative rows of the points, see px_rows
 };
 
-template <int N1, int NF, int CW>
+template <class T>
+struct alignas(4 * sizeof(T)) Vec4 {
+  T x, y, z, w;
+};
+template <class T>
+struct alignas(16) VecN {  // 16 bytes
+  static constexpr int N = 16 / sizeof(T);
+  T v[N];
+};
+
+template <class T, int N1, int NF, int CW>
 struct PxSmem {
+  static constexpr bool D = sizeof(T) == 8;
   static constexpr int S = N1 * N1 * N1, NT = N1 * N1, MT = NF * NF;
-  static constexpr int TP = MT == 16 ? 20 : 12;  // triangle row stride: 16-byte rows on distinct banks
+  // triangle row stride: 16-byte rows on distinct banks
+  static constexpr int TP = D ? (MT == 16 ? 18 : 10) : (MT == 16 ? 20 : 12);
   static constexpr int FS = S | 1;               // field row stride (odd)
-  static constexpr int nH = 15 * N1 * TP;        // c-contracted fluxes; before: state, gradient inputs, fluxes; face fields
+  static constexpr int oDev = 64 * S / sizeof(T), oG = oDev + 4 * S;  // inside H, after the staged state (8 doubles per point)
+  static constexpr int need = D ? oG + 12 * S : cmax(oG + 12 * S, 6 * MX_XF * NT);
+  // c-contracted fluxes; before: state, gradient inputs, viscous fluxes; FP32: face fields
+  static constexpr int nH = cmax(15 * N1 * TP, need);
   static constexpr int nX = MX_XF * FS, nY = 5 * N1 * TP;
-  static constexpr int oX = nH, oY = (oX + nX + 3) / 4 * 4, oRef = oY + nY, oF = oRef + 8;
-  static constexpr int cell = (oF + 30 + 3) / 4 * 4;  // floats per cell
-  static constexpr int oDev = 16 * S, oG = oDev + 4 * S;  // inside H, after the staged state (8 doubles per point)
-  static_assert(oG + 12 * S <= nH && 6 * MX_XF * NT <= nH, "phases share the H block");
-  static constexpr int total = PX_WARPS * CW * cell * 4;
+  static constexpr int oX = (nH + 3) / 4 * 4, oY = (oX + nX + 3) / 4 * 4, oRef = oY + nY, oF = oRef + 8;
+  static constexpr int cell = (oF + 120 / (int)sizeof(T) + 3) / 4 * 4;  // T values per cell
+  static constexpr int total = PX_WARPS * CW * cell * (int)sizeof(T);
 };
 
-template <int N1, int NF, int CW, bool VISC>
-__global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
-    k_px_cell(const __grid_constant__ PxOps<float, N1, NF> op, PxGeom pg, float* __restrict__ XF, float* __restrict__ PFm,
-              float* __restrict__ RV, int FW, unsigned face_mask, const double* __restrict__ U, int nv,
-              const double* __restrict__ nut, float mu, int cell_base, int cell_end) {
-  using L = PxSmem<N1, NF, CW>;
+// rho H of the Euler flux, rho * (p / (0.4 max(rho, 1e-10)) + |u|^2 / 2) + p over
+// max(rho, 1e-10) times rho (core/fr_operators/flux_kernels.py:28-68)
+__device__ __forceinline__ double px_rhoH(double rho, double p, double u2) {
+  if (rho >= 1e-10) return GAMMA / (GAMMA - 1.0) * p + 0.5 * rho * u2;
+  const double rs = 1e-10;
+  const double rhoE = rho * (p / ((GAMMA - 1.0) * rs) + 0.5 * u2);
+  return rho * ((rhoE + p) / rs);
+}
+
+// T = float: the mixed form (face-point fields XF by extrapolation, point
+// fields PF only where a face point interpolates from them).  T = double: the
+// plain form; it writes the point fields, from which k_face extrapolates and
+// interpolates with every entry of the mesh's own operators.
+template <class T, int N1, int NF, int CW, bool VISC>
+__global__ void __launch_bounds__(32 * PX_WARPS, sizeof(T) == 8 ? 2 : (N1 == 3 ? 4 : 3))
+    k_px_cell(const __grid_constant__ PxOps<T, N1, NF> op, PxGeom<T> pg, float* __restrict__ XF, T* __restrict__ PF,
+              T* __restrict__ RV, int FW, unsigned face_mask, const double* __restrict__ U, int nv,
+              const double* __restrict__ nut, T mu, int cell_base, int cell_end) {
+  using L = PxSmem<T, N1, NF, CW>;
+  constexpr bool D = sizeof(T) == 8;
   constexpr int S = L::S, NT = L::NT, MT = L::MT, TP = L::TP, FS = L::FS, NP = NT;
   constexpr int CPR = 32 / S;                 // cells per round of the point phases
   constexpr int PR = (CW + CPR - 1) / CPR;    // rounds
-  extern __shared__ __align__(16) float smf[];
+  constexpr int VN = VecN<T>::N;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* smf = reinterpret_cast<T*>(smraw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int e0 = cell_base + (blockIdx.x * PX_WARPS + warp) * CW;
   const int nc = min(CW, cell_end - e0);
   if (nc <= 0) return;  // whole warps; no block barrier below
-  float* sw = smf + warp * CW * L::cell;
+  T* sw = smf + warp * CW * L::cell;
   // point lanes: the same solution point every round
   const int s = lane % S, pc = lane / S;
   const int tri = s / N1, cc = s % N1;
@@ -99,76 +132,79 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
   __syncwarp();
 
   // ---- primitives; deviations from the cell's reference point ----
-  float uf[PR][3], mut[PR];
+  T uf[PR][3], mut[PR];
 #pragma unroll
   for (int r = 0; r < PR; ++r) {
     const int c = r * CPR + pc;
     const bool in = pc < CPR && c < CW;
-    float* sc = sw + (in ? c : 0) * L::cell;
+    T* sc = sw + (in ? c : 0) * L::cell;
     double q[6] = {1.0, 0.0, 0.0, 0.0, 1.0, 1.0};
-    mut[r] = 0.f;
+    mut[r] = T(0);
     if (in && c < nc) {
       const double* d = reinterpret_cast<const double*>(sc);
       mxd::prim_T(d + s * nv, q);
-      if (VISC && nut) mut[r] = float(q[0] * d[7 * S + s]);
+      if (VISC && nut) mut[r] = T(q[0] * d[7 * S + s]);
     }
-    float dev[6];
-    constexpr int MID = S / 2;  // the point whose value is the cell's reference state
+    // FP32: deviations from the value at the cell's middle point, which carry
+    // the variation in 24 bits.  FP64 keeps the values; the reference state
+    // only enters the inviscid flux (below).
+    T dev[6];
+    constexpr int MID = S / 2;
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
       const float ref = __shfl_sync(0xffffffffu, float(q[v]), (pc < CPR ? pc : 0) * S + MID);
-      dev[v] = float(q[v] - double(ref));
-      if (in && s == MID) sc[L::oRef + v] = ref;
+      dev[v] = D ? T(q[v]) : T(q[v] - double(ref));
+      if (in && s == MID) sc[L::oRef + v] = T(ref);
     }
 #pragma unroll
-    for (int d = 0; d < 3; ++d) uf[r][d] = float(q[1 + d]);
+    for (int d = 0; d < 3; ++d) uf[r][d] = T(q[1 + d]);
     if (in) {
 #pragma unroll
       for (int v = 0; v < 5; ++v) sc[L::oX + v * FS + s] = dev[v];
-      if (VISC) *reinterpret_cast<float4*>(sc + L::oDev + 4 * s) = make_float4(dev[1], dev[2], dev[3], dev[5]);
+      if (VISC) *reinterpret_cast<Vec4<T>*>(sc + L::oDev + 4 * s) = Vec4<T>{dev[1], dev[2], dev[3], dev[5]};
     }
-    if (PFm && in && c < nc) {
-      float* o = PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+    if (!D && PF && in && c < nc) {
+      T* o = PF + ((size_t)(e0 + c) * S + s) * MX_PF;
 #pragma unroll
-      for (int v = 0; v < 5; ++v) o[10 + v] = float(q[v]);
+      for (int v = 0; v < 5; ++v) o[10 + v] = T(q[v]);
     }
   }
   __syncwarp();
 
-  float vis[PR][4];
+  T vis[PR][4];
   if constexpr (VISC) {
     // this lane's rows of the derivative operators
-    float d0[N1], d1[NT], d2[N1];
+    T d0[N1], d1[NT], d2[N1];
 #pragma unroll
     for (int l = 0; l < N1; ++l) {
-      d0[l] = op.D0[tri / N1][l];
-      d2[l] = op.D2[cc][l];
+      d0[l] = __ldg(pg.rows + l * S + s);
+      d2[l] = __ldg(pg.rows + (N1 + NT + l) * S + s);
     }
 #pragma unroll
-    for (int t = 0; t < NT; ++t) d1[t] = op.D1[tri][t];
-    float rd[PR];
+    for (int t = 0; t < NT; ++t) d1[t] = __ldg(pg.rows + (N1 + t) * S + s);
+    T rd[PR];
 #pragma unroll
     for (int r = 0; r < PR; ++r) {
       const int c = r * CPR + pc;
       const bool in = pc < CPR && c < CW;
-      float* sc = sw + (in ? c : 0) * L::cell;
-      float aj[9];
-      rd[r] = 0.f;
+      T* sc = sw + (in ? c : 0) * L::cell;
+      T aj[9];
+      rd[r] = T(0);
 #pragma unroll
-      for (int k = 0; k < 9; ++k) aj[k] = 0.f;
+      for (int k = 0; k < 9; ++k) aj[k] = T(0);
       if (in && c < nc) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) aj[k] = __ldg(pg.adjs + ((size_t)(e0 + c) * 9 + k) * S + s);
-        rd[r] = float(__ldg(pg.rdet + (size_t)(e0 + c) * S + s));
+        rd[r] = T(__ldg(pg.rdet + (size_t)(e0 + c) * S + s));
       }
       // reference-space gradients of u, v, w, T
-      const float4* dv = reinterpret_cast<const float4*>(sc + L::oDev);
-      float g[3][4];
+      const Vec4<T>* dv = reinterpret_cast<const Vec4<T>*>(sc + L::oDev);
+      T g[3][4];
 #pragma unroll
       for (int m = 0; m < 3; ++m)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) g[m][f] = 0.f;
-      auto acc = [](float (&o)[4], float w, const float4& x) {
+        for (int f = 0; f < 4; ++f) g[m][f] = T(0);
+      auto acc = [](T (&o)[4], T w, const Vec4<T>& x) {
         o[0] += w * x.x;
         o[1] += w * x.y;
         o[2] += w * x.z;
@@ -182,34 +218,34 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc(g[1], d1[t], dv[t * N1 + cc]);
       // physical gradients: inverse Jacobian = adjugate / det
-      float gr[4][3];
+      T gr[4][3];
 #pragma unroll
       for (int f = 0; f < 4; ++f)
 #pragma unroll
         for (int n = 0; n < 3; ++n)
           gr[f][n] = rd[r] * (g[0][f] * aj[n] + g[1][f] * aj[3 + n] + g[2][f] * aj[6 + n]);
-      const float sym[6] = {gr[0][0], gr[1][1], gr[2][2], 0.5f * (gr[0][1] + gr[1][0]), 0.5f * (gr[0][2] + gr[2][0]),
-                            0.5f * (gr[1][2] + gr[2][1])};
-      float G[3][4];
+      const T sym[6] = {gr[0][0], gr[1][1], gr[2][2], T(0.5) * (gr[0][1] + gr[1][0]), T(0.5) * (gr[0][2] + gr[2][0]),
+                        T(0.5) * (gr[1][2] + gr[2][1])};
+      T G[3][4];
       viscous_flux_sym(uf[r], sym, gr[3], mu, mut[r], G);
       if (in) {
-        float* x = sc + L::oX + 5 * FS + s;
+        T* x = sc + L::oX + 5 * FS + s;
 #pragma unroll
         for (int k = 0; k < 6; ++k) x[k * FS] = sym[k];
 #pragma unroll
         for (int k = 0; k < 3; ++k) x[(6 + k) * FS] = gr[3][k];
         x[9 * FS] = mut[r];
-        float4* gt = reinterpret_cast<float4*>(sc + L::oG);
+        Vec4<T>* gt = reinterpret_cast<Vec4<T>*>(sc + L::oG);
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-          float h[4];
+          T h[4];
 #pragma unroll
           for (int v = 0; v < 4; ++v) h[v] = aj[m * 3] * G[0][v] + aj[m * 3 + 1] * G[1][v] + aj[m * 3 + 2] * G[2][v];
-          gt[m * S + s] = make_float4(h[0], h[1], h[2], h[3]);
+          gt[m * S + s] = Vec4<T>{h[0], h[1], h[2], h[3]};
         }
       }
-      if (PFm && in && c < nc) {
-        float* o = PFm + ((size_t)(e0 + c) * S + s) * MX_PF;
+      if (!D && PF && in && c < nc) {
+        T* o = PF + ((size_t)(e0 + c) * S + s) * MX_PF;
 #pragma unroll
         for (int k = 0; k < 6; ++k) o[k] = sym[k];
 #pragma unroll
@@ -222,10 +258,10 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
 #pragma unroll
     for (int r = 0; r < PR; ++r) {
       const int c = r * CPR + pc;
-      const float* sc = sw + (pc < CPR && c < CW ? c : 0) * L::cell;
-      const float4* gt = reinterpret_cast<const float4*>(sc + L::oG);
-      float o[4] = {0.f, 0.f, 0.f, 0.f};
-      auto acc = [&](float w, const float4& x) {
+      const T* sc = sw + (pc < CPR && c < CW ? c : 0) * L::cell;
+      const Vec4<T>* gt = reinterpret_cast<const Vec4<T>*>(sc + L::oG);
+      T o[4] = {T(0), T(0), T(0), T(0)};
+      auto acc = [&](T w, const Vec4<T>& x) {
         o[0] += w * x.x;
         o[1] += w * x.y;
         o[2] += w * x.z;
@@ -244,56 +280,69 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
     __syncwarp();  // H is reused for the face-point fields
   }
 
-  // ---- extrapolation: one lane per (cell, field), the field in registers ----
-  constexpr int NFL = VISC ? MX_XF : 5;
-  for (int it = lane; it < CW * NFL; it += 32) {
-    const int c = it / NFL, f = it - c * NFL;
-    float* sc = sw + c * L::cell;
-    float x[S];
-    const float* xs = sc + L::oX + f * FS;
-#pragma unroll
-    for (int j = 0; j < S; ++j) x[j] = xs[j];
-    const float base = f < 5 ? sc[L::oRef + f] : 0.f;  // the extrapolation reproduces constants
-    float* o = sc + f * NP;                            // face k's point i at o[k * MX_XF * NP + i]
-#pragma unroll
-    for (int sd = 0; sd < 2; ++sd) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        float a0 = 0.f, a2 = 0.f;
-#pragma unroll
-        for (int l = 0; l < N1; ++l) {
-          a0 += op.E02[0][sd][l] * x[l * NT + i];
-          a2 += op.E02[1][sd][l] * x[i * N1 + l];
-        }
-        o[sd * MX_XF * NP + i] = base + a0;
-        o[(4 + sd) * MX_XF * NP + i] = base + a2;
+  if constexpr (D) {
+    // point fields of the face kernel: one contiguous block of 128-byte rows per cell
+    for (int c = 0; c < nc; ++c) {
+      const T* sc = sw + c * L::cell;
+      T* dst = PF + (size_t)(e0 + c) * S * PFW;
+      for (int t = lane; t < S * PFW; t += 32) {
+        const int j = t / PFW, f = t % PFW;
+        if (f < (VISC ? MX_XF : 5)) dst[t] = sc[L::oX + f * FS + j];
       }
-      if (face_mask >> (2 + sd) & 1) {
+    }
+    __syncwarp();
+  } else {
+    // ---- extrapolation: one lane per (cell, field), the field in registers ----
+    constexpr int NFL = VISC ? MX_XF : 5;
+    for (int it = lane; it < CW * NFL; it += 32) {
+      const int c = it / NFL, f = it - c * NFL;
+      T* sc = sw + c * L::cell;
+      float x[S];
+      const float* xs = sc + L::oX + f * FS;
+#pragma unroll
+      for (int j = 0; j < S; ++j) x[j] = xs[j];
+      const float base = f < 5 ? sc[L::oRef + f] : 0.f;  // the extrapolation reproduces constants
+      float* o = sc + f * NP;                            // face k's point i at o[k * MX_XF * NP + i]
+#pragma unroll
+      for (int sd = 0; sd < 2; ++sd) {
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-          float a1 = 0.f;
+          float a0 = 0.f, a2 = 0.f;
 #pragma unroll
-          for (int t = 0; t < NT; ++t) a1 += op.E1[sd][i / N1][t] * x[t * N1 + i % N1];
-          o[(2 + sd) * MX_XF * NP + i] = base + a1;
+          for (int l = 0; l < N1; ++l) {
+            a0 += op.E02[0][sd][l] * x[l * NT + i];
+            a2 += op.E02[1][sd][l] * x[i * N1 + l];
+          }
+          o[sd * MX_XF * NP + i] = base + a0;
+          o[(4 + sd) * MX_XF * NP + i] = base + a2;
+        }
+        if (face_mask >> (2 + sd) & 1) {
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            float a1 = 0.f;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) a1 += op.E1[sd][i / N1][t] * x[t * N1 + i % N1];
+            o[(2 + sd) * MX_XF * NP + i] = base + a1;
+          }
         }
       }
     }
-  }
-  __syncwarp();
-  // face-point fields of the faces that some slot reads, one contiguous block per face
-  for (int c = 0; c < nc; ++c) {
-    const float* sc = sw + c * L::cell;
-    float* dst = XF + (size_t)(e0 + c) * 6 * FW * NP;
-    if (VISC && FW == MX_XF) {
-      constexpr int HB = MX_XF * NP;  // floats per face block
-      for (int t = lane; t < 6 * HB / 2; t += 32) {
-        const bool use = (face_mask >> (2 * t / HB) & 1) | (face_mask >> ((2 * t + 1) / HB) & 1);
-        if (use) reinterpret_cast<float2*>(dst)[t] = reinterpret_cast<const float2*>(sc)[t];
-      }
-    } else {
-      for (int t = lane; t < 6 * 5 * NP; t += 32) {
-        const int k = t / (5 * NP), j = t - k * (5 * NP);
-        if (face_mask >> k & 1) dst[k * FW * NP + j] = sc[k * MX_XF * NP + j];
+    __syncwarp();
+    // face-point fields of the faces that some slot reads, one contiguous block per face
+    for (int c = 0; c < nc; ++c) {
+      const T* sc = sw + c * L::cell;
+      float* dst = XF + (size_t)(e0 + c) * 6 * FW * NP;
+      if (VISC && FW == MX_XF) {
+        constexpr int HB = MX_XF * NP;  // floats per face block
+        for (int t = lane; t < 6 * HB / 2; t += 32) {
+          const bool use = (face_mask >> (2 * t / HB) & 1) | (face_mask >> ((2 * t + 1) / HB) & 1);
+          if (use) reinterpret_cast<float2*>(dst)[t] = reinterpret_cast<const float2*>(sc)[t];
+        }
+      } else {
+        for (int t = lane; t < 6 * 5 * NP; t += 32) {
+          const int k = t / (5 * NP), j = t - k * (5 * NP);
+          if (face_mask >> k & 1) dst[k * FW * NP + j] = sc[k * MX_XF * NP + j];
+        }
       }
     }
   }
@@ -312,28 +361,31 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
   // ---- c2f, triangle part: one lane per (cell, variable, c-level) ----
   for (int it = lane; it < CW * 5 * N1; it += 32) {
     const int c = it / (5 * N1), vk = it - c * (5 * N1), v = vk / N1, k = vk - v * N1;
-    float* sc = sw + c * L::cell;
-    float x[NT];
+    T* sc = sw + c * L::cell;
+    T x[NT];
+    const T base = D ? sc[L::oRef + v] : T(0);
 #pragma unroll
-    for (int t = 0; t < NT; ++t) x[t] = sc[L::oX + v * FS + t * N1 + k];
-    float* y = sc + L::oY + vk * TP;
+    for (int t = 0; t < NT; ++t) x[t] = sc[L::oX + v * FS + t * N1 + k] - base;
+    T* y = sc + L::oY + vk * TP;
 #pragma unroll
-    for (int t4 = 0; t4 < (MT + 3) / 4; ++t4) {
-      float z[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int tv = 0; tv < (MT + VN - 1) / VN; ++tv) {
+      VecN<T> z;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (t4 * 4 + j < MT) {
+      for (int j = 0; j < VN; ++j) {
+        z.v[j] = T(0);
+        if (tv * VN + j < MT) {
 #pragma unroll
-          for (int t = 0; t < NT; ++t) z[j] += op.Ct[t4 * 4 + j][t] * x[t];
+          for (int t = 0; t < NT; ++t) z.v[j] += op.Ct[tv * VN + j][t] * x[t];
         }
-      *reinterpret_cast<float4*>(y + t4 * 4) = make_float4(z[0], z[1], z[2], z[3]);
+      }
+      *reinterpret_cast<VecN<T>*>(y + tv * VN) = z;
     }
   }
   // Euler flux at the reference state, FP64: lane = (cell, direction)
   if (lane < 3 * CW) {
     const int c = lane / 3, n = lane % 3;
-    float* sc = sw + c * L::cell;
-    const float* rf = sc + L::oRef;
+    T* sc = sw + c * L::cell;
+    const T* rf = sc + L::oRef;
     const double q[5] = {rf[0], rf[1], rf[2], rf[3], rf[4]};
     const double un = n == 0 ? q[1] : (n == 1 ? q[2] : q[3]);
     const double m = q[0] * un;
@@ -342,7 +394,7 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
     F[1] = m * q[1] + (n == 0 ? q[4] : 0.0);
     F[2] = m * q[2] + (n == 1 ? q[4] : 0.0);
     F[3] = m * q[3] + (n == 2 ? q[4] : 0.0);
-    F[4] = un * (GAMMA / (GAMMA - 1.0) * q[4] + 0.5 * q[0] * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]));
+    F[4] = un * px_rhoH(q[0], q[4], q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
   }
   __syncwarp();
 
@@ -351,9 +403,9 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
   // c part of W accumulated in registers ----
   for (int it = lane; it < CW * MT; it += 32) {
     const int c = it / MT, t = it - c * MT;
-    float* sc = sw + c * L::cell;
-    float af[9][NF];
-    {
+    T* sc = sw + c * L::cell;
+    T af[D ? 1 : 9][D ? 1 : NF];
+    if constexpr (!D) {
       const float* ap = pg.adjf + ((size_t)(e0 + (c < nc ? c : 0)) * 9 * MT + t) * NF;
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
@@ -369,35 +421,58 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
         }
       }
     }
-    float y[5][N1], qb[5];
+    T y[5][N1], qb[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       qb[v] = sc[L::oRef + v];
 #pragma unroll
       for (int k = 0; k < N1; ++k) y[v][k] = sc[L::oY + (v * N1 + k) * TP + t];
     }
-    float h[3][5][N1];
+    T h[3][5][N1];
 #pragma unroll
     for (int m = 0; m < 3; ++m)
 #pragma unroll
       for (int v = 0; v < 5; ++v)
 #pragma unroll
-        for (int k = 0; k < N1; ++k) h[m][v][k] = 0.f;
+        for (int k = 0; k < N1; ++k) h[m][v][k] = T(0);
 #pragma unroll
     for (int l = 0; l < NF; ++l) {
-      float dq[5], dF[3][5];
+      T dq[5], dF[3][5];
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        dq[v] = 0.f;
+        dq[v] = T(0);
 #pragma unroll
         for (int k = 0; k < N1; ++k) dq[v] += op.Cc[l][k] * y[v][k];
       }
-      mxd::euler_flux_delta(qb, dq, dF);
+      T al[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        if constexpr (D) al[k] = __ldg(pg.adjf + (((size_t)(e0 + (c < nc ? c : 0)) * NF + l) * 9 + k) * MT + t);
+        else al[k] = af[k][l];
+      }
+      if constexpr (D) {
+        // the flux itself (density floored as in the plain Euler flux), less
+        // the flux of the reference state
+        const double* Fr = reinterpret_cast<const double*>(sc + L::oF);
+        const T rho = qb[0] + dq[0], p = qb[4] + dq[4];
+        const T u[3] = {qb[1] + dq[1], qb[2] + dq[2], qb[3] + dq[3]};
+        const T rH = px_rhoH(rho, p, u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          const T m = rho * u[n];
+          dF[n][0] = m - Fr[n * 5];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) dF[n][1 + j] = m * u[j] + (n == j ? p : T(0)) - Fr[n * 5 + 1 + j];
+          dF[n][4] = rH * u[n] - Fr[n * 5 + 4];
+        }
+      } else {
+        mxd::euler_flux_delta<T>(qb, dq, dF);
+      }
 #pragma unroll
       for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-          const float ft = af[m * 3][l] * dF[0][v] + af[m * 3 + 1][l] * dF[1][v] + af[m * 3 + 2][l] * dF[2][v];
+          const T ft = al[m * 3] * dF[0][v] + al[m * 3 + 1] * dF[1][v] + al[m * 3 + 2] * dF[2][v];
 #pragma unroll
           for (int k = 0; k < N1; ++k) h[m][v][k] += op.Wc[m][k][l] * ft;
         }
@@ -414,22 +489,21 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
   // ---- W, triangle part: one lane per (cell, variable, c-level) ----
   for (int it = lane; it < CW * 5 * N1; it += 32) {
     const int c = it / (5 * N1), vk = it - c * (5 * N1), v = vk / N1, k = vk - v * N1;
-    float* sc = sw + c * L::cell;
-    float o[NT];
+    T* sc = sw + c * L::cell;
+    T o[NT];
 #pragma unroll
-    for (int j = 0; j < NT; ++j) o[j] = 0.f;
+    for (int j = 0; j < NT; ++j) o[j] = T(0);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      const float4* hp = reinterpret_cast<const float4*>(sc + (m * 5 * N1 + vk) * TP);
+      const VecN<T>* hp = reinterpret_cast<const VecN<T>*>(sc + (m * 5 * N1 + vk) * TP);
 #pragma unroll
-      for (int t4 = 0; t4 < (MT + 3) / 4; ++t4) {
-        const float4 x = hp[t4];
-        const float xv[4] = {x.x, x.y, x.z, x.w};
+      for (int tv = 0; tv < (MT + VN - 1) / VN; ++tv) {
+        const VecN<T> xv = hp[tv];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (t4 * 4 + i < MT) {
+        for (int i = 0; i < VN; ++i)
+          if (tv * VN + i < MT) {
 #pragma unroll
-            for (int j = 0; j < NT; ++j) o[j] += op.Wt[m][j][t4 * 4 + i] * xv[i];
+            for (int j = 0; j < NT; ++j) o[j] += op.Wt[m][j][tv * VN + i] * xv.v[i];
           }
       }
     }
@@ -443,30 +517,33 @@ __global__ void __launch_bounds__(32 * PX_WARPS, N1 == 3 ? 4 : 3)
   for (int r = 0; r < PR; ++r) {
     const int c = r * CPR + pc;
     if (pc < CPR && c < nc) {
-      float* sc = sw + c * L::cell;
+      T* sc = sw + c * L::cell;
       const size_t p = (size_t)(e0 + c) * S + s;
       const double md0 = __ldg(pg.MD + p * 3), md1 = __ldg(pg.MD + p * 3 + 1), md2 = __ldg(pg.MD + p * 3 + 2);
       const double rdet = __ldg(pg.rdet + p);
       const double* F = reinterpret_cast<const double*>(sc + L::oF);
-      const float* x = sc + L::oX + s;
-      float* o = RV + (size_t)(e0 + c) * 9 * S + s;
+      const T* x = sc + L::oX + s;
+      T* o = RV + (size_t)(e0 + c) * 9 * S + s;
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
         const double mdf = md0 * F[v] + md1 * F[5 + v] + md2 * F[10 + v];
-        o[v * S] = float(-(double(x[v * FS]) + mdf) * rdet);
+        o[v * S] = T(-(double(x[v * FS]) + mdf) * rdet);
         if (VISC && v > 0) o[(4 + v) * S] = x[(4 + v) * FS];
       }
     }
   }
 }
 
-// FP64 3 x 3 metric entries (npts per cell, 9 each) -> FP32 planes (N, 9, npts)
-__global__ void k_px_planes(const double* __restrict__ adj, size_t ncells, int npts, float* __restrict__ out) {
+// FP64 3 x 3 metric entries (npts per cell, 9 each) -> planes (N, 9, npts), or
+// with levels > 1 (N, levels, 9, npts / levels), point = j * levels + level
+template <class T>
+__global__ void k_px_planes(const double* __restrict__ adj, size_t ncells, int npts, int levels, T* __restrict__ out) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncells * npts * 9) return;
-  const int p = (int)(t % npts), k = (int)(t / npts % 9);
+  const int w = npts / levels;
+  const int j = (int)(t % w), k = (int)(t / w % 9), l = (int)(t / ((size_t)w * 9) % levels);
   const size_t c = t / ((size_t)npts * 9);
-  out[t] = float(adj[(c * npts + p) * 9 + k]);
+  out[t] = T(adj[(c * npts + (size_t)j * levels + l) * 9 + k]);
 }
 
 // ---- host: operator structure ----
