@@ -394,6 +394,12 @@ struct Launch {
     static const bool done = [] {
       const size_t smem = cell_smem();
       cudaFuncSetAttribute(k_cell<S, FN, NP, CPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if constexpr (S == 8) {
+        cudaFuncSetAttribute(k_face_staged<S, NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             FaceSmem<S, NP, false>::total);
+        cudaFuncSetAttribute(k_face_staged<S, NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             FaceSmem<S, NP, true>::total);
+      }
       cudaFuncSetAttribute(k_update<S, NP, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
       if constexpr (PXD) {
         cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -444,14 +450,22 @@ struct Launch {
     return cudaGetLastError();
   }
   static cudaError_t stage(afr_handle* h, StageArgs a, cudaStream_t st, StepTimer* tm = nullptr) {
-    constexpr int SPW = 32 / NP;  // slots per warp of the face kernel
-    const int nwarps = (h->slots.n + SPW - 1) / SPW;
-    if (nwarps > 0)
-      k_face<S, NP><<<(nwarps + FACE_WARPS - 1) / FACE_WARPS, 32 * FACE_WARPS, 0, st>>>(
-          h->g, h->ops, h->fc, h->bc, h->slots, h->PF, h->slot_rows, h->prm.mu, a.inviscid_only ? 0 : 1, h->J);
+    set_attrs();
+    if (h->slots.n > 0) {
+      if constexpr (S == 8) {
+        auto* fn = a.inviscid_only ? k_face_staged<S, NP, false> : k_face_staged<S, NP, true>;
+        const int sm = a.inviscid_only ? FaceSmem<S, NP, false>::total : FaceSmem<S, NP, true>::total;
+        fn<<<(h->N + FACE_WARPS - 1) / FACE_WARPS, 32 * FACE_WARPS, sm, st>>>(
+            h->g, h->ops, h->fc, h->bc, h->slots, h->PF, h->slot_rows, h->prm.mu, h->J);
+      } else {
+        constexpr int per = FACE_WARPS * (32 / NP);
+        auto* fn = a.inviscid_only ? k_face<S, NP, false> : k_face<S, NP, true>;
+        fn<<<(h->slots.n + per - 1) / per, 32 * FACE_WARPS, 0, st>>>(h->g, h->ops, h->fc, h->bc, h->slots, h->PF,
+                                                                     h->slot_rows, h->prm.mu, h->J);
+      }
+    }
     if (tm) tm->mark(st);
     const size_t smem = cell_smem();
-    set_attrs();
     a.N = h->N;
     a.slot_flags = h->slots.flags;
     const int ranges[3] = {0, h->n_prism, h->N};
@@ -1469,6 +1483,37 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     cudaStreamSynchronize(st);  // r leaves scope
   }
   {
+    // nonzeros of the extrapolation rows
+    std::vector<double> ew(12 * S * P, 0.0);
+    std::vector<int32_t> ei(12 * S * P, 0), en(12 * P, 0);
+    for (size_t gr = 0; gr < 12; ++gr)
+      for (size_t i = 0; i < P; ++i) {
+        const double* w = m->boundary_extrap + (gr * P + i) * S;
+        double big = 0.0, rest = 0.0;
+        for (size_t s2 = 0; s2 < S; ++s2) big = std::max(big, std::fabs(w[s2]));
+        int32_t n = 0;
+        for (size_t s2 = 0; s2 < S; ++s2)
+          if (!(std::fabs(w[s2]) <= 3e-15 * big)) {
+            ew[(gr * S + n) * P + i] = w[s2];
+            ei[(gr * S + n) * P + i] = (int32_t)s2;
+            ++n;
+          } else {
+            rest += w[s2];
+          }
+        for (int32_t k = 0; k < n; ++k) ew[(gr * S + k) * P + i] += rest / n;
+        en[gr * P + i] = n;
+      }
+    double* dw;
+    int32_t *di, *dn;
+    if ((rc = upload(h, &dw, ew.data(), ew.size(), st)) || (rc = upload(h, &di, ei.data(), ei.size(), st)) ||
+        (rc = upload(h, &dn, en.data(), en.size(), st)))
+      return bail(rc);
+    cudaStreamSynchronize(st);  // host vectors leave scope
+    h->ops.ex_w = dw;
+    h->ops.ex_i = di;
+    h->ops.ex_n = dn;
+  }
+  {
     double *ex, *gl, *gr;
     int32_t *dfp, *dco;
     if ((rc = upload(h, &ex, m->boundary_extrap, 12 * P * S, st))) return bail(rc);
@@ -1612,6 +1657,7 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     cudaMemcpy(codes.data(), sl, codes.size() * sizeof(int32_t), cudaMemcpyDeviceToHost);
     const size_t ns = codes.size();
     std::vector<int32_t> sf(ns), sc(ns), sflg(ns), s0(ns), s1(ns), si1(ns);
+    std::vector<int4> srec(prm->precision != AFR_PREC_MIXED && h->order > 0 ? 2 * ns : 0);
     for (size_t c = 0; c < N; ++c)
       for (int32_t k = ptr[c]; k < ptr[c + 1]; ++k) {
         const int f = codes[k] >> 1;
@@ -1626,14 +1672,25 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
         s0[k] = bnd ? -1 : (int32_t)(nbside ? m->ow_src0_cell[f] : m->nb_src0_cell[f]);
         si1[k] = (int32_t)i1;
         s1[k] = (bnd || i1 < 0) ? -1 : (int32_t)(nbside ? m->ow_src1_cell[i1] : m->nb_src1_cell[i1]);
+        if (!srec.empty()) {
+          // matrix rows: table rows of an indexed mesh, else the record's own
+          const bool ix = m->src_mat_table != nullptr;
+          const int32_t m0 = ix ? (nbside ? m->ow_src0_mat_index[f] : m->nb_src0_mat_index[f]) : f;
+          const int32_t m1 =
+              s1[k] < 0 ? 0 : (ix ? (nbside ? m->ow_src1_mat_index[i1] : m->nb_src1_mat_index[i1]) : (int32_t)i1);
+          srec[2 * (size_t)k] = make_int4(s0[k], m0, s1[k], m1);
+          srec[2 * (size_t)k + 1] = make_int4(f, sflg[k], (int)c, 0);
+        }
       }
     int32_t *d_f, *d_c, *d_fl, *d_0, *d_1, *d_i1;
     if ((rc = upload(h, &d_f, sf.data(), ns, st)) || (rc = upload(h, &d_c, sc.data(), ns, st)) ||
         (rc = upload(h, &d_fl, sflg.data(), ns, st)) || (rc = upload(h, &d_0, s0.data(), ns, st)) ||
         (rc = upload(h, &d_1, s1.data(), ns, st)) || (rc = upload(h, &d_i1, si1.data(), ns, st)))
       return bail(rc);
+    int4* d_rec = nullptr;
+    if (!srec.empty() && (rc = upload(h, &d_rec, srec.data(), srec.size(), st))) return bail(rc);
     cudaStreamSynchronize(st);
-    h->slots = SlotTable{(int32_t)ns, d_f, d_c, d_fl, d_0, d_1, d_i1};
+    h->slots = SlotTable{(int32_t)ns, d_f, d_c, d_fl, d_0, d_1, d_i1, d_rec};
     // FP64 jumps: the plain stage of orders 1-3 only
     if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = dalloc(h, &h->J, ns * P * 9))) return bail(rc);
   }
@@ -1670,7 +1727,8 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
   if ((rc = dalloc(h, &h->norm_part, N))) return bail(rc);
   if ((rc = dalloc(h, &h->norm_rho_part, N))) return bail(rc);
   if ((rc = dalloc(h, &h->red, 4))) return bail(rc);
-  if ((rc = dalloc(h, &h->red_part, (N * S + RED_CHUNK - 1) / RED_CHUNK + 1))) return bail(rc);
+  if ((rc = dalloc(h, &h->red_part, std::max((N * S + RED_CHUNK - 1) / RED_CHUNK, (N * S * h->nv + IMP_CHUNK - 1) / IMP_CHUNK) + 1)))
+    return bail(rc);
   if (prm->turb == AFR_TURB_SST) {
     if ((rc = dalloc(h, &h->pt, N * S * 5))) return bail(rc);
     if ((rc = dalloc(h, &h->cfp, F * P * 2))) return bail(rc);
@@ -1860,15 +1918,33 @@ int imp_norm(afr_handle* h, const ImpArgs& a, int mode, cudaStream_t st, double*
   return AFR_OK;
 }
 
-int filter_cells(afr_handle* h, double* U, cudaStream_t st) {
-  switch (h->order) {
-    case 0: k_filter_cells<1><<<h->N, 32, 0, st>>>(h->g, h->ops, U, h->nv); break;
-    case 1: k_filter_cells<8><<<h->N, 64, 0, st>>>(h->g, h->ops, U, h->nv); break;
-    case 2: k_filter_cells<27><<<h->N, 160, 0, st>>>(h->g, h->ops, U, h->nv); break;
-    default: k_filter_cells<64><<<h->N, 320, 0, st>>>(h->g, h->ops, U, h->nv); break;
+extern "C++" {  // a template inside the C block
+template <int S>
+cudaError_t dual_stage_launch(afr_handle* h, const ImpArgs& a, bool last, cudaStream_t st) {
+  static const cudaError_t attr = cudaFuncSetAttribute(k_dual_stage<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       DualDims<S>::bytes(7));
+  if (attr != cudaSuccess) return attr;
+  constexpr int per = DUAL_WARPS * DualDims<S>::CW;
+  const int ranges[3] = {0, h->n_prism, h->N};
+  for (int r = 0; r < 2; ++r) {
+    const int n = ranges[r + 1] - ranges[r];
+    if (n > 0)
+      k_dual_stage<S><<<(n + per - 1) / per, 32 * DUAL_WARPS, DualDims<S>::bytes(h->nv), st>>>(
+          a, h->ops, r, ranges[r], ranges[r + 1], last ? 1 : 0);
   }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? AFR_OK : cuda_fail(h, e, "filter");
+  return cudaGetLastError();
+}
+}  // extern "C++"
+
+int dual_stage(afr_handle* h, const ImpArgs& a, bool last, cudaStream_t st) {
+  cudaError_t e;
+  switch (h->order) {
+    case 0: e = dual_stage_launch<1>(h, a, last, st); break;
+    case 1: e = dual_stage_launch<8>(h, a, last, st); break;
+    case 2: e = dual_stage_launch<27>(h, a, last, st); break;
+    default: e = dual_stage_launch<64>(h, a, last, st);
+  }
+  return e == cudaSuccess ? AFR_OK : cuda_fail(h, e, "dual-time stage");
 }
 
 int copy_state(afr_handle* h, double* dst, const double* src, cudaStream_t st) {
@@ -1929,7 +2005,6 @@ int afr_step_dual_time(afr_handle* h, double* U, double* k, double* omega, doubl
   a.Uprev = has_prev ? U_prev : nullptr;
   a.dtphys = dt_physical;
   a.dtl = h->dt;
-  const unsigned gb = (unsigned)((npts + 255) / 256);
   double init = 0.0, prev = 0.0, cfl = 0.1;
   a.Ucur = U;
   if ((rc = imp_norm(h, a, 0, st, &init))) return rc;
@@ -1955,12 +2030,8 @@ int afr_step_dual_time(afr_handle* h, double* U, double* k, double* omega, doubl
       a.Ucur = s == 0 ? U : stg[s - 1];
       a.stage = s;
       a.Unext = stg[s];
-      k_dual_stage<<<gb, 256, 0, st>>>(a);
-      if ((rc = filter_cells(h, stg[s], st))) return rc;
+      if ((rc = dual_stage(h, a, s == 2, st))) return rc;
     }
-    // positivity and filter once more on the pseudo step's result (dual.py:137-139)
-    k_positivity<<<gb, 256, 0, st>>>(h->iX, (int64_t)npts, h->nv);
-    if ((rc = filter_cells(h, h->iX, st))) return rc;
     ImpArgs d = a;
     d.U0 = U;
     d.Ucur = h->iX;

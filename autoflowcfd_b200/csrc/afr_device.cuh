@@ -54,6 +54,13 @@ struct Ops {
   const double* fc2f[2];    // c2f (Fn, S)
   const double* fW[2];      // W (S, 3Fn)
   const double* ffilt[2];   // filt (S, S)
+  // nonzeros of the extrapolation rows (entries within 3e-15 of the row's
+  // largest are left out, their sum shared among the others): row group
+  // g = (type*3 + axis)*2 + side, entry k of face point i at [(g*S + k)*P + i],
+  // counts at [g*P + i]
+  const double* ex_w;
+  const int32_t* ex_i;
+  const int32_t* ex_n;
   const double* fextrap;    // extrap: 12 images of (P, S), ceil(P/8) * ceil(S/4) * 32 doubles each
 };
 
@@ -158,20 +165,24 @@ __device__ __forceinline__ void ausm_up(const T qL[5], const T qR[5], const T n[
   const T uR = qR[1], vR = qR[2], wR = qR[3];
   const T unL = uL * n[0] + vL * n[1] + wL * n[2];
   const T unR = uR * n[0] + vR * n[1] + wR * n[2];
-  const T aL = sqrt(fmax(T(GAMMA) * pL / rhoL, T(1e-10)));
-  const T aR = sqrt(fmax(T(GAMMA) * pR / rhoR, T(1e-10)));
-  const T ML = unL / fmax(aL, T(1e-10));
-  const T MR = unR / fmax(aR, T(1e-10));
+  // six divisions and three square roots: they are what the flux costs in FP64
+  const T prL = pL / rhoL, prR = pR / rhoR;
+  const T aL = sqrt(fmax(T(GAMMA) * prL, T(1e-10)));
+  const T aR = sqrt(fmax(T(GAMMA) * prR, T(1e-10)));
+  const T ML = unL / aL;  // aL, aR >= 1e-5
+  const T MR = unR / aR;
   const T a_half = T(0.5) * (aL + aR);
   const T rho_half = T(0.5) * (rhoL + rhoR);
-  const T Mbar2 = (sq(unL) + sq(unR)) / (T(2.0) * sq(a_half));
+  const T ra2 = T(1.0) / sq(a_half);
+  const T Mbar2 = T(0.5) * (sq(unL) + sq(unR)) * ra2;
   const T M0 = fmin(T(1.0), fmax(Mbar2, ma_ref * ma_ref));
-  T fa = sqrt(M0) * (T(2.0) - sqrt(M0));
+  const T sM0 = sqrt(M0);
+  T fa = sM0 * (T(2.0) - sM0);
   fa = fmax(fa, T(1e-6));
   const T mp = (fabs(ML) >= T(1.0)) ? T(0.5) * (ML + fabs(ML)) : T(0.25) * sq(ML + T(1.0)) + alpha * sq(sq(ML) - T(1.0));
   const T mm = (fabs(MR) >= T(1.0)) ? T(0.5) * (MR - fabs(MR)) : -T(0.25) * sq(MR - T(1.0)) - alpha * sq(sq(MR) - T(1.0));
   const T M_half = mp + mm;
-  const T Mp = -(Kp / fa) * fmax(T(1.0) - sigma_p * Mbar2, T(0.0)) * (pR - pL) / (rho_half * sq(a_half));
+  const T Mp = -Kp * fmax(T(1.0) - sigma_p * Mbar2, T(0.0)) * (pR - pL) * ra2 / (fa * rho_half);
   const T mdot = T(0.5) * (rhoL * aL + rhoR * aR) * (M_half + Mp);
   const T sgnL = (ML > T(0.0)) ? T(1.0) : ((ML < T(0.0)) ? T(-1.0) : T(0.0));
   const T sgnR = (MR > T(0.0)) ? T(1.0) : ((MR < T(0.0)) ? T(-1.0) : T(0.0));
@@ -185,8 +196,8 @@ __device__ __forceinline__ void ausm_up(const T qL[5], const T qR[5], const T n[
   out[1] = mdot * (up ? uL : uR) + p_half * n[0];
   out[2] = mdot * (up ? vL : vR) + p_half * n[1];
   out[3] = mdot * (up ? wL : wR) + p_half * n[2];
-  const T hL = T(GAMMA / (GAMMA - 1.0)) * pL / rhoL + T(0.5) * (sq(uL) + sq(vL) + sq(wL));
-  const T hR = T(GAMMA / (GAMMA - 1.0)) * pR / rhoR + T(0.5) * (sq(uR) + sq(vR) + sq(wR));
+  const T hL = T(GAMMA / (GAMMA - 1.0)) * prL + T(0.5) * (sq(uL) + sq(vL) + sq(wL));
+  const T hR = T(GAMMA / (GAMMA - 1.0)) * prR + T(0.5) * (sq(uR) + sq(vR) + sq(wR));
   out[4] = mdot * (up ? hL : hR);
 }
 

@@ -58,30 +58,66 @@ struct ImpArgs {
   double* Unext;
 };
 
-// one SSP-RK3 stage of the pseudo-time iteration on the dual residual, with
-// positivity; L = -R_dual(Ucur), dt = pseudo dt * CFL factor
-__global__ void k_dual_stage(ImpArgs a) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= a.npts) return;
-  const int nv = a.nv;
-  const double dt = a.dtl[p] * a.scale;
-  double un[8];
-#pragma unroll
-  for (int v = 0; v < 8; ++v) {
-    if (v >= nv) {
-      un[v] = 0.0;
-      continue;
-    }
-    const size_t i = (size_t)p * nv + v;
+// One SSP-RK3 stage of the pseudo-time iteration on the dual residual, with
+// positivity and the modal filter (L = -R_dual(Ucur), dt = pseudo dt * CFL
+// factor); with `last`, positivity and filter once more, as the scheme applies
+// them to the pseudo step's result (dual.py:137-139).  A warp owns CW cells:
+// the stage is elementwise, so its arrays are read as contiguous blocks, the
+// rows meet in shared memory, and the filter is one FP64 tensor product per
+// warp.  (Stage, filter and final positivity as launches of their own took 10,
+// 12 and 5 us each on 4,000 P2 prisms.)
+constexpr int DUAL_WARPS = 4;
+template <int S>
+struct DualDims {
+  static constexpr int CW = S <= 8 ? 8 : 3;
+  __host__ __device__ static constexpr int bytes(int nv) { return DUAL_WARPS * 2 * CW * S * nv * 8; }
+};
+
+template <int S>
+__global__ void __launch_bounds__(32 * DUAL_WARPS)
+    k_dual_stage(ImpArgs a, Ops ops, int ct, int cell_base, int cell_end, int last) {
+  constexpr int CW = DualDims<S>::CW;
+  extern __shared__ __align__(16) double smdual[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e0 = cell_base + (blockIdx.x * DUAL_WARPS + warp) * CW;
+  const int nc = min(CW, cell_end - e0);
+  if (nc <= 0) return;  // whole warps; no block barrier below
+  const int nv = a.nv, np = nc * S, ne = np * nv;
+  double* x = smdual + warp * 2 * CW * S * nv;
+  double* y = x + CW * S * nv;
+  const size_t base = (size_t)e0 * S;
+  for (int t = lane; t < ne; t += 32) {
+    const size_t i = base * nv + t;
+    const double dt = a.dtl[base + t / nv] * a.scale;
     const double L = -dual_residual(a.Rinv[i], a.Rvisc[i], a.Ucur[i], a.Un[i], a.Uprev, i, a.dtphys);
-    if (a.stage == 0) un[v] = a.U0[i] + dt * L;
-    else if (a.stage == 1) un[v] = (0.75 * a.U0[i] + 0.25 * a.Ucur[i]) + (0.25 * dt) * L;
-    else un[v] = (1.0 / 3.0 * a.U0[i] + 2.0 / 3.0 * a.Ucur[i]) + (2.0 / 3.0 * dt) * L;
+    if (a.stage == 0) x[t] = a.U0[i] + dt * L;
+    else if (a.stage == 1) x[t] = (0.75 * a.U0[i] + 0.25 * a.Ucur[i]) + (0.25 * dt) * L;
+    else x[t] = (1.0 / 3.0 * a.U0[i] + 2.0 / 3.0 * a.Ucur[i]) + (2.0 / 3.0 * dt) * L;
   }
-  positivity_point(un, nv);
+  __syncwarp();
+  for (int pass = 0; pass <= last; ++pass) {
+    for (int p = lane; p < np; p += 32) {
+      double un[8];
 #pragma unroll
-  for (int v = 0; v < 8; ++v)
-    if (v < nv) a.Unext[(size_t)p * nv + v] = un[v];
+      for (int v = 0; v < 8; ++v) un[v] = v < nv ? x[p * nv + v] : 0.0;
+      positivity_point(un, nv);
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        if (v < nv) {
+          x[p * nv + v] = un[v];
+          if (v >= 5) y[p * nv + v] = un[v];
+        }
+    }
+    __syncwarp();
+    dmma_warp_rb_f<(S + 7) / 8, (5 * CW + 7) / 8, S>(
+        S, 5 * nc, ops.ffilt[ct], [&](int j, int col) { return x[((col / 5) * S + j) * nv + col % 5]; },
+        [&](int m, int col, double v) { y[((col / 5) * S + m) * nv + col % 5] = v; });
+    __syncwarp();
+    double* z = x;
+    x = y;
+    y = z;
+  }
+  for (int t = lane; t < ne; t += 32) a.Unext[base * nv + t] = x[t];
 }
 
 // damped Picard update of the IMEX scheme with positivity:
@@ -109,42 +145,12 @@ __global__ void k_imex_update(ImpArgs a) {
     if (v < nv) a.Unext[(size_t)p * nv + v] = un[v];
 }
 
-// positivity alone, in place
-__global__ void k_positivity(double* U, int64_t npts, int nv) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npts) return;
-  double un[8];
-#pragma unroll
-  for (int v = 0; v < 8; ++v) un[v] = v < nv ? U[(size_t)p * nv + v] : 0.0;
-  positivity_point(un, nv);
-#pragma unroll
-  for (int v = 0; v < 8; ++v)
-    if (v < nv) U[(size_t)p * nv + v] = un[v];
-}
-
-// modal filter of the first five variables of every cell, in place: one CTA
-// per cell, each output summed over the cell's points in order
-// (np.einsum("sj,cjv->csv") of core/fr_solver/filter.py:29-42)
-template <int S>
-__global__ void k_filter_cells(Geom g, Ops ops, double* U, int nv) {
-  __shared__ double sm[S * 5];
-  const int c = blockIdx.x;
-  double* Uc = U + (size_t)c * S * nv;
-  for (int t = threadIdx.x; t < S * 5; t += blockDim.x) sm[t] = Uc[(t / 5) * nv + t % 5];
-  __syncthreads();
-  const double* F = ops.filt[cell_type(g, c)];
-  for (int t = threadIdx.x; t < S * 5; t += blockDim.x) {
-    const int s = t / 5, v = t % 5;
-    double acc = 0.0;
-    for (int j = 0; j < S; ++j) acc += __ldg(F + s * S + j) * sm[j * 5 + v];
-    Uc[s * nv + v] = acc;
-  }
-}
-
 // sums of squares in chunks of IMP_CHUNK elements (one partial per CTA), of
 //   mode 0: the dual residual of Ucur;  mode 1: Ucur - U0;
 //   mode 2: the IMEX total -inviscid(U^n) + -viscous(Ucur);  mode 3: inviscid + viscous (dU/dt)
-constexpr int IMP_CHUNK = 65536, IMP_THREADS = 256;
+// 4,096 elements per CTA: a 4,000-cell P2 case (540,000 elements) fills 132 CTAs
+// instead of nine (92 -> 5 us).
+constexpr int IMP_CHUNK = 4096, IMP_THREADS = 256;
 __global__ void __launch_bounds__(IMP_THREADS) k_imp_sumsq(ImpArgs a, int mode, double* part) {
   __shared__ double sh[IMP_THREADS];
   const size_t n = (size_t)a.npts * a.nv;

@@ -266,6 +266,7 @@ __device__ void suppress_outliers_cells(double* sRi, double* sRv, const double* 
 // one unused (128-byte rows)
 // ---------------------------------------------------------------------------
 constexpr int PFW = 16;
+constexpr int PFS = 17;  // row stride in shared memory (odd: consecutive rows on distinct banks)
 
 template <int S>
 struct PreTile {
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
                                              const double* __restrict__ nut, int want_grads,
                                              double* __restrict__ PF, int cell_base, int cell_end) {
   constexpr int CPB = PreTile<S>::CPB;
-  __shared__ double sPF[CPB * S * PFW];
+  __shared__ double sPF[CPB * S * PFS];
   __shared__ double f[CPB * S * 4];
   __shared__ double gc[CPB * S * 3 * 4];
   const int e0 = cell_base + blockIdx.x * CPB;
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
     double q[5];
     const double* u = U + p * nv;
     cons_to_prim(u, q);
-    double* o = sPF + t * PFW;
+    double* o = sPF + t * PFS;
     for (int v = 0; v < 5; ++v) o[v] = q[v];
     o[15] = 0.0;
     o[14] = nut ? fmax(u[0], 1e-10) * nut[p] : 0.0;
@@ -320,7 +321,7 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
           for (int m = 0; m < 3; ++m) acc += gc[(t * 3 + m) * 4 + q] * inv[m * 3 + n];
           gr[q][n] = acc;
         }
-      double* o = sPF + t * PFW + 5;
+      double* o = sPF + t * PFS + 5;
 #pragma unroll
       for (int n = 0; n < 3; ++n) {
         o[n] = gr[n][n];
@@ -331,11 +332,11 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
       o[5] = 0.5 * (gr[1][2] + gr[2][1]);
     }
   } else {
-    for (int t = threadIdx.x; t < nc * S * 9; t += blockDim.x) sPF[(t / 9) * PFW + 5 + t % 9] = 0.0;
+    for (int t = threadIdx.x; t < nc * S * 9; t += blockDim.x) sPF[(t / 9) * PFS + 5 + t % 9] = 0.0;
   }
   __syncthreads();
   double* out = PF + (size_t)e0 * S * PFW;
-  for (int t = threadIdx.x; t < nc * S * PFW; t += blockDim.x) out[t] = sPF[t];
+  for (int t = threadIdx.x; t < nc * S * PFW; t += blockDim.x) out[t] = sPF[(t / PFW) * PFS + t % PFW];
 }
 
 // ---------------------------------------------------------------------------
@@ -354,6 +355,9 @@ struct SlotTable {
   const int32_t* c0;        // (n) first interpolation source cell, -1 if none
   const int32_t* c1;        // (n) second source cell, -1 if none
   const int32_t* i1;        // (n) row of the compact second-source table
+  // (n, 2) what the FP64 face kernel needs of a slot: source cells and matrix
+  // rows (c0, m0, c1, m1), then face, flags
+  const int4* rec;
 };
 
 
@@ -442,110 +446,21 @@ __device__ __forceinline__ void dmma_warp_rb_f(int M, int N, const double* __res
     }
 }
 
-// Face kernel: one warp per group of SPW = 32 / NP slots (a slot is one side
-// of one face record whose correction lifts into a cell; lane = slot-in-group
-// * NP + flux point in the flux phase).  Per slot, the own side's
-// extrapolation E * [q, grads, mu_t] and the
-// other side's interpolation M_src0 * [q, grads, mu_t] (+ M_src1 * ...) are
-// FP64 tensor-core products into the warp's shared rows; the lanes then form
-// the ghost state, AUSM+up with the alignment fallback and the BR1 common
-// flux with the boundary penalty
-// (core/fr_residual/inviscid_kernel_colored.py:86-236,
-// core/fr_residual/viscous_flux_kernel.py:335-520) and write the jumps
-// J (n_slots, 9, NP: inviscid 5, viscous momentum and energy 4).  A weight of zero contributes nothing to the products
-// while the state is finite (the reference skips zero weights,
-// inviscid_kernel_colored.py:117-121; a non-finite state makes the step
-// non-finite either way).
-// Slot flags: bit0 neighbour side, bit1 boundary face, bits2-3 axis, bit4 side>0.
-constexpr int FACE_WARPS = 4;
-constexpr int FW_F = 15;  // doubles per face point and side
-
-template <int S, int NP>
-__global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Faces fc, Bc bc, SlotTable st,
-                                                          const double* __restrict__ PF,
-                                                          const double4* __restrict__ arow, double mu, int visc,
-                                                          double* __restrict__ J) {
-  constexpr int SPW = 32 / NP;  // slots per warp
-  constexpr int MT = (NP + 7) / 8;  // row tiles of the face points
-  __shared__ double sOw[FACE_WARPS][SPW * NP * FW_F];
-  __shared__ double sOt[FACE_WARPS][SPW * NP * FW_F];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sl0 = (blockIdx.x * FACE_WARPS + warp) * SPW;
-  if (sl0 >= st.n) return;  // whole warps leave together
-  const int nsl = min(SPW, st.n - sl0);
-  double* ow_s = sOw[warp];
-  double* ot_s = sOt[warp];
-  for (int j = 0; j < nsl; ++j) {
-    const int sl = sl0 + j;
-    const int f = st.face[sl];
-    const int e = st.cell[sl];
-    const int fl = st.flags[sl];
-    const bool is_owner = (fl & 1) == 0;
-    const bool bnd = (fl & 2) != 0;
-    const int ax = (fl >> 2) & 3;
-    const int sb = (fl & 16) ? 1 : 0;
-    const int ct = cell_type(g, e);
-    // own side: rows face points, columns [q(5), grads + mu_t(10)]
-    const double* Ef = ops.fextrap + (((size_t)ct * 3 + ax) * 2 + sb) * (MT * ((S + 3) / 4) * 32);
-    const double* pf = PF + (size_t)e * S * PFW;
-    double* ow = ow_s + j * NP * FW_F;
-    {
-      auto fb = [&](int s, int n) { return __ldg(pf + s * PFW + n); };
-      auto fc_ = [&](int i, int n, double x) { ow[i * FW_F + n] = x; };
-      if (visc) dmma_warp_rb_f<MT, 2, S>(NP, FW_F, Ef, fb, fc_);
-      else dmma_warp_rb_f<MT, 1, S>(NP, 5, Ef, fb, fc_);  // columns 5.. are not read without viscosity
-    }
-    // other side: the interpolation sources (the first, then the second added)
-    double* ot = ot_s + j * NP * FW_F;
-    if (!bnd) {
-      for (int src = 0; src < 2; ++src) {
-        const int c = src == 0 ? st.c0[sl] : st.c1[sl];
-        if (c < 0) {
-          if (src == 0)
-            for (int t = lane; t < NP * FW_F; t += 32) ot[t] = 0.0;
-          continue;
-        }
-        const double* M = src == 0 ? (is_owner ? fmat(fc.nb_m0, fc.nb_m0i, f, 0, NP, S)
-                                               : fmat(fc.ow_m0, fc.ow_m0i, f, 0, NP, S))
-                                   : (is_owner ? fmat(fc.nb_m1, fc.nb_m1i, st.i1[sl], 0, NP, S)
-                                               : fmat(fc.ow_m1, fc.ow_m1i, st.i1[sl], 0, NP, S));
-        const double* pc = PF + (size_t)c * S * PFW;
-        __syncwarp();
-        auto fa = [&](int i, int s) { return __ldg(M + s * NP + i); };
-        auto fb = [&](int s, int n) { return __ldg(pc + s * PFW + n); };
-        auto fc_ = [&](int i, int n, double x) {
-          if (src == 0) ot[i * FW_F + n] = x;
-          else ot[i * FW_F + n] += x;
-        };
-        if (visc) dmma_warp_rb<MT, 2, S>(NP, FW_F, fa, fb, fc_);
-        else dmma_warp_rb<MT, 1, S>(NP, 5, fa, fb, fc_);  // columns 5.. are not read without viscosity
-      }
-    }
-  }
-  __syncwarp();
-  // flux phase: lane = slot-in-group * NP + face point
-  const int j = lane / NP, i = lane % NP;
-  if (j >= nsl || lane >= SPW * NP) return;
-  const int sl = sl0 + j;
-  const int f = st.face[sl];
-  const int e = st.cell[sl];
-  const int fl = st.flags[sl];
-  const bool is_owner = (fl & 1) == 0;
-  const bool bnd = (fl & 2) != 0;
-  const double side = (fl & 16) ? 1.0 : -1.0;
-  double ow[FW_F], ot[FW_F];
-#pragma unroll
-  for (int k = 0; k < FW_F; ++k) ow[k] = (k < 5 || visc) ? ow_s[(j * NP + i) * FW_F + k] : 0.0;
+// the jumps of one slot point from its own side and the other side's fields
+template <int S, int NP, bool VISC, int NF>
+__device__ __forceinline__ void face_jump(const Geom& g, const Faces& fc, const Bc& bc, int sl, int i, int e, int f,
+                                          bool is_owner, bool bnd, double side, const double (&ow)[NF],
+                                          double (&ot)[NF], const double4* __restrict__ arow, double mu,
+                                          double* __restrict__ J) {
   const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
   if (bnd) {
     double n[3], gq[5];
     for (int d = 0; d < 3; ++d) n[d] = tn[d];
     ghost_state(bc, fc.bc_group[f], ow, n, gq);
-    for (int v = 0; v < 5; ++v) ot[v] = gq[v];
-    for (int k = 5; k < FW_F; ++k) ot[k] = ow[k];
-  } else {
 #pragma unroll
-    for (int k = 0; k < FW_F; ++k) ot[k] = (k < 5 || visc) ? ot_s[(j * NP + i) * FW_F + k] : 0.0;
+    for (int v = 0; v < 5; ++v) ot[v] = gq[v];
+#pragma unroll
+    for (int k = 5; k < NF; ++k) ot[k] = ow[k];
   }
   // pointwise fluxes; the own adjugate row and its norm are geometry, formed at
   // create (a negative norm marks the alignment fallback)
@@ -564,10 +479,10 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
   euler_flux(ow, Fp);
   double* Jo = J + (size_t)sl * 9 * NP + i;
   for (int v = 0; v < 5; ++v) Jo[v * NP] = Fc[v] * mag * side - (a0 * Fp[0][v] + a1 * Fp[1][v] + a2 * Fp[2][v]);
-  if (visc) {
-    double av[FW_F];  // the common flux: both sides' averages
+  if constexpr (VISC) {
+    double av[NF];  // the common flux: both sides' averages
 #pragma unroll
-    for (int k = 1; k < FW_F; ++k) av[k] = 0.5 * (ow[k] + ot[k]);
+    for (int k = 1; k < NF; ++k) av[k] = 0.5 * (ow[k] + ot[k]);
     double Gc[3][4], Go[3][4];
     viscous_flux_sym(av + 1, av + 5, av + 11, mu, av[14], Gc);
     viscous_flux_sym(ow + 1, ow + 5, ow + 11, mu, ow[14], Go);
@@ -588,6 +503,205 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4) k_face(Geom g, Ops ops, Fa
     }
     for (int v = 0; v < 4; ++v) Jo[(5 + v) * NP] = jv[v];
   }
+}
+
+// Face kernels.  A slot is one side of one face record whose correction lifts
+// into a cell; lane = (slot, flux point) forms the own side from the nonzeros
+// of its extrapolation row (Ops::ex_*: 3 or 9 of a P2 prism's 27 points), the
+// other side with the record's matrix (the second source added to the first),
+// the ghost state, AUSM+up with the alignment fallback and the BR1 common flux
+// with the boundary penalty
+// (core/fr_residual/inviscid_kernel_colored.py:86-236,
+// core/fr_residual/viscous_flux_kernel.py:335-520), and writes the jumps
+// J (n_slots, 9, NP: inviscid 5, viscous momentum and energy 4).
+// A weight of zero contributes nothing while the state is finite (the reference
+// skips zero weights, inviscid_kernel_colored.py:117-121; a non-finite state
+// makes the step non-finite either way).
+//
+// k_face (orders 2, 3): a warp per group of SPW = 32 / NP slots; the other
+// side's product is register-blocked on the FP64 tensor path, its operands
+// gathered straight from global memory.
+// k_face_staged (order 1, 8 x 4 matrices that fill a quarter of the tensor
+// tiles): a warp per cell; the rows of the cell and of its slots' source cells
+// arrive in shared memory by 16-byte asynchronous copies, all in flight at
+// once, and the products are plain multiply-adds.  24,576 P1 tets, inviscid: 83 us on
+// the tensor path, 64 us staged; 17,280 P2 prisms, viscous: 268 us staged.
+// Slot flags: bit0 neighbour side, bit1 boundary face, bits2-3 axis, bit4 side>0.
+constexpr int FACE_WARPS = 4;
+constexpr int FW_F = 15;  // fields per face point and side
+
+template <int S, int NP, bool VISC>
+struct FaceSmem {
+  static constexpr int SPW = 32 / NP;        // slots in flight per warp
+  static constexpr int RQ = VISC ? 8 : 3;    // 16-byte pieces of a point row (without viscosity only q)
+  static constexpr int RW = VISC ? 18 : 6;   // row stride: 16-byte accesses to eight rows hit distinct banks
+  static constexpr int warp = (1 + SPW) * S * RW;  // doubles: the cell's rows, then each slot's source rows
+  static constexpr int total = FACE_WARPS * warp * 8;
+};
+
+template <int S, int NP, bool VISC>
+__global__ void __launch_bounds__(32 * FACE_WARPS, VISC ? 3 : 4)
+    k_face_staged(Geom g, Ops ops, Faces fc, Bc bc, SlotTable st, const double* __restrict__ PF,
+                  const double4* __restrict__ arow, double mu, double* __restrict__ J) {
+  using L = FaceSmem<S, NP, VISC>;
+  constexpr int SPW = L::SPW, RQ = L::RQ, RW = L::RW, NF = VISC ? FW_F : 5;
+  extern __shared__ __align__(16) double smf64[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e = blockIdx.x * FACE_WARPS + warp;
+  if (e >= g.N) return;  // whole warps; warp-level synchronisation only
+  double* own = smf64 + warp * L::warp;
+  double* nb = own + S * RW;
+  auto stage = [&](double* dst, int c) {
+    const double* pf = PF + (size_t)c * S * PFW;
+    for (int t = lane; t < S * RQ; t += 32) {
+      const int r = t / RQ, q = t - r * RQ;
+      cp_async16(dst + r * RW + 2 * q, pf + r * PFW + 2 * q);
+    }
+  };
+  stage(own, e);
+  const int k0 = __ldg(fc.slot_ptr + e), k1 = __ldg(fc.slot_ptr + e + 1);
+  const int ct = cell_type(g, e);
+  const int j = lane / NP, i = lane % NP;
+  for (int kb = k0; kb < k1; kb += SPW) {
+    const int nsl = min(SPW, k1 - kb);
+    const bool live = j < nsl;  // lanes past the last slot follow it
+    const int sl = kb + (live ? j : 0);
+    const int4 r0 = __ldg(st.rec + 2 * (size_t)sl), r1 = __ldg(st.rec + 2 * (size_t)sl + 1);
+    for (int q = 0; q < nsl; ++q) {
+      const int c = __shfl_sync(0xffffffffu, r0.x, q * NP);
+      if (c >= 0) stage(nb + q * S * RW, c);
+    }
+    cp_async_wait_all();
+    __syncwarp();
+    const int f = r1.x, fl = r1.y;
+    const bool is_owner = (fl & 1) == 0;
+    const bool bnd = (fl & 2) != 0;
+    const double side = (fl & 16) ? 1.0 : -1.0;
+    double ow[NF], ot[NF];
+#pragma unroll
+    for (int k = 0; k < NF; ++k) ow[k] = ot[k] = 0.0;
+    auto add = [&](double (&o)[NF], double w, const double* row) {
+      const double2* x = reinterpret_cast<const double2*>(row);
+#pragma unroll
+      for (int q = 0; q < (NF + 1) / 2; ++q) {
+        const double2 v = x[q];
+        o[2 * q] += w * v.x;
+        if (2 * q + 1 < NF) o[2 * q + 1] += w * v.y;
+      }
+    };
+    {
+      const int gr = (ct * 3 + ((fl >> 2) & 3)) * 2 + ((fl & 16) ? 1 : 0);
+      const int n = __ldg(ops.ex_n + gr * NP + i);
+      const size_t at = (size_t)gr * S * NP + i;
+#pragma unroll 3
+      for (int k = 0; k < n; ++k)
+        add(ow, __ldg(ops.ex_w + at + (size_t)k * NP), own + __ldg(ops.ex_i + at + (size_t)k * NP) * RW);
+    }
+    const double* nr = nb + (live ? j : 0) * S * RW;
+    if (r0.x >= 0) {
+      const double* M = (is_owner ? fc.nb_m0 : fc.ow_m0) + (size_t)r0.y * S * NP + i;
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) add(ot, __ldg(M + s * NP), nr + s * RW);
+    }
+    if (__any_sync(0xffffffffu, r0.z >= 0)) {
+      // second sources, into the same rows
+      __syncwarp();
+      for (int q = 0; q < nsl; ++q) {
+        const int c = __shfl_sync(0xffffffffu, r0.z, q * NP);
+        if (c >= 0) stage(nb + q * S * RW, c);
+      }
+      cp_async_wait_all();
+      __syncwarp();
+      if (r0.z >= 0) {
+        const double* M = (is_owner ? fc.nb_m1 : fc.ow_m1) + (size_t)r0.w * S * NP + i;
+#pragma unroll 8
+        for (int s = 0; s < S; ++s) add(ot, __ldg(M + s * NP), nr + s * RW);
+      }
+    }
+    __syncwarp();  // the rows are consumed
+    if (live && lane < SPW * NP)
+      face_jump<S, NP, VISC>(g, fc, bc, sl, i, e, f, is_owner, bnd, side, ow, ot, arow, mu, J);
+  }
+}
+
+template <int S, int NP, bool VISC>
+__global__ void __launch_bounds__(32 * FACE_WARPS, 4)
+    k_face(Geom g, Ops ops, Faces fc, Bc bc, SlotTable st, const double* __restrict__ PF,
+           const double4* __restrict__ arow, double mu, double* __restrict__ J) {
+  constexpr int SPW = 32 / NP, MT = (NP + 7) / 8, NF = VISC ? FW_F : 5, NT = (NF + 7) / 8;
+  // own side from the rows' nonzeros at P2; at P3, where the reference's rows
+  // are up to full, on the tensor path too (24,576 P3 tets: 500 us with the rows)
+  constexpr bool ROWS = S <= 27;
+  __shared__ double sOt[FACE_WARPS][SPW * NP * NF];
+  __shared__ double sOw[ROWS ? 1 : FACE_WARPS][ROWS ? 1 : SPW * NP * NF];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sl0 = (blockIdx.x * FACE_WARPS + warp) * SPW;
+  if (sl0 >= st.n) return;  // whole warps; warp-level synchronisation only
+  const int nsl = min(SPW, st.n - sl0);
+  double* ot_s = sOt[warp];
+  for (int j = 0; j < nsl; ++j) {
+    const int4 r0 = __ldg(st.rec + 2 * (size_t)(sl0 + j)), r1 = __ldg(st.rec + 2 * (size_t)(sl0 + j) + 1);
+    const bool is_owner = (r1.y & 1) == 0;
+    double* ot = ot_s + j * NP * NF;
+    if constexpr (!ROWS) {
+      const int gr = (cell_type(g, r1.z) * 3 + ((r1.y >> 2) & 3)) * 2 + ((r1.y & 16) ? 1 : 0);
+      const double* pf = PF + (size_t)r1.z * S * PFW;
+      double* ow = sOw[warp] + j * NP * NF;
+      dmma_warp_rb_f<MT, NT, S>(
+          NP, NF, ops.fextrap + (size_t)gr * (MT * ((S + 3) / 4) * 32),
+          [&](int s, int n) { return __ldg(pf + s * PFW + n); }, [&](int i, int n, double x) { ow[i * NF + n] = x; });
+    }
+    for (int src = 0; src < 2; ++src) {
+      const int c = src == 0 ? r0.x : r0.z;
+      if (c < 0) {
+        if (src == 0)
+          for (int t = lane; t < NP * NF; t += 32) ot[t] = 0.0;
+        continue;
+      }
+      const double* M = (src == 0 ? (is_owner ? fc.nb_m0 : fc.ow_m0) : (is_owner ? fc.nb_m1 : fc.ow_m1)) +
+                        (size_t)(src == 0 ? r0.y : r0.w) * S * NP;
+      const double* pc = PF + (size_t)c * S * PFW;
+      __syncwarp();
+      dmma_warp_rb<MT, NT, S>(
+          NP, NF, [&](int i, int s) { return __ldg(M + s * NP + i); },
+          [&](int s, int n) { return __ldg(pc + s * PFW + n); },
+          [&](int i, int n, double x) {
+            if (src == 0) ot[i * NF + n] = x;
+            else ot[i * NF + n] += x;
+          });
+    }
+  }
+  __syncwarp();
+  const int j = lane / NP, i = lane % NP;
+  if (j >= nsl || lane >= SPW * NP) return;
+  const int sl = sl0 + j;
+  const int4 r1 = __ldg(st.rec + 2 * (size_t)sl + 1);
+  const int fl = r1.y, e = r1.z;
+  double ow[NF], ot[NF];
+#pragma unroll
+  for (int k = 0; k < NF; ++k) {
+    ow[k] = ROWS ? 0.0 : sOw[ROWS ? 0 : warp][ROWS ? 0 : (j * NP + i) * NF + k];
+    ot[k] = ot_s[(j * NP + i) * NF + k];
+  }
+  if constexpr (ROWS) {
+    const int gr = (cell_type(g, e) * 3 + ((fl >> 2) & 3)) * 2 + ((fl & 16) ? 1 : 0);
+    const int n = __ldg(ops.ex_n + gr * NP + i);
+    const size_t at = (size_t)gr * S * NP + i;
+    const double* pf = PF + (size_t)e * S * PFW;
+#pragma unroll 3
+    for (int k = 0; k < n; ++k) {
+      const double w = __ldg(ops.ex_w + at + (size_t)k * NP);
+      const double2* x = reinterpret_cast<const double2*>(pf + __ldg(ops.ex_i + at + (size_t)k * NP) * PFW);
+#pragma unroll
+      for (int q = 0; q < (NF + 1) / 2; ++q) {
+        const double2 v = __ldg(x + q);
+        ow[2 * q] += w * v.x;
+        if (2 * q + 1 < NF) ow[2 * q + 1] += w * v.y;
+      }
+    }
+  }
+  face_jump<S, NP, VISC>(g, fc, bc, sl, i, e, r1.x, (fl & 1) == 0, (fl & 2) != 0, (fl & 16) ? 1.0 : -1.0, ow, ot, arow,
+                         mu, J);
 }
 
 // own adjugate row of the face's axis at every slot flux point (E * adj) and
@@ -630,8 +744,8 @@ constexpr int CELL_MAXSLOT = 6;  // slots per cell staged in shared memory (more
 
 template <int S, int FN, int CPB, int NPMAX>
 struct CellSmem {
-  static constexpr int oPF = 0;                    // CPB*S*16
-  static constexpr int oAdj = oPF + CPB * S * PFW; // CPB*S*9
+  static constexpr int oPF = 0;                    // CPB*S*PFS
+  static constexpr int oAdj = oPF + CPB * S * PFS; // CPB*S*9
   static constexpr int oU = oAdj + CPB * S * 9;    // CPB*S*US
   static constexpr int oDet = oU + CPB * S * US;    // CPB*S
   static constexpr int oRi = oDet + CPB * S;       // CPB*S*5
@@ -670,7 +784,8 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
 
   double* sAf = sm + L::oAf;
   // ---- load: asynchronous 8-byte copies, all in flight at once ----
-  for (int t = tid; t < nc * S * PFW; t += blockDim.x) cp_async8(sPF + t, a.PF + (size_t)e0 * S * PFW + t);
+  for (int t = tid; t < nc * S * PFW; t += blockDim.x) 
+    cp_async8(sPF + (t / PFW) * PFS + t % PFW, a.PF + (size_t)e0 * S * PFW + t);
   for (int t = tid; t < nc * S * 9; t += blockDim.x) cp_async8(sAdj + t, g.adj + (size_t)e0 * S * 9 + t);
   for (int t = tid; t < nc * S * nv; t += blockDim.x)
     cp_async8(sU + (t / nv) * US + t % nv, a.Ucur + (size_t)e0 * S * nv + t);
@@ -691,13 +806,13 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   {
     dmma_product_rb<(5 * CPB + 7) / 8>(
         FN, 5 * nc, S, ops.fc2f[ct],
-        [&](int s, int col) { return sPF[((col / 5) * S + s) * PFW + col % 5]; },
+        [&](int s, int col) { return sPF[((col / 5) * S + s) * PFS + col % 5]; },
         [&](int i, int col, double x) { sQf[((col / 5) * FN + i) * 5 + col % 5] = x; });
   }
   if (visc) {
     for (int t = tid; t < nc * S; t += blockDim.x) {
       double G[3][4];
-      const double* p = sPF + t * PFW;
+      const double* p = sPF + t * PFS;
       viscous_flux_sym(p + 1, p + 5, p + 11, a.mu, p[14], G);
       const double* am = sAdj + t * 9;
       for (int m = 0; m < 3; ++m) {

@@ -404,7 +404,12 @@ __global__ void __launch_bounds__(32 * PX_WARPS, sizeof(T) == 8 ? 2 : (N1 == 3 ?
   for (int it = lane; it < CW * MT; it += 32) {
     const int c = it / MT, t = it - c * MT;
     T* sc = sw + c * L::cell;
-    T af[D ? 1 : 9][D ? 1 : NF];
+    T af[D ? 1 : 9][D ? 1 : NF], an[D ? 9 : 1];
+    const T* ap = pg.adjf + (size_t)(e0 + (c < nc ? c : 0)) * NF * 9 * MT + t;
+    if constexpr (D) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) an[k] = __ldg(ap + k * MT);
+    }
     if constexpr (!D) {
       const float* ap = pg.adjf + ((size_t)(e0 + (c < nc ? c : 0)) * 9 * MT + t) * NF;
 #pragma unroll
@@ -447,8 +452,12 @@ __global__ void __launch_bounds__(32 * PX_WARPS, sizeof(T) == 8 ? 2 : (N1 == 3 ?
       T al[9];
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
-        if constexpr (D) al[k] = __ldg(pg.adjf + (((size_t)(e0 + (c < nc ? c : 0)) * NF + l) * 9 + k) * MT + t);
-        else al[k] = af[k][l];
+        if constexpr (D) {
+          al[k] = an[k];  // loaded one level ahead
+          if (l + 1 < NF) an[k] = __ldg(ap + ((l + 1) * 9 + k) * MT);
+        } else {
+          al[k] = af[k][l];
+        }
       }
       if constexpr (D) {
         // the flux itself (density floored as in the plain Euler flux), less
