@@ -367,8 +367,13 @@ cudaError_t sst_launch(afr_handle* h, const SstArgs& a, cudaStream_t st, StepTim
 
 template <int S, int FN, int NP, int N1D>
 struct Launch {
-  static constexpr int CPB = S <= 8 ? 8 : (S <= 27 ? 2 : 1);
-  static size_t cell_smem() { return sizeof(double) * CellSmem<S, FN, CPB, NP>::total; }
+  // cells per CTA of the generic cell kernel.  P3 without viscosity: three, whose
+  // 15 columns fill two tensor tiles and share each 98 KB pass over the W image
+  // (one cell's five columns leave three of eight idle); with viscosity their
+  // tiles would not fit.
+  static constexpr int CPB = S <= 8 ? 8 : (S <= 27 ? 2 : 1), CPBI = S == 64 ? 3 : CPB;
+  static constexpr int cell_smem_v = (int)sizeof(double) * CellSmem<S, FN, CPB, NP, true>::total;
+  static constexpr int cell_smem_i = (int)sizeof(double) * CellSmem<S, FN, CPBI, NP, false>::total;
   // structured prisms: one kernel forms the face-point fields and the volume terms
   static constexpr bool PXD = S == 8 || S == 27;
   static constexpr int PXN1 = S == 8 ? 2 : 3, PXNF = S == 8 ? 3 : 4, PXC = S == 8 ? 6 : 2;
@@ -392,8 +397,8 @@ struct Launch {
   // shared-memory limits of the plain form's kernels, once per process
   static void set_attrs() {
     static const bool done = [] {
-      const size_t smem = cell_smem();
-      cudaFuncSetAttribute(k_cell<S, FN, NP, CPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_cell<S, FN, NP, CPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_v);
+      cudaFuncSetAttribute(k_cell<S, FN, NP, CPBI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_i);
       if constexpr (S == 8) {
         cudaFuncSetAttribute(k_face_staged<S, NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              FaceSmem<S, NP, false>::total);
@@ -465,7 +470,6 @@ struct Launch {
       }
     }
     if (tm) tm->mark(st);
-    const size_t smem = cell_smem();
     a.N = h->N;
     a.slot_flags = h->slots.flags;
     const int ranges[3] = {0, h->n_prism, h->N};
@@ -480,7 +484,12 @@ struct Launch {
             h->ops, h->fc, a, r, h->RVd, h->J, h->pgd.rdet);
         continue;
       }
-      k_cell<S, FN, NP, CPB><<<(n + CPB - 1) / CPB, CELL_THREADS, smem, st>>>(h->g, h->ops, h->fc, a, h->J);
+      if (a.inviscid_only)
+        k_cell<S, FN, NP, CPBI, false><<<(n + CPBI - 1) / CPBI, CELL_THREADS, cell_smem_i, st>>>(h->g, h->ops, h->fc, a,
+                                                                                             h->J);
+      else
+        k_cell<S, FN, NP, CPB, true><<<(n + CPB - 1) / CPB, CELL_THREADS, cell_smem_v, st>>>(h->g, h->ops, h->fc, a,
+                                                                                         h->J);
     }
     return cudaGetLastError();
   }

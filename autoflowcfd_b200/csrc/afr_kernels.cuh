@@ -732,7 +732,8 @@ __global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __
 }
 
 // ---------------------------------------------------------------------------
-// cell kernel: CPB cells per CTA.  Volume terms (inviscid over-integrated
+// cell kernel: CPB cells per CTA (structured prisms of orders 1 and 2 take
+// k_px_cell and k_update).  Volume terms (inviscid over-integrated
 // divergence with W = f2c * D_fine folded at create, viscous divergence),
 // lifting of the face jumps of each cell's slots in ascending color order,
 // outlier suppression, then (stage >= 0) the SSP-RK3 Shu-Osher combination,
@@ -742,28 +743,33 @@ __global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __
 constexpr int CELL_THREADS = 256;
 constexpr int CELL_MAXSLOT = 6;  // slots per cell staged in shared memory (more: read from global)
 
-template <int S, int FN, int CPB, int NPMAX>
+// Doubles of each block.  Without viscosity only q of the point fields, the
+// inviscid jumps and residuals are held, so more CTAs fit an SM.
+template <int S, int FN, int CPB, int NPMAX, bool VISC>
 struct CellSmem {
-  static constexpr int oPF = 0;                    // CPB*S*PFS
-  static constexpr int oAdj = oPF + CPB * S * PFS; // CPB*S*9
-  static constexpr int oU = oAdj + CPB * S * 9;    // CPB*S*US
-  static constexpr int oDet = oU + CPB * S * US;    // CPB*S
+  static constexpr int PS = VISC ? PFS : 5;        // point-field row stride
+  static constexpr int JF = VISC ? 9 : 5;          // jump fields
+  static constexpr int oPF = 0;                    // CPB*S*PS
+  static constexpr int oAdj = oPF + CPB * S * PS;  // CPB*S*9
+  static constexpr int oU = oAdj + (VISC ? CPB * S * 9 : 0);  // CPB*S*US
+  static constexpr int oDet = oU + CPB * S * US;   // CPB*S: det, then 1 / det
   static constexpr int oRi = oDet + CPB * S;       // CPB*S*5
   static constexpr int oRv = oRi + CPB * S * 5;    // CPB*S*5
-  static constexpr int oQf = oRv + CPB * S * 5;    // CPB*FN*5
+  static constexpr int oQf = oRv + (VISC ? CPB * S * 5 : 0);  // CPB*FN*5
   static constexpr int oFt = oQf + CPB * FN * 5;   // CPB*FN*15
-  static constexpr int oGt = oFt + CPB * FN * 15;  // CPB*S*15
-  static constexpr int oJ = oGt + CPB * S * 15;    // staged jumps of the CTA's slots
-  static constexpr int oWp = oJ + CPB * CELL_MAXSLOT * NPMAX * 9;  // 2 halves of the W divergence
-  static constexpr int oAf = oWp + 2 * CPB * S * 5;  // CPB*FN*9 adjugates at the fine points
-  static constexpr int work = oAf + CPB * FN * 9;     // CPB*2*OUT_WORK (outliers) + 32
-  static constexpr int total = work + CPB * 2 * OUT_WORK + 32;
+  static constexpr int oGt = oFt + CPB * FN * 15;  // CPB*S*15; with or without viscosity the norm terms (2*CPB*S)
+  static constexpr int oJ = oGt + (VISC ? CPB * S * 15 : CPB * S * 2);  // staged jumps of the CTA's slots
+  static constexpr int oAf = oJ + CPB * CELL_MAXSLOT * NPMAX * JF;      // CPB*FN*9 adjugates at the fine points
+  static constexpr int work = oAf + CPB * FN * 9;  // CPB*2*OUT_WORK (outliers)
+  static constexpr int oG = work + CPB * 2 * OUT_WORK;  // g_left, g_right (8)
+  static constexpr int oI = oG + 8;                // ints: lifting maps (6*S), slot flags, slot pointers
+  static constexpr int total = oI + (6 * S + CPB * CELL_MAXSLOT + CPB + 2) / 2 + 1;
 };
 
-template <int S, int FN, int NP, int CPB>
+template <int S, int FN, int NP, int CPB, bool VISC>
 __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces fc, StageArgs a,
                                                           const double* __restrict__ J) {
-  using L = CellSmem<S, FN, CPB, NP>;
+  using L = CellSmem<S, FN, CPB, NP, VISC>;
   extern __shared__ double sm[];
   double* sPF = sm + L::oPF;
   double* sAdj = sm + L::oAdj;
@@ -775,18 +781,27 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   double* sFt = sm + L::oFt;
   double* sGt = sm + L::oGt;
   double* work = sm + L::work;
+  double* sG = sm + L::oG;
+  int* sDfp = reinterpret_cast<int*>(sm + L::oI);
+  int* sDco = sDfp + 3 * S;
+  int* sFl = sDco + 3 * S;
+  int* sPtr = sFl + CPB * CELL_MAXSLOT;
   const int e0 = a.cell_base + blockIdx.x * CPB;
   const int nc = min(CPB, a.cell_end - e0);
   const int ct = cell_type(g, e0);  // a launch covers cells of one type
   const int nv = a.nv;
-  const bool visc = !a.inviscid_only;
+  constexpr bool visc = VISC;
+  constexpr int PS = L::PS;
   const int tid = threadIdx.x;
 
   double* sAf = sm + L::oAf;
   // ---- load: asynchronous 8-byte copies, all in flight at once ----
-  for (int t = tid; t < nc * S * PFW; t += blockDim.x) 
-    cp_async8(sPF + (t / PFW) * PFS + t % PFW, a.PF + (size_t)e0 * S * PFW + t);
-  for (int t = tid; t < nc * S * 9; t += blockDim.x) cp_async8(sAdj + t, g.adj + (size_t)e0 * S * 9 + t);
+  for (int t = tid; t < nc * S * (VISC ? PFW : 5); t += blockDim.x) {
+    const int p = t / (VISC ? PFW : 5), k = t % (VISC ? PFW : 5);
+    cp_async8(sPF + p * PS + k, a.PF + ((size_t)e0 * S + p) * PFW + k);
+  }
+  if (VISC)
+    for (int t = tid; t < nc * S * 9; t += blockDim.x) cp_async8(sAdj + t, g.adj + (size_t)e0 * S * 9 + t);
   for (int t = tid; t < nc * S * nv; t += blockDim.x)
     cp_async8(sU + (t / nv) * US + t % nv, a.Ucur + (size_t)e0 * S * nv + t);
   for (int t = tid; t < nc * S; t += blockDim.x) cp_async8(sDet + t, g.det + (size_t)e0 * S + t);
@@ -795,9 +810,26 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   const int k_beg = fc.slot_ptr[e0], k_end = fc.slot_ptr[e0 + nc];
   const bool staged = (k_end - k_beg) <= CPB * CELL_MAXSLOT;
   double* sJ = sm + L::oJ;
-  if (staged)
-    for (int t = tid; t < (k_end - k_beg) * NP * 9; t += blockDim.x)
-      cp_async8(sJ + t, J + (size_t)k_beg * NP * 9 + t);
+  constexpr int JF = L::JF;
+  if (staged) {
+    for (int t = tid; t < (k_end - k_beg) * NP * JF; t += blockDim.x) {
+      const int k = t / (NP * JF), r = t - k * (NP * JF);
+      cp_async8(sJ + t, J + (size_t)(k_beg + k) * 9 * NP + r);
+    }
+    for (int t = tid; t < k_end - k_beg; t += blockDim.x) sFl[t] = __ldg(a.slot_flags + k_beg + t);
+  }
+  // the lifting's maps: read per slot and point below, where each was a chain
+  // of dependent global loads
+  constexpr int N1D = S == 8 ? 2 : (S == 27 ? 3 : 4);
+  for (int t = tid; t < 3 * S; t += blockDim.x) {
+    sDfp[t] = __ldg(ops.dist_fp + t);
+    sDco[t] = __ldg(ops.dist_co + t);
+  }
+  if (tid < N1D) {
+    sG[tid] = ops.g_left[tid];
+    sG[4 + tid] = ops.g_right[tid];
+  }
+  if (tid <= nc) sPtr[tid] = __ldg(fc.slot_ptr + e0 + tid);
   cp_async_wait_all();
   __syncthreads();
 
@@ -806,13 +838,13 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   {
     dmma_product_rb<(5 * CPB + 7) / 8>(
         FN, 5 * nc, S, ops.fc2f[ct],
-        [&](int s, int col) { return sPF[((col / 5) * S + s) * PFS + col % 5]; },
+        [&](int s, int col) { return sPF[((col / 5) * S + s) * PS + col % 5]; },
         [&](int i, int col, double x) { sQf[((col / 5) * FN + i) * 5 + col % 5] = x; });
   }
-  if (visc) {
+  if constexpr (VISC) {
     for (int t = tid; t < nc * S; t += blockDim.x) {
       double G[3][4];
-      const double* p = sPF + t * PFS;
+      const double* p = sPF + t * PS;
       viscous_flux_sym(p + 1, p + 5, p + 11, a.mu, p[14], G);
       const double* am = sAdj + t * 9;
       for (int m = 0; m < 3; ++m) {
@@ -823,6 +855,7 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
     }
   }
   __syncthreads();
+  for (int t = tid; t < nc * S; t += blockDim.x) sDet[t] = 1.0 / sDet[t];  // each use within an ulp of a division
   // ---- Euler fluxes at fine points, contravariant with adj_fine ----
   for (int t = tid; t < nc * FN; t += blockDim.x) {
     const int b = t / FN, i = t % FN;
@@ -841,20 +874,24 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   // the fine-point fluxes, viscous D3 (S x 3S) to the point fluxes; rows the
   // solution points, columns (cell, variable) ----
   {
-    dmma_product_f(
-        S, 5 * nc, FN * 3, ops.fW[ct],
-        [&](int k, int col) { return sFt[(col / 5) * FN * 15 + k * 5 + col % 5]; },
-        [&](int s, int col, double x) {
-          const int b = col / 5;
-          sRi[(b * S + s) * 5 + col % 5] = -x / sDet[b * S + s];
-        });
-    if (visc) {
+    auto fb = [&](int k, int col) { return sFt[(col / 5) * FN * 15 + k * 5 + col % 5]; };
+    auto fo = [&](int s, int col, double x) {
+      const int b = col / 5;
+      sRi[(b * S + s) * 5 + col % 5] = -x * sDet[b * S + s];
+    };
+    // with as many row tiles as warps, each warp keeps its operator fragment for
+    // every column tile
+    if constexpr ((S + 7) / 8 >= CELL_THREADS / 32 && 5 * CPB > 8)
+      dmma_product_rb<(5 * CPB + 7) / 8>(S, 5 * nc, FN * 3, ops.fW[ct], fb, fo);
+    else
+      dmma_product_f(S, 5 * nc, FN * 3, ops.fW[ct], fb, fo);
+    if constexpr (VISC) {
       dmma_product_f(
           S, 5 * nc, S * 3, ops.fD3[ct],
           [&](int k, int col) { return sGt[(col / 5) * S * 15 + k * 5 + col % 5]; },
           [&](int s, int col, double x) {
             const int b = col / 5;
-            sRv[(b * S + s) * 5 + col % 5] = x / sDet[b * S + s];
+            sRv[(b * S + s) * 5 + col % 5] = x * sDet[b * S + s];
           });
     }
   }
@@ -862,20 +899,19 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_cell(Geom g, Ops ops, Faces
   // ---- lift the face jumps of each cell's slots, ascending color order ----
   for (int t = tid; t < nc * S * 5; t += blockDim.x) {
     const int b = t / (S * 5), r = t % (S * 5), s = r / 5, v = r % 5;
-    const int e = e0 + b;
-    const double rdj = 1.0 / sDet[b * S + s];  // each term within an ulp of g' J / det
+    const double rdj = sDet[b * S + s];  // each term within an ulp of g' J / det
     double ci = 0.0, cv = 0.0;
-    for (int k = fc.slot_ptr[e]; k < fc.slot_ptr[e + 1]; ++k) {
-      const int fl = a.slot_flags[k];
+    for (int k = sPtr[b]; k < sPtr[b + 1]; ++k) {
+      const int fl = staged ? sFl[k - k_beg] : a.slot_flags[k];
       const int ax = (fl >> 2) & 3;
-      const int fp = ops.dist_fp[ax * S + s];
-      const double gw = ((fl & 16) ? ops.g_right : ops.g_left)[ops.dist_co[ax * S + s]];
-      const double* Jk = staged ? sJ + (k - k_beg) * 9 * NP + fp : J + (size_t)k * 9 * NP + fp;
+      const int fp = sDfp[ax * S + s];
+      const double gw = sG[((fl & 16) ? 4 : 0) + sDco[ax * S + s]];
+      const double* Jk = staged ? sJ + (k - k_beg) * JF * NP + fp : J + (size_t)k * 9 * NP + fp;
       ci += -(gw * Jk[v * NP]) * rdj;
-      if (visc && v > 0) cv += (gw * Jk[(4 + v) * NP]) * rdj;
+      if (VISC && v > 0) cv += (gw * Jk[(4 + v) * NP]) * rdj;
     }
     sRi[t] = sRi[t] + ci;
-    if (visc) sRv[t] = sRv[t] + cv;
+    if constexpr (VISC) sRv[t] = sRv[t] + cv;
   }
   __syncthreads();
   suppress_outliers_cells<S>(sRi, sRv, sU, nc, visc, work);
