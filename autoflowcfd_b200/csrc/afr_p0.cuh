@@ -54,8 +54,6 @@ __global__ void __launch_bounds__(128) k_p0_face(Geom g, Faces fc, Bc bc, P0Tab 
   double Fc[5];
   ausm_up(qo, qn, n, Fc);
   const double A = t.area[f];
-  double* out = t.flux + (size_t)f * 8;
-  for (int v = 0; v < 5; ++v) out[v] = Fc[v] * A;
   double jv[3] = {0.0, 0.0, 0.0};
   const int pc = t.pen[f];
   if (visc && pc) {
@@ -73,7 +71,11 @@ __global__ void __launch_bounds__(128) k_p0_face(Geom g, Faces fc, Bc bc, P0Tab 
     const double scale = eta * sqrt(a0 * a0 + a1 * a1 + a2 * a2) * side;
     for (int v = 1; v < 4; ++v) jv[v - 1] = -scale * (qo[v] - gq[v]);
   }
-  for (int v = 0; v < 3; ++v) out[5 + v] = jv[v];
+  double2* out = reinterpret_cast<double2*>(t.flux + (size_t)f * 8);  // one 64-byte record
+  out[0] = make_double2(Fc[0] * A, Fc[1] * A);
+  out[1] = make_double2(Fc[2] * A, Fc[3] * A);
+  out[2] = make_double2(Fc[4] * A, jv[0]);
+  if (visc && pc) out[3] = make_double2(jv[1], jv[2]);  // read behind the penalty code only
 }
 
 // one thread per cell: gather the face contributions, then (stage >= 0) the
@@ -87,14 +89,19 @@ __global__ void __launch_bounds__(128) k_p0_cell(Geom g, Ops ops, Faces fc, P0Ta
   const bool visc = !a.inviscid_only;
   double ri[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const double rvol = 1.0 / t.volume[c];
+  // four records' loads in flight, added in ascending order
+#pragma unroll 4
   for (int k = t.cptr[c]; k < t.cptr[c + 1]; ++k) {
-    const int code = t.cref[k];
-    const double* F = t.flux + (size_t)(code >> 1) * 8;
-    if (code & 1) {
-      for (int v = 0; v < 5; ++v) ri[v] += F[v] * rvol;
-    } else {
-      for (int v = 0; v < 5; ++v) ri[v] -= F[v] * rvol;
-    }
+    const int code = __ldg(t.cref + k);
+    const double2* F = reinterpret_cast<const double2*>(t.flux + (size_t)(code >> 1) * 8);
+    const double2 f0 = __ldg(F), f1 = __ldg(F + 1);
+    const double f4 = __ldg(t.flux + (size_t)(code >> 1) * 8 + 4);
+    const double w = (code & 1) ? rvol : -rvol;
+    ri[0] += f0.x * w;
+    ri[1] += f0.y * w;
+    ri[2] += f1.x * w;
+    ri[3] += f1.y * w;
+    ri[4] += f4 * w;
   }
   // viscous corrections of the owner-primary boundary slots, ascending color
   double rv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
