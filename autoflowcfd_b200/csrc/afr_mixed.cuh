@@ -540,8 +540,10 @@ __device__ __forceinline__ void mx_face_jump(const Faces& fc, const SlotTable& s
   const int sl = t / NP, i = t % NP;
   const float4 ar = mf.arow[t];
   const float a0 = ar.x, a1 = ar.y, a2 = ar.z;
-  const float mag = fmaxf(fabsf(ar.w), 1e-30f), rm = side / mag;
-  float dir[3] = {a0 * rm, a1 * rm, a2 * rm};
+  const float mag = fmaxf(fabsf(ar.w), 1e-30f);
+  // divided, not multiplied by 1 / mag: the second rounding would show in the
+  // step's error (P1: 6.8e-9 -> 7.3e-9)
+  float dir[3] = {a0 / mag * side, a1 / mag * side, a2 / mag * side};
   if (ar.w < 0.f) {  // alignment fallback: the face normal, outward from this side
     const int f = st.face[sl];
     const double* tnp = fc.tnormal + ((size_t)f * NP + i) * 3;
@@ -1415,9 +1417,10 @@ __global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow
   {
     // the direction is compared with the face normal in the face kernel's own FP32 arithmetic
     const float4 ar = make_float4(float(a0), float(a1), float(a2), float(sqrt(a0 * a0 + a1 * a1 + a2 * a2)));
-    const float mag = fmaxf(ar.w, 1e-30f), rm = (sb ? 1.f : -1.f) / mag, sg = is_owner ? 1.f : -1.f;
+    const float mag = fmaxf(ar.w, 1e-30f), sd = sb ? 1.f : -1.f, sg = is_owner ? 1.f : -1.f;
     const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
-    const float al = ar.x * rm * (sg * float(tn[0])) + ar.y * rm * (sg * float(tn[1])) + ar.z * rm * (sg * float(tn[2]));
+    const float al = ar.x / mag * sd * (sg * float(tn[0])) + ar.y / mag * sd * (sg * float(tn[1])) +
+                     ar.z / mag * sd * (sg * float(tn[2]));
     arow[t] = make_float4(ar.x, ar.y, ar.z, al < 0.5f ? -mag : ar.w);
   }
   if (bnd) {
