@@ -382,13 +382,13 @@ struct Launch {
   static bool px_range(const afr_handle* h, int r) { return PXD && h->px && r == 0; }
   static cudaError_t px_cell(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
     if constexpr (PXD) {
-      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
+      const int nb = (n + PXC * px_warps(PXN1) - 1) / (PXC * px_warps(PXN1));
       const auto* op = [&] {
         if constexpr (S == 8) return &h->px1;
         else return &h->px2;
       }();
       auto* fn = visc ? k_px_cell<float, PXN1, PXNF, PXC, true> : k_px_cell<float, PXN1, PXNF, PXC, false>;
-      fn<<<nb, 32 * PX_WARPS, PxS::total, st>>>(*op, h->pg, h->mb.XF, h->px_points ? h->mb.PFm : nullptr, h->mb.RV,
+      fn<<<nb, 32 * px_warps(PXN1), PxS::total, st>>>(*op, h->pg, h->mb.XF, h->px_points ? h->mb.PFm : nullptr, h->mb.RV,
                                                 h->mb.FW, h->px_faces, U, h->nv, nut, (float)h->prm.mu, 0, n);
       return cudaGetLastError();
     }
@@ -423,13 +423,13 @@ struct Launch {
   static cudaError_t px_cell64(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
     if constexpr (PXD) {
       set_attrs();
-      const int nb = (n + PXC * PX_WARPS - 1) / (PXC * PX_WARPS);
+      const int nb = (n + PXC * px_warps(PXN1) - 1) / (PXC * px_warps(PXN1));
       const auto* op = [&] {
         if constexpr (S == 8) return &h->pxd1;
         else return &h->pxd2;
       }();
       auto* fn = visc ? k_px_cell<double, PXN1, PXNF, PXC, true> : k_px_cell<double, PXN1, PXNF, PXC, false>;
-      fn<<<nb, 32 * PX_WARPS, PxSD::total, st>>>(*op, h->pgd, nullptr, h->PF, h->RVd, 0, 0u, U, h->nv, nut,
+      fn<<<nb, 32 * px_warps(PXN1), PxSD::total, st>>>(*op, h->pgd, nullptr, h->PF, h->RVd, 0, 0u, U, h->nv, nut,
                                                  h->prm.mu, 0, n);
       return cudaGetLastError();
     }

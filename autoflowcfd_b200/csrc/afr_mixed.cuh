@@ -1150,9 +1150,12 @@ __device__ __noinline__ Vals<PL> outlier_exact(Vals<PL> X, Vals<PL> u, int grp, 
 }
 }  // namespace mxd
 
-// T: float (mixed form) or double (plain form of structured prisms).
+// T: float (mixed form) or double (plain form of structured prisms).  Register
+// caps from timing four, five and six CTAs per SM: P2 float 203 us at five (214
+// at six, 221 at four; 91,200 prisms), P1 float 131 us at six (135 at five; 256,000),
+// P2 double 54 us at four (60 at three; 17,280).
 template <int S, int NP, class T>
-__global__ void __launch_bounds__(128, S == 64 || sizeof(T) == 8 ? 3 : 5)
+__global__ void __launch_bounds__(128, S == 64 ? 3 : (sizeof(T) == 8 ? 4 : (S == 8 ? 6 : 5)))
     k_update(Ops ops, Faces fc, StageArgs a, int ct, const T* __restrict__ RV, const T* __restrict__ Jm,
              const double* __restrict__ rdet) {
   using L = MxUpd<S>;

@@ -34,7 +34,9 @@
 
 namespace afr {
 
-constexpr int PX_WARPS = 4;
+// warps per CTA: P1's 16 KB per warp fill an SM better in pairs (14 warps instead
+// of 12; 256,000 prisms: 319 -> 298 us), P2 is limited by registers
+__host__ __device__ constexpr int px_warps(int n1) { return n1 == 2 ? 2 : 4; }
 
 template <class T, int N1, int NF>
 struct PxOps {
@@ -82,7 +84,7 @@ struct PxSmem {
   static constexpr int nX = MX_XF * FS, nY = 5 * N1 * TP;
   static constexpr int oX = (nH + 3) / 4 * 4, oY = (oX + nX + 3) / 4 * 4, oRef = oY + nY, oF = oRef + 8;
   static constexpr int cell = (oF + 120 / (int)sizeof(T) + 3) / 4 * 4;  // T values per cell
-  static constexpr int total = PX_WARPS * CW * cell * (int)sizeof(T);
+  static constexpr int total = px_warps(N1) * CW * cell * (int)sizeof(T);
 };
 
 // rho H of the Euler flux, rho * (p / (0.4 max(rho, 1e-10)) + |u|^2 / 2) + p over
@@ -99,7 +101,7 @@ __device__ __forceinline__ double px_rhoH(double rho, double p, double u2) {
 // plain form; it writes the point fields, from which k_face extrapolates and
 // interpolates with every entry of the mesh's own operators.
 template <class T, int N1, int NF, int CW, bool VISC>
-__global__ void __launch_bounds__(32 * PX_WARPS, sizeof(T) == 8 ? 2 : (N1 == 3 ? 4 : 3))
+__global__ void __launch_bounds__(32 * px_warps(N1), sizeof(T) == 8 ? (N1 == 3 ? 2 : 4) : (N1 == 3 ? 4 : 7))
     k_px_cell(const __grid_constant__ PxOps<T, N1, NF> op, PxGeom<T> pg, float* __restrict__ XF, T* __restrict__ PF,
               T* __restrict__ RV, int FW, unsigned face_mask, const double* __restrict__ U, int nv,
               const double* __restrict__ nut, T mu, int cell_base, int cell_end) {
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(32 * PX_WARPS, sizeof(T) == 8 ? 2 : (N1 == 3 ?
   extern __shared__ __align__(16) unsigned char smraw[];
   T* smf = reinterpret_cast<T*>(smraw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int e0 = cell_base + (blockIdx.x * PX_WARPS + warp) * CW;
+  const int e0 = cell_base + (blockIdx.x * px_warps(N1) + warp) * CW;
   const int nc = min(CW, cell_end - e0);
   if (nc <= 0) return;  // whole warps; no block barrier below
   T* sw = smf + warp * CW * L::cell;
