@@ -394,27 +394,24 @@ struct Launch {
     }
     return cudaErrorNotSupported;
   }
-  // shared-memory limits of the plain form's kernels, once per process
-  static void set_attrs() {
-    static const bool done = [] {
-      cudaFuncSetAttribute(k_cell<S, FN, NP, CPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_v);
-      cudaFuncSetAttribute(k_cell<S, FN, NP, CPBI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_i);
-      if constexpr (S == 8) {
-        cudaFuncSetAttribute(k_face_staged<S, NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             FaceSmem<S, NP, false>::total);
-        cudaFuncSetAttribute(k_face_staged<S, NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             FaceSmem<S, NP, true>::total);
-      }
-      cudaFuncSetAttribute(k_update<S, NP, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
-      if constexpr (PXD) {
-        cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             PxSD::total);
-        cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             PxSD::total);
-      }
-      return true;
-    }();
-    (void)done;
+  // shared-memory limits of the plain form's kernels on the current device (at create)
+  static cudaError_t set_attrs() {
+    cudaFuncSetAttribute(k_cell<S, FN, NP, CPB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_v);
+    cudaFuncSetAttribute(k_cell<S, FN, NP, CPBI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cell_smem_i);
+    if constexpr (S == 8) {
+      cudaFuncSetAttribute(k_face_staged<S, NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           FaceSmem<S, NP, false>::total);
+      cudaFuncSetAttribute(k_face_staged<S, NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           FaceSmem<S, NP, true>::total);
+    }
+    cudaFuncSetAttribute(k_update<S, NP, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxUpd<S>::bytes(7, 4));
+    if constexpr (PXD) {
+      cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           PxSD::total);
+      cudaFuncSetAttribute(k_px_cell<double, PXN1, PXNF, PXC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           PxSD::total);
+    }
+    return cudaGetLastError();
   }
   // the plain form's structured prisms
   static bool px64_range(const afr_handle* h, int r) {
@@ -422,7 +419,6 @@ struct Launch {
   }
   static cudaError_t px_cell64(afr_handle* h, const double* U, const double* nut, bool visc, int n, cudaStream_t st) {
     if constexpr (PXD) {
-      set_attrs();
       const int nb = (n + PXC * px_warps(PXN1) - 1) / (PXC * px_warps(PXN1));
       const auto* op = [&] {
         if constexpr (S == 8) return &h->pxd1;
@@ -455,7 +451,6 @@ struct Launch {
     return cudaGetLastError();
   }
   static cudaError_t stage(afr_handle* h, StageArgs a, cudaStream_t st, StepTimer* tm = nullptr) {
-    set_attrs();
     if (h->slots.n > 0) {
       if constexpr (S == 8) {
         auto* fn = a.inviscid_only ? k_face_staged<S, NP, false> : k_face_staged<S, NP, true>;
@@ -630,6 +625,7 @@ struct Launch {
 // kernel stand in for the three kernels of a stage.  Gradients (the force
 // integral's pre-pass) use the generic one-point kernels.
 struct LaunchP0 {
+  static cudaError_t set_attrs() { return cudaSuccess; }
   static cudaError_t pre(afr_handle* h, const double* U, const double* nut, bool grads, cudaStream_t st) {
     constexpr int CPB = PreTile<1>::CPB;
     const int ranges[3] = {0, h->n_prism, h->N};
@@ -955,6 +951,10 @@ static void release_alloc(afr_handle* h, const double*& p, size_t n) {
 static int plain_setup(afr_handle* h, cudaStream_t st) {
   const size_t N = h->N, S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism;
   int rc;
+  {
+    const cudaError_t e = dispatch(h, [](auto L) { return decltype(L)::set_attrs(); });
+    if (e != cudaSuccess) return cuda_fail(h, e, "kernel attributes");
+  }
   if ((rc = dalloc(h, &h->slot_rows, ns * P))) return rc;
   double *adjs = nullptr, *adjf = nullptr, *md = nullptr, *rdet = nullptr;
   if (h->px64 && ((rc = dalloc(h, &adjs, NP * S * 9)) || (rc = dalloc(h, &adjf, NP * Fn * 9)) ||
@@ -1691,10 +1691,14 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
           srec[2 * (size_t)k + 1] = make_int4(f, sflg[k], (int)c, 0);
         }
       }
-    int32_t *d_f, *d_c, *d_fl, *d_0, *d_1, *d_i1;
+    // the mixed form's face kernel finds its sources per slot, the plain form's
+    // in the records
+    const bool mixed = prm->precision == AFR_PREC_MIXED;
+    int32_t *d_f, *d_c, *d_fl, *d_0 = nullptr, *d_1 = nullptr, *d_i1 = nullptr;
     if ((rc = upload(h, &d_f, sf.data(), ns, st)) || (rc = upload(h, &d_c, sc.data(), ns, st)) ||
-        (rc = upload(h, &d_fl, sflg.data(), ns, st)) || (rc = upload(h, &d_0, s0.data(), ns, st)) ||
-        (rc = upload(h, &d_1, s1.data(), ns, st)) || (rc = upload(h, &d_i1, si1.data(), ns, st)))
+        (rc = upload(h, &d_fl, sflg.data(), ns, st)) ||
+        (mixed && ((rc = upload(h, &d_0, s0.data(), ns, st)) || (rc = upload(h, &d_1, s1.data(), ns, st)) ||
+                   (rc = upload(h, &d_i1, si1.data(), ns, st)))))
       return bail(rc);
     int4* d_rec = nullptr;
     if (!srec.empty() && (rc = upload(h, &d_rec, srec.data(), srec.size(), st))) return bail(rc);
@@ -1889,6 +1893,15 @@ int afr_step(afr_handle* h, double* U, double* k, double* omega, double* nu_t, d
 namespace {
 int imp_buffers(afr_handle* h) {
   if (h->iRinv) return AFR_OK;
+  cudaError_t e = cudaSuccess;
+  const auto lim = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  switch (h->order) {
+    case 0: e = cudaFuncSetAttribute(k_dual_stage<1>, lim, DualDims<1>::bytes(7)); break;
+    case 1: e = cudaFuncSetAttribute(k_dual_stage<8>, lim, DualDims<8>::bytes(7)); break;
+    case 2: e = cudaFuncSetAttribute(k_dual_stage<27>, lim, DualDims<27>::bytes(7)); break;
+    default: e = cudaFuncSetAttribute(k_dual_stage<64>, lim, DualDims<64>::bytes(7));
+  }
+  if (e != cudaSuccess) return cuda_fail(h, e, "dual-time kernel");
   const size_t n = (size_t)h->N * h->S * h->nv;
   int rc;
   if ((rc = dalloc(h, &h->iRinv, n)) || (rc = dalloc(h, &h->iRvisc, n)) || (rc = dalloc(h, &h->iRscr, n)) ||
@@ -1930,9 +1943,6 @@ int imp_norm(afr_handle* h, const ImpArgs& a, int mode, cudaStream_t st, double*
 extern "C++" {  // a template inside the C block
 template <int S>
 cudaError_t dual_stage_launch(afr_handle* h, const ImpArgs& a, bool last, cudaStream_t st) {
-  static const cudaError_t attr = cudaFuncSetAttribute(k_dual_stage<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       DualDims<S>::bytes(7));
-  if (attr != cudaSuccess) return attr;
   constexpr int per = DUAL_WARPS * DualDims<S>::CW;
   const int ranges[3] = {0, h->n_prism, h->N};
   for (int r = 0; r < 2; ++r) {
