@@ -1,7 +1,9 @@
 // Mixed-precision form of the FR residual-and-update stage.
 //
-// The operator contractions run on the tensor cores (tcgen05, BF16 inputs,
-// FP32 accumulation in tensor memory) as three-term hi+lo split products,
+// Prisms whose operators are tensor products take the FP32 cell kernel
+// (afr_prism.cuh) in place of k_mx_pre and k_mx_vol.  Elsewhere (tets, P3) the
+// operator contractions run on the tensor cores (tcgen05, BF16 inputs, FP32
+// accumulation in tensor memory) as three-term hi+lo split products,
 // D = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi, which carry about 16 significant bits
 // of each factor.  Pointwise fluxes are FP32.  FP64 is kept for the state, the
 // geometry metrics, the primitive recovery from the conserved state, the

@@ -68,8 +68,9 @@ class B200FRSolver:
         global_dt_factor: > 0 selects time-accurate global stepping
             dt = factor * min(dt_local).
         precision: "fp64" (plain form, FP64 throughout) or "mixed" (operator
-            contractions as BF16 hi+lo split tensor-core products with FP32
-            accumulation, FP32 fluxes; FP64 state, metrics, norms and Cd/Cl).
+            contractions in FP32 on tensor-product prisms, elsewhere as BF16
+            hi+lo split tensor-core products with FP32 accumulation; FP32
+            fluxes; FP64 state, metrics, norms and Cd/Cl).
         device: CUDA device.
         mixed_ignore_conditioning: build the mixed form even for operators
             whose row l1 norms exceed its FP32-accumulation bound (to measure

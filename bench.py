@@ -10,8 +10,8 @@ generated mesh of the reference's own hex-splitting template.
 
 A step is one ``afr_step`` (local dt, SST source/transport/update, three RK
 stages).  metric = DOF-updates/s = n_cells * 27 SPs * 5 variables * 3 stages
-per step / time.  ``value`` is the mixed-precision form (BF16 hi+lo split
-tensor-core contractions, FP32 fluxes, FP64 state) timed with device-resident
+per step / time.  ``value`` is the mixed-precision form (FP32 contractions
+and fluxes on the structured prisms, FP64 state) timed with device-resident
 inputs; the plain FP64 form runs in the same process from the same start
 state (``plain_fp64``), and ``accuracy`` compares the two forms per field over
 steps 1-6 (before the SST growth) and Cd.
@@ -109,57 +109,82 @@ C2_BYTES_PER_CELL_STAGE = 3 * 8 * 7 * 27 + 8 * 10 * 27 + 8 * 9 * 64 + 8 * 3 * 9 
     + 8 * 27 + 8 * 6 * 27 / 3
 
 # DRAM bytes per cell and launch of the mixed stage kernels, measured with ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum) on the 76,800-prism P2 SST
+# (dram__bytes.sum.per_second x duration) on a 91,200-prism P2 SST
 # case; a full-size launch moves these times the number of cells.
-MEASURED_TRAFFIC_PER_CELL = {"k_mx_pre": 8353.0, "k_mx_face": 7101.0, "k_mx_vol": 9921.0, "k_mx_update": 6126.0}
+MEASURED_TRAFFIC_PER_CELL = {"k_px_cell": 9250.0, "k_mx_face": 5337.0, "k_update": 5820.0}
 
 
-def mixed_algorithmic_bytes(case, nv=7):
-    """Minimum bytes each per-stage kernel of the mixed form must move (every
-    array it reads or writes once, in the layout the form stores).
-
-    k_mx_pre: state, FP32 inverse-Jacobian rows (3 x 16 B), nu_t in; FP32
-    point fields (20 per point) and face-point fields (18 per face point, 6*P
-    per cell) out.
-    k_mx_face: both sides' face-point fields, the slot's adjugate row (16 B),
-    other-side index (1 B), true normal (24 B) per slot flux point, jumps out.
-    k_mx_vol: state, FP32 point fields, FP32 adjugate rows at solution and fine
-    points (3 x 16 B each), reciprocal det, metric divergence in; FP32 volume
-    terms (10 per point) out.
-    k_mx_update: volume terms, jumps, current and step-start state, dt,
-    reciprocal det in; next state out."""
-    N, S, Fn = int(case["n_cells"]), int(case["n_sps"]), int(case["n_fine"])
-    P = case["true_normal"].shape[1]
+def _slot_counts(case):
+    """Residual slots (primary face sides) of a case and its points per face."""
     isb = case["is_boundary"].astype(bool)
     slots = int(np.sum(case["owner_is_primary"].astype(bool))) + \
         int(np.sum(~isb & case["neighbor_is_primary"].astype(bool)))
-    sp = slots * P
-    pre = N * S * (8 * (nv + 1) + 48) + N * S * 20 * 4 + N * 18 * 6 * P * 4
-    face = sp * (2 * 18 * 4 + 16 + 1 + 24 + 10 * 4) + slots * 24
-    vol = N * S * (8 * (nv + 1 + 3) + 48) + N * S * 20 * 4 + N * Fn * 48 + N * S * 10 * 4
-    upd = N * S * 10 * 4 + sp * 10 * 4 + N * S * 8 * (3 * nv + 2) + slots * 4
-    return {"k_mx_pre": pre, "k_mx_face": face, "k_mx_vol": vol, "k_mx_update": upd}
+    return slots, case["true_normal"].shape[1]
 
 
-def algorithmic_bytes(case, nv=7):
-    """Minimum bytes each per-stage kernel of the plain FP64 form must move (every array once).
+def mixed_algorithmic_bytes(case, nv=7):
+    """Minimum bytes each per-stage kernel of the mixed form must move on
+    structured prisms (every array it reads or writes once, in the layout the
+    form stores).
 
-    k_face: point fields of every cell (18 doubles per point), adjugates, the
-    interpolation matrices of every residual slot, normals, slot metadata, and
-    the jumps it writes (10 doubles per slot flux point).
-    k_cell: point fields, adjugates, fine-point adjugates, det, dt, current and
-    step-start state, the state it writes, and the jumps it reads."""
+    k_px_cell: state, nu_t, FP32 adjugates at solution and fine points (36 B
+    each), reciprocal det, metric divergence in; face-point fields (15 per
+    point of the five faces that slots read) and FP32 volume terms (9 per
+    point) out.
+    k_mx_face: every slot's own face-point row once (a pair reads both sides'),
+    adjugate row (16 B), half a 16 B pair record in; jumps (9) out.
+    k_update: volume terms, jumps, current and step-start state, dt,
+    reciprocal det in; next state out."""
     N, S, Fn = int(case["n_cells"]), int(case["n_sps"]), int(case["n_fine"])
-    P = case["true_normal"].shape[1]
+    slots, P = _slot_counts(case)
+    sp = slots * P
+    px = N * S * (8 * (nv + 1) + 36 + 8 + 24) + N * Fn * 36 + sp * 15 * 4 + N * S * 9 * 4
+    face = sp * (15 * 4 + 16 + 8 + 9 * 4)
+    upd = N * S * 9 * 4 + sp * 9 * 4 + N * S * 8 * (3 * nv + 2) + slots * 4
+    return {"k_px_cell": px, "k_mx_face": face, "k_update": upd}
+
+
+def prism_fp64_algorithmic_bytes(case, nv=7):
+    """The same of the plain FP64 form on structured prisms.
+
+    k_px_cell: state, nu_t, adjugates at solution and fine points (72 B each),
+    reciprocal det, metric divergence in; point fields (16 per point) and
+    volume terms (9) out.
+    k_face: every cell's point fields once, the interpolation matrices of every
+    slot, adjugate row (32 B) and record (32 B per slot) in; jumps (9) out.
+    k_update: as in the mixed form, FP64 volume terms and jumps."""
+    N, S, Fn = int(case["n_cells"]), int(case["n_sps"]), int(case["n_fine"])
+    slots, P = _slot_counts(case)
+    sp = slots * P
     isb = case["is_boundary"].astype(bool)
     opr = case["owner_is_primary"].astype(bool)
     npr = case["neighbor_is_primary"].astype(bool)
-    slots = int(np.sum(opr)) + int(np.sum(~isb & npr))
     mats = int(np.sum(opr & ~isb)) + int(np.sum(~isb & npr)) + \
         int(np.sum(case["nb_src1_idx"][opr & ~isb] >= 0)) + int(np.sum(case["ow_src1_idx"][~isb & npr] >= 0))
-    jumps = slots * P * 10 * 8
-    face = N * S * 8 * (18 + 9) + mats * P * S * 8 + slots * (P * 3 * 8 + 24) + jumps
-    cell = N * S * 8 * (18 + 9 + 1 + 1 + 3 * nv) + N * Fn * 9 * 8 + jumps + slots * 4
+    px = N * S * (8 * (nv + 1) + 72 + 8 + 24) + N * Fn * 72 + N * S * (16 + 9) * 8
+    face = N * S * 16 * 8 + mats * P * S * 8 + sp * 32 + slots * 32 + sp * 72
+    upd = N * S * 72 + sp * 72 + N * S * 8 * (3 * nv + 2) + slots * 4
+    return {"k_px_cell": px, "k_face": face, "k_update": upd}
+
+
+def algorithmic_bytes(case, nv=7):
+    """Minimum bytes the generic per-stage kernels of the plain FP64 form must
+    move (every array once; Euler runs).
+
+    k_face: q of every cell's points, the interpolation matrices of every
+    residual slot, adjugate rows and records, and the jumps it writes.
+    k_cell: q, fine-point adjugates, det, dt, current and step-start state, the
+    state it writes, and the jumps it reads."""
+    N, S, Fn = int(case["n_cells"]), int(case["n_sps"]), int(case["n_fine"])
+    slots, P = _slot_counts(case)
+    isb = case["is_boundary"].astype(bool)
+    opr = case["owner_is_primary"].astype(bool)
+    npr = case["neighbor_is_primary"].astype(bool)
+    mats = int(np.sum(opr & ~isb)) + int(np.sum(~isb & npr)) + \
+        int(np.sum(case["nb_src1_idx"][opr & ~isb] >= 0)) + int(np.sum(case["ow_src1_idx"][~isb & npr] >= 0))
+    jumps = slots * P * 5 * 8
+    face = N * S * 8 * 5 + mats * P * S * 8 + slots * (P * 32 + 32) + jumps
+    cell = N * S * 8 * (5 + 1 + 1 + 3 * nv) + N * Fn * 9 * 8 + jumps + slots * 4
     return {"k_face": face, "k_cell": cell}
 
 
@@ -491,12 +516,12 @@ def run_ensemble(args):
         "metric": "DOF-updates/s, batched uneven ensemble (all cases, per RK stage)", "value": ens.dof_per_step() / (ms * 1e-3),
         "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None,
-        "dtype": "bf16x2 split tensor-core contractions (f32 accumulate), f32 fluxes, f64 state" if args.form != "fp64" else "f64",
+        "dtype": "f32 contractions and fluxes, f64 state" if args.form != "fp64" else "f64",
         "data": "synthetic (seeded case draw)",
         "config": {"workload": "C4 batched uneven ensemble: laminar NS Re 1e5, jittered prism boxes with wall bump",
                    "n_cases": len(specs), "cases_p1": n1, "cases_p2": len(specs) - n1, "n_cells": ens.n_cells,
                    "hex_cells_range": [2000, 64000], "mach_range": [0.05, 0.3], "launch": "one CUDA graph per step "
-                   "(per order group: pre, face, volume, update launches per RK stage)",
+                   "(per order group: cell, face, update launches per RK stage)",
                    "autotune_per_group": choices, "mesh_gen_s": round(t_gen, 1), "create_s": round(t_create, 1)},
         "norms": {"min": float(np.min(norms)), "max": float(np.max(norms)), "finite_cases": int(np.isfinite(norms).sum())},
         "case_status_nonfinite": int(np.sum(status != 0)),
@@ -978,7 +1003,7 @@ def run_serve(args):
     line = {
         "metric": "serving: solves/hour, p50/p99 latency (s)", "value": summary["solves_per_hour"],
         "unit": "solves/hour", "n_gpus": 1, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "bf16x2 split tensor-core contractions (f32 accumulate), f32 fluxes, f64 state",
+        "dtype": "f32 contractions and fluxes, f64 state",
         "data": "synthetic (seeded Poisson request stream)",
         "config": {"workload": "C5 serving: Poisson 4 req/s, prism boxes 8k-200k hex, P1/P2, Mach 0.05-0.25, "
                                "parametric wall bump", "requests": len(reqs), "physics": args.turb,
@@ -1062,7 +1087,7 @@ def main():
     U, k, om, nut, mu = initial_state(case, spec)
     rho, u, p, *_ = flow_conditions()
     t_gen = time.perf_counter() - t_gen
-    bytes_fp64 = algorithmic_bytes(case)
+    bytes_fp64 = prism_fp64_algorithmic_bytes(case)
     bytes_mx = mixed_algorithmic_bytes(case)
     stream = torch.cuda.current_stream()
 
@@ -1108,11 +1133,12 @@ def main():
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
     bd = head["breakdown"]
     if forms[0] == "mixed":
-        kern_ms = {"k_mx_pre": bd["k_pre_ms_per_launch"], "k_mx_face": bd["k_face_ms_per_launch"],
-                   "k_mx_vol": bd["k_cell_ms_per_launch"], "k_mx_update": bd["k_update_ms_per_launch"]}
+        kern_ms = {"k_px_cell": bd["k_pre_ms_per_launch"], "k_mx_face": bd["k_face_ms_per_launch"],
+                   "k_update": bd["k_update_ms_per_launch"]}
         alg = bytes_mx
     else:
-        kern_ms = {"k_face": bd["k_face_ms_per_launch"], "k_cell": bd["k_cell_ms_per_launch"]}
+        kern_ms = {"k_px_cell": bd["k_pre_ms_per_launch"], "k_face": bd["k_face_ms_per_launch"],
+                   "k_update": bd["k_cell_ms_per_launch"]}
         alg = bytes_fp64
     per_kernel = {kk: {"ms_per_launch": kern_ms[kk], "algorithmic_bytes": alg[kk],
                        "achieved_gbs": alg[kk] / (kern_ms[kk] * 1e-3) / 1e9 if kern_ms[kk] else None}
@@ -1123,7 +1149,7 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "bf16x2 split tensor-core contractions (f32 accumulate), f32 fluxes, f64 state" if mixed_head
+        "dtype": "f32 contractions and fluxes, f64 state" if mixed_head
         else "f64",
         "data": "synthetic (seeded generated mesh and state)",
         "config": {"workload": ("C2 P2 RANS-SST: 96x80x72 hex -> 1,105,920 prisms" if spec is FULL
@@ -1138,7 +1164,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                      "frac": (achieved / hbm_peak) if achieved else None,
                      "traffic": (MEASURED_TRAFFIC_PER_CELL[dom] * N) if dom in MEASURED_TRAFFIC_PER_CELL else None,
-                     "traffic_source": "ncu DRAM bytes per cell on 76,800 prisms, scaled to this launch",
+                     "traffic_source": "ncu DRAM bytes per cell on 91,200 prisms, scaled to this launch",
                      "kernel": dom, "algorithmic_bytes_per_launch": alg[dom], "per_kernel": per_kernel,
                      "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},
         # whole step against HBM: the reference-layout algorithmic bytes per

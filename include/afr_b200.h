@@ -62,9 +62,10 @@ enum { AFR_TURB_NONE = 0, AFR_TURB_SST = 1 };
 /* Arithmetic form of the residual-and-update stage.  AFR_PREC_FP64 is FP64
  * throughout.  AFR_PREC_MIXED runs the operator contractions (c2f, the
  * folded f2c*D_fine divergence, the viscous D_3d divergence, the gradients
- * and the extrapolation to faces) on the tensor cores as BF16 hi+lo split
- * products with FP32 accumulation and the pointwise fluxes in FP32, keeping
- * FP64 for the state, geometry metrics, primitive recovery, residual sums,
+ * and the extrapolation to faces) in FP32 where the prism operators are tensor
+ * products, and elsewhere on the tensor cores as BF16 hi+lo split products
+ * with FP32 accumulation; pointwise fluxes are FP32.  It keeps FP64 for the
+ * state, geometry metrics, primitive recovery, residual sums,
  * RK update, norm and Cd/Cl.  Viscous terms are built up to P2 in the mixed
  * form (P3 mixed handles must be inviscid).  A contraction accumulated in FP32
  * carries about 2^-24 * (operator row l1 norm) * |x|, so afr_create refuses
@@ -284,8 +285,8 @@ int afr_rms_norm_noalloc(const double* x, int64_t n, double* out, void* stream);
 
 /* Launch-shape autotuner of the mixed form: times one residual evaluation of
  * the state U (nu_t for SST handles) for each candidate pre-pass CTAs per SM,
- * face-kernel block size (64/128/256) and update-kernel cells per CTA (half /
- * base / double), one parameter at a time, and keeps the fastest in the
+ * face-kernel block size (64/128/256) and update-kernel warps per CTA (1 / 2 /
+ * 4), one parameter at a time, and keeps the fastest in the
  * handle.  U is not modified.  choice_out (3 ints, may be NULL) receives the
  * choices; plain-form handles keep their fixed shapes (choices -1).  No
  * counterpart in the reference (launch shapes have none there). */
@@ -296,7 +297,7 @@ int afr_autotune(afr_handle* h, const double* U, const double* nu_t, int32_t* ch
  * by 512 tensor-memory columns per SM), the runtime occupancy query's value
  * for the pre-pass (one for any kernel that uses tensor memory), volume-kernel
  * CTAs per SM, the runtime query's value for it, face-kernel block,
- * update-kernel variant (0 half, 1 base, 2 double cells per CTA) and the
+ * update-kernel variant (0, 1, 2: 1, 2, 4 warps per CTA) and the
  * device's SM count.
  * Plain-form handles report -1 except the SM count.  No counterpart in the
  * reference. */
