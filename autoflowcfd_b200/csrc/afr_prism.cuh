@@ -149,12 +149,14 @@ __global__ void __launch_bounds__(32 * px_warps(N1), sizeof(T) == 8 ? (N1 == 3 ?
     }
     // FP32: deviations from the value at the cell's middle point, which carry
     // the variation in 24 bits.  FP64 keeps the values; the reference state
-    // only enters the inviscid flux (below).
+    // only enters the inviscid flux (below), and any finite one serves: zero
+    // where the middle point's value is beyond FP32's range.
     T dev[6];
     constexpr int MID = S / 2;
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
-      const float ref = __shfl_sync(0xffffffffu, float(q[v]), (pc < CPR ? pc : 0) * S + MID);
+      float ref = __shfl_sync(0xffffffffu, float(q[v]), (pc < CPR ? pc : 0) * S + MID);
+      if (D && !isfinite(ref)) ref = 0.f;
       dev[v] = D ? T(q[v]) : T(q[v] - double(ref));
       if (in && s == MID) sc[L::oRef + v] = T(ref);
     }
