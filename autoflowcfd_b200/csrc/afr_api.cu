@@ -39,8 +39,7 @@ struct afr_handle {
   double* PF = nullptr;       // (N,S,16) point fields of the state being evaluated
   double* J = nullptr;        // (n_slots,9,P) face jumps of the residual slots
   SlotTable slots{};
-  double* Ua = nullptr;
-  double* Ub = nullptr;
+  double* Ua = nullptr;       // (N,S,nv) the state between the stages
   double* dt = nullptr;
   double* norm_part = nullptr;
   double* norm_rho_part = nullptr;
@@ -52,7 +51,7 @@ struct afr_handle {
   SstFace* sst_faces = nullptr;
   uint8_t* cd_wall = nullptr;
   double* area_w = nullptr;
-  int32_t* cd_faces = nullptr;
+  int4* cd_faces = nullptr;   // wall faces of the force integral: face, owner, axis, side > 0
   int n_cd_faces = 0;
   double* cd_part = nullptr;  // (n_cd_faces, 6)
   unsigned* status = nullptr;
@@ -156,16 +155,17 @@ int upload_i32(afr_handle* h, int32_t** dst, const T* src, size_t n, cudaStream_
   return e == cudaSuccess ? AFR_OK : cuda_fail(h, e, "upload sync");
 }
 
-__global__ void k_form_adj(const double* det, const double* inv, double* adj, size_t npts) {
+// inverse Jacobians -> adjugates, in place
+__global__ void k_form_adj(const double* det, double* adj, size_t npts) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npts * 9) return;
-  adj[t] = det[t / 9] * inv[t];  // compute_adj_j, core/fr_operators/volume_contract.py:47-80
+  adj[t] = det[t / 9] * adj[t];  // compute_adj_j, core/fr_operators/volume_contract.py:47-80
 }
 
 // |volume|^(1/3) per cell, the length of the local time step (core/fr_solver/cfl.py)
-__global__ void k_cube_root_abs(const double* v, size_t n, double* out) {
+__global__ void k_cube_root_abs(double* v, size_t n) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) out[t] = pow(fabs(v[t]), 1.0 / 3.0);
+  if (t < n) v[t] = pow(fabs(v[t]), 1.0 / 3.0);
 }
 
 __global__ void k_metric_flux_scale(const double* adj, double* mfs, size_t npts) {
@@ -236,15 +236,13 @@ __global__ void k_fill_scaled(double* x, size_t n, const double* v, double facto
 
 // per wall face: pressure and viscous force partials (postprocess/fr_coefficients.py:105-133)
 template <int S, int NP>
-__global__ void k_force(Geom g, Ops ops, Faces fc, const int32_t* faces, int nf, const double* U, int nv,
+__global__ void k_force(Geom g, Ops ops, Faces fc, const int4* faces, int nf, const double* U, int nv,
                         const double* PF, const double* nut, const double* area_w, double mu, double* part) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nf) return;
-  const int f = faces[t];
-  const int oc = fc.owner[f];
-  const int ct = cell_type(g, oc);
-  const int ax = fc.o_axis[f];
-  const double* E = ops.extrap + (((size_t)ct * 3 + ax) * 2 + (fc.o_side[f] < 0.0 ? 0 : 1)) * NP * S;
+  const int4 rec = faces[t];
+  const int f = rec.x, oc = rec.y;
+  const double* E = ops.extrap + (((size_t)cell_type(g, oc) * 3 + rec.z) * 2 + rec.w) * NP * S;
   double fp[3] = {0, 0, 0}, fv[3] = {0, 0, 0};
   for (int i = 0; i < NP; ++i) {
     double pf = 0.0, mt = 0.0, sg[6] = {0, 0, 0, 0, 0, 0};  // S00, S11, S22, S01, S02, S12
@@ -260,7 +258,7 @@ __global__ void k_force(Geom g, Ops ops, Faces fc, const int32_t* faces, int nf,
       for (int k = 0; k < 6; ++k) sg[k] += w * PF[p * PFW + 5 + k];
     }
     const double* n = fc.tnormal + ((size_t)f * NP + i) * 3;
-    const double aw = area_w[(size_t)f * NP + i];
+    const double aw = area_w[(size_t)t * NP + i];
     for (int d = 0; d < 3; ++d) fp[d] += pf * n[d] * aw;
     const double mtot = mu + mt;
     const double div = sg[0] + sg[1] + sg[2];
@@ -946,55 +944,54 @@ static void release_alloc(afr_handle* h, const double*& p, size_t n) {
 }
 
 // Tables of the plain form at orders 1-3: the slots' own adjugate rows, and for
-// structured prisms the metrics in lane order, the metric divergence MD and
-// 1/det.  The fine-point adjugates stay only for cells on the generic kernels.
+// structured prisms the metric divergence MD, 1/det and the metrics in lane order
+// (in place: no kernel after this one reads theirs in the reference's order).
 static int plain_setup(afr_handle* h, cudaStream_t st) {
-  const size_t N = h->N, S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism;
+  const size_t S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism;
   int rc;
   {
     const cudaError_t e = dispatch(h, [](auto L) { return decltype(L)::set_attrs(); });
     if (e != cudaSuccess) return cuda_fail(h, e, "kernel attributes");
   }
   if ((rc = dalloc(h, &h->slot_rows, ns * P))) return rc;
-  double *adjs = nullptr, *adjf = nullptr, *md = nullptr, *rdet = nullptr;
-  if (h->px64 && ((rc = dalloc(h, &adjs, NP * S * 9)) || (rc = dalloc(h, &adjf, NP * Fn * 9)) ||
-                  (rc = dalloc(h, &md, N * S * 3)) || (rc = dalloc(h, &rdet, N * S)) ||
+  double *md = nullptr, *rdet = nullptr;
+  if (h->px64 && ((rc = dalloc(h, &md, NP * S * 3)) || (rc = dalloc(h, &rdet, NP * S)) ||
                   (rc = dalloc(h, &h->RVd, NP * S * 9))))
     return rc;
-  const unsigned nb = (unsigned)((ns * P + 127) / 128), nmd = (unsigned)((N * S * 3 + 255) / 256);
+  const unsigned nb = (unsigned)((ns * P + 127) / 128), nmd = (unsigned)((NP * S * 3 + 255) / 256);
   switch (h->order) {
     case 1:
       if (ns) k_slot_rows<8, 4><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
-      if (h->px64) k_mx_md<8, 27><<<nmd, 256, 0, st>>>(h->g, h->ops, md);
+      if (h->px64) k_mx_md<8, 27><<<nmd, 256, 0, st>>>(h->g, h->ops, NP, md);
       break;
     case 2:
       if (ns) k_slot_rows<27, 9><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
-      if (h->px64) k_mx_md<27, 64><<<nmd, 256, 0, st>>>(h->g, h->ops, md);
+      if (h->px64) k_mx_md<27, 64><<<nmd, 256, 0, st>>>(h->g, h->ops, NP, md);
       break;
     default:
       if (ns) k_slot_rows<64, 16><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
   }
   if (h->px64) {
     const int nf = h->order == 1 ? 3 : 4;
-    k_px_planes<<<(unsigned)((NP * Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, (int)Fn, nf, adjf);
-    k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, (int)S, 1, adjs);
-    k_mx_rdet<<<(unsigned)((N * S + 255) / 256), 256, 0, st>>>(h->g.det, N * S, rdet);
-    h->pgd = PxGeom<double>{adjs, adjf, md, rdet, h->px_rows};
+    k_px_planes<<<(unsigned)NP, 128, 0, st>>>(h->g.adj_fine, (int)Fn, nf, const_cast<double*>(h->g.adj_fine));
+    k_px_planes<<<(unsigned)NP, 128, 0, st>>>(h->g.adj, (int)S, 1, const_cast<double*>(h->g.adj));
+    k_mx_rdet<<<(unsigned)((NP * S + 255) / 256), 256, 0, st>>>(h->g.det, NP * S, rdet);
+    h->pgd = PxGeom<double>{h->g.adj, h->g.adj_fine, md, rdet, h->px_rows};
   }
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return cuda_fail(h, e, "plain-form set-up");
-  if (h->px64 && h->n_prism == h->N) {
-    release_alloc(h, h->g.adj_fine, N * Fn * 9);
-    release_alloc(h, h->g.adj, N * S * 9);
-  }
-  return AFR_OK;
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? AFR_OK : cuda_fail(h, e, "plain-form set-up");
 }
+
+// host copies of the residual slots' columns (face and cell: mixed form only)
+struct HostSlots {
+  std::vector<int32_t> flags, face, cell;
+};
 
 // Tables of the mixed-precision form: operator images, metric divergence,
 // interior-penalty lengths, per-slot adjugate rows and the conforming-face
 // match of the other side's face point.
-static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<double>* Wkeep, cudaStream_t st) {
+static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<double>* Wkeep, const HostSlots& hs,
+                       cudaStream_t st) {
   const int S = h->S, Fn = h->Fn, P = h->P;
   const size_t N = h->N;
   if (h->order == 3 && !h->prm.inviscid_only)
@@ -1113,15 +1110,15 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
     using LL = decltype(L);
     const size_t nmd = N * S * 3;
     switch (h->order) {
-      case 1: k_mx_md<8, 27><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, md);
+      case 1: k_mx_md<8, 27><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<8><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
               if (ns) k_mx_match<8, 4><<<(unsigned)((ns * 4 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
               break;
-      case 2: k_mx_md<27, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, md);
+      case 2: k_mx_md<27, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<27><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
               if (ns) k_mx_match<27, 9><<<(unsigned)((ns * 9 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
               break;
-      default: k_mx_md<64, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, md);
+      default: k_mx_md<64, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<64><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
               if (ns) k_mx_match<64, 16><<<(unsigned)((ns * 16 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
               break;
@@ -1133,8 +1130,8 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
       k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv, nsrows, invs32);
     }
     if (h->px) {
-      k_px_planes<<<(unsigned)((NP * h->Fn * 9 + 255) / 256), 256, 0, st>>>(h->g.adj_fine, NP, h->Fn, 1, padjf);
-      k_px_planes<<<(unsigned)((NP * S * 9 + 255) / 256), 256, 0, st>>>(h->g.adj, NP, S, 1, padjs);
+      k_px_planes<<<(unsigned)NP, 128, 0, st>>>(h->g.adj_fine, h->Fn, 1, padjf);
+      k_px_planes<<<(unsigned)NP, 128, 0, st>>>(h->g.adj, S, 1, padjs);
     }
     k_mx_rdet<<<(unsigned)((N * (size_t)S + 255) / 256), 256, 0, st>>>(h->g.det, N * (size_t)S, rdet);
     cudaError_t r = cudaGetLastError();
@@ -1152,11 +1149,8 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   if (ns > 0) {
     const size_t nt = ns * P;
     std::vector<uint8_t> hofp(nt);
-    std::vector<int32_t> hface(ns), hflag(ns), hcell(ns);
+    const std::vector<int32_t>&hface = hs.face, &hflag = hs.flags, &hcell = hs.cell;
     e = cudaMemcpy(hofp.data(), ofp, nt, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(hface.data(), h->slots.face, ns * 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(hflag.data(), h->slots.flags, ns * 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(hcell.data(), h->slots.cell, ns * 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
     std::vector<int32_t> nb_slot(h->F, -1);
     for (size_t sl = 0; sl < ns; ++sl) {
@@ -1225,24 +1219,17 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   // The dense per-record interpolation matrices are read afterwards only by
   // the general (unmatched) face points and by the SST face kernel: release
   // them when neither exists.
-  if (ns && h->prm.turb != AFR_TURB_SST) {
-    std::vector<uint8_t> o(ns * P);
-    e = cudaMemcpy(o.data(), ofp, o.size(), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form set-up");
-    bool all_matched = true;
-    for (uint8_t v : o) all_matched = all_matched && v != MX_OFP_GENERAL;
-    if (all_matched) {
-      // (an indexed mesh's four pointers share one table: freed once)
-      const double* mats[4] = {h->fc.nb_m0, h->fc.nb_m1, h->fc.ow_m0, h->fc.ow_m1};
-      for (int i = 0; i < 4; ++i) {
-        auto it = std::find(h->allocs.begin(), h->allocs.end(), (void*)mats[i]);
-        if (it == h->allocs.end()) continue;
-        h->allocs.erase(it);
-        cudaFree((void*)mats[i]);
-        h->bytes -= std::max<size_t>(h->mat_elems[i], 1) * sizeof(double);
-      }
-      h->fc.nb_m0 = h->fc.nb_m1 = h->fc.ow_m0 = h->fc.ow_m1 = nullptr;
+  if (ns && h->prm.turb != AFR_TURB_SST && !h->px_points) {
+    // (an indexed mesh's four pointers share one table: freed once)
+    const double* mats[4] = {h->fc.nb_m0, h->fc.nb_m1, h->fc.ow_m0, h->fc.ow_m1};
+    for (int i = 0; i < 4; ++i) {
+      auto it = std::find(h->allocs.begin(), h->allocs.end(), (void*)mats[i]);
+      if (it == h->allocs.end()) continue;
+      h->allocs.erase(it);
+      cudaFree((void*)mats[i]);
+      h->bytes -= std::max<size_t>(h->mat_elems[i], 1) * sizeof(double);
     }
+    h->fc.nb_m0 = h->fc.nb_m1 = h->fc.ow_m0 = h->fc.ow_m1 = nullptr;
   }
   return AFR_OK;
 }
@@ -1360,45 +1347,6 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     return bail(fail(h, AFR_ENOMEM, "pinned status word"));
   *h->status_host = 0;
 
-  // ---- geometry ----
-  double *det = nullptr, *inv = nullptr, *detf = nullptr, *invf = nullptr;
-  if ((rc = upload(h, &det, m->det_jacs, N * S, st))) return bail(rc);
-  if ((rc = upload(h, &inv, m->inv_jacs, N * S * 9, st))) return bail(rc);
-  double *adj, *adjf, *vol, *mfs, *wd = nullptr;
-  if ((rc = dalloc(h, &adj, N * S * 9))) return bail(rc);
-  if ((rc = dalloc(h, &adjf, N * Fn * 9))) return bail(rc);
-  if ((rc = dalloc(h, &mfs, N * S))) return bail(rc);
-  if ((rc = upload(h, &vol, m->cell_volumes, N, st))) return bail(rc);
-  if (m->wall_distance && (rc = upload(h, &wd, m->wall_distance, N * S, st))) return bail(rc);
-  {
-    // fine-point Jacobians are only needed to form adj_fine: stage them through
-    // a temporary allocation released right after
-    cudaError_t e1 = cudaMalloc((void**)&detf, N * Fn * sizeof(double));
-    cudaError_t e2 = cudaMalloc((void**)&invf, N * Fn * 9 * sizeof(double));
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-      cudaFree(detf);
-      cudaFree(invf);
-      return bail(fail(h, AFR_ENOMEM, "cudaMalloc failed for fine Jacobians"));
-    }
-    cudaMemcpyAsync(detf, m->det_jacs_fine, N * Fn * sizeof(double), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(invf, m->inv_jacs_fine, N * Fn * 9 * sizeof(double), cudaMemcpyHostToDevice, st);
-    const size_t nf = N * Fn * 9, nc = N * S * 9;
-    k_form_adj<<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(detf, invf, adjf, N * Fn);
-    k_form_adj<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(det, inv, adj, N * S);
-    if (m->metric_flux_scale)
-      cudaMemcpyAsync(mfs, m->metric_flux_scale, N * S * sizeof(double), cudaMemcpyHostToDevice, st);
-    else
-      k_metric_flux_scale<<<(unsigned)((N * S + 255) / 256), 256, 0, st>>>(adj, mfs, N * S);
-    cudaError_t e = cudaStreamSynchronize(st);
-    cudaFree(detf);
-    cudaFree(invf);
-    if (e != cudaSuccess) return bail(cuda_fail(h, e, "geometry set-up"));
-  }
-  double* hvol;
-  if ((rc = dalloc(h, &hvol, N))) return bail(rc);
-  k_cube_root_abs<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(vol, N, hvol);
-  h->g = Geom{h->N, h->n_prism, det, inv, adj, adjf, vol, mfs, wd, hvol};
-
   // ---- operators ----
   // fragment-major image of an M x K operator whose element (m, k) is
   // A[m * rs + k * cs] (layout in Ops)
@@ -1432,17 +1380,11 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     const double* f2c_h = m->f2c[t] ? m->f2c[t] : (p0 ? one : nullptr);
     if (!m->D_3d[t] || !c2f_h || !dfn_h || !f2c_h || !m->filter[t])
       return bail(fail(h, AFR_EINVAL, "missing operator for a present cell type"));
-    double *d3, *d3g, *c2f, *dfn, *f2c, *flt;
-    if ((rc = upload(h, &d3, m->D_3d[t], S * S * 3, st))) return bail(rc);
+    double* flt;
     std::vector<double> g2(3 * S * S);
     for (size_t s = 0; s < S; ++s)
       for (int mm = 0; mm < 3; ++mm)
         for (size_t j = 0; j < S; ++j) g2[(s * 3 + mm) * S + j] = m->D_3d[t][s * 3 * S + j * 3 + mm];
-    if ((rc = upload(h, &d3g, g2.data(), g2.size(), st))) return bail(rc);
-    cudaStreamSynchronize(st);
-    if ((rc = upload(h, &c2f, c2f_h, Fn * S, st))) return bail(rc);
-    if ((rc = upload(h, &dfn, dfn_h, Fn * Fn * 3, st))) return bail(rc);
-    if ((rc = upload(h, &f2c, f2c_h, S * Fn, st))) return bail(rc);
     if ((rc = upload(h, &flt, m->filter[t], S * S, st))) return bail(rc);
     // W = f2c * D_fine (S x 3Fn), summed in ascending fine-point order
     std::vector<double> Wh(S * 3 * Fn, 0.0);
@@ -1470,11 +1412,6 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
       h->ops.ffilt[t] = fflt;
     }
     Wkeep[t] = Wh;
-    h->ops.D3[t] = d3;
-    h->ops.D3g[t] = d3g;
-    h->ops.c2f[t] = c2f;
-    h->ops.Dfine[t] = dfn;
-    h->ops.f2c[t] = f2c;
     h->ops.filt[t] = flt;
   }
   // tensor-product structure of the prism operators (afr_prism.cuh).  The
@@ -1543,36 +1480,69 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     h->ops.dist_co = dco;
   }
 
+  // ---- geometry ----
+  // The inverse Jacobians (at solution and fine points) are uploaded into the
+  // arrays of the adjugates and scaled there by det.  Those at solution points
+  // are kept for the cells whose kernels read them.
+  const bool plain_px = h->px64 && prm->precision == AFR_PREC_FP64 && prm->turb != AFR_TURB_SST;
+  const size_t inv0 = plain_px ? (size_t)h->n_prism : 0;
+  double *det, *inv = nullptr, *detf = nullptr, *adj, *adjf, *mfs, *wd = nullptr, *hvol;
+  if ((rc = upload(h, &det, m->det_jacs, N * S, st)) || (rc = upload(h, &adj, m->inv_jacs, N * S * 9, st)) ||
+      (rc = upload(h, &adjf, m->inv_jacs_fine, N * Fn * 9, st)) || (rc = dalloc(h, &mfs, N * S)) ||
+      (rc = upload(h, &hvol, m->cell_volumes, N, st)) ||
+      (inv0 < N && (rc = dalloc(h, &inv, (N - inv0) * S * 9))) ||
+      (m->wall_distance && (rc = upload(h, &wd, m->wall_distance, N * S, st))))
+    return bail(rc);
+  if (cudaMalloc((void**)&detf, N * Fn * sizeof(double)) != cudaSuccess)  // for this block only
+    return bail(fail(h, AFR_ENOMEM, "cudaMalloc failed for fine Jacobians"));
+  {
+    const size_t nf = N * Fn * 9, nc = N * S * 9;
+    cudaMemcpyAsync(detf, m->det_jacs_fine, N * Fn * sizeof(double), cudaMemcpyHostToDevice, st);
+    if (inv) cudaMemcpyAsync(inv, adj + inv0 * S * 9, (N - inv0) * S * 9 * sizeof(double), cudaMemcpyDeviceToDevice, st);
+    k_form_adj<<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(detf, adjf, N * Fn);
+    k_form_adj<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(det, adj, N * S);
+    if (m->metric_flux_scale)
+      cudaMemcpyAsync(mfs, m->metric_flux_scale, N * S * sizeof(double), cudaMemcpyHostToDevice, st);
+    else
+      k_metric_flux_scale<<<(unsigned)((N * S + 255) / 256), 256, 0, st>>>(adj, mfs, N * S);
+    k_cube_root_abs<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(hvol, N);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    cudaFree(detf);
+    if (e != cudaSuccess) return bail(cuda_fail(h, e, "geometry set-up"));
+  }
+  h->g = Geom{h->N, h->n_prism, det, inv, (int32_t)inv0, adj, adjf, mfs, wd, hvol};
+
   // ---- faces ----
   Faces& fc = h->fc;
   fc.F = h->F;
   {
-    int32_t *own, *nbr, *c0n, *i1n, *c1n, *c0o, *i1o, *c1o, *bcg;
-    int8_t *oax, *nax;
-    uint8_t* isb;
-    double *osd, *nsd, *tn, *m0n, *m1n, *m0o, *m1o;
-    if ((rc = upload_i32(h, &own, m->owner_cell, F, st, tmp))) return bail(rc);
-    if ((rc = upload_i32(h, &nbr, m->neighbor_cell, F, st, tmp))) return bail(rc);
-    std::vector<int8_t> ax8(F);
-    for (size_t f = 0; f < F; ++f) ax8[f] = (int8_t)m->owner_axis[f];
-    if ((rc = upload(h, &oax, ax8.data(), F, st))) return bail(rc);
-    cudaStreamSynchronize(st);
-    for (size_t f = 0; f < F; ++f) ax8[f] = (int8_t)std::max<int64_t>(m->neighbor_axis[f], 0);
-    if ((rc = upload(h, &nax, ax8.data(), F, st))) return bail(rc);
-    cudaStreamSynchronize(st);
-    if ((rc = upload(h, &osd, m->owner_side, F, st))) return bail(rc);
-    if ((rc = upload(h, &nsd, m->neighbor_side, F, st))) return bail(rc);
-    if ((rc = upload(h, &isb, m->is_boundary, F, st))) return bail(rc);
+    int32_t *own = nullptr, *nbr = nullptr, *bcg;
+    int8_t *oax = nullptr, *nax = nullptr;
+    uint8_t* isb = nullptr;
+    double *osd = nullptr, *nsd = nullptr, *tn, *m0n, *m1n, *m0o, *m1o;
     if ((rc = upload(h, &tn, m->true_normal, F * P * 3, st))) return bail(rc);
-    if ((rc = upload_i32(h, &c0n, m->nb_src0_cell, F, st, tmp))) return bail(rc);
-    if ((rc = upload_i32(h, &i1n, m->nb_src1_idx, F, st, tmp))) return bail(rc);
-    if ((rc = upload_i32(h, &c1n, m->nb_src1_cell, (size_t)m->n_nb_src1, st, tmp))) return bail(rc);
+    if (prm->precision == AFR_PREC_MIXED || h->order == 0) {
+      if ((rc = upload_i32(h, &own, m->owner_cell, F, st, tmp)) || (rc = upload_i32(h, &nbr, m->neighbor_cell, F, st, tmp)))
+        return bail(rc);
+      std::vector<int8_t> ax8(F), nx8(F);
+      for (size_t f = 0; f < F; ++f) {
+        ax8[f] = (int8_t)m->owner_axis[f];
+        nx8[f] = (int8_t)std::max<int64_t>(m->neighbor_axis[f], 0);
+      }
+      if ((rc = upload(h, &oax, ax8.data(), F, st)) || (rc = upload(h, &nax, nx8.data(), F, st)) ||
+          (rc = upload(h, &osd, m->owner_side, F, st)) || (rc = upload(h, &nsd, m->neighbor_side, F, st)) ||
+          (rc = upload(h, &isb, m->is_boundary, F, st)))
+        return bail(rc);
+      cudaStreamSynchronize(st);  // ax8 and nx8 leave scope
+    }
     // interpolation matrices: an indexed mesh keeps its table of distinct
     // matrices on the device with per-record row indices; a dense mesh keeps
-    // its per-record arrays with identity indices
+    // its per-record arrays with identity indices (the mixed form's; the plain
+    // form's slot records hold theirs)
     const bool indexed = m->src_mat_table != nullptr;
     const size_t n1n = (size_t)m->n_nb_src1, n1o = (size_t)m->n_ow_src1;
-    int32_t *m0ni, *m1ni, *m0oi, *m1oi;
+    const bool row_idx = prm->precision == AFR_PREC_MIXED;
+    int32_t *m0ni = nullptr, *m1ni = nullptr, *m0oi = nullptr, *m1oi = nullptr;
     if (indexed) {
       if (m->n_src_mats <= 0) return bail(fail(h, AFR_EINVAL, "empty matrix table"));
       const int32_t* idx[4] = {m->nb_src0_mat_index, m->nb_src1_mat_index, m->ow_src0_mat_index, m->ow_src1_mat_index};
@@ -1584,10 +1554,9 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
       if ((rc = upload(h, &m0n, tabT.data(), tabT.size(), st))) return bail(rc);
       cudaStreamSynchronize(st);
       m1n = m0o = m1o = m0n;
-      if ((rc = upload_i32(h, &m0ni, idx[0], F, st, tmp))) return bail(rc);
-      if ((rc = upload_i32(h, &m1ni, idx[1], n1n, st, tmp))) return bail(rc);
-      if ((rc = upload_i32(h, &m0oi, idx[2], F, st, tmp))) return bail(rc);
-      if ((rc = upload_i32(h, &m1oi, idx[3], n1o, st, tmp))) return bail(rc);
+      if (row_idx && ((rc = upload(h, &m0ni, idx[0], F, st)) || (rc = upload(h, &m1ni, idx[1], n1n, st)) ||
+                      (rc = upload(h, &m0oi, idx[2], F, st)) || (rc = upload(h, &m1oi, idx[3], n1o, st))))
+        return bail(rc);
       h->mat_elems[0] = (size_t)m->n_src_mats * P * S;
     } else {
       const double* dense[4] = {m->nb_src0_mat, m->nb_src1_mat, m->ow_src0_mat, m->ow_src1_mat};
@@ -1598,28 +1567,27 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
         if ((rc = upload(h, dst[k], t.data(), t.size(), st))) return bail(rc);
         cudaStreamSynchronize(st);  // t leaves scope
       }
-      std::vector<int32_t> iota(std::max<size_t>(F, std::max(n1n, n1o)));
-      for (size_t r = 0; r < iota.size(); ++r) iota[r] = (int32_t)r;
-      if ((rc = upload(h, &m0ni, iota.data(), F, st))) return bail(rc);
-      m0oi = m0ni;
-      if ((rc = upload(h, &m1ni, iota.data(), n1n, st))) return bail(rc);
-      if ((rc = upload(h, &m1oi, iota.data(), n1o, st))) return bail(rc);
-      cudaStreamSynchronize(st);  // iota leaves scope
+      if (row_idx) {
+        std::vector<int32_t> iota(std::max<size_t>(F, std::max(n1n, n1o)));
+        for (size_t r = 0; r < iota.size(); ++r) iota[r] = (int32_t)r;
+        if ((rc = upload(h, &m0ni, iota.data(), F, st)) || (rc = upload(h, &m1ni, iota.data(), n1n, st)) ||
+            (rc = upload(h, &m1oi, iota.data(), n1o, st)))
+          return bail(rc);
+        m0oi = m0ni;
+        cudaStreamSynchronize(st);  // iota leaves scope
+      }
       h->mat_elems[0] = F * P * S;
       h->mat_elems[1] = n1n * P * S;
       h->mat_elems[2] = F * P * S;
       h->mat_elems[3] = n1o * P * S;
     }
-    if ((rc = upload_i32(h, &c0o, m->ow_src0_cell, F, st, tmp))) return bail(rc);
-    if ((rc = upload_i32(h, &i1o, m->ow_src1_idx, F, st, tmp))) return bail(rc);
-    if ((rc = upload_i32(h, &c1o, m->ow_src1_cell, (size_t)m->n_ow_src1, st, tmp))) return bail(rc);
     if ((rc = upload(h, &bcg, m->bc_group, F, st))) return bail(rc);
     fc.owner = own; fc.neighbor = nbr; fc.o_axis = oax; fc.n_axis = nax; fc.o_side = osd; fc.n_side = nsd;
-    fc.is_bnd = isb; fc.tnormal = tn; fc.nb_c0 = c0n; fc.nb_m0 = m0n; fc.nb_i1 = i1n; fc.nb_c1 = c1n; fc.nb_m1 = m1n;
-    fc.ow_c0 = c0o; fc.ow_m0 = m0o; fc.ow_i1 = i1o; fc.ow_c1 = c1o; fc.ow_m1 = m1o; fc.bc_group = bcg;
+    fc.is_bnd = isb; fc.tnormal = tn; fc.nb_m0 = m0n; fc.nb_m1 = m1n; fc.ow_m0 = m0o; fc.ow_m1 = m1o; fc.bc_group = bcg;
     fc.nb_m0i = m0ni; fc.nb_m1i = m1ni; fc.ow_m0i = m0oi; fc.ow_m1i = m1oi;
   }
   // slot lists: faces visited in ascending (color, face index)
+  HostSlots hs;
   {
     std::vector<int32_t> order(F);
     for (size_t f = 0; f < F; ++f) order[f] = (int32_t)f;
@@ -1631,8 +1599,9 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
       const double side = nb ? m->neighbor_side[f] : m->owner_side[f];
       return (f << 4) | (ax << 2) | (nb ? 2 : 0) | (side > 0.0 ? 1 : 0);
     };
-    auto build = [&](bool transport, int32_t** dptr, int32_t** dslot) -> int {
-      std::vector<int32_t> cnt(N + 1, 0);
+    // per-cell slot ranges and codes; uploaded by the caller where a kernel reads them
+    auto build = [&](bool transport, std::vector<int32_t>& cnt, std::vector<int32_t>& slots) {
+      cnt.assign(N + 1, 0);
       auto visit = [&](auto&& emit) {
         for (int32_t f : order) {
           const bool bnd = m->is_boundary[f] != 0;
@@ -1647,26 +1616,38 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
       };
       visit([&](int32_t c, int32_t) { cnt[c + 1]++; });
       for (size_t i = 0; i < N; ++i) cnt[i + 1] += cnt[i];
-      std::vector<int32_t> pos(cnt.begin(), cnt.end() - 1), slots(cnt[N]);
+      std::vector<int32_t> pos(cnt.begin(), cnt.end() - 1);
+      slots.resize(cnt[N]);
       visit([&](int32_t c, int32_t code) { slots[pos[c]++] = code; });
-      int r = upload(h, dptr, cnt.data(), N + 1, st);
-      if (r) return r;
-      r = upload(h, dslot, slots.data(), slots.size(), st);
-      if (r) return r;
-      return cudaStreamSynchronize(st) == cudaSuccess ? AFR_OK : AFR_ECUDA;
     };
-    int32_t *sp, *sl, *tp, *tl;
-    if ((rc = build(false, &sp, &sl))) return bail(rc);
-    if ((rc = build(true, &tp, &tl))) return bail(rc);
-    fc.slot_ptr = sp; fc.slot = sl; fc.tslot_ptr = tp; fc.tslot = tl;
-    // slot table of the residual slots, in the same (cell, color) order
-    std::vector<int32_t> ptr(N + 1), codes;
-    cudaMemcpy(ptr.data(), sp, (N + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost);
-    codes.resize(ptr[N]);
-    cudaMemcpy(codes.data(), sl, codes.size() * sizeof(int32_t), cudaMemcpyDeviceToHost);
+    std::vector<int32_t> ptr, codes;
+    if (prm->turb == AFR_TURB_SST) {
+      int32_t *tp, *tl;
+      build(true, ptr, codes);
+      if ((rc = upload(h, &tp, ptr.data(), N + 1, st)) || (rc = upload(h, &tl, codes.data(), codes.size(), st)))
+        return bail(rc);
+      cudaStreamSynchronize(st);  // ptr and codes are filled again
+      fc.tslot_ptr = tp; fc.tslot = tl;
+    }
+    build(false, ptr, codes);
+    int32_t *sp, *sl = nullptr;
+    if ((rc = upload(h, &sp, ptr.data(), N + 1, st)) ||
+        (h->order == 0 && (rc = upload(h, &sl, codes.data(), codes.size(), st))))
+      return bail(rc);
+    fc.slot_ptr = sp; fc.slot = sl;
+    // slot table of the residual slots, in the same (cell, color) order: the plain
+    // form's kernels find a slot's sources in its record, the mixed form's in the
+    // columns, which its set-up reads too
+    const bool mixed = prm->precision == AFR_PREC_MIXED, plain = !mixed && h->order > 0;
     const size_t ns = codes.size();
-    std::vector<int32_t> sf(ns), sc(ns), sflg(ns), s0(ns), s1(ns), si1(ns);
-    std::vector<int4> srec(prm->precision != AFR_PREC_MIXED && h->order > 0 ? 2 * ns : 0);
+    const bool ix = m->src_mat_table != nullptr;  // else a record's own matrix row
+    hs.flags.resize(ns);
+    if (mixed) {
+      hs.face.resize(ns);
+      hs.cell.resize(ns);
+    }
+    std::vector<int32_t> s0(mixed ? ns : 0), s1(mixed ? ns : 0), si1(mixed ? ns : 0);
+    std::vector<int4> srec(plain ? 2 * ns : 0);
     for (size_t c = 0; c < N; ++c)
       for (int32_t k = ptr[c]; k < ptr[c + 1]; ++k) {
         const int f = codes[k] >> 1;
@@ -1674,38 +1655,36 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
         const bool bnd = m->is_boundary[f] != 0;
         const int ax = (int)(nbside ? m->neighbor_axis[f] : m->owner_axis[f]);
         const double side = nbside ? m->neighbor_side[f] : m->owner_side[f];
-        sf[k] = f;
-        sc[k] = (int32_t)c;
-        sflg[k] = (nbside ? 1 : 0) | (bnd ? 2 : 0) | (ax << 2) | (side > 0.0 ? 16 : 0);
+        const int32_t fl = (nbside ? 1 : 0) | (bnd ? 2 : 0) | (ax << 2) | (side > 0.0 ? 16 : 0);
         const int64_t i1 = nbside ? m->ow_src1_idx[f] : m->nb_src1_idx[f];
-        s0[k] = bnd ? -1 : (int32_t)(nbside ? m->ow_src0_cell[f] : m->nb_src0_cell[f]);
-        si1[k] = (int32_t)i1;
-        s1[k] = (bnd || i1 < 0) ? -1 : (int32_t)(nbside ? m->ow_src1_cell[i1] : m->nb_src1_cell[i1]);
-        if (!srec.empty()) {
-          // matrix rows: table rows of an indexed mesh, else the record's own
-          const bool ix = m->src_mat_table != nullptr;
+        const int32_t c0 = bnd ? -1 : (int32_t)(nbside ? m->ow_src0_cell[f] : m->nb_src0_cell[f]);
+        const int32_t c1 = (bnd || i1 < 0) ? -1 : (int32_t)(nbside ? m->ow_src1_cell[i1] : m->nb_src1_cell[i1]);
+        hs.flags[k] = fl;
+        if (mixed) {
+          hs.face[k] = f;
+          hs.cell[k] = (int32_t)c;
+          s0[k] = c0;
+          s1[k] = c1;
+          si1[k] = (int32_t)i1;
+        } else if (plain) {
           const int32_t m0 = ix ? (nbside ? m->ow_src0_mat_index[f] : m->nb_src0_mat_index[f]) : f;
           const int32_t m1 =
-              s1[k] < 0 ? 0 : (ix ? (nbside ? m->ow_src1_mat_index[i1] : m->nb_src1_mat_index[i1]) : (int32_t)i1);
-          srec[2 * (size_t)k] = make_int4(s0[k], m0, s1[k], m1);
-          srec[2 * (size_t)k + 1] = make_int4(f, sflg[k], (int)c, 0);
+              c1 < 0 ? 0 : (ix ? (nbside ? m->ow_src1_mat_index[i1] : m->nb_src1_mat_index[i1]) : (int32_t)i1);
+          srec[2 * (size_t)k] = make_int4(c0, m0, c1, m1);
+          srec[2 * (size_t)k + 1] = make_int4(f, fl, (int)c, 0);
         }
       }
-    // the mixed form's face kernel finds its sources per slot, the plain form's
-    // in the records
-    const bool mixed = prm->precision == AFR_PREC_MIXED;
-    int32_t *d_f, *d_c, *d_fl, *d_0 = nullptr, *d_1 = nullptr, *d_i1 = nullptr;
-    if ((rc = upload(h, &d_f, sf.data(), ns, st)) || (rc = upload(h, &d_c, sc.data(), ns, st)) ||
-        (rc = upload(h, &d_fl, sflg.data(), ns, st)) ||
-        (mixed && ((rc = upload(h, &d_0, s0.data(), ns, st)) || (rc = upload(h, &d_1, s1.data(), ns, st)) ||
+    int32_t *d_fl, *d_f = nullptr, *d_c = nullptr, *d_0 = nullptr, *d_1 = nullptr, *d_i1 = nullptr;
+    int4* d_rec = nullptr;
+    if ((rc = upload(h, &d_fl, hs.flags.data(), ns, st)) || (plain && (rc = upload(h, &d_rec, srec.data(), 2 * ns, st))) ||
+        (mixed && ((rc = upload(h, &d_f, hs.face.data(), ns, st)) || (rc = upload(h, &d_c, hs.cell.data(), ns, st)) ||
+                   (rc = upload(h, &d_0, s0.data(), ns, st)) || (rc = upload(h, &d_1, s1.data(), ns, st)) ||
                    (rc = upload(h, &d_i1, si1.data(), ns, st)))))
       return bail(rc);
-    int4* d_rec = nullptr;
-    if (!srec.empty() && (rc = upload(h, &d_rec, srec.data(), srec.size(), st))) return bail(rc);
     cudaStreamSynchronize(st);
-    h->slots = SlotTable{(int32_t)ns, d_f, d_c, d_fl, d_0, d_1, d_i1, d_rec};
+    h->slots = SlotTable{(int32_t)ns, d_fl, d_f, d_c, d_0, d_1, d_i1, d_rec};
     // FP64 jumps: the plain stage of orders 1-3 only
-    if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = dalloc(h, &h->J, ns * P * 9))) return bail(rc);
+    if (plain && (rc = dalloc(h, &h->J, ns * P * 9))) return bail(rc);
   }
   // ---- boundary condition table ----
   {
@@ -1721,12 +1700,16 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     cudaStreamSynchronize(st);
   }
   if (m->cd_wall_face && m->true_area_weight) {
-    std::vector<int32_t> cdf;
+    std::vector<int4> cdf;
+    std::vector<double> aw;  // (force faces, P)
     for (size_t f = 0; f < F; ++f)
-      if (m->cd_wall_face[f] && m->owner_is_primary[f]) cdf.push_back((int32_t)f);
+      if (m->cd_wall_face[f] && m->owner_is_primary[f]) {
+        cdf.push_back(make_int4((int)f, (int)m->owner_cell[f], (int)m->owner_axis[f], m->owner_side[f] < 0.0 ? 0 : 1));
+        aw.insert(aw.end(), m->true_area_weight + f * P, m->true_area_weight + (f + 1) * P);
+      }
     h->n_cd_faces = (int)cdf.size();
     if ((rc = upload(h, &h->cd_faces, cdf.data(), cdf.size(), st))) return bail(rc);
-    if ((rc = upload(h, &h->area_w, m->true_area_weight, F * P, st))) return bail(rc);
+    if ((rc = upload(h, &h->area_w, aw.data(), aw.size(), st))) return bail(rc);
     if ((rc = dalloc(h, &h->cd_part, cdf.size() * 6))) return bail(rc);
     cudaStreamSynchronize(st);
   }
@@ -1735,7 +1718,6 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
   // them only for the force integral, which allocates them for its call
   if (prm->precision != AFR_PREC_MIXED && (rc = dalloc(h, &h->PF, N * S * PFW))) return bail(rc);
   if ((rc = dalloc(h, &h->Ua, N * S * h->nv))) return bail(rc);
-  if ((rc = dalloc(h, &h->Ub, N * S * h->nv))) return bail(rc);
   if ((rc = dalloc(h, &h->dt, N * S))) return bail(rc);
   if ((rc = dalloc(h, &h->norm_part, N))) return bail(rc);
   if ((rc = dalloc(h, &h->norm_rho_part, N))) return bail(rc);
@@ -1743,7 +1725,15 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
   if ((rc = dalloc(h, &h->red_part, std::max((N * S + RED_CHUNK - 1) / RED_CHUNK, (N * S * h->nv + IMP_CHUNK - 1) / IMP_CHUNK) + 1)))
     return bail(rc);
   if (prm->turb == AFR_TURB_SST) {
-    if ((rc = dalloc(h, &h->pt, N * S * 5))) return bail(rc);
+    // the plain form's point fields are dead while the SST kernels run: their
+    // rows of 16 hold sp8 and pt
+    if (h->PF) {
+      static_assert(PFW >= 13, "sp8 (8) and pt (5) in a point-field row");
+      h->sp8 = h->PF;
+      h->pt = h->PF + N * S * 8;
+    } else if ((rc = dalloc(h, &h->pt, N * S * 5)) || (rc = dalloc(h, &h->sp8, N * S * 8))) {
+      return bail(rc);
+    }
     if ((rc = dalloc(h, &h->cfp, F * P * 2))) return bail(rc);
     // face records of the transport
     const int32_t *i0 = nullptr, *i1 = nullptr;  // matrix rows (dense meshes: the record's own)
@@ -1768,9 +1758,8 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     }
     if ((rc = upload(h, &h->sst_faces, rec.data(), F, st))) return bail(rc);
     cudaStreamSynchronize(st);  // rec leaves scope
-    if ((rc = dalloc(h, &h->sp8, N * S * 8))) return bail(rc);
   }
-  if (prm->precision == AFR_PREC_MIXED && (rc = mixed_setup(h, m, Wkeep, st))) return bail(rc);
+  if (prm->precision == AFR_PREC_MIXED && (rc = mixed_setup(h, m, Wkeep, hs, st))) return bail(rc);
   if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = plain_setup(h, st))) return bail(rc);
   if (h->order == 0 && (rc = p0_setup(h, m, st))) return bail(rc);
   cudaError_t e = cudaStreamSynchronize(st);
@@ -1846,8 +1835,8 @@ static int step_impl(afr_handle* h, double* U, double* k, double* omega, double*
       nl += 3;
       if (r != cudaSuccess) return r;
     }
-    const double* cur[3] = {U, h->Ua, h->Ub};
-    double* nxt[3] = {h->Ua, h->Ub, U};
+    const double* cur[3] = {U, h->Ua, h->Ua};  // the second stage works in place
+    double* nxt[3] = {h->Ua, h->Ua, U};
     for (int stg = 0; stg < 3; ++stg) {
       StageArgs a = base_args(h);
       a.Ucur = cur[stg];
@@ -2042,7 +2031,7 @@ int afr_step_dual_time(afr_handle* h, double* U, double* k, double* omega, doubl
     prev = cur;
     a.scale = cfl;
     // SSP-RK3 of the dual residual from U (the stage-0 residual is the one above)
-    double* stg[3] = {h->Ua, h->Ub, h->iX};
+    double* stg[3] = {h->Ua, h->Ua, h->iX};
     for (int s = 0; s < 3; ++s) {
       if (s > 0 && (rc = eval_both(h, stg[s - 1], nut, h->iRinv, h->iRvisc, st))) return rc;
       a.U0 = U;

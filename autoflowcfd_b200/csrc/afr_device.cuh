@@ -33,11 +33,6 @@ enum DevStatus : uint32_t {
 
 // Per-cell-type operator set (index 0 = prism, 1 = tet), all row-major doubles.
 struct Ops {
-  const double* D3[2];      // (S, S, 3): D3[s*3S + j*3 + m]
-  const double* D3g[2];     // (3S, S):   gradient form, row s*3+m, col j
-  const double* c2f[2];     // (Fn, S)
-  const double* Dfine[2];   // (Fn, Fn*3)
-  const double* f2c[2];     // (S, Fn)
   const double* W[2];       // (S, 3Fn) = f2c * D_fine, folded once at create
   const double* filt[2];    // (S, S)
   const double* extrap;     // (2, 3, 2, P, S)
@@ -49,8 +44,8 @@ struct Ops {
   // (element (m, k) of an M x K operator at [((m/8) * ceil(K/4) + k/4) * 32 +
   // (m%8) * 4 + k%4], zero outside the operator): one warp's fragment load is
   // 256 contiguous bytes
-  const double* fD3[2];     // D3 as (S, 3S)
-  const double* fD3g[2];    // D3g (3S, S)
+  const double* fD3[2];     // D_3d (S, 3S), column j*3 + m
+  const double* fD3g[2];    // its gradient form (3S, S), row s*3 + m, column j
   const double* fc2f[2];    // c2f (Fn, S)
   const double* fW[2];      // W (S, 3Fn)
   const double* ffilt[2];   // filt (S, S)
@@ -67,10 +62,14 @@ struct Ops {
 struct Geom {
   int32_t N, n_prism;
   const double* det;        // (N, S)
-  const double* inv;        // (N, S, 3, 3)
-  const double* adj;        // (N, S, 3, 3)  det * inv, formed once at create
-  const double* adj_fine;   // (N, Fn, 3, 3)
-  const double* volume;     // (N)
+  // inverse Jacobians (N - inv0, S, 3, 3) of cells inv0 and up: the structured
+  // prisms of the plain form have none without SST (their gradients use adj / det)
+  const double* inv;
+  int32_t inv0;
+  // det * inv, formed once at create: (N, S, 3, 3), at fine points (N, Fn, 3, 3);
+  // structured prisms of the plain form: in lane order, see PxGeom
+  const double* adj;
+  const double* adj_fine;
   const double* mfs;        // (N, S) sum_m |adj[m,:]|
   const double* wall_dist;  // (N, S) or null
   const double* hvol;       // (N) |volume|^(1/3), the local-dt length (formed once at create)
@@ -82,6 +81,8 @@ struct Geom {
 // colored kernels add corrections into a cell.
 struct Faces {
   int32_t F;
+  // sides of the records: mixed form and order 0 (the plain form's slot records
+  // hold what it needs of them)
   const int32_t* owner;       // (F)
   const int32_t* neighbor;    // (F), -1 on boundary
   const int8_t* o_axis;       // (F)
@@ -95,25 +96,20 @@ struct Faces {
   // of the distinct matrices when the mesh gives one (a few dozen on
   // generated meshes), else the dense per-record arrays with identity
   // indices.  fmat() gives record r's face point i; weight s is at [s * P].
-  const int32_t* nb_c0;       // (F) neighbor-side sources (owner side reads)
-  const double* nb_m0;        // matrices of nb_m0i
+  // The row indices are the mixed form's; the plain form's are in its slot records.
+  const double* nb_m0;        // neighbor-side sources (owner side reads): first source
   const int32_t* nb_m0i;      // (F)
-  const int32_t* nb_i1;       // (F) index into the compact second source, -1 if none
-  const int32_t* nb_c1;       // (n1)
-  const double* nb_m1;
+  const double* nb_m1;        // compact second source
   const int32_t* nb_m1i;      // (n1)
-  const int32_t* ow_c0;       // owner-side sources (neighbor side reads)
-  const double* ow_m0;
+  const double* ow_m0;        // owner-side sources (neighbor side reads)
   const int32_t* ow_m0i;
-  const int32_t* ow_i1;
-  const int32_t* ow_c1;
   const double* ow_m1;
   const int32_t* ow_m1i;
   const int32_t* bc_group;    // (F) row of the BC table
   // residual slots: primary sides, ascending color
   const int32_t* slot_ptr;    // (N+1)
-  const int32_t* slot;        // face*2 + (0 owner, 1 neighbor)
-  // transport slots: every face side (owner always, neighbor if interior)
+  const int32_t* slot;        // face*2 + (0 owner, 1 neighbor); order 0 only
+  // transport slots (SST only): every face side (owner always, neighbor if interior)
   const int32_t* tslot_ptr;   // (N+1)
   const int32_t* tslot;       // face << 4 | axis << 2 | (neighbor side) << 1 | (side > 0)
 };

@@ -17,8 +17,7 @@ namespace afr {
 struct StageArgs {
   const double* Ucur;   // state the residual is evaluated on (N,S,nv)
   const double* U0;     // step-start state (RK combination)
-  const double* U1;     // stage-1 state (RK stage 2 combination)
-  double* Unext;        // output state (N,S,nv)
+  double* Unext;        // output state (N,S,nv); may be Ucur or U0: a warp or CTA writes only the cells it read
   const double* PF;     // (N,S,16) point fields of Ucur (k_pre)
   const double* nut;    // (N,S) kinematic eddy viscosity or null
   const double* dt;     // (N,S)
@@ -310,8 +309,14 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
     __syncthreads();
     for (int t = threadIdx.x; t < nc * S; t += blockDim.x) {
       double inv[9];
-      const double* ip = g.inv + ((size_t)e0 * S + t) * 9;
-      for (int k = 0; k < 9; ++k) inv[k] = __ldg(ip + k);
+      if (e0 >= g.inv0) {
+        const double* ip = g.inv + ((size_t)(e0 - g.inv0) * S + t) * 9;
+        for (int k = 0; k < 9; ++k) inv[k] = __ldg(ip + k);
+      } else {  // adjugate planes of a structured prism
+        const double* ap = g.adj + (size_t)(e0 + t / S) * 9 * S + t % S;
+        const double rd = 1.0 / __ldg(g.det + (size_t)e0 * S + t);
+        for (int k = 0; k < 9; ++k) inv[k] = __ldg(ap + k * S) * rd;
+      }
       double gr[4][3];  // rows u, v, w, T
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -349,14 +354,15 @@ __global__ void __launch_bounds__(128) k_pre(Geom g, Ops ops, const double* __re
 // ---------------------------------------------------------------------------
 struct SlotTable {
   int32_t n;                // number of slots
+  const int32_t* flags;     // (n)
+  // mixed form
   const int32_t* face;      // (n)
   const int32_t* cell;      // (n) cell the slot lifts into
-  const int32_t* flags;     // (n)
   const int32_t* c0;        // (n) first interpolation source cell, -1 if none
   const int32_t* c1;        // (n) second source cell, -1 if none
   const int32_t* i1;        // (n) row of the compact second-source table
-  // (n, 2) what the FP64 face kernel needs of a slot: source cells and matrix
-  // rows (c0, m0, c1, m1), then face, flags
+  // plain form: (n, 2) what a slot's face points need: source cells and matrix
+  // rows (c0, m0, c1, m1), then face, flags, cell
   const int4* rec;
 };
 
@@ -712,7 +718,8 @@ __global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (size_t)st.n * NP) return;
   const int sl = (int)(t / NP), i = (int)(t % NP);
-  const int f = st.face[sl], e = st.cell[sl], fl = st.flags[sl];
+  const int4 rc = __ldg(st.rec + 2 * (size_t)sl + 1);
+  const int f = rc.x, fl = rc.y, e = rc.z;
   const int ax = (fl >> 2) & 3, sb = (fl & 16) ? 1 : 0;
   const double* Er = ops.extrap + ((((size_t)cell_type(g, e) * 3 + ax) * 2 + sb) * NP + i) * S;
   double a0 = 0.0, a1 = 0.0, a2 = 0.0;

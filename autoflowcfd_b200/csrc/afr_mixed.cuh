@@ -1484,9 +1484,9 @@ __global__ void k_mx_rows_f32(const double* __restrict__ adj_fine, size_t nrows,
 
 // MD[c,s,n] = sum_{i,m} W[s, i*3+m] adj_fine[c,i,m,n]  (W's columns follow D_fine: i*3+m)
 template <int S, int FN>
-__global__ void k_mx_md(Geom g, Ops ops, double* MD) {
+__global__ void k_mx_md(Geom g, Ops ops, size_t ncells, double* MD) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)g.N * S * 3) return;
+  if (t >= ncells * S * 3) return;
   const int n = (int)(t % 3);
   const int s = (int)((t / 3) % S);
   const size_t c = t / (3 * S);

@@ -51,9 +51,9 @@ struct PxOps {
 // per-cell metrics in the order the lanes read them
 template <class T>
 struct PxGeom {
-  const T* adjs;       // (N, 9, S) solution-point adjugates, entry m*3 + n
+  const T* adjs;       // (n_prism, 9, S) solution-point adjugates, entry m*3 + n
   // fine-point adjugates (fine point = triangle point * NF + c-level): FP32
-  // (N, 9, MT, NF), a lane's c-line in one vector; FP64 (N, NF, 9, MT), level by level
+  // (n_prism, 9, MT, NF), a lane's c-line in one vector; FP64 (n_prism, NF, 9, MT), level by level
   const T* adjf;
   const double* MD;    // (N, S, 3)
   const double* rdet;  // (N, S)
@@ -547,16 +547,21 @@ __global__ void __launch_bounds__(32 * px_warps(N1), sizeof(T) == 8 ? (N1 == 3 ?
   }
 }
 
-// FP64 3 x 3 metric entries (npts per cell, 9 each) -> planes (N, 9, npts), or
-// with levels > 1 (N, levels, 9, npts / levels), point = j * levels + level
+// FP64 3 x 3 metric entries (npts <= 64 per cell, 9 each) -> planes (N, 9, npts),
+// or with levels > 1 (N, levels, 9, npts / levels), point = j * levels + level.
+// A CTA per cell, through shared memory: out may be adj (a second copy of the
+// metrics would be a quarter of a P2 handle).
 template <class T>
-__global__ void k_px_planes(const double* __restrict__ adj, size_t ncells, int npts, int levels, T* __restrict__ out) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncells * npts * 9) return;
+__global__ void __launch_bounds__(128) k_px_planes(const double* adj, int npts, int levels, T* out) {
+  __shared__ double sh[64 * 9];
+  const size_t base = (size_t)blockIdx.x * npts * 9;
+  for (int t = threadIdx.x; t < npts * 9; t += blockDim.x) sh[t] = adj[base + t];
+  __syncthreads();
   const int w = npts / levels;
-  const int j = (int)(t % w), k = (int)(t / w % 9), l = (int)(t / ((size_t)w * 9) % levels);
-  const size_t c = t / ((size_t)npts * 9);
-  out[t] = T(adj[(c * npts + (size_t)j * levels + l) * 9 + k]);
+  for (int t = threadIdx.x; t < npts * 9; t += blockDim.x) {
+    const int j = t % w, k = t / w % 9, l = t / (w * 9);
+    out[base + t] = T(sh[(j * levels + l) * 9 + k]);
+  }
 }
 
 // ---- host: operator structure ----
