@@ -1,5 +1,5 @@
-// Mixed-precision cell kernel of prisms whose operators have tensor-product
-// structure in the collapsed coordinates (a, b, c): point s = (a*N1 + b)*N1 + c.
+// Cell kernel of prisms, FP32 (mixed form) and FP64 (plain form), whose operators
+// have tensor-product structure in the collapsed coordinates (a, b, c): point s = (a*N1 + b)*N1 + c.
 //
 //   D_3d[.,.,0]  couples points of one a-line (same b, c), the same weights on
 //   every line; D_3d[.,.,2] likewise along c; D_3d[.,.,1] couples the points of
@@ -9,10 +9,12 @@
 //   c2f and the folded W = f2c*D_fine (per reference axis m) are Kronecker
 //   products triangle (x) c-line.
 //
-// The reference's prism operators have this structure to rounding (entries
-// outside it are 1e-16 to 6e-15 of the largest); afr_create tests for it
-// (px_operators) and takes this kernel instead of k_mx_pre + k_mx_vol, which
-// stay for every other operator set (tets, P3).
+// The reference's prism operators have this structure to rounding: entries
+// outside it are at most 2e-15 of the largest in D_3d, boundary_extrap and c2f,
+// and W is off by 6e-15 (P1) and 1.1e-13 (P2) of its rows' l1 norms.  afr_create
+// tests for it (px_operators) and takes this kernel instead of k_mx_pre +
+// k_mx_vol (mixed) or k_pre + k_cell's volume terms (plain), which stay for every
+// other operator set (tets, P3).
 //
 // Why: with the structure a P2 cell needs 9 k multiply-adds instead of the
 // 45 k of the dense products, so plain FP32 (whose products carry 24 bits
@@ -26,9 +28,10 @@
 // another's loads and arithmetic.  CW is chosen so that the items of the
 // phases fill the 32 lanes: P2, CW = 2: 27 + 27 points, 30 (cell, variable,
 // c-level), 32 (cell, fine triangle point), 30 (cell, field); P1, CW = 6: 48,
-// 60, 54 and 90 in two or three rounds.  The operators arrive as a kernel
-// parameter: every index into them is a compile-time constant, so they are
-// operands from the constant bank and cost no loads.
+// 60, 54 and 90 in two or three rounds.  The operators of the extrapolation, c2f
+// and W arrive as a kernel parameter: every index into them is a compile-time
+// constant, so they are operands from the constant bank and cost no loads.  The
+// derivatives differ from point to point; a lane loads its point's rows once.
 #pragma once
 #include "afr_mixed.cuh"
 
@@ -650,10 +653,14 @@ inline std::vector<double> px_rows(const double* D) {
 }
 
 // The structured operators of a prism set and their worst deviation from the
-// given ones: D (S, S, 3), E (3, 2, P, S), c2f (Fn, S), f2c (S, Fn), Df (Fn, Fn, 3).
+// given ones: D (S, S, 3), E (3, 2, P, S), c2f (Fn, S), relative to the largest
+// entry, and the folded W = f2c * Df (S, Fn, 3), as the row's summed deviation
+// over its l1 norm: what the contraction can be off by, in terms of its input.
+// f2c (S, Fn) and Df (Fn, Fn, 3) only give W's factors: neither is applied by
+// itself, and noise that is small in each can add up in their product.
 template <int N1, int NF>
 inline double px_operators(const double* D, const double* E, const double* c2f, const double* f2c, const double* Df,
-                           PxOps<double, N1, NF>& o) {
+                           const double* W, PxOps<double, N1, NF>& o) {
   constexpr int NT = N1 * N1, S = NT * N1, MT = NF * NF, FN = MT * NF, P = NT;
   double dev = px_lines<N1>(D, o.D0, o.D1, o.D2);
   auto e = [&](int ax, int sd, int i, int s) { return E[(((size_t)ax * 2 + sd) * P + i) * S + s]; };
@@ -685,11 +692,11 @@ inline double px_operators(const double* D, const double* E, const double* c2f, 
   if (!(dev < 1.0)) return INFINITY;
   for (int i = 0; i < MT * NT; ++i) o.Ct[i / NT][i % NT] = T[i];
   for (int i = 0; i < NF * N1; ++i) o.Cc[i / N1][i % N1] = c[i];
-  // W = f2c * D_fine from the factors of both: (T (x) c) * (a-line, plane, c-line)
-  dev = std::max(dev, px_kron(NT, N1, MT, NF, [&](int i, int j) { return f2c[(size_t)i * FN + j]; }, T, c));
+  // W's factors from those of f2c and D_fine: (T (x) c) * (a-line, plane, c-line)
   double f0[NF][NF], f1[MT][MT], f2[NF][NF];
-  dev = std::max(dev, px_lines<NF>(Df, f0, f1, f2));
-  if (!(dev < 1.0)) return INFINITY;
+  if (!(px_kron(NT, N1, MT, NF, [&](int i, int j) { return f2c[(size_t)i * FN + j]; }, T, c) < 1.0) ||
+      !(px_lines<NF>(Df, f0, f1, f2) < 1.0))
+    return INFINITY;
   for (int r = 0; r < NT; ++r)
     for (int t = 0; t < MT; ++t) {
       double w0 = 0.0, w1 = 0.0;
@@ -706,6 +713,17 @@ inline double px_operators(const double* D, const double* E, const double* c2f, 
       o.Wc[0][k][l] = o.Wc[1][k][l] = c[k * NF + l];
       o.Wc[2][k][l] = w2;
     }
+  for (int s = 0; s < S; ++s) {
+    double off = 0.0, l1 = 0.0;
+    for (int i = 0; i < FN; ++i)
+      for (int m = 0; m < 3; ++m) {
+        const double w = W[((size_t)s * FN + i) * 3 + m];
+        off += std::fabs(w - o.Wt[m][s / N1][i / NF] * o.Wc[m][s % N1][i % NF]);
+        l1 += std::fabs(w);
+      }
+    if (!(l1 <= 1e300) || l1 == 0.0) return INFINITY;
+    dev = std::max(dev, off / l1);
+  }
   return dev;
 }
 

@@ -104,6 +104,28 @@ def test_structured_prisms_against_oracle_and_generic_kernels(order, shape):
     assert rel(mx[2], f64[2]) < 1e-6
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("order", [1, 2])
+def test_noise_that_adds_up_in_the_folded_operator_leaves_the_structure(order, precision):
+    """f2c entries off by 1.2e-13 of its largest, signed so that the row's products
+    with D_fine add up: the folded W, which the kernels apply, is off by 1.6e-12 (P1)
+    and 2e-11 (P2) of that row's l1 norm, over both forms' limits.  Viscous
+    residuals do not see f2c: their bits tell the kernels apart."""
+    case, U, nut = make("prism", (2, 2, 2), order)
+    f2c, D = case["f2c_prism"], case["Dfine_prism"].reshape(case["Dfine_prism"].shape[0], -1)
+    v = np.random.default_rng(0).choice([-1.0, 1.0], f2c.shape[1])
+    for _ in range(50):
+        v = np.sign(D @ np.sign(v @ D))
+    noise = 1.2e-13 * np.abs(f2c).max() * v
+    assert np.abs(noise @ D).sum() > 1.5e-12 * np.abs(f2c[0] @ D).sum()
+    noisy = dict(case)
+    noisy["f2c_prism"] = f2c.copy()
+    noisy["f2c_prism"][0] += noise
+    good, other = evaluate(case, U, nut, precision), evaluate(noisy, U, nut, precision)
+    assert np.any(good[1] != other[1])
+    assert rel(good[1], other[1]) < (1e-11 if precision == "fp64" else 2e-2)
+
+
 def test_viscous_tets_against_oracle():
     """The generic cell kernel's viscous tiles and the staged P1 faces on tets."""
     case, U, nut = make("tet", (3, 3, 3), 1)
