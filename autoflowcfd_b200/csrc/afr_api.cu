@@ -83,6 +83,7 @@ struct afr_handle {
   double4* slot_rows = nullptr;  // (n_slots, P) own adjugate rows (plain form)
   unsigned px_faces = 0;  // bit (axis*2 + side): faces whose point fields some slot reads
   bool px_points = false;  // some face point interpolates from the point fields
+  bool face_rows = false;  // P2 Euler runs of the plain form: k_face takes the own side from the rows' nonzeros
   int mx_pre_blocks = 0, mx_cell_blocks = 0;  // resident CTAs of the persistent kernels
   int mx_pre_per_sm = 0, mx_pre_max_per_sm = 0, n_sms = 0;
   int mx_pre_occ = 0, mx_vol_occ = 0;          // occupancy-API CTAs per SM, before the tensor-memory cap
@@ -457,7 +458,9 @@ struct Launch {
             h->g, h->ops, h->fc, h->bc, h->slots, h->PF, h->slot_rows, h->prm.mu, h->J);
       } else {
         constexpr int per = FACE_WARPS * (32 / NP);
-        auto* fn = a.inviscid_only ? k_face<S, NP, false> : k_face<S, NP, true>;
+        auto* fn = a.inviscid_only ? k_face<S, NP, false, false> : k_face<S, NP, true, false>;
+        if constexpr (S == 27)
+          if (a.inviscid_only && h->face_rows) fn = k_face<S, NP, false, true>;
         fn<<<(h->slots.n + per - 1) / per, 32 * FACE_WARPS, 0, st>>>(h->g, h->ops, h->fc, h->bc, h->slots, h->PF,
                                                                      h->slot_rows, h->prm.mu, h->J);
       }
@@ -1435,6 +1438,7 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     // nonzeros of the extrapolation rows
     std::vector<double> ew(12 * S * P, 0.0);
     std::vector<int32_t> ei(12 * S * P, 0), en(12 * P, 0);
+    size_t nonzeros = 0, rows = 0;  // of the cell types present
     for (size_t gr = 0; gr < 12; ++gr)
       for (size_t i = 0; i < P; ++i) {
         const double* w = m->boundary_extrap + (gr * P + i) * S;
@@ -1451,7 +1455,13 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
           }
         for (int32_t k = 0; k < n; ++k) ew[(gr * S + k) * P + i] += rest / n;
         en[gr * P + i] = n;
+        if (gr < 6 ? h->n_prism > 0 : h->N > h->n_prism) {
+          nonzeros += n;
+          ++rows;
+        }
       }
+    // a quarter of the points: between P2 prisms (5.1 of 27) and P2 tets (15.9), see k_face
+    h->face_rows = 4 * nonzeros <= rows * S;
     double* dw;
     int32_t *di, *dn;
     if ((rc = upload(h, &dw, ew.data(), ew.size(), st)) || (rc = upload(h, &di, ei.data(), ei.size(), st)) ||

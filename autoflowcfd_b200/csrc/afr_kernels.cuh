@@ -512,8 +512,7 @@ __device__ __forceinline__ void face_jump(const Geom& g, const Faces& fc, const 
 }
 
 // Face kernels.  A slot is one side of one face record whose correction lifts
-// into a cell; lane = (slot, flux point) forms the own side from the nonzeros
-// of its extrapolation row (Ops::ex_*: 3 or 9 of a P2 prism's 27 points), the
+// into a cell; lane = (slot, flux point) forms the own side by extrapolation, the
 // other side with the record's matrix (the second source added to the first),
 // the ghost state, AUSM+up with the alignment fallback and the BR1 common flux
 // with the boundary penalty
@@ -524,11 +523,19 @@ __device__ __forceinline__ void face_jump(const Geom& g, const Faces& fc, const 
 // skips zero weights, inviscid_kernel_colored.py:117-121; a non-finite state
 // makes the step non-finite either way).
 //
-// k_face (orders 2, 3): a warp per group of SPW = 32 / NP slots; the other
-// side's product is register-blocked on the FP64 tensor path, its operands
-// gathered straight from global memory.
+// k_face (orders 2, 3): a warp per group of SPW = 32 / NP slots; both sides'
+// products are register-blocked on the FP64 tensor path, their operands
+// gathered straight from global memory.  ROWS: the own side from the nonzeros of
+// its extrapolation row instead (Ops::ex_*), by the lane itself.  That pays only
+// without viscosity, where the product's five columns leave three of a tile's
+// eight idle, and where the rows are sparse: step of 17,280 P2 prisms (5.1
+// nonzeros of 27 on average) 728 us with, 746 without; residual of 10,368 P2 tets
+// (15.9) 245 and 224.  With viscosity the rows cost more on every mesh: 17,280 P2
+// prisms 1,144 and 1,090 us per step, 1,332 and 1,275 with SST; both residuals of
+// 10,368 P2 tets 593 and 511, of 10,080 P3 prisms 1,386 and 1,182, of 6,000 P3
+// tets 910 and 629.
 // k_face_staged (order 1, 8 x 4 matrices that fill a quarter of the tensor
-// tiles): a warp per cell; the rows of the cell and of its slots' source cells
+// tiles): a warp per cell, the own side from the row's nonzeros; the rows of the cell and of its slots' source cells
 // arrive in shared memory by 16-byte asynchronous copies, all in flight at
 // once, and the products are plain multiply-adds.  24,576 P1 tets, inviscid: 83 us on
 // the tensor path, 64 us staged; 17,280 P2 prisms, viscous: 268 us staged.
@@ -630,14 +637,11 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, VISC ? 3 : 4)
   }
 }
 
-template <int S, int NP, bool VISC>
+template <int S, int NP, bool VISC, bool ROWS>
 __global__ void __launch_bounds__(32 * FACE_WARPS, 4)
     k_face(Geom g, Ops ops, Faces fc, Bc bc, SlotTable st, const double* __restrict__ PF,
            const double4* __restrict__ arow, double mu, double* __restrict__ J) {
   constexpr int SPW = 32 / NP, MT = (NP + 7) / 8, NF = VISC ? FW_F : 5, NT = (NF + 7) / 8;
-  // own side from the rows' nonzeros at P2; at P3, where the reference's rows
-  // are up to full, on the tensor path too (24,576 P3 tets: 500 us with the rows)
-  constexpr bool ROWS = S <= 27;
   __shared__ double sOt[FACE_WARPS][SPW * NP * NF];
   __shared__ double sOw[ROWS ? 1 : FACE_WARPS][ROWS ? 1 : SPW * NP * NF];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

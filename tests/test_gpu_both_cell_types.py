@@ -73,7 +73,10 @@ def test_prisms_and_tets_in_one_handle(order, precision):
                                 "z_min": {"type": "WALL", "is_no_slip": True}})
     a = B200FRSolver(alone, mu_molecular=MU, rho_inf=RHO, vel_inf=60.0, p_inf=P, precision=precision)
     a.set_state_from_cpu(U[:n])
-    assert np.array_equal(a.compute_inviscid_residual().cpu().numpy(), gi[:n])
+    alone_i = a.compute_inviscid_residual().cpu().numpy()
+    # P2 plain Euler faces extrapolate from the rows' nonzeros or by the full product, by the mesh's mean row: the
+    # order of the sums, as against the oracle above
+    assert rel(gi[:n], alone_i) < 1e-11 if (order, precision) == (2, "fp64") else np.array_equal(gi[:n], alone_i)
     assert np.array_equal(a.compute_viscous_residual().cpu().numpy(), gv[:n])
     ref = a.compute_aerodynamic_coefficients()
     a.cleanup()
