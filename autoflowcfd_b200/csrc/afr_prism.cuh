@@ -147,7 +147,12 @@ __global__ void __launch_bounds__(32 * px_warps(N1), sizeof(T) == 8 ? (N1 == 3 ?
     mut[r] = T(0);
     if (in && c < nc) {
       const double* d = reinterpret_cast<const double*>(sc);
-      mxd::prim_T(d + s * nv, q);
+      if constexpr (D) {  // quotients as in k_pre: a reciprocal of rho would round twice
+        cons_to_prim(d + s * nv, q);
+        q[5] = q[4] / (q[0] * R_AIR);
+      } else {
+        mxd::prim_T(d + s * nv, q);
+      }
       if (VISC && nut) mut[r] = T(q[0] * d[7 * S + s]);
     }
     // FP32: deviations from the value at the cell's middle point, which carry
