@@ -34,16 +34,15 @@ def test_one_cells_extreme_value_stays_with_its_neighbours(precision, order, pla
         s = B200FRSolver(case, mu_molecular=E.MU, rho_inf=E.RHO_INF, vel_inf=spec.velocity, p_inf=E.P_INF,
                          precision=precision)
         s.set_state_from_cpu(V)
-        try:
-            out.append(s.compute_inviscid_residual().cpu().numpy())
-        except RuntimeError:
-            out.append(None)
+        out.append(s.compute_inviscid_residual().cpu().numpy())  # reports no state of its own: any error is a failure
         s.cleanup()
     clean, bad = out
     assert np.all(np.isfinite(clean))
-    if bad is not None:
-        far = [c for c in range(N) if c not in near]
-        assert np.array_equal(bad[far], clean[far])
+    far = [c for c in range(N) if c not in near]
+    assert np.array_equal(bad[far], clean[far])
+    assert np.any(bad[victim] != clean[victim])
+    if planted == 1e200 and precision == "fp64":  # a finite value: finite terms, cleared where the rule says so
+        assert np.all(np.isfinite(bad))
 
 
 @pytest.mark.parametrize("order", [1, 2])
