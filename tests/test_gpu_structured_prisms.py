@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from autoflowcfd_b200 import boxgeom, boxmesh
+from fields import per_field, scalar, worst
 from oracle import fr_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -18,7 +19,7 @@ RHO, P = 1.225, 101325.0
 SHAPES = [(2, 2, 2), (3, 3, 2), (5, 3, 3), (3, 3, 3)]
 
 
-def make(kind, shape, order):
+def make(kind, shape, order, wall_distance=False):
     u = 60.0
     cfg = {n: {"type": "FARFIELD", "Q_free": [RHO, u, 0.0, 0.0, P]} for n in boxmesh.PLANE_NAMES}
     cfg["z_min"] = {"type": "WALL", "is_no_slip": True}
@@ -30,7 +31,8 @@ def make(kind, shape, order):
         box = boxmesh.prism_box(*shape, (0.4, 0.3, 0.2), jitter=0.1, seed=3)
     else:
         box = boxmesh.tet_box(*shape, (0.4, 0.3, 0.2), jitter=0.05, seed=3, periodic=True)
-    case = boxgeom.build_case(box, order, cfg if kind == "prism" else None, want_sps_coords=True)
+    case = boxgeom.build_case(box, order, cfg if kind == "prism" else None, wall_distance=wall_distance,
+                              want_sps_coords=True)
     x = case.pop("sps_coords")
     rng = np.random.default_rng(17)
     s = lambda a: np.sin((x * a).sum(-1) * 9.0 + rng.uniform(0, 6))  # noqa: E731
@@ -63,12 +65,16 @@ def evaluate(case, U, nut, precision):
     return out
 
 
-def oracle(case, U, nut):
+def dense(case):
     c = dict(case)
     tab = c.pop("src_mat_table")
     for k in ("nb_src0_mat", "nb_src1_mat", "ow_src0_mat", "ow_src1_mat"):
         c[k] = tab[c.pop(k + "_index")]
-    m = O.Mesh.from_case(c)
+    return O.Mesh.from_case(c)
+
+
+def oracle(case, U, nut):
+    m = dense(case)
     return O.inviscid_residual(m, U), O.viscous_residual(m, U, 2e-3, np.maximum(U[..., 0], 1e-10) * nut)
 
 
@@ -134,3 +140,54 @@ def test_viscous_tets_against_oracle():
     ri, rv = oracle(case, U, nut)
     out = evaluate(case, U, nut, "fp64")
     assert rel(out[0], ri) < 1e-10 and rel(out[1], rv) < 1e-10
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("order", [1, 2])
+def test_structured_sst_kernels_at_tile_edges(order, shape):
+    """The mixed form's SST kernels of structured prisms (four P1 cells or one P2
+    cell per warp) against the plain form's, which run the generic ones: one update
+    of the same fields.  Operators 2e-15 apart, twice differentiated: 1e-12 of the
+    fields; the sources, which differences of them make, 1e-9."""
+    import torch
+
+    from autoflowcfd_b200.solver import B200FRSolver
+
+    case, U, nut = make("prism", shape, order, wall_distance=True)
+    k = 0.5 * nut / nut.mean()
+    w = k / nut
+    U = np.concatenate([U, (U[..., 0] * k)[..., None], (U[..., 0] * w)[..., None]], -1)
+    out = []
+    for precision in ("fp64", "mixed"):
+        s = B200FRSolver(case, turb_model_name="SST", mu_molecular=2e-3, rho_inf=RHO, vel_inf=60.0, p_inf=P,
+                         precision=precision)
+        s.set_state_from_cpu(U)
+        s.set_turbulence(k, w, nut)
+        dt = torch.full(k.shape, 1e-6, dtype=torch.float64, device="cuda")
+        diag = [d.cpu().numpy() for d in s.compute_turbulence_source(dt, diag=True)]
+        out.append(([a.cpu().numpy() for a in (s.k, s.omega, s.nu_t)], diag))
+        s.cleanup()
+    (f64, d64), (fmx, dmx) = out
+    assert np.any(f64[0] != k) and np.any(f64[1] != w)  # the update moved them
+    assert all(scalar(a, b)[1] < 1e-12 for a, b in zip(fmx, f64))
+    assert all(scalar(a, b)[1] < 1e-9 for a, b in zip(dmx, d64))
+
+
+@pytest.mark.parametrize("order", [0, 1, 2, 3])
+def test_dual_time_stage_at_tile_edges(order):
+    """Pseudo-time stages with the positivity and filter in the same kernel (eight
+    cells per warp up to P1, three above): 100 cells leave remainders of both.  Two
+    physical steps (BDF1, BDF2) against the oracle."""
+    from autoflowcfd_b200.solver import B200FRSolver
+
+    case, U, _ = make("prism", (5, 5, 2), order)
+    ref = O.Solver(dense(case), U.copy(), 2e-3, time_scheme="dual_time", dt_step=1e-4, dual_time_inner_iter=2)
+    s = B200FRSolver(case, mu_molecular=2e-3, rho_inf=RHO, vel_inf=60.0, p_inf=P, time_scheme="dual_time",
+                     dual_time_inner_iter=2)
+    s.set_state_from_cpu(U)
+    for _ in range(2):
+        n_ref, n = ref.step(), s.step(1e-4)
+        assert worst(per_field(s.U, ref.U)) < 1e-12
+        assert abs(n - n_ref) <= 1e-9 * n_ref
+    assert worst(per_field(ref.U, U)) > 1e-9  # the steps moved the state
+    s.cleanup()
