@@ -197,32 +197,7 @@ __device__ __forceinline__ void ausm_up(const T qL[5], const T qR[5], const T n[
   out[4] = mdot * (up ? hL : hR);
 }
 
-// gv[a*3+b] = d u_a / d x_b, gT[3], viscous flux G (3,5)
-template <class T>
-__device__ __forceinline__ void viscous_flux(const T q[5], const T gv[9], const T gT[3], T mu, T mu_t, T G[3][5]) {
-  const T mt = mu + mu_t;
-  const T S00 = gv[0], S11 = gv[4], S22 = gv[8];
-  const T S01 = T(0.5) * (gv[1] + gv[3]);
-  const T S02 = T(0.5) * (gv[2] + gv[6]);
-  const T S12 = T(0.5) * (gv[5] + gv[7]);
-  const T div = gv[0] + gv[4] + gv[8];
-  const T lam = T(-2.0 / 3.0) * mt;
-  const T t00 = T(2.0) * mt * S00 + lam * div;
-  const T t11 = T(2.0) * mt * S11 + lam * div;
-  const T t22 = T(2.0) * mt * S22 + lam * div;
-  const T t01 = T(2.0) * mt * S01, t02 = T(2.0) * mt * S02, t12 = T(2.0) * mt * S12;
-  const T cp = T(GAMMA * R_AIR / (GAMMA - 1.0));
-  const T k = mu * cp / T(PR) + mu_t * cp / T(PR_T);
-  const T u = q[1], v = q[2], w = q[3];
-  G[0][0] = T(0.0); G[0][1] = t00; G[0][2] = t01; G[0][3] = t02;
-  G[1][0] = T(0.0); G[1][1] = t01; G[1][2] = t11; G[1][3] = t12;
-  G[2][0] = T(0.0); G[2][1] = t02; G[2][2] = t12; G[2][3] = t22;
-  G[0][4] = (u * t00 + v * t01 + w * t02) + (-k * gT[0]);
-  G[1][4] = (u * t01 + v * t11 + w * t12) + (-k * gT[1]);
-  G[2][4] = (u * t02 + v * t12 + w * t22) + (-k * gT[2]);
-}
-
-// viscous_flux from the symmetric gradient sg = (S00, S11, S22, S01, S02, S12),
+// viscous flux from the symmetric gradient sg = (S00, S11, S22, S01, S02, S12),
 // S_ij = (d_j u_i + d_i u_j) / 2, the only combinations of the velocity
 // gradient it contains; components 1..4 (the mass flux is zero)
 template <class T>

@@ -29,7 +29,7 @@
 
 namespace {
 
-constexpr int FP_MAX = 16, SPS_MAX = 64, N1D_MAX = 4, JOB_WARPS = 4;
+constexpr int FP_MAX = 16, SPS_MAX = 64, JOB_WARPS = 4;
 constexpr int NEWTON_MAX_ITER = 50, LINE_SEARCH_MAX = 20;
 __constant__ int c_face_axis[6] = {0, 0, 1, 1, 2, 2};
 __constant__ double c_face_side[6] = {-1.0, 1.0, -1.0, 1.0, -1.0, 1.0};

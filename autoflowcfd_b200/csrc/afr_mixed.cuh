@@ -141,24 +141,6 @@ __device__ __forceinline__ void prefetch_l2(const void* base, size_t total, size
   }
 }
 
-// two consecutive K positions (idx even) of one row: hi and lo parts as
-// packed bf16x2 words, one conversion per part
-__device__ __forceinline__ void st_split2(uint16_t* img, int img_elems, int idx, float x0, float x1) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-  const float2 hf = __bfloat1622float2(h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - hf.x, x1 - hf.y);
-  *reinterpret_cast<__nv_bfloat162*>(img + idx) = h;
-  *reinterpret_cast<__nv_bfloat162*>(img + img_elems + idx) = l;
-}
-
-// (cell, point pair) enumeration with the cell fastest in groups of 8: lanes
-// of a warp cover 8 cells x 4 consecutive pairs (8 points, one 16-byte row each)
-__device__ __forceinline__ void cell_pair(int idx, int npts, int& c, int& p0) {
-  const int rest = idx >> 3;
-  p0 = 2 * (rest % (npts / 2));
-  c = (rest / (npts / 2)) * 8 + (idx & 7);
-}
-
 using afr::cp_async8;
 using afr::cp_async_wait_all;
 

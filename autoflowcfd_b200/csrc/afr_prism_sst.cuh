@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(32 * PXS_WARPS)
   if (nc <= 0) return;  // whole warps; no block barrier below
   const int s = lane % S, c = lane / S < CPR ? lane / S : 0;
   const bool on = lane / S < nc;
-  const int tri = s / N1, cc = s % N1;
+  const int cc = s % N1;
   const int nv = a.nv;
   double* sw = smd + warp * CPR * L::cell;
   for (int b = 0; b < nc; ++b) {

@@ -126,11 +126,5 @@ __device__ __forceinline__ void tmem_ldn(uint32_t taddr, float* v) {
   for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// hi + lo BF16 split of an FP32 value: x ~= hi + lo to about 2^-16 relative
-__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& lo) {
-  hi = __float2bfloat16_rn(x);
-  lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-}
-
 }  // namespace tc
 }  // namespace afr
