@@ -1115,15 +1115,15 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
     switch (h->order) {
       case 1: k_mx_md<8, 27><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<8><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
-              if (ns) k_mx_match<8, 4><<<(unsigned)((ns * 4 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
+              if (ns) k_mx_match<8, 4><<<(unsigned)((ns * 4 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, h->status, 1e-6);
               break;
       case 2: k_mx_md<27, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<27><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
-              if (ns) k_mx_match<27, 9><<<(unsigned)((ns * 9 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
+              if (ns) k_mx_match<27, 9><<<(unsigned)((ns * 9 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, h->status, 1e-6);
               break;
       default: k_mx_md<64, 64><<<(unsigned)((nmd + 255) / 256), 256, 0, st>>>(h->g, h->ops, N, md);
               k_mx_hcell<64><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(h->g, hc);
-              if (ns) k_mx_match<64, 16><<<(unsigned)((ns * 16 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, 1e-6);
+              if (ns) k_mx_match<64, 16><<<(unsigned)((ns * 16 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, h->status, 1e-6);
               break;
     }
     const size_t nrows = N * (size_t)h->Fn * 3, nsrows = N * (size_t)S * 3;
@@ -1141,40 +1141,28 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
     return r != cudaSuccess ? r : LL::mx_grids(h);
   });
   if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form set-up");
-  unsigned s = 0;
-  e = cudaMemcpyAsync(&s, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+  unsigned used = 0;  // what k_mx_match found, through the status word
+  e = cudaMemcpyAsync(&used, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form set-up");
   cudaMemsetAsync(h->status, 0, sizeof(unsigned), st);
+  h->px_faces = used & 0x3fu;
+  h->px_points = (used & MX_GENERAL) != 0;
   // pair the matched slot points of interior faces across the face's two
   // slots: owner point (slot s, i) matched to the neighbour's face point j,
   // whose own match points back at (s's face, i)
   if (ns > 0) {
     const size_t nt = ns * P;
     std::vector<uint8_t> hofp(nt);
-    const std::vector<int32_t>&hface = hs.face, &hflag = hs.flags, &hcell = hs.cell;
+    const std::vector<int32_t>&hface = hs.face, &hflag = hs.flags;
     e = cudaMemcpy(hofp.data(), ofp, nt, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
     std::vector<int32_t> nb_slot(h->F, -1);
-    for (size_t sl = 0; sl < ns; ++sl) {
-      const int fl = hflag[sl];
-      if (fl & 1) nb_slot[hface[sl]] = (int32_t)sl;
-      h->px_faces |= 1u << (((fl >> 2) & 3) * 2 + ((fl & 16) ? 1 : 0));
-      if (fl & 2) continue;  // boundary: no other side
-      for (int i = 0; i < P; ++i) {
-        const int o = hofp[sl * P + i];
-        if (o == MX_OFP_GENERAL) h->px_points = true;
-        else h->px_faces |= 1u << (o / P);
-      }
-    }
-    std::vector<MxPair> pairs;
+    for (size_t sl = 0; sl < ns; ++sl)
+      if (hflag[sl] & 1) nb_slot[hface[sl]] = (int32_t)sl;
+    std::vector<int2> pairs;
     std::vector<uint8_t> taken(nt, 0);
     if (N * 6 * P >= ((size_t)1 << 31)) return fail(h, AFR_EUNSUPPORTED, "more than 2^31 face points");
-    auto row = [&](size_t sl, int i) -> uint32_t {
-      const int fl = hflag[sl];
-      const uint32_t face = ((fl >> 2) & 3) * 2 + ((fl & 16) ? 1 : 0);
-      return (((uint32_t)hcell[sl] * 6 + face) * P + i) | ((fl & 16) ? 0x80000000u : 0u);
-    };
     pairs.reserve(nt / 2);
     for (size_t sl = 0; sl < ns; ++sl) {
       const int fl = hflag[sl];
@@ -1190,21 +1178,26 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
         if (o == MX_OFP_GENERAL || o / P != code2) continue;
         const size_t t2 = (size_t)s2 * P + o % P;
         if (hofp[t2] != code * P + i || taken[t2]) continue;
-        pairs.push_back(MxPair{(int32_t)t, (int32_t)t2, row(sl, i), row(s2, o % P)});
+        pairs.push_back(make_int2((int)t, (int)t2));
         taken[t] = taken[t2] = 1;
       }
     }
     std::vector<int32_t> rest;
     for (size_t t = 0; t < nt; ++t)
       if (!taken[t]) rest.push_back((int32_t)t);
-    int32_t* dpairs = nullptr;
     int32_t* drest = nullptr;
-    if (!pairs.empty() && (rc = upload(h, &dpairs, reinterpret_cast<const int32_t*>(pairs.data()), pairs.size() * 4, st)))
-      return rc;
+    if (!pairs.empty()) {
+      if ((rc = dalloc(h, &h->mx_pairs, pairs.size()))) return rc;
+      // through the jumps, which are larger (36 bytes per slot point, at most 4 here) and not in use yet
+      int2* tmp = reinterpret_cast<int2*>(jm);
+      e = cudaMemcpyAsync(tmp, pairs.data(), pairs.size() * sizeof(int2), cudaMemcpyHostToDevice, st);
+      k_mx_pairs<<<(unsigned)((pairs.size() + 255) / 256), 256, 0, st>>>(h->slots, tmp, (int)pairs.size(), P, h->mx_pairs);
+      if (e == cudaSuccess) e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
+    }
     if (!rest.empty() && (rc = upload(h, &drest, rest.data(), rest.size(), st))) return rc;
     e = cudaStreamSynchronize(st);  // host vectors leave scope
     if (e != cudaSuccess) return cuda_fail(h, e, "mixed-form face pairs");
-    h->mx_pairs = reinterpret_cast<MxPair*>(dpairs);
     h->mx_rest = drest;
     h->mx_npairs = (int)pairs.size();
     h->mx_nrest = (int)rest.size();

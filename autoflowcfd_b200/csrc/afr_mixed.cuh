@@ -1382,9 +1382,13 @@ __global__ void __launch_bounds__(128, S == 64 ? 3 : (sizeof(T) == 8 ? 4 : (S ==
 // ---------------------------------------------------------------------------
 // own adjugate row at each slot flux point (E * adj, FP64 then rounded) and the
 // face point of the other side whose extrapolation row equals the slot's
-// interpolation row to tol relative (MX_OFP_GENERAL where none does)
+// interpolation row to tol relative (MX_OFP_GENERAL where none does).  used: bit
+// axis*2 + side of every face whose face-point fields a slot reads, and MX_GENERAL
+// where some point interpolates from point fields
+constexpr unsigned MX_GENERAL = 1u << 8;
 template <int S, int NP>
-__global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow, uint8_t* ofp, double tol) {
+__global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow, uint8_t* ofp, unsigned* used,
+                           double tol) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= st.n * NP) return;
   const int sl = t / NP, i = t % NP;
@@ -1410,6 +1414,10 @@ __global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow
                      ar.z / mag * sd * (sg * float(tn[2]));
     arow[t] = make_float4(ar.x, ar.y, ar.z, al < 0.5f ? -mag : ar.w);
   }
+  auto mark = [used](unsigned bits) {
+    if (bits & ~*(volatile unsigned*)used) atomicOr(used, bits);  // few threads find a bit unset
+  };
+  mark(1u << (ax * 2 + sb));
   if (bnd) {
     ofp[t] = 0;
     return;
@@ -1420,6 +1428,7 @@ __global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow
   const int expect = is_owner ? fc.neighbor[f] : fc.owner[f];
   const bool one_cell = (c0 == expect || c0 < 0) && (c1 == expect || c1 < 0) && (c0 >= 0 || c1 >= 0);
   if (!one_cell) {
+    mark(MX_GENERAL);
     ofp[t] = MX_OFP_GENERAL;
     return;
   }
@@ -1445,8 +1454,21 @@ __global__ void k_mx_match(Geom g, Ops ops, Faces fc, SlotTable st, float4* arow
       best = j;
     }
   }
-  ofp[t] = (best >= 0 && best_err <= tol * fmax(mmax, 1e-300)) ? (uint8_t)((oax * 2 + osb) * NP + best)
-                                                                 : MX_OFP_GENERAL;
+  const bool matched = best >= 0 && best_err <= tol * fmax(mmax, 1e-300);
+  mark(matched ? 1u << (oax * 2 + osb) : MX_GENERAL);
+  ofp[t] = matched ? (uint8_t)((oax * 2 + osb) * NP + best) : MX_OFP_GENERAL;
+}
+
+// the records of matched slot points: their face-point rows and sides
+__global__ void k_mx_pairs(SlotTable st, const int2* __restrict__ pts, int n, int NP, MxPair* __restrict__ out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int2 t = pts[j];
+  auto row = [&](int p) -> uint32_t {
+    const int sl = p / NP, fl = st.flags[sl], face = ((fl >> 2) & 3) * 2 + ((fl & 16) ? 1 : 0);
+    return (((uint32_t)st.cell[sl] * 6 + face) * NP + p % NP) | ((fl & 16) ? 0x80000000u : 0u);
+  };
+  out[j] = MxPair{t.x, t.y, row(t.x), row(t.y)};
 }
 
 // 1 / det per solution point

@@ -46,9 +46,9 @@ struct PxOps {
   static constexpr int NT = N1 * N1, MT = NF * NF;
   T E02[2][2][N1];   // extrapolation along a (0) and c (1): [which][side][point of the line]
   T E1[2][N1][NT];   // extrapolation to the b faces: [side][a of the face point][triangle point]
-  // The factors below start at an odd entry: read as vectors (at even or aligned
-  // ones) they go through registers, one by one they are operands.  102,660 P2
-  // prisms, step: 2,028 us at an odd entry, 2,058 aligned to four, 2,086 at an even one.
+  // The factors below start at an odd entry, where the compiler cannot combine
+  // their loads.  102,660 P2 prisms, step: 2,028 us there, 2,058 aligned to four
+  // entries, 2,086 at an even one (registers and spills are the same).
   T odd[1];
   T Ct[MT][NT], Cc[NF][N1];        // c2f = Ct (x) Cc
   T Wt[3][NT][MT], Wc[3][N1][NF];  // W per axis = Wt (x) Wc

@@ -65,9 +65,12 @@ enum { AFR_TURB_NONE = 0, AFR_TURB_SST = 1 };
  * and the extrapolation to faces) in FP32 where the prism operators are tensor
  * products, and elsewhere on the tensor cores as BF16 hi+lo split products
  * with FP32 accumulation; pointwise fluxes are FP32.  It keeps FP64 for the
- * state, geometry metrics, primitive recovery, residual sums,
+ * state, geometry metrics, primitive recovery, SST closure, residual sums,
  * RK update, norm and Cd/Cl.  Viscous terms are built up to P2 in the mixed
- * form (P3 mixed handles must be inviscid).  A contraction accumulated in FP32
+ * form (P3 mixed handles must be inviscid).  The SST gradients of tensor-product
+ * prisms leave out the operators' entries outside that structure (rounding
+ * noise, 2e-15 of the largest): omega of a growing closure moves by 2.3e-8 in
+ * twelve steps by that alone.  A contraction accumulated in FP32
  * carries about 2^-24 * (operator row l1 norm) * |x|, so afr_create refuses
  * the mixed form (AFR_EUNSUPPORTED) when a present cell type's operators have
  * row l1 norms above 1e6: the reference's collapsed-tet operators at P2 and P3
