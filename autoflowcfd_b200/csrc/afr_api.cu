@@ -51,7 +51,7 @@ struct afr_handle {
   SstFace* sst_faces = nullptr;
   uint8_t* cd_wall = nullptr;
   double* area_w = nullptr;
-  int4* cd_faces = nullptr;   // wall faces of the force integral: face, owner, axis, side > 0
+  int4* cd_faces = nullptr;   // wall faces of the force integral: row of the normals, owner, axis, side > 0
   int n_cd_faces = 0;
   double* cd_part = nullptr;  // (n_cd_faces, 6)
   unsigned* status = nullptr;
@@ -949,30 +949,42 @@ static void release_alloc(afr_handle* h, const double*& p, size_t n) {
 // Tables of the plain form at orders 1-3: the slots' own adjugate rows, and for
 // structured prisms the metric divergence MD, 1/det and the metrics in lane order
 // (in place: no kernel after this one reads theirs in the reference's order).
-static int plain_setup(afr_handle* h, cudaStream_t st) {
-  const size_t S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism;
+// nrow: the faces' rows among those whose normals are kept (boundary and force
+// faces), changed to all faces where an interior slot needs its own.
+static int plain_setup(afr_handle* h, const afr_mesh_desc* m, std::vector<int32_t>& nrow, cudaStream_t st) {
+  const size_t S = h->S, P = h->P, Fn = h->Fn, ns = h->slots.n, NP = h->n_prism, F = h->F;
+  const bool sst = h->prm.turb == AFR_TURB_SST;  // its face kernel reads every face's
   int rc;
+  // all normals, for the slots' alignment test: in the point fields, not in use yet, where they fit
+  double* normals = h->PF;
+  const bool own = F * P * 3 > (size_t)h->N * S * PFW;
+  if (own && cudaMalloc((void**)&normals, F * P * 3 * sizeof(double)) != cudaSuccess)
+    return fail(h, AFR_ENOMEM, "cudaMalloc failed for face normals");
+  auto release_normals = [&] {
+    if (own) cudaFree(normals);
+  };
+  cudaMemcpyAsync(normals, m->true_normal, F * P * 3 * sizeof(double), cudaMemcpyHostToDevice, st);
   {
     const cudaError_t e = dispatch(h, [](auto L) { return decltype(L)::set_attrs(); });
-    if (e != cudaSuccess) return cuda_fail(h, e, "kernel attributes");
+    if (e != cudaSuccess) return release_normals(), cuda_fail(h, e, "kernel attributes");
   }
-  if ((rc = dalloc(h, &h->slot_rows, ns * P))) return rc;
+  if ((rc = dalloc(h, &h->slot_rows, ns * P))) return release_normals(), rc;
   double *md = nullptr, *rdet = nullptr;
   if (h->px64 && ((rc = dalloc(h, &md, NP * S * 3)) || (rc = dalloc(h, &rdet, NP * S)) ||
                   (rc = dalloc(h, &h->RVd, NP * S * 9))))
-    return rc;
+    return release_normals(), rc;
   const unsigned nb = (unsigned)((ns * P + 127) / 128), nmd = (unsigned)((NP * S * 3 + 255) / 256);
   switch (h->order) {
     case 1:
-      if (ns) k_slot_rows<8, 4><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+      if (ns) k_slot_rows<8, 4><<<nb, 128, 0, st>>>(h->g, h->ops, normals, h->slots, h->slot_rows, h->status);
       if (h->px64) k_mx_md<8, 27><<<nmd, 256, 0, st>>>(h->g, h->ops, NP, md);
       break;
     case 2:
-      if (ns) k_slot_rows<27, 9><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+      if (ns) k_slot_rows<27, 9><<<nb, 128, 0, st>>>(h->g, h->ops, normals, h->slots, h->slot_rows, h->status);
       if (h->px64) k_mx_md<27, 64><<<nmd, 256, 0, st>>>(h->g, h->ops, NP, md);
       break;
     default:
-      if (ns) k_slot_rows<64, 16><<<nb, 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, h->slot_rows);
+      if (ns) k_slot_rows<64, 16><<<nb, 128, 0, st>>>(h->g, h->ops, normals, h->slots, h->slot_rows, h->status);
   }
   if (h->px64) {
     const int nf = h->order == 1 ? 3 : 4;
@@ -981,7 +993,34 @@ static int plain_setup(afr_handle* h, cudaStream_t st) {
     k_mx_rdet<<<(unsigned)((NP * S + 255) / 256), 256, 0, st>>>(h->g.det, NP * S, rdet);
     h->pgd = PxGeom<double>{h->g.adj, h->g.adj_fine, md, rdet, h->px_rows};
   }
-  const cudaError_t e = cudaGetLastError();
+  unsigned fallback = 0;  // through the status word
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&fallback, h->status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->status, 0, sizeof(unsigned), st);
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  release_normals();
+  if (e == cudaSuccess) e = e2;
+  if (e != cudaSuccess) return cuda_fail(h, e, "plain-form set-up");
+  double* tn;
+  int32_t* bcg;
+  if (fallback || sst) {
+    for (size_t f = 0; f < F; ++f) nrow[f] = (int32_t)f;
+    k_slot_face_rows<<<(unsigned)((ns + 127) / 128), 128, 0, st>>>(h->slots);
+    if ((rc = upload(h, &tn, m->true_normal, F * P * 3, st)) || (rc = upload(h, &bcg, m->bc_group, F, st))) return rc;
+    e = cudaGetLastError();
+  } else {
+    std::vector<double> n;
+    std::vector<int32_t> g;
+    for (size_t f = 0; f < F; ++f)
+      if (nrow[f] >= 0) {
+        n.insert(n.end(), m->true_normal + f * P * 3, m->true_normal + (f + 1) * P * 3);
+        g.push_back(m->bc_group[f]);
+      }
+    if ((rc = upload(h, &tn, n.data(), n.size(), st)) || (rc = upload(h, &bcg, g.data(), g.size(), st))) return rc;
+    e = cudaStreamSynchronize(st);  // n and g leave scope
+  }
+  h->fc.tnormal = tn;
+  h->fc.bc_group = bcg;
   return e == cudaSuccess ? AFR_OK : cuda_fail(h, e, "plain-form set-up");
 }
 
@@ -1076,15 +1115,20 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
   h->mo.MD = md;
   h->mo.hcell = hc;
   float4 *adjf32 = nullptr, *adjs32 = nullptr, *invs32 = nullptr;
-  if (tcr && ((rc = dalloc(h, &adjf32, N * (size_t)h->Fn * 3)) || (rc = dalloc(h, &adjs32, N * (size_t)S * 3)) ||
-              (rc = dalloc(h, &invs32, N * (size_t)S * 3))))
+  const size_t T0 = h->px ? h->n_prism : 0, NT = N - T0;  // cells of the tensor-core kernels
+  if (tcr && ((rc = dalloc(h, &adjf32, NT * (size_t)h->Fn * 3)) || (rc = dalloc(h, &adjs32, NT * (size_t)S * 3)) ||
+              (rc = dalloc(h, &invs32, NT * (size_t)S * 3))))
     return rc;
   float *padjs = nullptr, *padjf = nullptr;
   const size_t NP = h->n_prism;
   if (h->px && ((rc = dalloc(h, &padjs, NP * S * 9)) || (rc = dalloc(h, &padjf, NP * h->Fn * 9)))) return rc;
-  h->mo.adjf = adjf32;
-  h->mo.adjs = adjs32;
-  h->mo.invs = invs32;
+  // indexed by cell number: cell T0's rows come first
+  auto from = [&](float4* p, size_t pts) {
+    return reinterpret_cast<const float4*>(reinterpret_cast<uintptr_t>(p) - T0 * pts * 3 * sizeof(float4));
+  };
+  h->mo.adjf = from(adjf32, h->Fn);
+  h->mo.adjs = from(adjs32, S);
+  h->mo.invs = from(invs32, S);
   double* rdet;
   if ((rc = dalloc(h, &rdet, N * (size_t)S))) return rc;
   h->mo.rdet = rdet;
@@ -1126,11 +1170,11 @@ static int mixed_setup(afr_handle* h, const afr_mesh_desc* m, const std::vector<
               if (ns) k_mx_match<64, 16><<<(unsigned)((ns * 16 + 127) / 128), 128, 0, st>>>(h->g, h->ops, h->fc, h->slots, arow, ofp, h->status, 1e-6);
               break;
     }
-    const size_t nrows = N * (size_t)h->Fn * 3, nsrows = N * (size_t)S * 3;
+    const size_t nrows = NT * (size_t)h->Fn * 3, nsrows = NT * (size_t)S * 3;
     if (tcr) {
-      k_mx_rows_f32<<<(unsigned)((nrows + 255) / 256), 256, 0, st>>>(h->g.adj_fine, nrows, adjf32);
-      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.adj, nsrows, adjs32);
-      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv, nsrows, invs32);
+      k_mx_rows_f32<<<(unsigned)((nrows + 255) / 256), 256, 0, st>>>(h->g.adj_fine + T0 * h->Fn * 9, nrows, adjf32);
+      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.adj + T0 * S * 9, nsrows, adjs32);
+      k_mx_rows_f32<<<(unsigned)((nsrows + 255) / 256), 256, 0, st>>>(h->g.inv + T0 * S * 9, nsrows, invs32);
     }
     if (h->px) {
       k_px_planes<<<(unsigned)NP, 128, 0, st>>>(h->g.adj_fine, h->Fn, 1, padjf);
@@ -1522,12 +1566,13 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
   Faces& fc = h->fc;
   fc.F = h->F;
   {
-    int32_t *own = nullptr, *nbr = nullptr, *bcg;
+    int32_t *own = nullptr, *nbr = nullptr, *bcg = nullptr;
     int8_t *oax = nullptr, *nax = nullptr;
     uint8_t* isb = nullptr;
-    double *osd = nullptr, *nsd = nullptr, *tn, *m0n, *m1n, *m0o, *m1o;
-    if ((rc = upload(h, &tn, m->true_normal, F * P * 3, st))) return bail(rc);
-    if (prm->precision == AFR_PREC_MIXED || h->order == 0) {
+    double *osd = nullptr, *nsd = nullptr, *tn = nullptr, *m0n, *m1n, *m0o, *m1o;
+    if (prm->precision == AFR_PREC_MIXED || h->order == 0) {  // plain form: see plain_setup
+      if ((rc = upload(h, &tn, m->true_normal, F * P * 3, st)) || (rc = upload(h, &bcg, m->bc_group, F, st)))
+        return bail(rc);
       if ((rc = upload_i32(h, &own, m->owner_cell, F, st, tmp)) || (rc = upload_i32(h, &nbr, m->neighbor_cell, F, st, tmp)))
         return bail(rc);
       std::vector<int8_t> ax8(F), nx8(F);
@@ -1587,13 +1632,13 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
       h->mat_elems[2] = F * P * S;
       h->mat_elems[3] = n1o * P * S;
     }
-    if ((rc = upload(h, &bcg, m->bc_group, F, st))) return bail(rc);
     fc.owner = own; fc.neighbor = nbr; fc.o_axis = oax; fc.n_axis = nax; fc.o_side = osd; fc.n_side = nsd;
     fc.is_bnd = isb; fc.tnormal = tn; fc.nb_m0 = m0n; fc.nb_m1 = m1n; fc.ow_m0 = m0o; fc.ow_m1 = m1o; fc.bc_group = bcg;
     fc.nb_m0i = m0ni; fc.nb_m1i = m1ni; fc.ow_m0i = m0oi; fc.ow_m1i = m1oi;
   }
   // slot lists: faces visited in ascending (color, face index)
   HostSlots hs;
+  std::vector<int32_t> nrow;  // plain form: the faces' rows among the kept normals, -1: none
   {
     std::vector<int32_t> order(F);
     for (size_t f = 0; f < F; ++f) order[f] = (int32_t)f;
@@ -1654,6 +1699,12 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     }
     std::vector<int32_t> s0(mixed ? ns : 0), s1(mixed ? ns : 0), si1(mixed ? ns : 0);
     std::vector<int4> srec(plain ? 2 * ns : 0);
+    if (plain) {
+      nrow.resize(F);
+      int32_t rows = 0;
+      for (size_t f = 0; f < F; ++f)
+        nrow[f] = m->is_boundary[f] || (m->cd_wall_face && m->cd_wall_face[f]) ? rows++ : -1;
+    }
     for (size_t c = 0; c < N; ++c)
       for (int32_t k = ptr[c]; k < ptr[c + 1]; ++k) {
         const int f = codes[k] >> 1;
@@ -1677,7 +1728,7 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
           const int32_t m1 =
               c1 < 0 ? 0 : (ix ? (nbside ? m->ow_src1_mat_index[i1] : m->nb_src1_mat_index[i1]) : (int32_t)i1);
           srec[2 * (size_t)k] = make_int4(c0, m0, c1, m1);
-          srec[2 * (size_t)k + 1] = make_int4(f, fl, (int)c, 0);
+          srec[2 * (size_t)k + 1] = make_int4(f, fl, (int)c, std::max(nrow[f], 0));
         }
       }
     int32_t *d_fl, *d_f = nullptr, *d_c = nullptr, *d_0 = nullptr, *d_1 = nullptr, *d_i1 = nullptr;
@@ -1703,20 +1754,6 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     if ((rc = upload(h, &bq, m->bc_Q, nb * 5, st))) return bail(rc);
     if ((rc = upload(h, &bp, m->bc_p_out, nb, st))) return bail(rc);
     h->bc = Bc{m->n_bc, bt, bn, bw, bq, bp};
-    cudaStreamSynchronize(st);
-  }
-  if (m->cd_wall_face && m->true_area_weight) {
-    std::vector<int4> cdf;
-    std::vector<double> aw;  // (force faces, P)
-    for (size_t f = 0; f < F; ++f)
-      if (m->cd_wall_face[f] && m->owner_is_primary[f]) {
-        cdf.push_back(make_int4((int)f, (int)m->owner_cell[f], (int)m->owner_axis[f], m->owner_side[f] < 0.0 ? 0 : 1));
-        aw.insert(aw.end(), m->true_area_weight + f * P, m->true_area_weight + (f + 1) * P);
-      }
-    h->n_cd_faces = (int)cdf.size();
-    if ((rc = upload(h, &h->cd_faces, cdf.data(), cdf.size(), st))) return bail(rc);
-    if ((rc = upload(h, &h->area_w, aw.data(), aw.size(), st))) return bail(rc);
-    if ((rc = dalloc(h, &h->cd_part, cdf.size() * 6))) return bail(rc);
     cudaStreamSynchronize(st);
   }
   // ---- scratch ----
@@ -1766,7 +1803,21 @@ int afr_create(const afr_mesh_desc* m, const afr_params* prm, void* stream, afr_
     cudaStreamSynchronize(st);  // rec leaves scope
   }
   if (prm->precision == AFR_PREC_MIXED && (rc = mixed_setup(h, m, Wkeep, hs, st))) return bail(rc);
-  if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = plain_setup(h, st))) return bail(rc);
+  if (prm->precision != AFR_PREC_MIXED && h->order > 0 && (rc = plain_setup(h, m, nrow, st))) return bail(rc);
+  if (m->cd_wall_face && m->true_area_weight) {
+    std::vector<int4> cdf;
+    std::vector<double> aw;  // (force faces, P)
+    for (size_t f = 0; f < F; ++f)
+      if (m->cd_wall_face[f] && m->owner_is_primary[f]) {
+        cdf.push_back(make_int4(nrow.empty() ? (int)f : nrow[f], (int)m->owner_cell[f], (int)m->owner_axis[f], m->owner_side[f] < 0.0 ? 0 : 1));
+        aw.insert(aw.end(), m->true_area_weight + f * P, m->true_area_weight + (f + 1) * P);
+      }
+    h->n_cd_faces = (int)cdf.size();
+    if ((rc = upload(h, &h->cd_faces, cdf.data(), cdf.size(), st))) return bail(rc);
+    if ((rc = upload(h, &h->area_w, aw.data(), aw.size(), st))) return bail(rc);
+    if ((rc = dalloc(h, &h->cd_part, cdf.size() * 6))) return bail(rc);
+    cudaStreamSynchronize(st);
+  }
   if (h->order == 0 && (rc = p0_setup(h, m, st))) return bail(rc);
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return bail(cuda_fail(h, e, "afr_create"));

@@ -90,7 +90,9 @@ struct Faces {
   const double* o_side;       // (F) +-1
   const double* n_side;       // (F)
   const uint8_t* is_bnd;      // (F)
-  const double* tnormal;      // (F, P, 3)
+  // (F, P, 3).  Plain form without SST: the boundary faces' rows only, unless some
+  // interior slot falls back to its face normal; slot and force records hold the row.
+  const double* tnormal;
   // Interpolation matrices stored transposed, (rows, S, P) with the face
   // point fastest, one matrix per record through a row index: a shared table
   // of the distinct matrices when the mesh gives one (a few dozen on
@@ -105,7 +107,7 @@ struct Faces {
   const int32_t* ow_m0i;
   const double* ow_m1;
   const int32_t* ow_m1i;
-  const int32_t* bc_group;    // (F) row of the BC table
+  const int32_t* bc_group;    // row of the BC table, in the rows of tnormal
   // residual slots: primary sides, ascending color
   const int32_t* slot_ptr;    // (N+1)
   const int32_t* slot;        // face*2 + (0 owner, 1 neighbor); order 0 only

@@ -362,8 +362,8 @@ struct SlotTable {
   const int32_t* c1;        // (n) second source cell, -1 if none
   const int32_t* i1;        // (n) row of the compact second-source table
   // plain form: (n, 2) what a slot's face points need: source cells and matrix
-  // rows (c0, m0, c1, m1), then face, flags, cell
-  const int4* rec;
+  // rows (c0, m0, c1, m1), then face, flags, cell, row of tnormal and bc_group
+  int4* rec;
 };
 
 
@@ -452,7 +452,8 @@ __device__ __forceinline__ void dmma_warp_rb_f(int M, int N, const double* __res
     }
 }
 
-// the jumps of one slot point from its own side and the other side's fields
+// the jumps of one slot point from its own side and the other side's fields; f:
+// the slot's row of tnormal and bc_group (read by boundary and fallback slots)
 template <int S, int NP, bool VISC, int NF>
 __device__ __forceinline__ void face_jump(const Geom& g, const Faces& fc, const Bc& bc, int sl, int i, int e, int f,
                                           bool is_owner, bool bnd, double side, const double (&ow)[NF],
@@ -586,7 +587,7 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, VISC ? 3 : 4)
     }
     cp_async_wait_all();
     __syncwarp();
-    const int f = r1.x, fl = r1.y;
+    const int f = r1.w, fl = r1.y;
     const bool is_owner = (fl & 1) == 0;
     const bool bnd = (fl & 2) != 0;
     const double side = (fl & 16) ? 1.0 : -1.0;
@@ -710,15 +711,17 @@ __global__ void __launch_bounds__(32 * FACE_WARPS, 4)
       }
     }
   }
-  face_jump<S, NP, VISC>(g, fc, bc, sl, i, e, r1.x, (fl & 1) == 0, (fl & 2) != 0, (fl & 16) ? 1.0 : -1.0, ow, ot, arow,
+  face_jump<S, NP, VISC>(g, fc, bc, sl, i, e, r1.w, (fl & 1) == 0, (fl & 2) != 0, (fl & 16) ? 1.0 : -1.0, ow, ot, arow,
                          mu, J);
 }
 
 // own adjugate row of the face's axis at every slot flux point (E * adj) and
 // its norm, negative where the row's direction falls back to the face normal
-// (alignment below 0.5, core/fr_residual/inviscid_kernel_colored.py:104-108)
+// (alignment below 0.5, core/fr_residual/inviscid_kernel_colored.py:104-108);
+// normals (F, P, 3); fallback: set where an interior slot does
 template <int S, int NP>
-__global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __restrict__ arow) {
+__global__ void k_slot_rows(Geom g, Ops ops, const double* __restrict__ normals, SlotTable st,
+                            double4* __restrict__ arow, unsigned* fallback) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (size_t)st.n * NP) return;
   const int sl = (int)(t / NP), i = (int)(t % NP);
@@ -737,9 +740,16 @@ __global__ void k_slot_rows(Geom g, Ops ops, Faces fc, SlotTable st, double4* __
   double mag = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
   if (mag < 1e-300) mag = 1e-300;
   const double side = sb ? 1.0 : -1.0, sg = (fl & 1) == 0 ? 1.0 : -1.0;
-  const double* tn = fc.tnormal + ((size_t)f * NP + i) * 3;
+  const double* tn = normals + ((size_t)f * NP + i) * 3;
   const double al = a0 / mag * side * (sg * tn[0]) + a1 / mag * side * (sg * tn[1]) + a2 / mag * side * (sg * tn[2]);
   arow[t] = make_double4(a0, a1, a2, al < 0.5 ? -mag : mag);
+  if (al < 0.5 && !(fl & 2)) *fallback = 1u;
+}
+
+// every slot's normals at its face's row
+__global__ void k_slot_face_rows(SlotTable st) {
+  const int sl = blockIdx.x * blockDim.x + threadIdx.x;
+  if (sl < st.n) st.rec[2 * (size_t)sl + 1].w = st.rec[2 * (size_t)sl + 1].x;
 }
 
 // ---------------------------------------------------------------------------

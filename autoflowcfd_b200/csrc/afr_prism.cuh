@@ -166,6 +166,10 @@ __global__ void __launch_bounds__(32 * px_warps(N1), sizeof(T) == 8 ? (N1 == 3 ?
     constexpr int MID = S / 2;
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
+      if (v == 5 && (D || !VISC)) {  // the temperature: gradients only
+        dev[5] = T(q[5]);
+        continue;
+      }
       float ref = __shfl_sync(0xffffffffu, float(q[v]), (pc < CPR ? pc : 0) * S + MID);
       if (D && !isfinite(ref)) ref = 0.f;
       dev[v] = D ? T(q[v]) : T(q[v] - double(ref));
